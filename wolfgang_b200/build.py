@@ -52,9 +52,9 @@ CXX_FLAGS = ["-std=c++20", "-O2", "-fPIC", "-ffp-contract=off", "-Wall",
 # anything still taken from a static archive.
 SHARED_LINK = ["-l:libstdc++.so.6", "-Wl,--exclude-libs,ALL"]
 
-CU_SOURCES = ["wg_runtime.cu", "wg_commute.cu", "wg_simplify.cu", "wg_bucket.cu", "wg_expect.cu", "wg_group.cu",
+CU_SOURCES = ["wg_runtime.cu", "wg_commute.cu", "wg_sort.cu", "wg_simplify.cu", "wg_bucket.cu", "wg_expect.cu", "wg_group.cu",
               "wg_batch.cu", "wg_tune.cu"]
-CU_HEADERS = ["wg_common.cuh", "wg_scan.cuh"]
+CU_HEADERS = ["wg_common.cuh", "wg_scan.cuh", "wg_sort.cuh", "wg_sort_block.cuh"]
 HOST_SOURCES = ["pauli_sum.cpp", "device.cpp"]
 HOST_HEADERS = ["abi.hpp", "guards.hpp"]
 

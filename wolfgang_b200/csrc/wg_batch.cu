@@ -357,7 +357,7 @@ void build_batch(wg_products_batch_s& b, const uint64_t* const* lhs_x, const uin
                                                 static_cast<uint32_t>(np), N, W, keys.as<uint64_t>(),
                                                 idx.as<uint32_t>(), raw.as<uint32_t>()));
     wg::check_launch("launch batch keys");
-    wg::radix_sort_keys(device, N, K, keys, idx, s);  // stable: nested-loop order within equal keys
+    wg::radix_sort_keys(device, N, K, keys, idx, s, true);  // stable: nested-loop order within equal keys
     b.code.reset(sizeof(uint32_t) * N, s);
     pbatch_gather_kernel<<<g, kThreads, 0, s>>>(idx.as<uint32_t>(), raw.as<uint32_t>(), N, b.code.as<uint32_t>());
     wg::check_launch("launch batch gather");

@@ -2014,26 +2014,6 @@ void compress(const wg::Scratch& rec, size_t T, int KW, const SigWords& sig, wg:
 }
 
 // Significant bits of the packed keys (host copy) and their count.
-// Under WG_SORT_AUTO, keys that vary in few 8-bit digits go to the LSD
-// pipeline, which streams the items once per varying digit: measured on the
-// B200, the bucketed path's time per item is that of about 5.5 LSD passes at
-// two mask words (config 2: 73 ms bucketed, 329 ms for its 25 LSD passes)
-// and it does not shrink with the key width, while narrow keys need few
-// passes (a 20-qubit operator: 6).  kLsdDigits is the largest varying-digit
-// count that the LSD pipeline takes, by mask words.
-constexpr int kLsdDigits[3] = {0, 8, 5};
-
-int varying_digits(const SigWords& sw, int KW) {
-  int d = 0;
-  for (int w = 0; w < KW; ++w)
-    for (int b = 0; b < 64; b += 8) d += ((sw.w[w] >> b) & 0xffu) != 0;
-  return d;
-}
-
-bool lsd_for_narrow_keys(const SigWords& sw, int KW) {
-  return wg::sort_algorithm() == WG_SORT_AUTO && varying_digits(sw, KW) <= kLsdDigits[KW / 2];
-}
-
 int read_sig(const wg::Scratch& sig, int KW, SigWords& out, cudaStream_t s) {
   unsigned long long h[4] = {0, 0, 0, 0};
   wg::check_cuda(cudaMemcpyAsync(h, sig.get(), sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, s),
@@ -2099,7 +2079,7 @@ bool bucket_products_once(int device, int W, const uint64_t* lx, const uint64_t*
   pack(rx, rz, rc, n_r, W, bk, sig.as<unsigned long long>(), device, s);
   SigWords sw{};
   const int total = read_sig(sig, KW, sw, s);
-  if (total < 1 || total > 255 || lsd_for_narrow_keys(sw, KW)) return false;
+  if (total < 1 || total > 255) return false;
   compress(ak, n_l, KW, sw, ac2, device, s);
   compress(bk, n_r, KW, sw, bc2, device, s);
   const ThrSpec thr{thr_mode, atol, rtol, thr_fixed};
@@ -2123,7 +2103,7 @@ bool bucket_simplify_once(int device, int W, const uint64_t* x, const uint64_t* 
   pack(x, z, c, n, W, tk, sig.as<unsigned long long>(), device, s);
   SigWords sw{};
   const int total = read_sig(sig, KW, sw, s);
-  if (total < 1 || total > 255 || lsd_for_narrow_keys(sw, KW)) return false;
+  if (total < 1 || total > 255) return false;
   compress(tk, n, KW, sw, tc2, device, s);
   const ThrSpec thr{thr_mode, atol, rtol, 0.0};
   const Outs out{ox, oz, oc, U};

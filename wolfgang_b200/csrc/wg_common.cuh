@@ -208,8 +208,8 @@ class Workspace {
 };
 
 // Stable LSD radix sort of n items by K structure-of-arrays key words (word 0
-// most significant) carrying a 32-bit item index (wg_simplify.cu).
-void radix_sort_keys(int device, size_t n, int K, Scratch& keys, Scratch& idx, cudaStream_t s);
+// most significant) carrying a 32-bit item index (wg_sort.cu; `alike`: see there).
+void radix_sort_keys(int device, size_t n, int K, Scratch& keys, Scratch& idx, cudaStream_t s, bool alike = false);
 
 // Bucketed sort-reduce (wg_bucket.cu).  thr_mode: 0 cull at thr_fixed, 1 at
 // atol + rtol*max|c|, 2 at atol (empty result when some |c| is infinite).

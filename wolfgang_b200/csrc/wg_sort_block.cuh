@@ -1,0 +1,260 @@
+// wg_sort_block.cuh -- key packing, and a stable sort of a few thousand
+// multi-word keys by one CTA.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <vector>
+
+#include "wg_common.cuh"
+#include "wg_sort.cuh"
+
+namespace wg {
+
+// Dynamic shared memory above 48 KB must be allowed per kernel and device; the
+// call is cheap and idempotent.
+template <class K>
+void allow_smem(K kernel, size_t bytes) {
+  check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+             "set kernel shared memory");
+}
+
+}  // namespace wg
+
+namespace wgo {
+
+// The bits of a key (word(k), K words) under the masks `bits`, packed to the
+// front of `words` words, handed out in order as put(w, value).
+template <class Word, class Put>
+__device__ __forceinline__ void pack_key(const unsigned long long* __restrict__ bits, int K, Word&& word, Put&& put,
+                                         int words) {
+  uint64_t cur = 0;
+  int at = 0, base = 0;
+  for (int k = 0; k < K; ++k) {
+    const uint64_t m = bits[k];
+    uint64_t v = word(k) & m;
+    while (v) {
+      const int b = 63 - __clzll(static_cast<long long>(v));
+      v ^= uint64_t{1} << b;
+      const int r = base + __popcll(m & ~((uint64_t{2} << b) - 1));
+      while (r >= 64 * (at + 1)) {
+        put(at++, cur);
+        cur = 0;
+      }
+      cur |= 0x8000000000000000ull >> (r & 63);
+    }
+    base += __popcll(m);
+  }
+  while (at < words) {
+    put(at++, cur);
+    cur = 0;
+  }
+}
+
+// Per list y: found[y][0][k] = OR of key word k, found[y][1][k] = OR of its
+// complement, pop[y] = set bits in all.
+template <class A, class C>
+__global__ void __launch_bounds__(256) key_bits_kernel(A a, size_t na, C c, size_t nc, int K,
+                                                       unsigned long long* __restrict__ found,
+                                                       unsigned long long* __restrict__ pop) {
+  const int y = blockIdx.y;
+  const size_t n = y == 0 ? na : nc;
+  unsigned long long set = 0;
+  for (int k = 0; k < K; ++k) {
+    uint64_t one = 0, none = 0;
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+      const uint64_t v = y == 0 ? a(i, k) : c(i, k);
+      one |= v;
+      none |= ~v;
+      set += __popcll(v);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      one |= __shfl_xor_sync(0xffffffffu, one, o);
+      none |= __shfl_xor_sync(0xffffffffu, none, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      if (one) atomicOr(found + (2 * y) * K + k, static_cast<unsigned long long>(one));
+      if (none) atomicOr(found + (2 * y + 1) * K + k, static_cast<unsigned long long>(none));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) set += __shfl_xor_sync(0xffffffffu, set, o);
+  if ((threadIdx.x & 31) == 0 && set) atomicAdd(pop + y, set);
+}
+
+// masks[k] = bits of word k that vary in either list
+static __global__ void key_masks_kernel(const unsigned long long* __restrict__ found, int K, int lists,
+                                        unsigned long long* __restrict__ masks) {
+  for (int k = threadIdx.x; k < K; k += blockDim.x) {
+    unsigned long long m = 0;
+    for (int y = 0; y < lists; ++y) m |= found[2 * y * K + k] & found[(2 * y + 1) * K + k];
+    masks[k] = m;
+  }
+}
+
+// Which key bits vary over one list (nc == 0), or over the XORs of the keys of
+// two.  Word(i, k) of a list gives its item i's key word k.  Synchronises s.
+template <class A, class C>
+KeyBits key_bits(int device, int K, size_t na, const A& a, size_t nc, const C& c, cudaStream_t s) {
+  KeyBits kb{};
+  kb.side_by_side = nc > 0;
+  kb.K = K;
+  const int lists = nc > 0 ? 2 : 1;
+  const size_t words = 4 * static_cast<size_t>(K) + 2;
+  wg::Scratch found(sizeof(uint64_t) * words, s);
+  kb.masks.reset(sizeof(uint64_t) * K, s);
+  wg::check_cuda(cudaMemsetAsync(found.get(), 0, sizeof(uint64_t) * words, s), "clear key bits");
+  auto* f = found.as<unsigned long long>();
+  const dim3 grid(wg::grid_for(std::max(na, nc), 256, device, 4), lists);
+  WG_TIMED("key_bits_kernel", s, (key_bits_kernel<A, C><<<grid, 256, 0, s>>>(a, na, c, nc, K, f, f + 4 * K)));
+  wg::check_launch("launch key bits");
+  key_masks_kernel<<<1, 256, 0, s>>>(f, K, lists, kb.masks.as<unsigned long long>());
+  wg::check_launch("launch key masks");
+  std::vector<unsigned long long> h(words);
+  wg::check_cuda(cudaMemcpyAsync(h.data(), f, sizeof(uint64_t) * words, cudaMemcpyDeviceToHost, s), "read key bits");
+  wg::check_cuda(cudaStreamSynchronize(s), "read key bits");
+  for (int k = 0; k < K; ++k) {
+    unsigned long long vary = 0, ored = 0;
+    for (int y = 0; y < lists; ++y) {
+      vary |= h[2 * y * K + k] & h[(2 * y + 1) * K + k];
+      ored |= h[2 * y * K + k];
+    }
+    kb.B += __builtin_popcountll(vary);
+    kb.ored += __builtin_popcountll(ored);
+    for (int b = 0; b < 64; b += 8) kb.ored_digits += ((ored >> b) & 0xffu) != 0;
+  }
+  const double B = std::max(1, kb.B);
+  const double p = std::min(1.0, static_cast<double>(h[4 * K]) / (B * static_cast<double>(na)));
+  const double q = nc > 0 ? std::min(1.0, static_cast<double>(h[4 * K + 1]) / (B * static_cast<double>(nc))) : 0.0;
+  kb.density = p * (1.0 - q) + q * (1.0 - p);
+  return kb;
+}
+
+// ------------------------------------------------------- sort by one CTA
+
+constexpr int kBlockSortThreads = 1024;
+constexpr int kBlockSortItems = 8192;
+constexpr int kBlockSortWarps = kBlockSortThreads / 32;
+constexpr int kBlockSortRounds = kBlockSortItems / kBlockSortThreads;
+
+struct BlockSort {
+  uint16_t order[2][kBlockSortItems];
+  uint32_t count[kDigits * (kBlockSortWarps + 1)];  // [digit][warp], padded against bank conflicts
+  uint32_t total[kDigits];
+  unsigned long long one, none;
+};
+
+// The items 0..n-1 (n <= kBlockSortItems) in stable ascending order of their
+// keys (word(k, item), word 0 most significant), by LSD passes over 8-bit
+// windows of the bits that vary.  Returns a shared array; ends with a barrier.
+// A pass's time is that of its five barriers and the keys' loads (L1 or L2).
+template <class Word>
+__device__ const uint16_t* block_sort(BlockSort& sm, int n, int K, Word&& word) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rounds = (n + kBlockSortThreads - 1) / kBlockSortThreads;
+  const int w0 = warp * 32 * rounds;  // a warp's places are consecutive
+  const uint32_t below = (1u << lane) - 1u;
+  int cur = 0;
+  for (int i = tid; i < n; i += kBlockSortThreads) sm.order[0][i] = static_cast<uint16_t>(i);
+  for (int k = K - 1; k >= 0; --k) {
+    if (tid == 0) sm.one = sm.none = 0;
+    __syncthreads();
+    {
+      uint64_t one = 0, none = 0;
+      for (int i = tid; i < n; i += kBlockSortThreads) {
+        const uint64_t v = word(k, i);
+        one |= v;
+        none |= ~v;
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        one |= __shfl_xor_sync(0xffffffffu, one, o);
+        none |= __shfl_xor_sync(0xffffffffu, none, o);
+      }
+      if (lane == 0) {
+        if (one) atomicOr(&sm.one, static_cast<unsigned long long>(one));
+        if (none) atomicOr(&sm.none, static_cast<unsigned long long>(none));
+      }
+    }
+    __syncthreads();
+    uint64_t vary = sm.one & sm.none;
+    while (vary) {
+      const int shift = __ffsll(static_cast<long long>(vary)) - 1;
+      vary &= ~(uint64_t{255} << shift);
+      const uint16_t* from = sm.order[cur];
+      uint16_t* to = sm.order[cur ^ 1];
+      for (int i = tid; i < kDigits * (kBlockSortWarps + 1); i += kBlockSortThreads) sm.count[i] = 0;
+      __syncthreads();
+      uint32_t digit[kBlockSortRounds], rank[kBlockSortRounds];
+#pragma unroll
+      for (int r = 0; r < kBlockSortRounds; ++r) {
+        const int p = w0 + 32 * r + lane;
+        digit[r] = r < rounds && p < n ? static_cast<uint32_t>(word(k, from[p]) >> shift) & 255u : kDigits;
+      }
+#pragma unroll
+      for (int r = 0; r < kBlockSortRounds; ++r) {
+        if (r < rounds) {
+          const uint32_t same = __match_any_sync(0xffffffffu, digit[r]);
+          const uint32_t at = digit[r] * (kBlockSortWarps + 1) + warp;
+          const uint32_t before = digit[r] < kDigits ? sm.count[at] : 0;
+          __syncwarp();
+          const uint32_t mine = __popc(same & below);
+          if (mine == 0 && digit[r] < kDigits) sm.count[at] = before + __popc(same);
+          __syncwarp();
+          rank[r] = before + mine;
+        }
+      }
+      __syncthreads();
+      // per digit: the warps' first places; a warp takes 8 digits, a lane a warp's count
+#pragma unroll
+      for (int e = 0; e < kDigits / kBlockSortWarps; ++e) {
+        const int d = warp * (kDigits / kBlockSortWarps) + e;
+        const uint32_t c = sm.count[d * (kBlockSortWarps + 1) + lane];
+        uint32_t incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += v;
+        }
+        sm.count[d * (kBlockSortWarps + 1) + lane] = incl - c;
+        if (lane == 31) sm.total[d] = incl;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        uint32_t c[kDigits / 32], sum = 0;
+#pragma unroll
+        for (int e = 0; e < kDigits / 32; ++e) {
+          c[e] = sm.total[lane * (kDigits / 32) + e];
+          sum += c[e];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += v;
+        }
+        uint32_t at = incl - sum;
+#pragma unroll
+        for (int e = 0; e < kDigits / 32; ++e) {
+          sm.total[lane * (kDigits / 32) + e] = at;
+          at += c[e];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < kBlockSortRounds; ++r) {
+        const int p = w0 + 32 * r + lane;
+        if (r < rounds && p < n)
+          to[sm.total[digit[r]] + sm.count[digit[r] * (kBlockSortWarps + 1) + warp] + rank[r]] = from[p];
+      }
+      cur ^= 1;
+      __syncthreads();
+    }
+  }
+  __syncthreads();
+  return sm.order[cur];
+}
+
+}  // namespace wgo
