@@ -5,32 +5,33 @@
 //   P|b> = i^y (-1)^{popc(z&b)} |b^x>,  y = popc(x&z),
 //   e_k = <psi|P_k|psi> = sum_b conj(psi[b^x]) i^y (-1)^{popc(z&b)} psi[b]  (real),
 //   E = sum_k c_k e_k.
-// Terms sharing an x-mask form a group.  For x != 0 the pair (b, b^x) with one
-// chosen bit of x clear in b gives t = conj(psi[b^x]) psi[b] and, since
-// (-1)^{popc(z&(b^x))} = (-1)^{popc(z&b)} (-1)^y,
-//   e_k = {2R, -2I, -2R, 2I}[y mod 4],  R = sum s_k(b) Re t,  I = sum s_k(b) Im t,
-// over half the basis; one pass over the pairs serves every term of the group.
-// For x == 0, e_k = sum_b s_k(b) |psi_b|^2.
+// Terms sharing an x-mask form a group: with t_b = conj(psi[b^x]) psi[b] and
+// s_k(b) = (-1)^{popc(z_k&b)},
+//   e_k = sum_b s_k(b) {Re, -Im, -Re, Im}[y mod 4] t_b.
+// b and b^x give the same summand, so half of the b's do where they are known
+// apart by a bit above the tile.
 //
-// Forward schedule.  The qubit index splits into a tile (low t bits, 2^t
-// amplitudes, t <= 19) and the tile number.  Groups whose x agree above the
-// tile bits form a class; every group of a class pairs tile T1 with the same
-// tile T1 ^ (x >> t).  Work items run class by class and tile pair by tile
-// pair, so the groups of a class read a tile pair while it is in L2.  A group
-// is cut into sub-groups of at most 16 terms; an item is (sub-group, tile
-// pair, chunk of 2^16 pairs).  Each thread walks its pairs in Gray-code order,
-// so one bit of b flips per step and the sign vector of all the sub-group's
-// terms updates with one XOR (bit-sliced: bit kk of plane q says whether z_kk
-// has bit q).
+// Tiles.  The amplitudes are cut into tiles of 2^12 (the low 12 bits of b; of
+// 2^n, at least 2^9, for fewer qubits).  Groups whose x agree above the tile
+// bits form a class: every group of a class pairs tile J with tile J ^ (x >> 12).
+// A CTA keeps tile J in registers, brings the other one into shared memory
+// once for all groups of the class, and the next one while it computes
+// (before, every group read both from L2).  A group is cut into sub-groups of
+// at most 8 terms of even y (which take Re t) and 8 of odd y (Im t).
 //
-// Adjoint: (H psi)[j] = sum_g F_g(j^x_g) psi[j^x_g],
-//   F_g(b) = sum_{k in g} c_k i^{y_k} (-1)^{popc(z_k&b)},
-// output-stationary: a thread owns 16 outputs, walked in Gray-code order.
-// Terms are cut into pieces of at most 8; F over a piece is a lookup in a
-// table of its 2^8 sign patterns, so a group costs one lookup per piece.
+// Forward.  A warp holds 32 x 16 amplitudes of the tile.  The sums of 8 terms
+// over them are matrix products: signs (8 terms x 4 amplitudes) times t (4
+// amplitudes x 8), FP64 m8n8k4, 16 of them a component whatever the number of
+// terms; what is left of the columns is added up with the terms' signs.
 //
-// Every partial sum is stored per chunk and reduced in a fixed order: results
-// are deterministic run to run.
+// Adjoint.  (H psi)[j] = sum_g F_g(j^x) psi[j^x].  F's real part at j is an entry
+// of a table of the 2^8 sign patterns of the sub-group's even terms, its
+// imaginary part one of the odd terms': two 8-byte shared-memory reads an
+// amplitude.  The patterns are a linear function of j, the XOR of a word for the
+// tile, the warp, the lane and the thread's own amplitudes.
+//
+// Every partial sum is stored and reduced in a fixed order: results are
+// deterministic run to run.
 
 #include <cuda_runtime.h>
 
@@ -47,74 +48,79 @@ namespace {
 using wgd::c128;
 
 constexpr int kThreads = 256;
-constexpr int kTileBits = 19;            // amplitudes per tile: 2^19
-constexpr int kSubTerms = 16;            // terms per forward sub-group
-constexpr int kChunkLog = 16;            // pairs per forward item: 2^16
-constexpr int kPiece = 8;                // terms per adjoint table
-constexpr int kQuadTerms = 4 * kPiece;   // terms per adjoint quad (four tables)
-constexpr int kAdjR = 16;                // outputs per thread in the adjoint
-constexpr int kAdjTileLog = 12;          // outputs per adjoint item: 2^12
-constexpr int kAdjQuadChunk = 2048;      // quads whose tile sign masks a CTA stages at a time
+constexpr int kTileBits = 12;            // amplitudes per tile: 2^12 at most
+constexpr int kTileMin = 9;              // and 2^9 at least (zeros above 2^n)
+constexpr int kTileMax = 1 << kTileBits;
+constexpr int kPiece = 8;                // terms per sub-group of either parity of y
+constexpr int kSegSubs = 16;             // sub-groups of one class staged at a time (adjoint)
+constexpr int kSegEntries = 2048;        // and their table entries
+constexpr int kChunkPieces = 32;         // pieces of one forward item
+constexpr int kFwdThreads = 512;         // two sets of 256 x 16 amplitudes = a tile
+constexpr int kFwdInner = 8;             // warps of a set
+constexpr int kAdjThreads = 512;         // x 8 amplitudes = a tile
 constexpr uint32_t kDiagFlag = 4;        // ty bit: the term's group has x == 0
+constexpr uint32_t kTwiceFlag = 8;       // ty bit: the forward pass meets every pair of the group twice
 
-enum SubKind : uint32_t { kDiag = 0, kLowX = 1, kHighX = 2 };
-
-struct ClassDev {
-  uint32_t units;    // tile pairs (or tiles) of the class
-  uint32_t ipu;      // items per unit: the chunks of every sub-group
-  uint32_t s0, s1;   // sub-group range
-  int pivot_hi;      // lowest set bit of x >> t (kind kHighX)
-  int pad;
+// A piece of a sub-group: terms [t0, t0 + nk), all of even or all of odd y.
+struct __align__(16) FwdPiece {
+  uint32_t xlo;              // x within the tile
+  uint32_t xhi;              // and above it
+  uint32_t t0;
+  uint16_t nk, odd;
+  uint32_t zlo[kPiece];      // z within the tile
+  uint32_t zhi[kPiece];      // and above it
 };
+static_assert(sizeof(FwdPiece) == 80, "copied in 16-byte pieces");
 
-struct SubDev {
-  uint64_t x;
-  uint64_t pbase;    // first partial of the sub-group's terms
-  uint32_t t0, nk;   // terms [t0, t0 + nk) in sorted order
-  uint32_t imag;     // bit kk: term kk reads Im t
-  uint32_t chunks;   // chunks per unit
-  uint32_t cpre;     // chunk offset of the sub-group within its class's unit
-  uint32_t chlog;    // pairs per chunk: 2^chlog
-  uint32_t nch;      // partials per term: units * chunks
-  uint32_t kind;     // SubKind
-  int pivot;         // lowest set bit of x (kind kLowX)
-  int pad;
+// A sub-group: terms [t0, t0 + nre) of even y, then nim of odd y.  A sign word has the even terms' signs in bits
+// 3-10, the odd ones' in bits 19-26: byte offsets into the tables.
+struct __align__(16) AdjSub {
+  uint32_t xlo;
+  uint32_t tab;              // first entry of its tables: 2^nre, then 2^nim
+  uint32_t t0;
+  uint16_t nre, nim;
+  uint32_t mixed;            // some coefficient is neither real nor imaginary (set with the coefficients)
+  uint32_t pad[3];
+  uint32_t zhi[2 * kPiece];  // z above the tile
+  uint32_t own[8];           // signs for the thread's amplitudes (tile bits m-3 to m-1)
+  uint32_t warp[16];         // for tile bits 5 to m-4
+  uint32_t lane[32];         // for tile bits 0-4
 };
+static_assert(sizeof(AdjSub) == 320, "copied in 16-byte pieces");
 
-struct QuadDev {
-  uint64_t x;
-  uint32_t t0, nk;      // terms [t0, t0 + nk), at most 32
-  uint32_t tbase[4];    // table offsets of the four pieces
-  uint32_t plane[4];    // sign planes of bits 8..11 (Gray steps of the adjoint)
+// Consecutive sub-groups of one class.
+struct __align__(16) SegDev {
+  uint32_t xhi;          // x above the tile
+  uint32_t s0, subs;     // sub-groups [s0, s0 + subs)
+  uint32_t tab, entries; // their table entries
+  uint32_t pad[3];
 };
 
 // Device-side description of one operator (kernel parameter, by value).
 struct PlanDev {
-  int n, t;
-  uint32_t T, G, NC, S, Q;
-  uint64_t items;            // forward items
-  const uint64_t* cls_item;  // [NC+1] item prefix per class
-  const ClassDev* cls;       // [NC]
-  const SubDev* sub;         // [S]
-  const uint32_t* zpl;       // [S][64] sign planes
-  const QuadDev* quad;       // [Q]
-  const uint64_t* tz;        // [T] sorted z-masks
-  const uint32_t* ty;        // [T] y mod 4 | kDiagFlag
+  int n, m;                  // qubits, tile bits
+  uint32_t T, G, S, NP, NS;  // terms, groups, sub-groups, pieces, segments
+  uint32_t tiles;            // 2^(n - m)
+  uint32_t chunks, ranges;   // forward items: chunks of pieces x ranges of tiles
+  const FwdPiece* piece;     // [NP]
+  AdjSub* asub;              // [S]
+  const SegDev* seg;         // [NS]
+  const uint32_t* chunk;     // [chunks + 1] first piece of a chunk
+  const uint32_t* ty;        // [T] y mod 4 | flags
   const uint32_t* torig;     // [T] original index of sorted term
-  const uint64_t* tpbase;    // [T] first partial of the term
-  const uint32_t* tnch;      // [T] partials of the term
   const double* coeffs;      // [2T] original-order coefficients
-  double* td;                // [2T] sorted c_k * i^y
-  double* table;             // [2 * entries] adjoint tables
-  double* partial;           // forward partial sums
-  uint32_t* stid;            // [Q][256] adjoint: bit kk = parity(z_kk & l) for lane offset l
+  double* table;             // adjoint tables of the part of c_k (-i)^y that its y makes it
+                             // (real where y is even)
+  double* other;             // and of the other part (read where AdjSub::mixed)
+  double* partial;           // [T][ranges] forward partial sums
 };
 
 struct wg_plan_host {
   int device;
   PlanDev dev;
   size_t n_groups = 0;
-  wg::Scratch blob, coeffs, td, table, partial, stid;
+  std::vector<uint32_t> bounds;  // segments of the adjoint's splits: splits + 1 bounds
+  wg::Scratch blob, coeffs, table, partial;
 };
 
 }  // namespace
@@ -124,11 +130,6 @@ struct wg_expect_plan_s {
 };
 
 namespace {
-
-__device__ __forceinline__ uint64_t insert_zero(uint64_t h, int p) {
-  const uint64_t lo = h & ((uint64_t{1} << p) - 1);
-  return ((h >> p) << (p + 1)) | lo;
-}
 
 template <typename Amp>
 __device__ __forceinline__ c128 load_amp(const void* psi, uint64_t i);
@@ -156,14 +157,19 @@ struct BatchDev {
   const PlanDev* plans;       // [np]
   const uint64_t* item_base;  // [np+1] forward items per pair
   const uint64_t* term_base;  // [np+1] flat term offsets
-  const uint64_t* tile_base;  // [np+1] adjoint items (0 for pairs without H psi)
+  const uint64_t* tile_base;  // [np+1] adjoint items (0 for pairs without H psi): tiles x splits
+  const uint64_t* amp_base;   // [np+1] amplitudes of the pairs whose adjoint is split
+  const uint32_t* splits;     // [np] parts of the segments an adjoint tile is split into
+  const uint32_t* split_at;   // [np] first entry of the pair's splits + 1 segment bounds
+  const uint32_t* bounds;
   const void* const* psis;    // [np]
   double* const* evals;       // [np] e_k outputs (original order)
   double* const* results;     // [np] E outputs or null
   double* const* hpsis;       // [np] H psi outputs or null
+  double2* const* parts;      // [np] splits x 2^n partial H psi, or null
   unsigned long long* counters;  // [2] forward / adjoint work queues
   uint32_t np;
-  uint64_t n_items, n_terms, n_tiles;
+  uint64_t n_items, n_terms, n_tiles, n_amps;
 };
 
 template <typename T>
@@ -178,176 +184,291 @@ __device__ __forceinline__ uint32_t upper_index(const T* base, uint32_t n, T v) 
   return lo;
 }
 
-// ------------------------------------------------------------- forward
+// ------------------------------------------------------------- tiles
 
-struct FwdShared {
-  uint32_t zpl[64];
-  uint64_t gmask[8];   // Gray level l: bit of b that flips
-  uint32_t gpl[8];     // Gray level l: sign plane of that bit
-  double red[kThreads / 32][kSubTerms];
-  unsigned long long item;
-};
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* to, const void* from) {
+  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(to));
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(from) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
 
-template <typename Amp, int KIND, int NK>
-__device__ __forceinline__ void forward_item(const PlanDev& P, const void* psi, const SubDev& sd, uint32_t u,
-                                             uint32_t ch, const ClassDev& cd, FwdShared& sh) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint64_t CH = uint64_t{1} << sd.chlog;
-  const int K = CH >= kThreads ? static_cast<int>(CH / kThreads) : 1;
-  const bool active = static_cast<uint64_t>(tid) < CH;
-  const int t = P.t;
-  const uint64_t x = sd.x;
-  // Gray-step tables: level l flips pair-index bit 8 + l, i.e. bit q(l) of b
-  if (tid < 8) {
-    const int j = 8 + tid;
-    const int q = KIND == kLowX ? j + (j >= sd.pivot ? 1 : 0) : j;
-    sh.gmask[tid] = q < 64 ? uint64_t{1} << q : 0;
-    sh.gpl[tid] = q < 64 ? sh.zpl[q] : 0u;
-  }
-  __syncthreads();
-  double accr[NK], acci[NK];
-#pragma unroll
-  for (int kk = 0; kk < NK; ++kk) accr[kk] = acci[kk] = 0.0;
-  double tre = 0.0, tim = 0.0;
-  if (active) {
-    const uint64_t h0 = static_cast<uint64_t>(ch) * CH + tid;
-    uint64_t b;
-    if (KIND == kDiag) b = (static_cast<uint64_t>(u) << t) | h0;
-    else if (KIND == kHighX) b = (insert_zero(u, cd.pivot_hi) << t) | h0;
-    else b = insert_zero((static_cast<uint64_t>(u) << (t - 1)) | h0, sd.pivot);
-    uint32_t S = 0;
-    for (uint32_t kk = 0; kk < sd.nk; ++kk) S |= static_cast<uint32_t>(__popcll(P.tz[sd.t0 + kk] & b) & 1) << kk;
-    const uint64_t m0 = sh.gmask[0];
-    const uint32_t p0 = sh.gpl[0];
-    // one pair: t = conj(psi[b ^ x]) psi[b]; every term with odd sign parity
-    // adds t to its masked sum (Re or Im is taken at the end)
-    auto pair = [&](uint64_t bb, uint32_t SS) {
-      const c128 a = load_amp<Amp>(psi, bb);
-      double vre, vim = 0.0;
-      if (KIND == kDiag) {
-        vre = a.re * a.re + a.im * a.im;
-      } else {
-        const c128 w = load_amp<Amp>(psi, bb ^ x);
-        vre = w.re * a.re + w.im * a.im;
-        vim = w.re * a.im - w.im * a.re;
+// Two tile buffers.  complex128 amplitudes are copied as they are, the next
+// tile into the other buffer; complex64 ones are copied into the second
+// buffer and widened from there into the first (once for all groups of a
+// class: the conversions would cost as much as the products).
+template <typename Amp>
+struct TileBuffers {
+  static constexpr bool kWide = sizeof(Amp) == 16;
+  double2* b0;
+  double2* b1;
+  int cur = 0;
+
+  // starts the copy of tile J (2^m amplitudes from J << m on, of 2^n); the
+  // caller commits
+  __device__ __forceinline__ void fetch(const void* psi, uint64_t J, int m, int n, int slot) {
+    const uint64_t base = J << m;
+    const int size = 1 << m, have = n < m ? 1 << n : size;
+    const Amp* from = static_cast<const Amp*>(psi) + base;
+    if constexpr (kWide) {
+      double2* to = slot ? b1 : b0;
+      for (int i = threadIdx.x; i < size; i += blockDim.x) {
+        if (i < have) copy_async<16>(to + i, from + i);
+        else to[i] = make_double2(0.0, 0.0);
       }
-      tre += vre;
-      if (KIND != kDiag) tim += vim;
-#pragma unroll
-      for (int kk = 0; kk < NK; ++kk) {
-        if ((SS >> kk) & 1u) {
-          accr[kk] += vre;
-          if (KIND != kDiag) acci[kk] += vim;
-        }
-      }
-    };
-    for (int k = 0; k < K; k += 2) {
-      if (k > 0) {
-        const int l = __ffs(k) - 1;  // >= 1
-        b ^= sh.gmask[l];
-        S ^= sh.gpl[l];
-      }
-      pair(b, S);
-      if (k + 1 < K) {
-        b ^= m0;
-        S ^= p0;
-        pair(b, S);
+    } else {
+      float2* to = reinterpret_cast<float2*>(b1);
+      for (int i = threadIdx.x; i < size; i += blockDim.x) {
+        if (i < have) copy_async<8>(to + i, from + i);
+        else to[i] = make_float2(0.0f, 0.0f);
       }
     }
   }
-  // per-term value: (sum of all) - 2 (sum over odd sign parity)
-#pragma unroll
-  for (int kk = 0; kk < NK; ++kk) {
-    const bool im = KIND != kDiag && ((sd.imag >> kk) & 1u);
-    const double v = im ? tim - 2.0 * acci[kk] : tre - 2.0 * accr[kk];
-    const double w = warp_sum(v);
-    if (lane == 0) sh.red[warp][kk] = w;
+  // complex64: the fetched tile, widened (all copies of this thread are done;
+  // each thread widens what it fetched)
+  __device__ __forceinline__ void widen(int m) {
+    const float2* from = reinterpret_cast<const float2*>(b1);
+    for (int i = threadIdx.x; i < (1 << m); i += blockDim.x) {
+      const float2 v = from[i];
+      b0[i] = make_double2(static_cast<double>(v.x), static_cast<double>(v.y));
+    }
   }
-  __syncthreads();
-  if (tid < static_cast<int>(sd.nk)) {
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w) s += sh.red[w][tid];
-    P.partial[sd.pbase + static_cast<uint64_t>(tid) * sd.nch + static_cast<uint64_t>(u) * sd.chunks + ch] = s;
-  }
+};
+
+// v with its sign flipped where bit 31 of `sign` is set
+__device__ __forceinline__ double flip(double v, uint32_t sign) {
+  return __hiloint2double(__double2hiint(v) ^ static_cast<int>(sign & 0x80000000u), __double2loint(v));
+}
+// ------------------------------------------------------------- forward
+
+struct FwdShared {
+  double2 tile[2][kTileMax];
+  double acc[kFwdInner][kChunkPieces * 32];  // by warp, piece, term and column quarter
+  FwdPiece piece[kChunkPieces];
+  uint32_t seg_xhi[kChunkPieces];
+  uint32_t seg_at[kChunkPieces + 1];
+  uint32_t segs;
+  unsigned long long item;
+};
+static_assert(sizeof(FwdShared) <= 227 * 1024, "shared memory of an SM");
+
+// C (8 x 8) += A (8 x 4) B (4 x 8) in FP64.  Lane l holds A[l / 4][l % 4],
+// B[l % 4][l / 4] and C[l / 4][2 (l % 4) + {0, 1}].
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
 }
 
-template <typename Amp, int KIND>
-__device__ __forceinline__ void forward_dispatch(const PlanDev& P, const void* psi, const SubDev& sd, uint32_t u,
-                                                 uint32_t ch, const ClassDev& cd, FwdShared& sh) {
-  switch ((sd.nk + 1) >> 1) {
-    case 0:
-    case 1: forward_item<Amp, KIND, 2>(P, psi, sd, u, ch, cd, sh); break;
-    case 2: forward_item<Amp, KIND, 4>(P, psi, sd, u, ch, cd, sh); break;
-    case 3: forward_item<Amp, KIND, 6>(P, psi, sd, u, ch, cd, sh); break;
-    case 4: forward_item<Amp, KIND, 8>(P, psi, sd, u, ch, cd, sh); break;
-    case 5: forward_item<Amp, KIND, 10>(P, psi, sd, u, ch, cd, sh); break;
-    case 6: forward_item<Amp, KIND, 12>(P, psi, sd, u, ch, cd, sh); break;
-    case 7: forward_item<Amp, KIND, 14>(P, psi, sd, u, ch, cd, sh); break;
-    default: forward_item<Amp, KIND, 16>(P, psi, sd, u, ch, cd, sh); break;
+// Where a thread's amplitudes lie in a tile of 2^m: M is m where it is known
+// at compile time (12 bits: the shifts become constants), else 0.
+template <int M>
+struct Layout {
+  int m_;
+  __device__ __forceinline__ int m() const { return M ? M : m_; }
+  __device__ __forceinline__ uint32_t off16(int r) const { return static_cast<uint32_t>(r) << (m() - 4); }
+  __device__ __forceinline__ uint32_t off8(int r) const { return static_cast<uint32_t>(r) << (m() - 3); }
+};
+
+// Adds a piece's sums over tile J to acc (the lane's place): a is the thread's
+// part of tile J, src the tile that x pairs it with.  Amplitude bits of the
+// tile: 0-1 lane % 4 (the products' inner index, with t's bits m-4 to m-2), 2-4
+// lane / 4 (the columns, with t's bit m-1), 5 to m-5 the warp.
+template <int M>
+__device__ __forceinline__ void forward_piece(const Layout<M>& lay, const FwdPiece& pd, const double2* src,
+                                              const c128 (&a)[16], uint32_t J, int tt, int lane, double* acc) {
+  constexpr uint32_t kSign = 0x80000000u;
+  const int m = lay.m();
+  const uint32_t at = static_cast<uint32_t>(tt) ^ pd.xlo;
+  double t[16];
+  if (pd.odd) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const double2 v = src[at ^ lay.off16(q)];
+      t[q] = fma(v.x, a[q].im, -(v.y * a[q].re));
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const double2 v = src[at ^ lay.off16(q)];
+      t[q] = fma(v.x, a[q].re, v.y * a[q].im);
+    }
   }
+  // the lane's term is lane / 4; its sign at the lane's and warp's share of the inner bits
+  const uint32_t zlo = pd.zlo[lane >> 2], zhi = pd.zhi[lane >> 2];
+  const uint32_t where = static_cast<uint32_t>(tt) & ~28u;
+  const uint32_t one = 0x3ff00000u ^ (static_cast<uint32_t>(__popc((zlo & where) ^ (zhi & J))) << 31);
+  const uint32_t e0 = (zlo << (35 - m)) & kSign, e1 = (zlo << (34 - m)) & kSign, e2 = (zlo << (33 - m)) & kSign;
+  double c00 = 0.0, c01 = 0.0, c10 = 0.0, c11 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    uint32_t hi = one;
+    if (k & 1) hi ^= e0;
+    if (k & 2) hi ^= e1;
+    if (k & 4) hi ^= e2;
+    const double s = __hiloint2double(static_cast<int>(hi), 0);
+    mma_f64(c00, c01, s, t[k]);
+    mma_f64(c10, c11, s, t[8 + k]);
+  }
+  const uint32_t bit2 = zlo << 29;
+  const double v = (c00 + flip(c01, bit2)) + flip(c10 + flip(c11, bit2), zlo << (32 - m));
+  *acc += flip(v, static_cast<uint32_t>(__popc((zlo >> 3) & (lane & 3))) << 31);
 }
 
+// A CTA takes (chunk of pieces, range of tiles) items.  24 qubits, 20,000 terms
+// in 1,699 groups: 50 ms (before, with 16 masked sums a pair: 87 ms); 20 qubits,
+// 4,096 terms in 2,526 groups: 2.2 ms (4.5).  Bound by instruction issue: the
+// matrix products are 15 of the 50 ms, a tile's fetch hides behind them.
 template <typename Amp>
-__global__ void __launch_bounds__(kThreads) expect_forward_kernel(BatchDev B) {
-  __shared__ FwdShared sh;
+__global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(BatchDev B) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  FwdShared& sh = *reinterpret_cast<FwdShared*>(raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   while (true) {
-    if (threadIdx.x == 0) sh.item = atomicAdd(B.counters, 1ull);
+    __syncthreads();
+    if (tid == 0) sh.item = atomicAdd(B.counters, 1ull);
     __syncthreads();
     const uint64_t item = sh.item;
     if (item >= B.n_items) break;
     const uint32_t p = upper_index<uint64_t>(B.item_base, B.np + 1, item);
     const PlanDev& P = B.plans[p];
-    const uint64_t r = item - B.item_base[p];
-    const uint32_t c = upper_index<uint64_t>(P.cls_item, P.NC + 1, r);
-    const ClassDev cd = P.cls[c];
-    const uint64_t rc = r - P.cls_item[c];
-    const uint32_t u = static_cast<uint32_t>(rc / cd.ipu);
-    const uint32_t r2 = static_cast<uint32_t>(rc - static_cast<uint64_t>(u) * cd.ipu);
-    // sub-group: last s in [s0, s1) with cpre <= r2
-    uint32_t lo = cd.s0, hi = cd.s1;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (P.sub[mid].cpre <= r2) lo = mid;
-      else hi = mid;
-    }
-    const SubDev sd = P.sub[lo];
-    const uint32_t ch = r2 - sd.cpre;
-    for (int q = threadIdx.x; q < 64; q += kThreads) sh.zpl[q] = q < P.n ? P.zpl[static_cast<uint64_t>(lo) * 64 + q] : 0u;
-    __syncthreads();
     const void* psi = B.psis[p];
-    if (sd.kind == kDiag) forward_dispatch<Amp, kDiag>(P, psi, sd, u, ch, cd, sh);
-    else if (sd.kind == kLowX) forward_dispatch<Amp, kLowX>(P, psi, sd, u, ch, cd, sh);
-    else forward_dispatch<Amp, kHighX>(P, psi, sd, u, ch, cd, sh);
+    const uint32_t r = static_cast<uint32_t>(item - B.item_base[p]);
+    // ranges outermost: the CTAs that run together meet the same tiles in L2
+    const uint32_t range = r / P.chunks, chunk = r - range * P.chunks;
+    const uint32_t piece0 = P.chunk[chunk], pieces = P.chunk[chunk + 1] - piece0;
+    const int m = P.m, n = P.n;
+    const uint32_t J0 = static_cast<uint32_t>(static_cast<uint64_t>(P.tiles) * range / P.ranges);
+    const uint32_t J1 = static_cast<uint32_t>(static_cast<uint64_t>(P.tiles) * (range + 1) / P.ranges);
+    // the chunk's pieces, and its runs of equal xhi
+    {
+      const uint4* from = reinterpret_cast<const uint4*>(P.piece + piece0);
+      uint4* to = reinterpret_cast<uint4*>(sh.piece);
+      for (uint32_t i = tid; i < pieces * (sizeof(FwdPiece) / 16); i += kFwdThreads) to[i] = from[i];
+      for (int i = tid; i < kFwdInner * kChunkPieces * 32; i += kFwdThreads) (&sh.acc[0][0])[i] = 0.0;
+      if (warp == 0) {
+        const uint32_t xhi = lane < static_cast<int>(pieces) ? P.piece[piece0 + lane].xhi : 0;
+        const uint32_t before = __shfl_up_sync(0xffffffffu, xhi, 1);
+        const bool head = lane < static_cast<int>(pieces) && (lane == 0 || xhi != before);
+        const uint32_t heads = __ballot_sync(0xffffffffu, head);
+        if (head) {
+          const int at = __popc(heads & ((1u << lane) - 1u));
+          sh.seg_xhi[at] = xhi;
+          sh.seg_at[at] = lane;
+        }
+        if (lane == 0) {
+          sh.segs = __popc(heads);
+          sh.seg_at[__popc(heads)] = pieces;
+        }
+      }
+    }
     __syncthreads();
+    const uint32_t segs = sh.segs;
+    // thread tt of the tile holds amplitudes tt + (q << m-4); the sets of
+    // threads (two for tiles of 2^12, more for smaller ones) take the pieces in
+    // turn: while one brings its operands in, the other's products run
+    const int tt = tid & ((1 << (m - 4)) - 1);
+    const uint32_t slice = tid >> (m - 4), slices = kFwdThreads >> (m - 4);
+    // (tile, segment) steps: a segment with x above the tile pairs J with
+    // J ^ xhi once, from the side whose lowest bit of xhi is clear
+    auto next_step = [&](uint32_t& J, uint32_t& g) {
+      while (J < J1) {
+        for (; g < segs; ++g) {
+          const uint32_t xhi = sh.seg_xhi[g];
+          if (xhi == 0 || !((J >> (__ffs(static_cast<int>(xhi)) - 1)) & 1u)) return true;
+        }
+        g = 0;
+        ++J;
+      }
+      return false;
+    };
+    TileBuffers<Amp> buf{sh.tile[0], sh.tile[1]};
+    constexpr bool kWide = TileBuffers<Amp>::kWide;
+    uint32_t J = J0, g = 0, have = 0xffffffffu;
+    bool more = next_step(J, g);
+    int slot = 0;
+    if (more) buf.fetch(psi, J ^ sh.seg_xhi[g], m, n, 0);
+    copy_commit();
+    c128 a[16];
+    while (more) {
+      uint32_t Jn = J, gn = g + 1;
+      const bool more_n = next_step(Jn, gn);
+      if (kWide) {
+        if (more_n) buf.fetch(psi, Jn ^ sh.seg_xhi[gn], m, n, slot ^ 1);
+        copy_commit();
+      }
+      if (have != J) {
+        have = J;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const uint64_t b = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(q) << (m - 4));
+          a[q] = (b >> n) == 0 ? load_amp<Amp>(psi, b) : c128{0.0, 0.0};
+        }
+      }
+      if (kWide) {
+        copy_wait<1>();
+      } else {
+        copy_wait<0>();
+        buf.widen(m);
+      }
+      __syncthreads();
+      if (!kWide) {
+        if (more_n) buf.fetch(psi, Jn ^ sh.seg_xhi[gn], m, n, 0);
+        copy_commit();
+      }
+      const double2* src = kWide && slot ? buf.b1 : buf.b0;
+      const uint32_t i1 = sh.seg_at[g + 1];
+      double* acc = sh.acc[tt >> 5] + lane;
+      if (m == kTileBits) {
+        const Layout<kTileBits> lay{m};
+        for (uint32_t i = sh.seg_at[g]; i < i1; ++i)
+          if ((i & 1u) == slice) forward_piece(lay, sh.piece[i], src, a, J, tt, lane, acc + 32 * i);
+      } else {
+        const Layout<0> lay{m};
+        for (uint32_t i = sh.seg_at[g]; i < i1; ++i)
+          if ((i & (slices - 1)) == slice) forward_piece(lay, sh.piece[i], src, a, J, tt, lane, acc + 32 * i);
+      }
+      __syncthreads();
+      J = Jn;
+      g = gn;
+      more = more_n;
+      slot ^= 1;
+    }
+    copy_wait<0>();
+    __syncthreads();
+    for (uint32_t k = tid; k < pieces * kPiece; k += kFwdThreads) {
+      const FwdPiece& pd = sh.piece[k / kPiece];
+      if (k % kPiece >= pd.nk) continue;
+      double s = 0.0;
+#pragma unroll
+      for (int v = 0; v < kFwdInner; ++v) {
+        const double* row = sh.acc[v] + 4 * k;
+        s += (row[0] + row[1]) + (row[2] + row[3]);
+      }
+      P.partial[static_cast<uint64_t>(pd.t0 + k % kPiece) * P.ranges + range] = s;
+    }
   }
 }
 
-// e_k from the chunk partials (summed in chunk order), scaled by the pairing
-// factor and scattered to original term order; flat over every pair's terms.
+// e_k from the ranges' partial sums (in order), scaled by the pairing factor
+// and scattered to original term order; flat over every pair's terms.
 __global__ void __launch_bounds__(kThreads) expect_finish_terms_kernel(BatchDev B) {
   for (uint64_t f = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; f < B.n_terms;
        f += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
     const uint32_t p = upper_index<uint64_t>(B.term_base, B.np + 1, f);
     const PlanDev& P = B.plans[p];
     const uint32_t k = static_cast<uint32_t>(f - B.term_base[p]);
-    const double* part = P.partial + P.tpbase[k];
-    const uint32_t nch = P.tnch[k];
+    const double* part = P.partial + static_cast<uint64_t>(k) * P.ranges;
     double s = 0.0;
-    for (uint32_t c = 0; c < nch; ++c) s += part[c];
+    for (uint32_t c = 0; c < P.ranges; ++c) s += part[c];
     const uint32_t ty = P.ty[k];
-    double e;
-    if (ty & kDiagFlag) {
-      e = s;
-    } else {
-      switch (ty & 3u) {
-        case 0: e = 2.0 * s; break;
-        case 1: e = -2.0 * s; break;
-        case 2: e = -2.0 * s; break;
-        default: e = 2.0 * s; break;
-      }
-    }
-    B.evals[p][P.torig[k]] = e;
+    const double e = ((ty & 3u) == 1 || (ty & 3u) == 2) ? -s : s;
+    B.evals[p][P.torig[k]] = ty & (kDiagFlag | kTwiceFlag) ? e : 2.0 * e;
   }
 }
 
@@ -388,149 +509,256 @@ __global__ void __launch_bounds__(kThreads) expect_total_kernel(BatchDev B) {
 
 // ------------------------------------------------------------- adjoint
 
-// Output-stationary adjoint over all pairs' tiles (persistent work queue): a
-// thread owns the outputs j = tile0 + tid + 256 gray(r), r < R.
+struct AdjStage {
+  AdjSub sub[kSegSubs];
+  double table[kSegEntries];
+};
+
+struct AdjShared {
+  double2 tile[2][kTileMax];
+  AdjStage stage[2];
+  unsigned long long item;
+};
+static_assert(sizeof(AdjShared) <= 227 * 1024, "shared memory of an SM");
+
+__device__ __forceinline__ double entry(const double* table, uint32_t bytes) {
+  return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(table) + bytes);
+}
+
+// Adds one sub-group's share of H psi in tile J to the thread's 8 amplitudes.
+// table: its staged tables; other: its tables of the other parts, in memory.
+template <int M>
+__device__ __forceinline__ void adjoint_sub(const Layout<M>& lay, const AdjSub& sd, const double* table,
+                                            const double* other, const double2* src, c128 (&acc)[8], uint32_t J,
+                                            int tt, int lane) {
+  constexpr uint32_t kOffsets = 8 * 255u;
+  // lanes 0-7 and 16-23 give the signs of the terms in the tile
+  const uint32_t mine = lane & 8 ? 0u : sd.zhi[(lane & 7) | ((lane & 16) >> 1)];
+  const uint32_t S = (__ballot_sync(0xffffffffu, __popc(mine & J) & 1) << 3) ^ sd.lane[lane] ^ sd.warp[tt >> 5];
+  const uint32_t nre = sd.nre, nim = sd.nim;
+  const uint32_t at = static_cast<uint32_t>(tt) ^ sd.xlo;
+  const double* tim = table + (1u << nre);
+  const uint4 o0 = reinterpret_cast<const uint4*>(sd.own)[0], o1 = reinterpret_cast<const uint4*>(sd.own)[1];
+  const uint32_t own[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+  if (sd.mixed) {
+    // complex coefficients: both tables add to both parts of F
+    const double* oim = other + (1u << nre);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const uint32_t q = S ^ own[r], qr = q & kOffsets, qi = (q >> 16) & kOffsets;
+      const double fre = entry(table, qr) + entry(oim, qi), fim = entry(tim, qi) + entry(other, qr);
+      const double2 v = src[at ^ lay.off8(r)];
+      acc[r].re = fma(-v.y, fim, fma(v.x, fre, acc[r].re));
+      acc[r].im = fma(v.y, fre, fma(v.x, fim, acc[r].im));
+    }
+  } else if (nim == 0) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const double fre = entry(table, (S ^ own[r]) & kOffsets);
+      const double2 v = src[at ^ lay.off8(r)];
+      acc[r].re = fma(v.x, fre, acc[r].re);
+      acc[r].im = fma(v.y, fre, acc[r].im);
+    }
+  } else if (nre == 0) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const double fim = entry(tim, ((S ^ own[r]) >> 16) & kOffsets);
+      const double2 v = src[at ^ lay.off8(r)];
+      acc[r].re = fma(-v.y, fim, acc[r].re);
+      acc[r].im = fma(v.x, fim, acc[r].im);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const uint32_t q = S ^ own[r];
+      const double fre = entry(table, q & kOffsets), fim = entry(tim, (q >> 16) & kOffsets);
+      const double2 v = src[at ^ lay.off8(r)];
+      acc[r].re = fma(-v.y, fim, fma(v.x, fre, acc[r].re));
+      acc[r].im = fma(v.y, fre, fma(v.x, fim, acc[r].im));
+    }
+  }
+}
+
+// Output-stationary: a CTA owns tile J of H psi, 8 amplitudes a thread, and
+// walks the segments of its split.  Bound by shared-memory wavefronts (71 % of
+// the cycles; 8 an amplitude and sub-group at least: 4 for psi, 2 for either
+// table): 44 ms on 24 qubits with 20,000 terms (80 ms with tables of complex
+// entries and psi read through L1).
 template <typename Amp>
-__global__ void __launch_bounds__(kThreads) expect_adjoint_kernel(BatchDev B) {
-  __shared__ unsigned long long s_item;
-  __shared__ uint32_t s_hi[kAdjQuadChunk];  // per quad of the chunk: parity(z & (hi ^ x)) masks
-  const int tid = threadIdx.x;
+__global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(BatchDev B) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  AdjShared& sh = *reinterpret_cast<AdjShared*>(raw);
+  const int tid = threadIdx.x, lane = tid & 31;
+  constexpr bool kWide = TileBuffers<Amp>::kWide;
   while (true) {
-    if (tid == 0) s_item = atomicAdd(B.counters + 1, 1ull);
     __syncthreads();
-    const uint64_t item = s_item;
+    if (tid == 0) sh.item = atomicAdd(B.counters + 1, 1ull);
     __syncthreads();
+    const uint64_t item = sh.item;
     if (item >= B.n_tiles) break;
     const uint32_t p = upper_index<uint64_t>(B.tile_base, B.np + 1, item);
     const PlanDev& P = B.plans[p];
     const void* psi = B.psis[p];
-    double* hpsi = B.hpsis[p];
-    const int tlog = P.n < kAdjTileLog ? P.n : kAdjTileLog;
-    const uint64_t TS = uint64_t{1} << tlog;
-    const int R = TS >= kThreads ? static_cast<int>(TS / kThreads) : 1;
-    const bool active = static_cast<uint64_t>(tid) < TS;
-    // b = j0 ^ x splits into the tile's bits and the lane's: j0 = hi + tid
-    // with hi a multiple of TS (>= 256 or 0), so a term's sign parity(z & b)
-    // is parity(z & (hi ^ x)) -- staged per quad by the CTA, once per tile --
-    // XOR parity(z & tid), the plan's stid table.
-    const uint64_t hi = (item - B.tile_base[p]) * TS;
-    const uint64_t j0 = hi + tid;
-    c128 acc[kAdjR];
+    const uint32_t splits = B.splits[p];
+    const uint64_t rest = item - B.tile_base[p];
+    // tiles outermost: the CTAs that run together share tiles and segments
+    const uint32_t J = static_cast<uint32_t>(rest / splits), split = static_cast<uint32_t>(rest - static_cast<uint64_t>(J) * splits);
+    const uint32_t g0 = B.bounds[B.split_at[p] + split], g1 = B.bounds[B.split_at[p] + split + 1];
+    const int m = P.m, n = P.n;
+    const int tt = tid & ((1 << (m - 3)) - 1);
+    const uint32_t slice = tid >> (m - 3), slices = kAdjThreads >> (m - 3);
+    TileBuffers<Amp> buf{sh.tile[0], sh.tile[1]};
+    auto fetch_stage = [&](const SegDev& sg, int slot) {
+      AdjStage& st = sh.stage[slot];
+      const char* from = reinterpret_cast<const char*>(P.asub + sg.s0);
+      char* to = reinterpret_cast<char*>(st.sub);
+      for (uint32_t i = tid; i < sg.subs * (sizeof(AdjSub) / 16); i += kAdjThreads)
+        copy_async<16>(to + 16 * i, from + 16 * i);
+      for (uint32_t i = tid; i < sg.entries / 2; i += kAdjThreads)
+        copy_async<16>(st.table + 2 * i, P.table + sg.tab + 2 * i);
+    };
+    c128 acc[8];
 #pragma unroll
-    for (int r = 0; r < kAdjR; ++r) acc[r] = {0.0, 0.0};
-    const double2* tab = reinterpret_cast<const double2*>(P.table);
-    for (uint32_t q0 = 0; q0 < P.Q; q0 += kAdjQuadChunk) {
-      const uint32_t qn = min(static_cast<uint32_t>(kAdjQuadChunk), P.Q - q0);
-      __syncthreads();  // the previous chunk's masks are read
-      for (uint32_t qq = tid; qq < qn; qq += kThreads) {
-        const QuadDev* qd = P.quad + q0 + qq;
-        const uint64_t hb = hi ^ qd->x;
-        const uint32_t nk = qd->nk, t0 = qd->t0;
-        uint32_t m = 0;
-        for (uint32_t kk = 0; kk < nk; ++kk) m |= static_cast<uint32_t>(__popcll(P.tz[t0 + kk] & hb) & 1) << kk;
-        s_hi[qq] = m;
+    for (int r = 0; r < 8; ++r) acc[r] = {0.0, 0.0};
+    int slot = 0, stage = 0;
+    SegDev sg = P.seg[g0], nx = P.seg[min(g0 + 1, g1 - 1)];
+    buf.fetch(psi, J ^ sg.xhi, m, n, 0);
+    fetch_stage(sg, 0);
+    copy_commit();
+    bool fresh = true;  // the segment's tile is not the one before's
+    for (uint32_t g = g0; g < g1; ++g) {
+      const bool last = g + 1 == g1;
+      const SegDev after = P.seg[min(g + 2, g1 - 1)];  // a step ahead of its use
+      const bool fresh_n = !last && nx.xhi != sg.xhi;
+      if (kWide) {
+        if (fresh_n) buf.fetch(psi, J ^ nx.xhi, m, n, slot ^ 1);
+        if (!last) fetch_stage(nx, stage ^ 1);
+        copy_commit();
+        copy_wait<1>();
+      } else {
+        copy_wait<0>();
+        if (fresh) buf.widen(m);
       }
       __syncthreads();
-      if (!active) continue;
-      for (uint32_t qq = 0; qq < qn; ++qq) {
-        const uint32_t qi = q0 + qq;
-        const QuadDev* qd = P.quad + qi;  // read in place: its small arrays are indexed at run time
-        const uint32_t nk = qd->nk;
-        uint64_t b = j0 ^ qd->x;
-        uint32_t S = s_hi[qq] ^ P.stid[static_cast<size_t>(qi) * kThreads + tid];
-        const int np = static_cast<int>((nk + kPiece - 1) / kPiece);
-        uint32_t pl[4], tb[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          pl[q] = qd->plane[q];
-          tb[q] = qd->tbase[q];
+      if (!kWide) {
+        if (fresh_n) buf.fetch(psi, J ^ nx.xhi, m, n, 0);
+        if (!last) fetch_stage(nx, stage ^ 1);
+        copy_commit();
+      }
+      const double2* src = kWide && slot ? buf.b1 : buf.b0;
+      const AdjStage& st = sh.stage[stage];
+      if (m == kTileBits) {
+        const Layout<kTileBits> lay{m};
+        for (uint32_t i = 0; i < sg.subs; ++i) {
+          const AdjSub& sd = st.sub[i];
+          adjoint_sub(lay, sd, st.table + (sd.tab - sg.tab), P.other + sd.tab, src, acc, J, tt, lane);
         }
+      } else {
+        const Layout<0> lay{m};
+        for (uint32_t i = 0; i < sg.subs; ++i) {
+          if ((i & (slices - 1)) != slice) continue;
+          const AdjSub& sd = st.sub[i];
+          adjoint_sub(lay, sd, st.table + (sd.tab - sg.tab), P.other + sd.tab, src, acc, J, tt, lane);
+        }
+      }
+      __syncthreads();
+      if (fresh_n) slot ^= 1;
+      fresh = fresh_n;
+      stage ^= 1;
+      sg = nx;
+      nx = after;
+    }
+    copy_wait<0>();
+    if (slices > 1) {
+      // the slices' sums, slice by slice (the tile buffers are free)
+      __syncthreads();
 #pragma unroll
-        for (int r = 0; r < kAdjR; ++r) {
-          if (r < R) {
-            if (r > 0) {
-              // Gray step flips output bit 8 + ctz(r), and the same bit of b
-              const int j = (r & 1) ? 0 : (r & 2) ? 1 : (r & 4) ? 2 : 3;
-              b ^= uint64_t{1} << (8 + j);
-              S ^= pl[j];
-            }
-            const double2 f0 = tab[tb[0] + (S & 0xffu)];
-            double fre = f0.x, fim = f0.y;
+      for (int r = 0; r < 8; ++r) {
+        const uint32_t j = tt + (static_cast<uint32_t>(r) << (m - 3));
+        sh.tile[0][(slice << m) + j] = make_double2(acc[r].re, acc[r].im);
+      }
+      __syncthreads();
+      if (slice == 0) {
 #pragma unroll
-            for (int pc = 1; pc < 4; ++pc) {
-              if (pc < np) {
-                const double2 f = tab[tb[pc] + ((S >> (kPiece * pc)) & 0xffu)];
-                fre += f.x;
-                fim += f.y;
-              }
-            }
-            const c128 v = load_amp<Amp>(psi, b);
-            acc[r].re += v.re * fre - v.im * fim;
-            acc[r].im += v.re * fim + v.im * fre;
+        for (int r = 0; r < 8; ++r) {
+          const uint32_t j = tt + (static_cast<uint32_t>(r) << (m - 3));
+          for (uint32_t v = 1; v < slices; ++v) {
+            const double2 o = sh.tile[0][(v << m) + j];
+            acc[r].re += o.x;
+            acc[r].im += o.y;
           }
         }
       }
     }
-    if (!active) continue;
-    uint64_t j = j0;
+    if (slice == 0) {
+      double2* out = splits > 1 ? B.parts[p] + (static_cast<uint64_t>(split) << n) : reinterpret_cast<double2*>(B.hpsis[p]);
 #pragma unroll
-    for (int r = 0; r < kAdjR; ++r) {
-      if (r < R) {
-        if (r > 0) j ^= uint64_t{1} << (8 + ((r & 1) ? 0 : (r & 2) ? 1 : (r & 4) ? 2 : 3));
-        reinterpret_cast<double2*>(hpsi)[j] = make_double2(acc[r].re, acc[r].im);
+      for (int r = 0; r < 8; ++r) {
+        const uint64_t j = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(r) << (m - 3));
+        if ((j >> n) == 0) out[j] = make_double2(acc[r].re, acc[r].im);
       }
     }
+  }
+}
+
+// H psi of the pairs whose segments were split, summed over the splits in order.
+__global__ void __launch_bounds__(kThreads) expect_join_kernel(BatchDev B) {
+  for (uint64_t f = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; f < B.n_amps;
+       f += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    const uint32_t p = upper_index<uint64_t>(B.amp_base, B.np + 1, f);
+    const uint64_t j = f - B.amp_base[p];
+    const double2* part = B.parts[p] + j;
+    const uint32_t splits = B.splits[p];
+    const int n = B.plans[p].n;
+    double2 s = part[0];
+    for (uint32_t k = 1; k < splits; ++k) {
+      const double2 v = part[static_cast<uint64_t>(k) << n];
+      s.x += v.x;
+      s.y += v.y;
+    }
+    reinterpret_cast<double2*>(B.hpsis[p])[j] = s;
   }
 }
 
 // ------------------------------------------------------------- plan build
 
-// stid[q][l] bit kk = parity(z_kk & l) over the terms of quad q, for the
-// adjoint's lane offsets l < 256 (z-masks only: built once per plan).
-__global__ void plan_stid_kernel(PlanDev P) {
-  const uint32_t l = threadIdx.x;
-  for (uint32_t q = blockIdx.x; q < P.Q; q += gridDim.x) {
-    const QuadDev* qd = P.quad + q;
-    const uint32_t nk = qd->nk, t0 = qd->t0;
-    uint32_t m = 0;
-    for (uint32_t kk = 0; kk < nk; ++kk) m |= static_cast<uint32_t>(__popcll(P.tz[t0 + kk] & l) & 1) << kk;
-    P.stid[static_cast<size_t>(q) * kThreads + l] = m;
-  }
-}
-
-// td[i] = c[torig[i]] * i^{y_i} (sorted order).
-__global__ void plan_coeffs_kernel(PlanDev P) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.T; i += gridDim.x * blockDim.x) {
-    const uint32_t o = P.torig[i];
-    const c128 d = wgd::rotate(c128{P.coeffs[2 * o], P.coeffs[2 * o + 1]}, P.ty[i] & 3u);
-    P.td[2 * i] = d.re;
-    P.td[2 * i + 1] = d.im;
-  }
-}
-
-// Adjoint tables: entry s of a piece = sum over its terms of td * (-1)^{bit kk of s},
-// in term order; one block per quad.
+// The adjoint's tables from the coefficients, a warp per sub-group: entry q of
+// a piece is the sum of its terms' c_k (-i)^y_k (i^y, and (-1)^y for the signs,
+// which are those at j where the adjoint needs them at j ^ x), with the sign of
+// bit kk of q, in order.
 __global__ void plan_tables_kernel(PlanDev P) {
-  for (uint32_t qi = blockIdx.x; qi < P.Q; qi += gridDim.x) {
-    const QuadDev qd = P.quad[qi];
-    for (uint32_t pc = 0; pc * kPiece < qd.nk; ++pc) {
-      const uint32_t t0 = qd.t0 + pc * kPiece;
-      const uint32_t np = min(static_cast<uint32_t>(kPiece), qd.nk - pc * kPiece);
-      for (uint32_t s = threadIdx.x; s < (1u << np); s += blockDim.x) {
-        double re = 0.0, im = 0.0;
-        for (uint32_t kk = 0; kk < np; ++kk) {
-          const double dre = P.td[2 * (t0 + kk)], dim = P.td[2 * (t0 + kk) + 1];
-          if ((s >> kk) & 1u) {
-            re -= dre;
-            im -= dim;
-          } else {
-            re += dre;
-            im += dim;
-          }
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < P.S; i += (gridDim.x * blockDim.x) >> 5) {
+    AdjSub& sd = P.asub[i];
+    // lane kk holds term kk of the sub-group
+    double own = 0.0, other = 0.0;
+    if (lane < static_cast<uint32_t>(sd.nre) + sd.nim) {
+      const uint32_t k = sd.t0 + lane, o = P.torig[k];
+      const c128 d = wgd::rotate(c128{P.coeffs[2 * o], P.coeffs[2 * o + 1]}, (4u - (P.ty[k] & 3u)) & 3u);
+      const bool odd = P.ty[k] & 1u;
+      own = odd ? d.im : d.re;
+      other = odd ? d.re : d.im;
+    }
+    const bool mixed = __any_sync(0xffffffffu, other != 0.0);  // true for a NaN
+    if (lane == 0) sd.mixed = mixed;
+    uint32_t first = 0, tab = sd.tab;
+    for (int half = 0; half < 2; ++half) {
+      const uint32_t nk = half ? sd.nim : sd.nre;
+      for (uint32_t q0 = 0; q0 < (1u << nk); q0 += 32) {
+        const uint32_t q = q0 + lane;
+        double a = 0.0, b = 0.0;
+        for (uint32_t kk = 0; kk < nk; ++kk) {
+          const double x = __shfl_sync(0xffffffffu, own, first + kk), y = __shfl_sync(0xffffffffu, other, first + kk);
+          a += (q >> kk) & 1u ? -x : x;
+          b += (q >> kk) & 1u ? -y : y;
         }
-        P.table[2 * (qd.tbase[pc] + s)] = re;
-        P.table[2 * (qd.tbase[pc] + s) + 1] = im;
+        if (q < (1u << nk)) {
+          P.table[tab + q] = a;
+          if (mixed) P.other[tab + q] = b;
+        }
       }
+      tab += 1u << nk;
+      first += nk;
     }
   }
 }
@@ -538,12 +766,8 @@ __global__ void plan_tables_kernel(PlanDev P) {
 void refresh_coeffs(const wg_plan_host& h, cudaStream_t s) {
   const PlanDev& P = h.dev;
   if (P.T == 0) return;
-  plan_coeffs_kernel<<<wg::grid_for(P.T, kThreads, h.device, 4), kThreads, 0, s>>>(P);
-  wg::check_launch("launch plan coefficients");
-  if (P.Q) {
-    plan_tables_kernel<<<std::min<uint32_t>(P.Q, 65535u), kThreads, 0, s>>>(P);
-    wg::check_launch("launch adjoint tables");
-  }
+  plan_tables_kernel<<<wg::grid_for(32 * static_cast<size_t>(P.S), kThreads, h.device, 8), kThreads, 0, s>>>(P);
+  wg::check_launch("launch adjoint tables");
 }
 
 // Appends raw bytes to the host image of the plan, 16-byte aligned.
@@ -568,7 +792,8 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   std::memset(&d, 0, sizeof(d));
   d.n = static_cast<int>(n);
   d.T = static_cast<uint32_t>(T);
-  d.t = std::min<int>(static_cast<int>(n), kTileBits);
+  d.m = std::max(kTileMin, std::min(static_cast<int>(n), kTileBits));
+  d.tiles = static_cast<int>(n) > d.m ? 1u << std::min<int>(31, static_cast<int>(n) - d.m) : 1u;
   p->coeffs.reset(std::max<size_t>(16, 16 * T), s);
   if (T) wg::check_cuda(cudaMemcpyAsync(p->coeffs.get(), c, 16 * T, cudaMemcpyDeviceToDevice, s), "copy coefficients");
   d.coeffs = p->coeffs.as<double>();
@@ -591,143 +816,166 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
     // the kernels index psi[b ^ x]: masks must stay below 2^n
     if ((bits >> n) != 0) wg::throw_invalid("Pauli masks set bits at or above num_qubits");
   }
-  // terms sorted by x (stable): groups
+  // terms sorted by x (stable): groups; by (x >> m, x) at once, since x sorts that way
   std::vector<uint32_t> order(T);
   std::iota(order.begin(), order.end(), 0u);
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return hx[a] < hx[b]; });
-  const int t = d.t;
-  std::vector<uint64_t> tz(T), tpbase(T);
-  std::vector<uint32_t> ty(T), torig(T), tnch(T);
-  std::vector<ClassDev> cls;
-  std::vector<uint64_t> cls_item{0};
-  std::vector<SubDev> sub;
-  std::vector<uint32_t> zpl;
-  std::vector<QuadDev> quad;
-  uint32_t table_entries = 0;
-  uint64_t pbase = 0;
-  size_t groups = 0;
-  for (size_t i = 0; i < T; ++i) {
-    const uint32_t o = order[i];
-    tz[i] = hz[o];
-    ty[i] = static_cast<uint32_t>(__builtin_popcountll(hx[o] & hz[o]) & 3) | (hx[o] == 0 ? kDiagFlag : 0u);
-    torig[i] = o;
-  }
-  size_t g0 = 0;
-  while (g0 < T) {
-    // one class: groups with equal x >> t
-    const uint64_t xhi = t < 64 ? (hx[order[g0]] >> t) : 0;
-    ClassDev cd{};
-    cd.s0 = static_cast<uint32_t>(sub.size());
-    cd.pivot_hi = xhi ? __builtin_ctzll(xhi) : 0;
-    const int rest = static_cast<int>(n) - t;  // tile-number bits
-    cd.units = xhi ? (rest > 0 ? 1u << (rest - 1) : 1u) : (1u << rest);
-    size_t gi = g0;
-    uint32_t cpre = 0;
-    std::vector<size_t> class_subs;
-    while (gi < T && (t < 64 ? (hx[order[gi]] >> t) : 0) == xhi) {
-      const uint64_t gx = hx[order[gi]];
-      size_t ge = gi;
-      while (ge < T && hx[order[ge]] == gx) ++ge;
-      ++groups;
-      // forward sub-groups
-      for (size_t s0 = gi; s0 < ge; s0 += kSubTerms) {
-        SubDev sd{};
-        sd.x = gx;
-        sd.t0 = static_cast<uint32_t>(s0);
-        sd.nk = static_cast<uint32_t>(std::min<size_t>(kSubTerms, ge - s0));
-        sd.kind = gx == 0 ? kDiag : (xhi ? kHighX : kLowX);
-        sd.pivot = gx ? __builtin_ctzll(gx) : 0;
-        const int replog = sd.kind == kLowX ? t - 1 : t;
-        sd.chlog = static_cast<uint32_t>(std::min(kChunkLog, replog));
-        sd.chunks = 1u << (replog - static_cast<int>(sd.chlog));
-        sd.nch = cd.units * sd.chunks;
-        sd.cpre = cpre;
-        cpre += sd.chunks;
-        sd.pbase = pbase;
-        pbase += static_cast<uint64_t>(sd.nk) * sd.nch;
-        for (uint32_t kk = 0; kk < sd.nk; ++kk) {
-          if (ty[s0 + kk] & 1u) sd.imag |= 1u << kk;
-          tpbase[s0 + kk] = sd.pbase + static_cast<uint64_t>(kk) * sd.nch;
-          tnch[s0 + kk] = sd.nch;
+  const int m = d.m;
+  std::vector<uint32_t> ty(T), torig(T), seg_cost, chunk{0};
+  std::vector<FwdPiece> piece;
+  std::vector<AdjSub> asub;
+  std::vector<SegDev> seg;
+  // the order of a piece's terms: those whose z are linearly independent on the
+  // lane bits first, so that the lanes' entries spread over the banks
+  auto spread = [&](uint32_t* first, uint32_t count) {
+    uint32_t basis[5] = {}, at = 0;
+    for (uint32_t i = 0; i < count; ++i) {
+      uint32_t v = static_cast<uint32_t>(hz[first[i]]) & 31u;
+      for (int b = 4; b >= 0 && v; --b) {
+        if (!((v >> b) & 1u)) continue;
+        if (basis[b]) {
+          v ^= basis[b];
+          continue;
         }
-        for (int q = 0; q < 64; ++q) {
-          uint32_t m = 0;
-          for (uint32_t kk = 0; kk < sd.nk; ++kk)
-            if (q < static_cast<int>(n) && ((tz[s0 + kk] >> q) & 1u)) m |= 1u << kk;
-          zpl.push_back(m);
-        }
-        sub.push_back(sd);
+        basis[b] = v;
+        std::rotate(first + at, first + i, first + i + 1);
+        ++at;
+        break;
       }
-      // adjoint quads
-      for (size_t q0 = gi; q0 < ge; q0 += kQuadTerms) {
-        QuadDev qd{};
-        qd.x = gx;
-        qd.t0 = static_cast<uint32_t>(q0);
-        qd.nk = static_cast<uint32_t>(std::min<size_t>(kQuadTerms, ge - q0));
-        for (uint32_t pc = 0; pc * kPiece < qd.nk; ++pc) {
-          const uint32_t np = std::min<uint32_t>(kPiece, qd.nk - pc * kPiece);
-          qd.tbase[pc] = table_entries;
-          table_entries += 1u << np;
-        }
-        for (int j = 0; j < 4; ++j) {
-          uint32_t m = 0;
-          const int bit = 8 + j;
-          for (uint32_t kk = 0; kk < qd.nk; ++kk)
-            if (bit < static_cast<int>(n) && ((tz[q0 + kk] >> bit) & 1u)) m |= 1u << kk;
-          qd.plane[j] = m;
-        }
-        quad.push_back(qd);
-      }
-      gi = ge;
     }
-    cd.s1 = static_cast<uint32_t>(sub.size());
-    cd.ipu = cpre;
-    cls.push_back(cd);
-    cls_item.push_back(cls_item.back() + static_cast<uint64_t>(cd.units) * cd.ipu);
-    g0 = gi;
+  };
+  size_t groups = 0;
+  uint64_t entries = 0;
+  std::vector<uint32_t> even, odd;
+  for (size_t g0 = 0, t0 = 0; g0 < T;) {
+    const uint64_t gx = hx[order[g0]];
+    size_t ge = g0;
+    even.clear();
+    odd.clear();
+    for (; ge < T && hx[order[ge]] == gx; ++ge) {
+      const uint32_t o = order[ge];
+      (__builtin_popcountll(gx & hz[o]) & 1 ? odd : even).push_back(o);
+    }
+    ++groups;
+    const size_t subs = std::max((even.size() + kPiece - 1) / kPiece, (odd.size() + kPiece - 1) / kPiece);
+    for (size_t i = 0; i < subs; ++i) {
+      AdjSub ad{};
+      ad.xlo = static_cast<uint32_t>(gx & ((uint64_t{1} << m) - 1));
+      ad.t0 = static_cast<uint32_t>(t0);
+      ad.tab = static_cast<uint32_t>(entries);
+      uint32_t plane[kTileBits] = {};  // sign word of tile bit q
+      for (int half = 0; half < 2; ++half) {
+        std::vector<uint32_t>& all = half ? odd : even;
+        const size_t from = std::min(all.size(), i * kPiece);
+        const uint32_t nk = static_cast<uint32_t>(std::min<size_t>(kPiece, all.size() - from));
+        (half ? ad.nim : ad.nre) = static_cast<uint16_t>(nk);
+        spread(all.data() + from, nk);
+        FwdPiece pd{};
+        pd.xlo = ad.xlo;
+        pd.xhi = static_cast<uint32_t>(gx >> m);
+        pd.t0 = static_cast<uint32_t>(t0);
+        pd.nk = static_cast<uint16_t>(nk);
+        pd.odd = static_cast<uint16_t>(half);
+        for (uint32_t kk = 0; kk < nk; ++kk, ++t0) {
+          const uint32_t o = all[from + kk];
+          torig[t0] = o;
+          ty[t0] = static_cast<uint32_t>(__builtin_popcountll(gx & hz[o]) & 3) |
+                   (gx == 0 ? kDiagFlag : (gx >> m) == 0 ? kTwiceFlag : 0u);
+          pd.zlo[kk] = static_cast<uint32_t>(hz[o] & ((uint64_t{1} << m) - 1));
+          pd.zhi[kk] = ad.zhi[half * kPiece + kk] = static_cast<uint32_t>(hz[o] >> m);
+          for (int q = 0; q < m; ++q) plane[q] |= static_cast<uint32_t>((hz[o] >> q) & 1u) << (3 + 16 * half + kk);
+        }
+        if (nk) piece.push_back(pd);
+        entries += uint64_t{1} << nk;
+      }
+      entries += entries & 1u;  // staged in 16-byte pieces
+      for (int q = 0; q < 5; ++q)
+        for (int l = 0; l < (1 << q); ++l) ad.lane[l | 1 << q] = ad.lane[l] ^ plane[q];
+      for (int q = 5; q < m - 3; ++q)
+        for (int l = 0; l < (1 << (q - 5)); ++l) ad.warp[l | 1 << (q - 5)] = ad.warp[l] ^ plane[q];
+      for (int q = 0; q < 3; ++q)
+        for (int l = 0; l < (1 << q); ++l) ad.own[l | 1 << q] = ad.own[l] ^ plane[m - 3 + q];
+      asub.push_back(ad);
+    }
+    g0 = ge;
   }
-  d.NC = static_cast<uint32_t>(cls.size());
-  d.S = static_cast<uint32_t>(sub.size());
-  d.Q = static_cast<uint32_t>(quad.size());
+  if (entries > 0xffffffffull) wg::throw_invalid("expectation plan: too many terms for its tables");
+  const size_t S = asub.size(), NP = piece.size();
+  auto xhi_of = [&](size_t i) { return static_cast<uint32_t>(hx[torig[asub[i].t0]] >> m); };
+  auto tab_end = [&](size_t i) { return i + 1 < S ? asub[i + 1].tab : static_cast<uint32_t>(entries); };
+  const auto& props = wg::device_props(device);
+  const size_t sms = static_cast<size_t>(props.sm_count);
+  // Segments: sub-groups of one class, at most kSegSubs; fewer where a few
+  // tiles could not occupy the device otherwise (the adjoint splits at segments).
+  const size_t slices = static_cast<size_t>(kTileMax) >> m;
+  const size_t seg_subs = std::min<size_t>(
+      kSegSubs, std::max<size_t>(slices, (S * d.tiles + 2 * sms - 1) / (2 * sms)));
+  for (size_t i = 0; i < S;) {
+    size_t e = i + 1;
+    while (e < S && e - i < seg_subs && xhi_of(e) == xhi_of(i) && tab_end(e) - asub[i].tab <= kSegEntries) ++e;
+    // work of a segment, in hundredths of a tile's fetch: the tile, and its
+    // sub-groups (in as many turns as the slices leave)
+    const bool same = !seg.empty() && seg.back().xhi == xhi_of(i);
+    seg.push_back(SegDev{xhi_of(i), static_cast<uint32_t>(i), static_cast<uint32_t>(e - i), asub[i].tab,
+                         tab_end(e - 1) - asub[i].tab, {}});
+    const uint32_t cost = (same ? 20u : 100u) + static_cast<uint32_t>((e - i + slices - 1) / slices) * 90u;
+    seg_cost.push_back((seg_cost.empty() ? 0u : seg_cost.back()) + cost);
+    i = e;
+  }
+  // The adjoint's tiles are split by segments until there are about four items
+  // an SM.  The plan alone sets the splits, so that a pair's H psi has the same
+  // bits in every batch.
+  {
+    const size_t NS = seg.size();
+    const size_t splits = std::max<size_t>(1, std::min<size_t>({(4 * sms + d.tiles / 2) / d.tiles, NS, 64}));
+    p->bounds.push_back(0);
+    for (size_t k = 1; k < splits; ++k) {
+      // the segment at which k / splits of the work is done; each split takes one at least
+      const uint32_t to = static_cast<uint32_t>(static_cast<uint64_t>(seg_cost.back()) * k / splits);
+      size_t at = static_cast<size_t>(std::lower_bound(seg_cost.begin(), seg_cost.end(), to) - seg_cost.begin()) + 1;
+      at = std::min(std::max<size_t>(at, p->bounds.back() + 1), NS - (splits - k));
+      p->bounds.push_back(static_cast<uint32_t>(at));
+    }
+    p->bounds.push_back(static_cast<uint32_t>(NS));
+  }
+  // Forward items: chunks of pieces (their sums stay in shared memory) times
+  // ranges of tiles; about eight items an SM where there is the work.
+  const size_t sets = (static_cast<size_t>(kFwdThreads) * 16) >> m;
+  const size_t chunk_pieces = std::min<size_t>(
+      kChunkPieces, std::max<size_t>(sets, (NP * d.tiles + 4 * sms - 1) / (4 * sms)));
+  for (size_t i = 0; i < NP; i += chunk_pieces) chunk.push_back(static_cast<uint32_t>(std::min(NP, i + chunk_pieces)));
+  d.chunks = static_cast<uint32_t>(chunk.size() - 1);
+  d.ranges = static_cast<uint32_t>(
+      std::max<size_t>(1, std::min<size_t>({d.tiles, 256, (8 * sms + d.chunks - 1) / d.chunks})));
+  d.S = static_cast<uint32_t>(S);
+  d.NP = static_cast<uint32_t>(NP);
+  d.NS = static_cast<uint32_t>(seg.size());
   d.G = static_cast<uint32_t>(groups);
-  d.items = cls_item.back();
   p->n_groups = groups;
   Blob blob;
-  const size_t o_ci = blob.put(cls_item), o_cls = blob.put(cls), o_sub = blob.put(sub), o_zpl = blob.put(zpl),
-               o_quad = blob.put(quad), o_tz = blob.put(tz), o_ty = blob.put(ty), o_torig = blob.put(torig),
-               o_tpb = blob.put(tpbase), o_tnch = blob.put(tnch);
+  const size_t o_piece = blob.put(piece), o_asub = blob.put(asub), o_seg = blob.put(seg), o_chunk = blob.put(chunk),
+               o_ty = blob.put(ty), o_torig = blob.put(torig);
   p->blob.reset(blob.bytes.size(), s);
   wg::check_cuda(cudaMemcpyAsync(p->blob.get(), blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice, s),
                  "upload plan");
   auto* base = static_cast<unsigned char*>(p->blob.get());
-  d.cls_item = reinterpret_cast<const uint64_t*>(base + o_ci);
-  d.cls = reinterpret_cast<const ClassDev*>(base + o_cls);
-  d.sub = reinterpret_cast<const SubDev*>(base + o_sub);
-  d.zpl = reinterpret_cast<const uint32_t*>(base + o_zpl);
-  d.quad = reinterpret_cast<const QuadDev*>(base + o_quad);
-  d.tz = reinterpret_cast<const uint64_t*>(base + o_tz);
+  d.piece = reinterpret_cast<const FwdPiece*>(base + o_piece);
+  d.asub = reinterpret_cast<AdjSub*>(base + o_asub);
+  d.seg = reinterpret_cast<const SegDev*>(base + o_seg);
+  d.chunk = reinterpret_cast<const uint32_t*>(base + o_chunk);
   d.ty = reinterpret_cast<const uint32_t*>(base + o_ty);
   d.torig = reinterpret_cast<const uint32_t*>(base + o_torig);
-  d.tpbase = reinterpret_cast<const uint64_t*>(base + o_tpb);
-  d.tnch = reinterpret_cast<const uint32_t*>(base + o_tnch);
-  p->td.reset(16 * T, s);
-  p->table.reset(16 * std::max<size_t>(1, table_entries), s);
-  p->partial.reset(8 * std::max<uint64_t>(1, pbase), s);
-  p->stid.reset(4 * kThreads * std::max<size_t>(1, d.Q), s);
-  d.td = p->td.as<double>();
+  p->table.reset(16 * entries, s);
+  p->partial.reset(8 * static_cast<uint64_t>(T) * d.ranges, s);
   d.table = p->table.as<double>();
+  d.other = d.table + entries;
   d.partial = p->partial.as<double>();
-  d.stid = p->stid.as<uint32_t>();
-  if (d.Q) {
-    plan_stid_kernel<<<std::min<uint32_t>(d.Q, 65535u), kThreads, 0, s>>>(d);
-    wg::check_launch("launch adjoint lane signs");
-  }
   refresh_coeffs(*p, s);
   // pageable source above: wait until the plan image is on the device
   wg::check_cuda(cudaStreamSynchronize(s), "build plan");
   // The plan outlives the caller's stream: release its buffers on the legacy
   // default stream.
-  for (wg::Scratch* b : {&p->blob, &p->coeffs, &p->td, &p->table, &p->partial, &p->stid}) b->rebind(nullptr);
+  for (wg::Scratch* b : {&p->blob, &p->coeffs, &p->table, &p->partial}) b->rebind(nullptr);
   return p.release();
 }
 
@@ -750,10 +998,17 @@ struct wg_expect_batch_s {
   int sms = 0;
   BatchDev dev{};
   wg::Scratch table;
+  wg::Scratch parts;  // partial H psi of the pairs whose adjoint is split
   std::vector<wg::Scratch> evtmp;
 };
 
 namespace {
+
+template <class K>
+void allow_smem(K kernel, size_t bytes) {
+  wg::check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+                 "set expectation shared memory");
+}
 
 wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int dtype, cudaStream_t s) {
   if (dtype != WG_DTYPE_C128 && dtype != WG_DTYPE_C64) wg::throw_invalid("psi dtype must be complex64 or complex128");
@@ -761,22 +1016,47 @@ wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int
   b->device = device;
   b->dtype = dtype;
   b->sms = wg::device_props(device).sm_count;
+  if (dtype == WG_DTYPE_C128) {
+    allow_smem(expect_forward_kernel<double2>, sizeof(FwdShared));
+    allow_smem(expect_adjoint_kernel<double2>, sizeof(AdjShared));
+  } else {
+    allow_smem(expect_forward_kernel<float2>, sizeof(FwdShared));
+    allow_smem(expect_adjoint_kernel<float2>, sizeof(AdjShared));
+  }
   const size_t np = specs.size();
   if (np > 0xffffffffull) wg::throw_invalid("too many pairs in one batch");
   std::vector<PlanDev> plans(np);
-  std::vector<uint64_t> item_base(np + 1, 0), term_base(np + 1, 0), tile_base(np + 1, 0);
+  std::vector<uint64_t> item_base(np + 1, 0), term_base(np + 1, 0), tile_base(np + 1, 0), amp_base(np + 1, 0);
+  std::vector<uint32_t> splits(np, 1), split_at(np, 0), bounds;
+  std::vector<uint64_t> part_at(np, 0);
   std::vector<const void*> psis(np);
   std::vector<double*> evals(np), results(np), hpsis(np);
+  std::vector<double2*> parts(np, nullptr);
   b->evtmp.resize(np);
+  uint64_t part_amps = 0;
   for (size_t i = 0; i < np; ++i) {
     const PlanDev& P = specs[i].plan->dev;
+    // tile numbers are 32 bits; no device holds a larger state
+    if (P.n > kTileBits + 31) wg::throw_invalid("expectation_statevector: the statevector exceeds device memory");
     plans[i] = P;
     psis[i] = specs[i].psi;
-    item_base[i + 1] = item_base[i] + (P.T ? P.items : 0);
+    item_base[i + 1] = item_base[i] + (P.T ? static_cast<uint64_t>(P.chunks) * P.ranges : 0);
     term_base[i + 1] = term_base[i] + P.T;
-    const int tlog = P.n < kAdjTileLog ? P.n : kAdjTileLog;
     const bool adj = specs[i].hpsi != nullptr && P.T != 0;
-    tile_base[i + 1] = tile_base[i] + (adj ? (uint64_t{1} << (P.n - tlog)) : 0);
+    tile_base[i + 1] = tile_base[i];
+    amp_base[i + 1] = amp_base[i];
+    if (adj) {
+      const auto& own = specs[i].plan->bounds;
+      splits[i] = static_cast<uint32_t>(own.size() - 1);
+      split_at[i] = static_cast<uint32_t>(bounds.size());
+      bounds.insert(bounds.end(), own.begin(), own.end());
+      tile_base[i + 1] += static_cast<uint64_t>(P.tiles) * splits[i];
+      if (splits[i] > 1) {
+        amp_base[i + 1] += uint64_t{1} << P.n;
+        part_at[i] = part_amps;
+        part_amps += static_cast<uint64_t>(splits[i]) << P.n;
+      }
+    }
     if (specs[i].term_values) {
       evals[i] = specs[i].term_values;
     } else {
@@ -787,44 +1067,62 @@ wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int
     results[i] = specs[i].result;
     hpsis[i] = specs[i].hpsi;
   }
-  // one device block: plans | item_base | term_base | tile_base | psis | evals | results | hpsis | counters
-  const size_t bytes = sizeof(PlanDev) * np + 8 * 3 * (np + 1) + 8 * 4 * np + 16;
-  std::vector<unsigned char> host(bytes, 0);
-  size_t off = 0;
+  if (part_amps) {
+    b->parts.reset(16 * part_amps, s);
+    b->parts.rebind(nullptr);
+    for (size_t i = 0; i < np; ++i)
+      if (splits[i] > 1) parts[i] = b->parts.as<double2>() + part_at[i];
+  }
+  if (bounds.empty()) bounds.push_back(0);
+  // one device block, 8-byte pieces first
+  std::vector<unsigned char> host;
   auto put = [&](const void* src, size_t n) {
-    std::memcpy(host.data() + off, src, n);
-    const size_t at = off;
-    off += n;
+    const size_t at = (host.size() + 15) & ~size_t{15};
+    host.resize(at + n);
+    std::memcpy(host.data() + at, src, n);
     return at;
   };
+  const unsigned long long zero[2] = {0, 0};
   const size_t o_plans = put(plans.data(), sizeof(PlanDev) * np);
   const size_t o_item = put(item_base.data(), 8 * (np + 1));
   const size_t o_term = put(term_base.data(), 8 * (np + 1));
   const size_t o_tile = put(tile_base.data(), 8 * (np + 1));
+  const size_t o_amp = put(amp_base.data(), 8 * (np + 1));
+  const size_t o_splits = put(splits.data(), 4 * np);
+  const size_t o_at = put(split_at.data(), 4 * np);
+  const size_t o_bounds = put(bounds.data(), 4 * bounds.size());
   const size_t o_psis = put(psis.data(), 8 * np);
   const size_t o_evals = put(evals.data(), 8 * np);
   const size_t o_res = put(results.data(), 8 * np);
   const size_t o_hpsi = put(hpsis.data(), 8 * np);
-  const size_t o_cnt = off;
-  b->table.reset(bytes, s);
+  const size_t o_parts = put(parts.data(), 8 * np);
+  const size_t o_cnt = put(zero, sizeof(zero));
+  b->table.reset(host.size(), s);
   b->table.rebind(nullptr);
   // pageable source: the call returns once the bytes are staged
-  wg::check_cuda(cudaMemcpyAsync(b->table.get(), host.data(), bytes, cudaMemcpyHostToDevice, s), "upload work table");
+  wg::check_cuda(cudaMemcpyAsync(b->table.get(), host.data(), host.size(), cudaMemcpyHostToDevice, s),
+                 "upload work table");
   auto* base = static_cast<unsigned char*>(b->table.get());
   BatchDev& d = b->dev;
   d.plans = reinterpret_cast<const PlanDev*>(base + o_plans);
   d.item_base = reinterpret_cast<const uint64_t*>(base + o_item);
   d.term_base = reinterpret_cast<const uint64_t*>(base + o_term);
   d.tile_base = reinterpret_cast<const uint64_t*>(base + o_tile);
+  d.amp_base = reinterpret_cast<const uint64_t*>(base + o_amp);
+  d.splits = reinterpret_cast<const uint32_t*>(base + o_splits);
+  d.split_at = reinterpret_cast<const uint32_t*>(base + o_at);
+  d.bounds = reinterpret_cast<const uint32_t*>(base + o_bounds);
   d.psis = reinterpret_cast<const void* const*>(base + o_psis);
   d.evals = reinterpret_cast<double* const*>(base + o_evals);
   d.results = reinterpret_cast<double* const*>(base + o_res);
   d.hpsis = reinterpret_cast<double* const*>(base + o_hpsi);
+  d.parts = reinterpret_cast<double2* const*>(base + o_parts);
   d.counters = reinterpret_cast<unsigned long long*>(base + o_cnt);
   d.np = static_cast<uint32_t>(np);
   d.n_items = item_base[np];
   d.n_terms = term_base[np];
   d.n_tiles = tile_base[np];
+  d.n_amps = amp_base[np];
   return b.release();
 }
 
@@ -833,17 +1131,16 @@ void run_batch(const wg_expect_batch_s& b, cudaStream_t s) {
   const BatchDev& d = b.dev;
   if (d.np == 0) return;
   wg::check_cuda(cudaMemsetAsync(d.counters, 0, 16, s), "reset work queues");
-  const unsigned persistent = static_cast<unsigned>(b.sms) * 8;
+  const unsigned persistent = static_cast<unsigned>(b.sms);  // one CTA an SM: its tiles fill the shared memory
   if (d.n_items) {
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(d.n_items, persistent));
-    if (b.dtype == WG_DTYPE_C128)
-      WG_TIMED("expect_forward_kernel", s, expect_forward_kernel<double2><<<grid, kThreads, 0, s>>>(d));
-    else
-      WG_TIMED("expect_forward_kernel", s, expect_forward_kernel<float2><<<grid, kThreads, 0, s>>>(d));
+    auto* kernel = b.dtype == WG_DTYPE_C128 ? expect_forward_kernel<double2> : expect_forward_kernel<float2>;
+    WG_TIMED("expect_forward_kernel", s, kernel<<<grid, kFwdThreads, sizeof(FwdShared), s>>>(d));
     wg::check_launch("launch expectation forward");
   }
+  const unsigned wave = static_cast<unsigned>(b.sms) * 8;
   if (d.n_terms) {
-    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((d.n_terms + kThreads - 1) / kThreads, persistent));
+    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((d.n_terms + kThreads - 1) / kThreads, wave));
     WG_TIMED("expect_finish_terms_kernel", s, expect_finish_terms_kernel<<<grid, kThreads, 0, s>>>(d));
     wg::check_launch("launch expectation finish");
   }
@@ -852,11 +1149,14 @@ void run_batch(const wg_expect_batch_s& b, cudaStream_t s) {
   wg::check_launch("launch expectation total");
   if (d.n_tiles) {
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(d.n_tiles, persistent));
-    if (b.dtype == WG_DTYPE_C128)
-      WG_TIMED("expect_adjoint_kernel", s, expect_adjoint_kernel<double2><<<grid, kThreads, 0, s>>>(d));
-    else
-      WG_TIMED("expect_adjoint_kernel", s, expect_adjoint_kernel<float2><<<grid, kThreads, 0, s>>>(d));
+    auto* kernel = b.dtype == WG_DTYPE_C128 ? expect_adjoint_kernel<double2> : expect_adjoint_kernel<float2>;
+    WG_TIMED("expect_adjoint_kernel", s, kernel<<<grid, kAdjThreads, sizeof(AdjShared), s>>>(d));
     wg::check_launch("launch expectation adjoint");
+  }
+  if (d.n_amps) {
+    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((d.n_amps + kThreads - 1) / kThreads, wave));
+    WG_TIMED("expect_join_kernel", s, expect_join_kernel<<<grid, kThreads, 0, s>>>(d));
+    wg::check_launch("launch expectation join");
   }
 }
 
@@ -875,6 +1175,7 @@ void run_specs(int device, const std::vector<RunSpec>& specs, int dtype, cudaStr
   run_batch(*b, s);
   // stream-ordered release after the kernels that read the tables
   b->table.rebind(s);
+  b->parts.rebind(s);
   for (auto& e : b->evtmp) e.rebind(s);
 }
 
