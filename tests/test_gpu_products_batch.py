@@ -171,3 +171,47 @@ def test_products_batch_nonfinite_and_huge_coefficients(cuda, oracle, rtol):
         for a, b in zip(g, oracle_pair(oracle, n, A, B, "simplify", 1e-12, rtol)):
             assert same_bits(a, b)
     batch.close()
+
+
+@pytest.mark.parametrize("n", [30, 100, 150])
+@pytest.mark.parametrize("rtol", [0.0, 0.02])
+def test_products_batch_tiles_and_culls(cuda, oracle, n, rtol):
+    """Pairs whose products end inside, at and behind a tile of 1,024, empty
+    pairs between them, one key of 3,000 products, and squares with small
+    integer coefficients, of which anticommuting products cancel exactly."""
+    import torch
+
+    from wolfgang_b200.products import ProductsBatch
+
+    rng = seeded("tiles", n, rtol)
+
+    def square(T, p):
+        _, x, z, c = random_operator(rng, n, T, p)
+        c = rng.integers(1, 4, size=T).astype(np.complex128)
+        return (n, x, z, c), (n, x.copy(), z.copy(), c.copy())
+
+    def plain(nl, nr):
+        return random_operator(rng, n, nl, 0.05), random_operator(rng, n, nr, 0.05)
+
+    def one_key(nl, nr):
+        A, B = random_operator(rng, n, 1, 0.2), random_operator(rng, n, 1, 0.2)
+        out = []
+        for (_, x, z, _), T in ((A, nl), (B, nr)):
+            out.append((n, np.repeat(x, T, 0), np.repeat(z, T, 0), rng.normal(size=T) + 1j * rng.normal(size=T)))
+        return tuple(out)
+
+    pairs = [plain(32, 32), plain(0, 5), square(40, 0.05), plain(1, 1), one_key(60, 50), plain(33, 31), square(70, 0.1),
+             plain(7, 0), plain(41, 50), one_key(2, 3)]
+    batch = ProductsBatch(pairs, atol=1e-12, rtol=rtol)
+    batch.run()
+    for _ in range(2):
+        for got, (A, B) in zip(batch.results(), pairs):
+            want = oracle_pair(oracle, n, A, B, "simplify", 1e-12, rtol)
+            assert all(same_bits(g, w) for g, w in zip(got, want))
+        # coefficients with which nothing cancels, then the squares again culled
+        for k, (A, B) in enumerate(pairs):
+            c = rng.normal(size=len(A[3])) + 1j * rng.normal(size=len(A[3]))
+            pairs[k] = ((A[0], A[1], A[2], c), B)
+            batch.set_coefficients(k, lhs=torch.from_numpy(c))
+        batch.run()
+    batch.close()

@@ -14,13 +14,14 @@
 //    sorted product keeps its pair-local index and phase (one 32-bit code),
 //    each run of equal keys (a segment) its start, pair and key.  All scratch
 //    of the numeric pass and the outputs (one slot per segment) are sized here.
-//  run (numeric, any number of times): one thread per segment forms its
-//    products' coefficients from the operands' current coefficient buffers and
-//    sums them in order; the cull threshold per pair (atol + rtol*max|c| over
-//    the pair's products, or the fused path's 1e-12); a scan of the survivors
-//    and their write-out in canonical order.  No allocation, no host copy, no
-//    host synchronisation: a run can be captured in a CUDA graph and replayed
-//    after the coefficients change.
+//  run (numeric, any number of times): one pass over the products, a CTA per
+//    1,024 of them: coefficients formed from the operands' current coefficient
+//    buffers, runs summed in order, sums culled (atol + rtol*max|c| over the
+//    pair's products, or the fused path's 1e-12) and written with their keys to
+//    the slots they have if nothing of their pair is culled.  Pairs of which
+//    something was are written once more, at the survivors' ranks.  No
+//    allocation, no host copy, no host synchronisation: a run can be captured
+//    in a CUDA graph and replayed after the coefficients change.
 //
 // Sizes: each pair has at most 2^30 products (index and phase share 32 bits)
 // and the batch fewer than 2^32 products in all.
@@ -63,6 +64,7 @@ struct PairNum {
   uint64_t div_m;
   uint64_t seg_base;  // first segment of the pair = first output slot
   uint64_t n_seg;
+  uint64_t item_end;  // end of the pair's (sorted) products
 };
 
 // How a run forms each pair's largest |product| (the rtol threshold):
@@ -159,128 +161,280 @@ __global__ void pbatch_count_kernel(const uint32_t* __restrict__ seg_pair, size_
 // product with a part beyond 2^1022 or not finite.
 __device__ __noinline__ double product_magnitude(double re, double im) { return wgd::hypot_ref(re, im); }
 
-// One thread per segment (a warp takes 32 consecutive segments): the
-// segment's products formed from the current coefficients and summed left to
-// right (FP64, no FMA: the reference's rounding); in SIMPLIFY mode the
-// largest |product| of each pair, for the rtol threshold (non-negative
-// doubles order like their bits; a NaN never replaces the running maximum,
-// std::max's rule) -- with rtol = 0 only the magnitudes that may be infinite
-// (a part beyond 2^1022 or not finite) are formed, since a finite maximum
-// leaves the threshold at atol.  want_max is a MaxMode.
-template <int want_max>
-__global__ void __launch_bounds__(kThreads) pbatch_sums_kernel(
-    const PairNum* __restrict__ pairs, const uint32_t* __restrict__ seg_start, const uint32_t* __restrict__ seg_pair,
-    const uint32_t* __restrict__ code, size_t S, double* __restrict__ segsum,
-    unsigned long long* __restrict__ pair_max) {
-  const int lane = threadIdx.x & 31;
-  const size_t warp = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
-  const size_t nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
-  for (size_t chunk = warp; chunk * 32 < S; chunk += nwarps) {
-    const size_t s = chunk * 32 + lane;
-    const bool valid = s < S;
-    const uint32_t p = valid ? seg_pair[s] : 0xffffffffu;
-    double mx = 0.0;
-    if (valid) {
-      const PairNum P = pairs[p];
-      const uint32_t b = seg_start[s], e = seg_start[s + 1];
-      const uint32_t nr = static_cast<uint32_t>(P.n_r);  // below 2^30
-      c128 acc{0.0, 0.0};
-      for (uint32_t j = b; j < e; ++j) {
-        const uint32_t cj = __ldg(code + j);
-        const uint32_t q = cj >> 2;
-        const uint32_t l = nr == 1 ? q : static_cast<uint32_t>(__umul64hi(static_cast<uint64_t>(q), P.div_m));
-        const uint32_t r = q - l * nr;
-        const double2 av = __ldg(reinterpret_cast<const double2*>(P.lc) + l);
-        const double2 bv = __ldg(reinterpret_cast<const double2*>(P.rc) + r);
-        const c128 prod = wgd::rotate(wgd::cmul(c128{av.x, av.y}, c128{bv.x, bv.y}), cj & 3u);
-        acc = wgd::cadd(acc, prod);
-        if (want_max == kMaxFull) {
-          const double m = wgd::hypot_ref(prod.re, prod.im);
-          if (mx < m) mx = m;
-        } else if (want_max == kMaxInf && !(fabs(prod.re) <= 0x1p1022 && fabs(prod.im) <= 0x1p1022)) {
-          const double m = product_magnitude(prod.re, prod.im);
-          if (mx < m) mx = m;
-        }
-      }
-      segsum[2 * s] = acc.re;
-      segsum[2 * s + 1] = acc.im;
-    }
-    if (want_max) {
-      const uint32_t p0 = __shfl_sync(0xffffffffu, p, 0);
-      if (__all_sync(0xffffffffu, p == p0 || !valid)) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-          const double other = __shfl_xor_sync(0xffffffffu, mx, o);
-          if (mx < other) mx = other;
-        }
-        if (lane == 0 && mx > 0.0) atomicMax(pair_max + p0, static_cast<unsigned long long>(__double_as_longlong(mx)));
-      } else if (valid && mx > 0.0) {
-        atomicMax(pair_max + p, static_cast<unsigned long long>(__double_as_longlong(mx)));
-      }
-    }
+// The product of a sorted position's code (FP64, no FMA: the reference's rounding).
+__device__ __forceinline__ c128 coded_product(const PairNum& P, uint32_t code) {
+  const uint32_t nr = static_cast<uint32_t>(P.n_r);  // below 2^30
+  const uint32_t q = code >> 2;
+  const uint32_t l = nr == 1 ? q : static_cast<uint32_t>(__umul64hi(static_cast<uint64_t>(q), P.div_m));
+  const double2 av = __ldg(reinterpret_cast<const double2*>(P.lc) + l);
+  const double2 bv = __ldg(reinterpret_cast<const double2*>(P.rc) + (q - l * nr));
+  return wgd::rotate(wgd::cmul(c128{av.x, av.y}, c128{bv.x, bv.y}), code & 3u);
+}
+
+// What a run learns of its pairs (cleared by every run).
+struct PairRun {
+  unsigned long long max;  // bits of the largest |product|, as far as the mode needs it
+  uint32_t culled;         // something of the pair is culled
+  uint32_t below;          // survivors in its first segment's tile below that segment
+};
+
+// The pair of sorted position j, not before pair p.
+__device__ __forceinline__ uint32_t pair_from(const PairNum* __restrict__ pairs, uint32_t p, uint64_t j) {
+  while (j >= pairs[p].item_end) ++p;
+  return p;
+}
+
+// rtol > 0: each pair's largest |product|, ahead of the pass that needs it
+// (non-negative doubles order like their bits; a NaN never replaces the running
+// maximum, std::max's rule).
+__global__ void __launch_bounds__(kThreads) pbatch_max_kernel(const PairNum* __restrict__ pairs,
+                                                              const uint32_t* __restrict__ code, size_t N,
+                                                              PairRun* __restrict__ run) {
+  uint32_t p = 0;
+  for (size_t j = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; j < N;
+       j += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    p = pair_from(pairs, p, j);
+    const c128 c = coded_product(pairs[p], code[j]);
+    const double m = wgd::hypot_ref(c.re, c.im);
+    if (m > __longlong_as_double(static_cast<long long>(run[p].max)))
+      atomicMax(&run[p].max, static_cast<unsigned long long>(__double_as_longlong(m)));
   }
 }
 
-// keep[s] = |sum| > threshold of the segment's pair (|.| = glibc's hypot).
-__global__ void pbatch_keep_kernel(const uint32_t* __restrict__ seg_pair, const double* __restrict__ segsum, size_t S,
-                                   int fused, double atol, double rtol, const unsigned long long* __restrict__ pair_max,
-                                   uint32_t* __restrict__ keep) {
-  for (size_t s = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; s < S;
-       s += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    double thr = 1.0e-12;  // the fused path's fixed cull (src/multiply.cpp:144, :226)
-    if (!fused) {
-      // atol + rtol * max|c| with one rounding each (src/simplify.cpp:156-160)
-      const double mx = __longlong_as_double(static_cast<long long>(pair_max[seg_pair[s]]));
-      thr = __dadd_rn(atol, __dmul_rn(rtol, mx));
-    }
-    // without NaNs the rounded |s| is never below max(|re|, |im|): most sums are
-    // decided without the full hypot
-    const double re = segsum[2 * s], im = segsum[2 * s + 1];
-    const bool plain = !isnan(re) && !isnan(im);
-    keep[s] = (plain && (fabs(re) > thr || fabs(im) > thr)) || wgd::hypot_ref(re, im) > thr;
-  }
-}
+constexpr int kTile = 1024;             // products whose segments a CTA owns: those that start there
+constexpr int kStage = kTile + kThreads;  // products staged at a time
 
-// Survivor s of pair p goes to output slot seg_base[p] + its rank in the pair.
-// WT = W for 1 or 2 mask words (16-byte loads and stores), 0 for any width.
-template <int WT>
-__global__ void pbatch_write_kernel(const PairNum* __restrict__ pairs, const uint32_t* __restrict__ seg_pair,
-                                    const uint64_t* __restrict__ seg_keys, const double* __restrict__ segsum,
-                                    const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pos, size_t S,
-                                    int Wrt, uint64_t* __restrict__ ox, uint64_t* __restrict__ oz,
-                                    double* __restrict__ oc) {
+// The numeric pass.  All threads form products (coalesced codes, gathers of
+// the operands' coefficients in flight together), a thread per segment adds its
+// products up from shared memory.  REDO: the pairs with culled segments again,
+// at the survivors' ranks (offset: survivors of all tiles before).  WT = W for 1
+// or 2 mask words (16-byte loads and stores), 0 for any width.
+// Bound by the latency and L1 lookups of the gathers (half of the products'
+// coefficients come from L2).  47,800,000 products of 64 pairs on 64 qubits:
+// 0.91 ms and 0.03 ms for the repetition's early exits.  Before, a thread per
+// segment chased start, code and coefficients one after another (0.99 ms), and
+// cull, scan and write-out re-read every sum (0.65 ms).  Ranks from a look-back
+// over the tiles measured 2.7 ms: the tiles of one large pair wait for one
+// another in a chain.
+template <int WT, int MAX, bool REDO>
+__global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
+    const PairNum* __restrict__ pairs, const uint32_t* __restrict__ tile_seg, const uint32_t* __restrict__ seg_start,
+    const uint32_t* __restrict__ seg_pair, const uint64_t* __restrict__ seg_keys, const uint32_t* __restrict__ code,
+    int Wrt, double atol, double rtol, PairRun* run, uint32_t* __restrict__ any, uint32_t* __restrict__ kept,
+    const uint32_t* __restrict__ tile_of, uint64_t* __restrict__ ox, uint64_t* __restrict__ oz,
+    double2* __restrict__ oc) {
+  if (REDO && *any == 0) return;
+  __shared__ double2 prod[kStage];
+  __shared__ uint32_t bits[kTile / 32];
+  __shared__ uint32_t rank[kTile / 32 + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int W = WT > 0 ? WT : Wrt;
-  for (size_t s = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; s < S;
-       s += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    if (!keep[s]) continue;
-    const uint64_t base = pairs[seg_pair[s]].seg_base;
-    const size_t o = base + (pos[s] - pos[base]);
-    const double2 c = reinterpret_cast<const double2*>(segsum)[s];
+  const uint32_t s0 = tile_seg[blockIdx.x], s1 = tile_seg[blockIdx.x + 1];
+  if (s0 == s1) {
+    if (!REDO && tid == 0) kept[blockIdx.x] = 0;
+    return;
+  }
+  if (REDO) {
+    // nothing to do unless a pair of the tile has culled segments
+    bool redo = false;
+    for (uint32_t p = seg_pair[s0]; p <= seg_pair[s1 - 1]; ++p) redo |= run[p].culled != 0;
+    if (!redo) return;
+  }
+  const uint32_t j0 = seg_start[s0], j1 = seg_start[s1];
+  const uint32_t staged = min(j1 - j0, static_cast<uint32_t>(kStage));
+  // products [from, from + count) into prod[0..]; the loads of a thread's
+  // products are in flight together
+  auto stage = [&](uint32_t p, uint32_t from, uint32_t count) {
+    constexpr int kPer = kStage / kThreads;
+    uint32_t c[kPer], own[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t i = k * kThreads + tid;
+      c[k] = i < count ? __ldg(code + from + i) : 0;
+    }
+    double2 u[kPer], v[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t i = k * kThreads + tid;
+      if (i < count) p = pair_from(pairs, p, from + i);
+      own[k] = p;
+      const PairNum& P = pairs[p];
+      const uint32_t nr = static_cast<uint32_t>(P.n_r), q = c[k] >> 2;  // below 2^30
+      const uint32_t l = nr == 1 ? q : static_cast<uint32_t>(__umul64hi(static_cast<uint64_t>(q), P.div_m));
+      u[k] = __ldg(reinterpret_cast<const double2*>(P.lc) + l);
+      v[k] = __ldg(reinterpret_cast<const double2*>(P.rc) + (q - l * nr));
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t i = k * kThreads + tid;
+      if (i >= count) break;
+      const c128 t = wgd::rotate(wgd::cmul(c128{u[k].x, u[k].y}, c128{v[k].x, v[k].y}), c[k] & 3u);
+      prod[i] = make_double2(t.re, t.im);
+      // with rtol = 0 only a magnitude that may be infinite matters (a part
+      // beyond 2^1022 or not finite): a finite maximum leaves the threshold at atol
+      if (!REDO && MAX == kMaxInf && !(fabs(t.re) <= 0x1p1022 && fabs(t.im) <= 0x1p1022)) {
+        const double m = product_magnitude(t.re, t.im);
+        if (m > 0.0) atomicMax(&run[own[k]].max, static_cast<unsigned long long>(__double_as_longlong(m)));
+      }
+    }
+  };
+  constexpr int kRounds = kTile / kThreads;
+  c128 sum[kRounds];
+  uint32_t pair[kRounds], begin[kRounds], end[kRounds];
+  bool keep[kRounds];
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    const uint32_t s = min(s0 + k * kThreads + tid, s1 - 1);
+    pair[k] = __ldg(seg_pair + s);
+    begin[k] = __ldg(seg_start + s) - j0;
+    end[k] = __ldg(seg_start + s + 1) - j0;
+  }
+  stage(seg_pair[s0], j0, staged);
+  __syncthreads();
+  ulonglong2 key[WT == 1 ? kRounds : 1];  // on their way while the sums are formed
+  if constexpr (WT == 1) {
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k)
+      key[k] = __ldg(reinterpret_cast<const ulonglong2*>(seg_keys) + min(s0 + k * kThreads + tid, s1 - 1));
+  }
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    sum[k] = {0.0, 0.0};
+    if (s0 + k * kThreads + tid >= s1) continue;
+    const uint32_t e = min(end[k], staged);
+    for (uint32_t q = begin[k]; q < e; ++q) sum[k] = wgd::cadd(sum[k], c128{prod[q].x, prod[q].y});
+  }
+  // the last segment may go on behind the staged products: all threads form
+  // them, its thread goes on adding
+  for (uint32_t from = j0 + staged; from < j1; from += kStage) {
+    const uint32_t count = min(j1 - from, static_cast<uint32_t>(kStage));
+    __syncthreads();
+    stage(seg_pair[s1 - 1], from, count);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k)
+      if (s0 + k * kThreads + tid == s1 - 1)
+        for (uint32_t q = 0; q < count; ++q) sum[k] = wgd::cadd(sum[k], c128{prod[q].x, prod[q].y});
+  }
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    keep[k] = false;
+    if (s0 + k * kThreads + tid < s1) {
+      const c128 acc = sum[k];
+      const uint32_t p = pair[k];
+      double thr = 1.0e-12;  // the fused path's fixed cull (src/multiply.cpp:144, :226)
+      // atol + rtol * max|c| with one rounding each (src/simplify.cpp:156-160)
+      if (MAX == kMaxInf) thr = atol;
+      else if (MAX == kMaxFull)
+        thr = __dadd_rn(atol, __dmul_rn(rtol, __longlong_as_double(static_cast<long long>(run[p].max))));
+      // without NaNs the rounded |s| is never below max(|re|, |im|): most sums are
+      // decided without the full hypot
+      const bool plain = !isnan(acc.re) && !isnan(acc.im);
+      keep[k] = (plain && (fabs(acc.re) > thr || fabs(acc.im) > thr)) || wgd::hypot_ref(acc.re, acc.im) > thr;
+      if (!REDO && !keep[k]) {
+        run[p].culled = 1;
+        *any = 1;
+      }
+    }
+    const uint32_t v = __ballot_sync(0xffffffffu, keep[k]);
+    if (lane == 0) bits[k * (kThreads / 32) + warp] = v;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    static_assert(kTile / 32 == 32, "one warp scans the tile");
+    const uint32_t c = __popc(bits[lane]);
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    rank[lane] = incl - c;
+    if (lane == 31) {
+      rank[32] = incl;
+      if (!REDO) kept[blockIdx.x] = incl;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    const uint32_t i = k * kThreads + tid, s = s0 + i;
+    if (s >= s1) continue;
+    const uint32_t p = pair[k];
+    const uint64_t base = pairs[p].seg_base;
+    const uint32_t below = rank[i >> 5] + __popc(bits[i >> 5] & ((1u << lane) - 1u));
+    size_t o = s;
+    if (!REDO) {
+      if (s == base) run[p].below = below;
+    } else {
+      if (!run[p].culled) continue;
+      // kept holds the survivors of all tiles before
+      o = base + (kept[blockIdx.x] + below) - (kept[tile_of[p]] + run[p].below);
+    }
+    if (!keep[k]) continue;
     if constexpr (WT == 1) {
-      const ulonglong2 k = reinterpret_cast<const ulonglong2*>(seg_keys)[s];
-      ox[o] = k.x;
-      oz[o] = k.y;
+      ox[o] = key[k].x;
+      oz[o] = key[k].y;
     } else if constexpr (WT == 2) {
-      const ulonglong2 kx = reinterpret_cast<const ulonglong2*>(seg_keys)[2 * s];
-      const ulonglong2 kz = reinterpret_cast<const ulonglong2*>(seg_keys)[2 * s + 1];
-      reinterpret_cast<ulonglong2*>(ox)[o] = kx;
-      reinterpret_cast<ulonglong2*>(oz)[o] = kz;
+      reinterpret_cast<ulonglong2*>(ox)[o] = __ldg(reinterpret_cast<const ulonglong2*>(seg_keys) + 2 * size_t(s));
+      reinterpret_cast<ulonglong2*>(oz)[o] = __ldg(reinterpret_cast<const ulonglong2*>(seg_keys) + 2 * size_t(s) + 1);
     } else {
       for (int w = 0; w < W; ++w) {
-        ox[o * W + w] = seg_keys[s * (2 * W) + w];
-        oz[o * W + w] = seg_keys[s * (2 * W) + W + w];
+        ox[o * W + w] = seg_keys[size_t(s) * (2 * W) + w];
+        oz[o * W + w] = seg_keys[size_t(s) * (2 * W) + W + w];
       }
     }
-    reinterpret_cast<double2*>(oc)[o] = c;
+    oc[o] = make_double2(sum[k].re, sum[k].im);
   }
 }
 
-__global__ void pbatch_counts_kernel(const PairNum* __restrict__ pairs, const uint32_t* __restrict__ pos,
-                                     size_t n_pairs, uint64_t* __restrict__ counts) {
-  for (size_t p = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; p < n_pairs;
-       p += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const PairNum P = pairs[p];
-    counts[p] = pos[P.seg_base + P.n_seg] - pos[P.seg_base];
+// One CTA, between the pass and its repetition: where something was culled,
+// the tiles' survivor counts become the survivors before each tile; the pairs'
+// counts.  rtol = 0: a pair with an infinite |product| has the threshold
+// atol + 0 * inf, a NaN, and keeps nothing.
+__global__ void __launch_bounds__(1024) pbatch_counts_kernel(const PairNum* __restrict__ pairs, size_t n_pairs,
+                                                             const uint32_t* __restrict__ tile_of, int infinite,
+                                                             const PairRun* __restrict__ run,
+                                                             const uint32_t* __restrict__ any, uint32_t* kept,
+                                                             size_t tiles, uint64_t* __restrict__ counts) {
+  __shared__ uint32_t sums[32];
+  __shared__ uint32_t carry;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (*any) {
+    if (tid == 0) carry = 0;
+    __syncthreads();
+    for (size_t t0 = 0; t0 < tiles; t0 += 1024) {
+      const size_t t = t0 + tid;
+      const uint32_t c = t < tiles ? kept[t] : 0;
+      uint32_t incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) sums[warp] = incl;
+      __syncthreads();
+      uint32_t before = carry;
+      for (int w = 0; w < warp; ++w) before += sums[w];
+      if (t < tiles) kept[t] = before + incl - c;
+      __syncthreads();
+      if (tid == 1023) carry = before + incl;
+      __syncthreads();
+    }
+    if (tid == 0) kept[tiles] = carry;
+    __syncthreads();
+  }
+  for (size_t p = tid; p < n_pairs; p += 1024) {
+    uint64_t c = pairs[p].n_seg;
+    if (c && run[p].culled) {
+      // up to where the next pair with segments begins
+      size_t q = p + 1;
+      while (q < n_pairs && pairs[q].n_seg == 0) ++q;
+      const uint32_t end = q < n_pairs ? kept[tile_of[q]] + run[q].below : kept[tiles];
+      c = end - (kept[tile_of[p]] + run[p].below);
+    }
+    if (infinite && isinf(__longlong_as_double(static_cast<long long>(run[p].max)))) c = 0;
+    counts[p] = c;
   }
 }
 
@@ -295,14 +449,16 @@ struct wg_products_batch_s {
   int mode = WG_PRODUCTS_SIMPLIFY;
   double atol = 0.0, rtol = 0.0;
   size_t n_pairs = 0, N = 0, S = 0;
-  unsigned sum_blocks = 0;  // grid of the segment-sum kernel
   std::vector<uint64_t> seg_base, n_seg;
   wg::Scratch pairs;            // PairNum[n_pairs]
   wg::Scratch code;             // uint32[N]: sorted products' index << 2 | phase
   wg::Scratch seg_start;        // uint32[S + 1]
   wg::Scratch seg_pair;         // uint32[S]
   wg::Scratch seg_keys;         // uint64[S][2W]
-  wg::Scratch segsum, keep, pos, scan_ws, pair_max;
+  wg::Scratch tile_seg;         // uint32[tiles + 1]: first segment that starts in a tile
+  wg::Scratch tile_of;          // uint32[n_pairs]: tile of a pair's first segment
+  wg::Scratch run, kept;        // PairRun[n_pairs] and `any`, cleared by every run; uint32[tiles + 1]
+  size_t tiles = 0;
   wg::Scratch out_x, out_z, out_c, counts;
 };
 
@@ -333,8 +489,8 @@ void build_batch(wg_products_batch_s& b, const uint64_t* const* lhs_x, const uin
     }
     masks[p] = PairMasks{lhs_x[p], lhs_z[p], rhs_x[p], rhs_z[p], n_rhs[p], item_base[p]};
     const uint64_t div_m = n_rhs[p] > 1 ? ~0ull / n_rhs[p] + 1 : 0ull;
-    nums[p] = PairNum{lhs_c[p], rhs_c[p], n_rhs[p], div_m, 0, 0};
     item_base[p + 1] = item_base[p] + P;
+    nums[p] = PairNum{lhs_c[p], rhs_c[p], n_rhs[p], div_m, 0, 0, item_base[p + 1]};
     if (item_base[p + 1] > 0xffffffffull) wg::throw_invalid("a product batch takes fewer than 2^32 products in all");
   }
   const size_t N = item_base[np];
@@ -381,6 +537,14 @@ void build_batch(wg_products_batch_s& b, const uint64_t* const* lhs_x, const uin
     const uint32_t n32 = static_cast<uint32_t>(N);
     wg::check_cuda(cudaMemcpyAsync(b.seg_start.as<uint32_t>() + S, &n32, sizeof(n32), cudaMemcpyHostToDevice, s),
                    "write segment end");
+    b.tiles = (N + kTile - 1) / kTile;
+    b.tile_seg.reset(sizeof(uint32_t) * (b.tiles + 1), s);
+    // the heads before a tile's first position: every kTile-th entry of the scan
+    wg::check_cuda(cudaMemcpy2DAsync(b.tile_seg.get(), sizeof(uint32_t), segid.get(), sizeof(uint32_t) * kTile,
+                                     sizeof(uint32_t), b.tiles, cudaMemcpyDeviceToDevice, s),
+                   "gather tile segments");
+    wg::check_cuda(cudaMemcpyAsync(b.tile_seg.as<uint32_t>() + b.tiles, &S, sizeof(S), cudaMemcpyHostToDevice, s),
+                   "write tile segment end");
     wg::Scratch cnt(sizeof(unsigned) * np, s);
     wg::check_cuda(cudaMemsetAsync(cnt.get(), 0, cnt.size(), s), "clear segment counts");
     pbatch_count_kernel<<<wg::grid_for(S, kThreads, device, 8), kThreads, 0, s>>>(b.seg_pair.as<uint32_t>(), S,
@@ -404,17 +568,22 @@ void build_batch(wg_products_batch_s& b, const uint64_t* const* lhs_x, const uin
   b.pairs.reset(sizeof(PairNum) * std::max<size_t>(np, 1), s);
   wg::check_cuda(cudaMemcpyAsync(b.pairs.get(), nums.data(), sizeof(PairNum) * np, cudaMemcpyHostToDevice, s),
                  "upload batch pairs");
-  b.segsum.reset(sizeof(double) * 2 * S, s);
-  b.keep.reset(sizeof(uint32_t) * S, s);
-  b.pos.reset(sizeof(uint32_t) * (S + 1), s);
-  b.scan_ws.reset(sizeof(uint32_t) * wgs::scan_workspace(S), s);
-  b.pair_max.reset(sizeof(unsigned long long) * std::max<size_t>(np, 1), s);
+  {
+    // the tile in which each pair's first segment starts (its first product's)
+    std::vector<uint32_t> tile_of(std::max<size_t>(np, 1), 0);
+    for (size_t p = 0; p < np; ++p) tile_of[p] = static_cast<uint32_t>(item_base[p] / kTile);
+    b.tile_of.reset(sizeof(uint32_t) * tile_of.size(), s);
+    wg::check_cuda(cudaMemcpyAsync(b.tile_of.get(), tile_of.data(), b.tile_of.size(), cudaMemcpyHostToDevice, s),
+                   "upload pair tiles");
+    wg::check_cuda(cudaStreamSynchronize(s), "upload pair tiles");
+  }
+  b.run.reset(sizeof(PairRun) * np + 16, s);
+  b.kept.reset(sizeof(uint32_t) * (b.tiles + 1), s);
   b.out_x.reset(sizeof(uint64_t) * S * W, s);
   b.out_z.reset(sizeof(uint64_t) * S * W, s);
   b.out_c.reset(sizeof(double) * 2 * S, s);
   b.counts.reset(sizeof(uint64_t) * std::max<size_t>(np, 1), s);
   wg::check_cuda(cudaMemsetAsync(b.counts.get(), 0, b.counts.size(), s), "clear batch counts");
-  b.sum_blocks = wg::grid_for(S, kThreads, device, 8);
   wg::check_cuda(cudaDeviceSynchronize(), "prepare product batch");
 }
 
@@ -428,32 +597,41 @@ void run_batch(wg_products_batch_s& b, cudaStream_t s) {
   }
   const bool fused = b.mode == WG_PRODUCTS_FUSED;
   const int max_mode = fused ? kMaxNone : b.rtol > 0.0 ? kMaxFull : kMaxInf;
-  if (!fused)
-    wg::check_cuda(cudaMemsetAsync(b.pair_max.get(), 0, sizeof(unsigned long long) * b.n_pairs, s), "clear maxima");
-  auto* sums = max_mode == kMaxNone ? pbatch_sums_kernel<kMaxNone>
-               : max_mode == kMaxInf ? pbatch_sums_kernel<kMaxInf> : pbatch_sums_kernel<kMaxFull>;
-  WG_TIMED("pbatch_sums_kernel", s,
-    sums<<<b.sum_blocks, kThreads, 0, s>>>(b.pairs.as<PairNum>(), b.seg_start.as<uint32_t>(),
-                                           b.seg_pair.as<uint32_t>(), b.code.as<uint32_t>(), S,
-                                           b.segsum.as<double>(), b.pair_max.as<unsigned long long>()));
-  wg::check_launch("launch batch sums");
-  const unsigned g = wg::grid_for(S, kThreads, device, 8);
-  WG_TIMED("pbatch_keep_kernel", s,
-    pbatch_keep_kernel<<<g, kThreads, 0, s>>>(b.seg_pair.as<uint32_t>(), b.segsum.as<double>(), S, fused ? 1 : 0,
-                                              b.atol, b.rtol, b.pair_max.as<unsigned long long>(),
-                                              b.keep.as<uint32_t>()));
-  wg::check_launch("launch batch cull");
-  wgs::exclusive_scan_ws<uint32_t>(b.keep.as<uint32_t>(), b.pos.as<uint32_t>(), S, b.pos.as<uint32_t>() + S,
-                                   b.scan_ws.as<uint32_t>(), s);
-  auto* write = b.W == 1 ? pbatch_write_kernel<1> : b.W == 2 ? pbatch_write_kernel<2> : pbatch_write_kernel<0>;
-  WG_TIMED("pbatch_write_kernel", s,
-    write<<<g, kThreads, 0, s>>>(b.pairs.as<PairNum>(), b.seg_pair.as<uint32_t>(), b.seg_keys.as<uint64_t>(),
-                                 b.segsum.as<double>(), b.keep.as<uint32_t>(), b.pos.as<uint32_t>(), S, b.W,
-                                 b.out_x.as<uint64_t>(), b.out_z.as<uint64_t>(), b.out_c.as<double>()));
-  wg::check_launch("launch batch write-out");
-  pbatch_counts_kernel<<<wg::grid_for(b.n_pairs, kThreads, device, 1), kThreads, 0, s>>>(
-      b.pairs.as<PairNum>(), b.pos.as<uint32_t>(), b.n_pairs, b.counts.as<uint64_t>());
-  wg::check_launch("launch batch counts");
+  wg::check_cuda(cudaMemsetAsync(b.run.get(), 0, b.run.size(), s), "clear batch state");
+  auto* run = b.run.as<PairRun>();
+  auto* any = reinterpret_cast<uint32_t*>(run + b.n_pairs);
+  auto* pairs = b.pairs.as<PairNum>();
+  auto* code = b.code.as<uint32_t>();
+  if (max_mode == kMaxFull) {
+    WG_TIMED("pbatch_max_kernel", s,
+      pbatch_max_kernel<<<wg::grid_for(b.N, kThreads, device, 8), kThreads, 0, s>>>(pairs, code, b.N, run));
+    wg::check_launch("launch batch maxima");
+  }
+  auto pass = [&](auto* kernel, const char* name) {
+    WG_TIMED(name, s,
+      kernel<<<static_cast<unsigned>(b.tiles), kThreads, 0, s>>>(
+          pairs, b.tile_seg.as<uint32_t>(), b.seg_start.as<uint32_t>(), b.seg_pair.as<uint32_t>(),
+          b.seg_keys.as<uint64_t>(), code, b.W, b.atol, b.rtol, run, any, b.kept.as<uint32_t>(),
+          b.tile_of.as<uint32_t>(), b.out_x.as<uint64_t>(), b.out_z.as<uint64_t>(), b.out_c.as<double2>()));
+    wg::check_launch("launch batch pass");
+  };
+  auto both = [&](auto* first, auto* again) {
+    pass(first, "pbatch_pass_kernel");
+    WG_TIMED("pbatch_counts_kernel", s,
+      pbatch_counts_kernel<<<1, 1024, 0, s>>>(pairs, b.n_pairs, b.tile_of.as<uint32_t>(), max_mode == kMaxInf ? 1 : 0,
+                                              run, any, b.kept.as<uint32_t>(), b.tiles, b.counts.as<uint64_t>()));
+    wg::check_launch("launch batch counts");
+    pass(again, "pbatch_redo_kernel");
+  };
+  auto width = [&](auto w) {
+    constexpr int WT = decltype(w)::value;
+    if (max_mode == kMaxNone) both(pbatch_pass_kernel<WT, kMaxNone, false>, pbatch_pass_kernel<WT, kMaxNone, true>);
+    else if (max_mode == kMaxInf) both(pbatch_pass_kernel<WT, kMaxInf, false>, pbatch_pass_kernel<WT, kMaxInf, true>);
+    else both(pbatch_pass_kernel<WT, kMaxFull, false>, pbatch_pass_kernel<WT, kMaxFull, true>);
+  };
+  if (b.W == 1) width(std::integral_constant<int, 1>{});
+  else if (b.W == 2) width(std::integral_constant<int, 2>{});
+  else width(std::integral_constant<int, 0>{});
 }
 
 }  // namespace
