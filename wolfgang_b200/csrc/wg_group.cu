@@ -7,11 +7,13 @@
 //   full: a term joins the first group all of whose members commute with it
 //                                                                  (:96-126)
 //   otherwise it opens a new group.  Groups list members in placement order.
-// The first-fit is sequential over terms; here it runs in chunks: a bound pass
-// over the whole GPU finds, for every term of a chunk, the first group that
-// accepts it at the chunk's start, and one warp then places the chunk's terms
-// in order starting from those bounds (see group_bound_kernel), so the result
-// equals the sequential first-fit.
+// A term's fate at a group depends only on the earlier terms that reached that
+// group, so the first-fit can be run group by group as well as term by term: the
+// terms stream, in order, through stages of 32 groups each.  A stage places the
+// terms that one of its groups accepts and passes the rest on, in order, and all
+// stages work at once on different parts of the stream (see Pipe below).  More
+// than 256 qubits: chunks of terms instead, a lower bound for each term over the
+// whole GPU and a warp that places them in order (group_bound_n_kernel).
 
 #include <cuda_runtime.h>
 
@@ -26,7 +28,7 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Sort keys for the deterministic order: word 0 = (maxw - weight) so that an
+// Sort keys for the deterministic order: word 0 = (64 W - weight) so that an
 // ascending sort puts heavier terms first, then the canonical key words.
 __global__ void order_keys_kernel(const uint64_t* __restrict__ x, const uint64_t* __restrict__ z, size_t T, int W,
                                   uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
@@ -39,7 +41,7 @@ __global__ void order_keys_kernel(const uint64_t* __restrict__ x, const uint64_t
       keys[static_cast<size_t>(1 + 2 * w) * T + i] = a;
       keys[static_cast<size_t>(2 + 2 * w) * T + i] = b;
     }
-    keys[i] = ~wgt;  // larger weight -> smaller key
+    keys[i] = static_cast<uint64_t>(64 * W) - wgt;  // larger weight -> smaller key
     idx[i] = static_cast<uint32_t>(i);
   }
 }
@@ -57,48 +59,81 @@ __global__ void gather_terms_kernel(const uint64_t* __restrict__ x, const uint64
   }
 }
 
-// First-fit over ordered terms (ox/oz in processing order), in chunks of
-// kChunk terms.  Group state only grows (a qwc basis gains bits, a full-mode
-// group gains members), so a term's set of accepting groups only shrinks as
-// terms are placed: the first group that accepts a term at the start of its
-// chunk is a lower bound on the group it joins.  group_bound_kernel finds
-// that bound for every term of a chunk at once (a warp per term, 32 groups per
-// ballot); group_resolve_kernel then places the chunk's terms one by one from
-// their bounds, checking groups from the bound upward against the current
-// state, which is the sequential first-fit's answer.  In full mode the bound
-// group itself was checked against every member present at the chunk's start,
-// so only the members it gained during the chunk are checked again.
-// qwc state: one basis row per group, rows[g] = [x words | z words] (2W
-// words, moved as 16-byte pieces).  full state: first[g] / last[g] /
-// next[pos] member lists in processing order; the bound pass also records
-// which of the 32 groups from the bound accepted the term at the chunk's start
-// (lbm), so that those need checking only against the chunk's own members.
-// Chunk lengths, measured on random 128-qubit terms (each qubit non-identity
-// with probability 0.05): qwc 1,024 (512: 88 ms, 1,024: 81 ms, 2,048: 122 ms
-// for 262,144 terms); full mode 96 (64: 88 ms, 96: 79 ms, 128: 81 ms, 256:
-// 114 ms, 512: 213 ms for 32,768 terms), where every failed bound costs
-// member-list walks and shorter chunks keep the bounds closer.
-constexpr int kChunk = 1024;     // terms per chunk (qwc); also the staging capacity
+constexpr int kChunk = 1024;     // terms per chunk (qwc), more than 256 qubits
 constexpr int kChunkFull = 96;   // terms per chunk in full mode
 constexpr int kBoundThreads = 256;
 constexpr int kResolveThreads = 256;
+// warps that search one term's bound in full mode, warp s every kBoundSplit-th
+// round of 32 groups from round s
+constexpr int kBoundSplit = 8;
+
+// ------------------------------------------------------------- pipeline
+//
+// Stage s holds groups 32 s to 32 s + 31, one per lane.  An empty group accepts
+// every term, so a stage with room takes the first term it sees that none of its
+// groups accepts, which is the sequential first-fit's new group.  The terms that
+// a stage passes on lie in one list for all stages: stage s writes its k-th after
+// it has read k or more of its predecessor's, so the predecessor's unread ones
+// are further on.  status[s] tells how many there are (and kDone when there will
+// be no more).  Stages take their number by a ticket, so that whoever a stage
+// waits for is already running; the waits are bounded all the same.
+constexpr int kStageGroups = 32;
+constexpr unsigned long long kDone = 1ull << 63;
+constexpr int kPollLimit = 1 << 26;
+
+struct Pipe {
+  const uint64_t* ox;            // terms in processing order
+  const uint64_t* oz;
+  uint32_t n;                    // terms that reach the first stage
+  int fresh;                     // they are the positions 0..n-1; else the list's first n entries
+  uint32_t* list;
+  unsigned long long* status;    // [stages], zeroed
+  uint32_t base;                 // first group of the first stage
+  uint32_t batch;                // terms taken at a time
+  uint32_t* group_of;
+  uint32_t* next;                // full mode: members that do not fit in shared memory, linked
+};
+
+struct PipeControl {
+  uint32_t ticket;
+  uint32_t timeout;
+  uint32_t groups;  // groups opened so far
+};
+
+// Terms that stage s can read, and whether more may come; waits until `want`
+// are there or the predecessor is done.
+__device__ __forceinline__ uint32_t wait_terms(const Pipe& p, uint32_t s, uint32_t have, uint32_t want,
+                                               PipeControl* ctl) {
+  if (s == 0) return min(want, p.n - have);
+  const volatile unsigned long long* st = p.status + s - 1;
+  for (int spins = 0;; ++spins) {
+    const unsigned long long v = *st;
+    const uint32_t there = static_cast<uint32_t>(v & ~kDone) - have;
+    if (there >= want || (v & kDone)) {
+      __threadfence();
+      return min(there, want);
+    }
+    if (spins > kPollLimit) {
+      ctl->timeout = 1;
+      return 0;
+    }
+    __nanosleep(64);
+  }
+}
+
+__device__ __forceinline__ uint32_t stream_term(const Pipe& p, uint32_t s, uint32_t k) {
+  return s == 0 && p.fresh ? k : __ldcg(p.list + k);
+}
 
 template <int W>
-__device__ __forceinline__ void load_row(const uint64_t* p, uint64_t (&r)[2 * W]) {
-  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p);
+__device__ __forceinline__ void load_term(const uint64_t* t, uint64_t (&r)[2 * W]) {
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(t);
 #pragma unroll
   for (int j = 0; j < W; ++j) {
     const ulonglong2 v = q[j];
     r[2 * j] = v.x;
     r[2 * j + 1] = v.y;
   }
-}
-
-template <int W>
-__device__ __forceinline__ void store_row(uint64_t* p, const uint64_t (&r)[2 * W]) {
-  ulonglong2* q = reinterpret_cast<ulonglong2*>(p);
-#pragma unroll
-  for (int j = 0; j < W; ++j) q[j] = make_ulonglong2(r[2 * j], r[2 * j + 1]);
 }
 
 // qwc: no qubit on which the term and the basis hold different non-identity
@@ -111,319 +146,367 @@ __device__ __forceinline__ bool row_accepts(const uint64_t (&t)[2 * W], const ui
   return d == 0;
 }
 
-// Every member from position m on (following next) commutes with the term.
 template <int W>
-__device__ __forceinline__ bool members_commute(const uint64_t (&t)[2 * W], const uint64_t* __restrict__ ox,
-                                                const uint64_t* __restrict__ oz, const uint32_t* next, uint32_t m) {
-  for (; m != UINT_MAX; m = next[m]) {
-    uint64_t acc = 0;
-#pragma unroll
-    for (int w = 0; w < W; ++w)
-      acc ^= (t[w] & oz[static_cast<size_t>(m) * W + w]) ^ (t[W + w] & ox[static_cast<size_t>(m) * W + w]);
-    if (__popcll(acc) & 1u) return false;
-  }
-  return true;
-}
-
-// The term anticommutes with the staged row (2W words in shared memory).
-template <int W>
-__device__ __forceinline__ bool anticommutes(const uint64_t (&t)[2 * W], const uint64_t* row) {
-  uint64_t r[2 * W];
-  load_row<W>(row, r);
+__device__ __forceinline__ bool anticommutes(const uint64_t (&t)[2 * W], const uint64_t (&r)[2 * W]) {
   uint64_t acc = 0;
 #pragma unroll
   for (int w = 0; w < W; ++w) acc ^= (t[w] & r[W + w]) ^ (t[W + w] & r[w]);
   return (__popcll(acc) & 1u) != 0;
 }
 
-// Full mode: the bound of each term of a chunk is searched by kBoundSplit
-// warps, warp s taking every kBoundSplit-th round of 32 groups from round s.
-// A warp records the first accepting group of its rounds with atomicMin on
-// lb[i] (set to UINT_MAX beforehand) and stops once its next round starts at
-// or above the smallest group recorded so far, so lb[i] ends as the first
-// accepting group overall.  Member lists make a round of checks long; the
-// split keeps a chunk of few terms from leaving most of the GPU idle.
-constexpr int kBoundSplit = 8;
+// Places up to 32 terms in order, by one warp: lane j has the groups that accept
+// term j (accepts) and the earlier ones of the 32 that it conflicts with
+// (against).  A group still accepts a term unless one of the 32 that it conflicts
+// with joined the group.  Terms that conflict with none that may be placed go
+// where they would go alone, all at once; the others one by one.  Returns the
+// lane's term's group, UINT_MAX for none; *joined: terms that joined the lane's
+// group.  sm: 32 words of the warp's own.
+__device__ __forceinline__ uint32_t place_terms(uint32_t accepts, uint32_t against, uint32_t* sm, uint32_t* joined) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t some = __ballot_sync(0xffffffffu, accepts != 0);
+  *joined = 0;
+  if (!some) return UINT_MAX;
+  uint32_t mine = UINT_MAX;
+  const bool alone = accepts != 0 && !(against & some);
+  sm[lane] = 0;
+  __syncwarp();
+  if (alone) {
+    mine = __ffs(accepts) - 1;
+    atomicOr(&sm[mine], 1u << lane);
+  }
+  __syncwarp();
+  uint32_t in = sm[lane];
+  for (uint32_t rest = some & ~__ballot_sync(0xffffffffu, alone); rest; rest &= rest - 1) {
+    const int j = __ffs(rest) - 1;
+    const uint32_t a = __shfl_sync(0xffffffffu, accepts, j), c = __shfl_sync(0xffffffffu, against, j);
+    const uint32_t ok = __ballot_sync(0xffffffffu, ((a >> lane) & 1u) && !(c & in));
+    const int g = __ffs(ok) - 1;  // -1: none
+    if (lane == j) mine = static_cast<uint32_t>(g);
+    if (lane == g) in |= 1u << j;
+  }
+  __syncwarp();
+  *joined = in;
+  return mine;
+}
 
+constexpr int kPlaceWarps = 4;    // qwc: warps that check and place
+constexpr int kBringWarps = 4;    // and that bring the next batch
+constexpr int kQwcThreads = 32 * (kPlaceWarps + kBringWarps);
+constexpr int kQwcMost = 512;     // most terms of a batch
+
+// qwc: the placing warps hold the stage's 32 bases, a group per lane, each the
+// same.  They take the batch's terms 32 at a time: each checks a quarter against
+// the bases as they are (independent checks, one ballot each), then all place
+// the 32 (place_terms), each for itself, and update their bases.  The other warps
+// bring the next batch in meanwhile, and for each 32 the table of which conflict.
+// What bounds the whole is the first stage, which sees every term, at about
+// 72 cycles each; one warp that read the groups' bases from shared memory,
+// 32 groups at a time, took 510.  65,536 terms on 128 qubits in 1,216 groups:
+// 2.5 ms (before: 17.6 and 1.0 ms for the bounds).
 template <int W>
-__global__ void __launch_bounds__(kBoundThreads) group_search_full_kernel(
-    const uint64_t* __restrict__ ox, const uint64_t* __restrict__ oz, uint32_t c0, uint32_t c1,
-    const uint32_t* __restrict__ first, const uint32_t* __restrict__ next, const uint32_t* __restrict__ n_groups,
-    uint32_t* lb) {
-  const uint32_t G0 = *n_groups;
-  const int lane = threadIdx.x & 31;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t units = (c1 - c0) * kBoundSplit;
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += nw) {
-    const uint32_t i = c0 + u / kBoundSplit, sub = u % kBoundSplit;
-    uint64_t t[2 * W];
+__global__ void __launch_bounds__(kQwcThreads) group_qwc_kernel(Pipe pipe, PipeControl* ctl) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  const uint32_t batch = pipe.batch;
+  uint64_t* rows = reinterpret_cast<uint64_t*>(raw);  // [2][batch][2W]
+  uint32_t* ids = reinterpret_cast<uint32_t*>(rows + 2 * static_cast<size_t>(batch) * (2 * W));  // [2][batch]
+  uint32_t* conflicts = ids + 2 * batch;  // [2][batch] earlier terms of its 32 that a term conflicts with
+  uint32_t* got = conflicts + 2 * batch;  // [batch] group in the stage, or UINT_MAX
+  __shared__ uint32_t s_stage, s_n[2], s_left[kQwcThreads / 32], s_accepts[2][32], s_in[kPlaceWarps][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int kBring = 32 * kBringWarps, kPer = kQwcMost / kBring, kFirst = 32 * kPlaceWarps;
+  if (tid == 0) s_stage = atomicAdd(&ctl->ticket, 1u);
+  __syncthreads();
+  const uint32_t stage = s_stage;
+  uint32_t read = 0, written = 0;  // terms taken from the stream, passed on
+  // the bringing warps: the next batch into buffer b
+  auto bring = [&](int b) {
+    if (tid == kFirst) s_n[b] = wait_terms(pipe, stage, read, batch, ctl);
+    asm volatile("bar.sync 1, %0;" ::"n"(kBring) : "memory");
+    const uint32_t n = s_n[b];
+    uint32_t id[kPer];
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      t[w] = ox[static_cast<size_t>(i) * W + w];
-      t[W + w] = oz[static_cast<size_t>(i) * W + w];
+    for (int e = 0; e < kPer; ++e) {
+      const uint32_t k = tid - kFirst + e * kBring;
+      id[e] = k < n ? stream_term(pipe, stage, read + k) : 0;
     }
-    for (uint32_t g0 = sub * 32; g0 < G0; g0 += 32 * kBoundSplit) {
-      // the smallest accepting group any warp has recorded, read once per warp
-      uint32_t best = 0;
-      if (lane == 0) best = *static_cast<volatile uint32_t*>(&lb[i]);
-      best = __shfl_sync(0xffffffffu, best, 0);
-      if (g0 >= best) break;
-      const uint32_t g = g0 + lane;
-      const bool ok = g < G0 && members_commute<W>(t, ox, oz, next, first[g]);
-      const unsigned b = __ballot_sync(0xffffffffu, ok);
-      if (b) {
-        if (lane == 0) atomicMin(&lb[i], g0 + __ffs(b) - 1);
-        break;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const uint32_t k = tid - kFirst + e * kBring;
+      if (k >= n) continue;
+      ids[b * batch + k] = id[e];
+      uint64_t* row = rows + (b * batch + k) * (2 * W);
+#pragma unroll
+      for (int w = 0; w < W; ++w) {
+        row[w] = __ldg(pipe.ox + static_cast<size_t>(id[e]) * W + w);
+        row[W + w] = __ldg(pipe.oz + static_cast<size_t>(id[e]) * W + w);
       }
     }
-  }
-}
-
-template <int W, bool FULL>
-__global__ void __launch_bounds__(kBoundThreads) group_bound_kernel(const uint64_t* __restrict__ ox,
-                                                                   const uint64_t* __restrict__ oz, uint32_t c0,
-                                                                   uint32_t c1, const uint64_t* __restrict__ rows,
-                                                                   const uint32_t* __restrict__ first,
-                                                                   const uint32_t* __restrict__ next,
-                                                                   const uint32_t* __restrict__ n_groups,
-                                                                   uint32_t* __restrict__ lb,
-                                                                   uint32_t* __restrict__ lbm) {
-  const uint32_t G0 = *n_groups;
-  const int lane = threadIdx.x & 31;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = c0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < c1; i += nw) {
-    uint64_t t[2 * W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-      t[w] = ox[static_cast<size_t>(i) * W + w];
-      t[W + w] = oz[static_cast<size_t>(i) * W + w];
+    asm volatile("bar.sync 1, %0;" ::"n"(kBring) : "memory");
+    for (uint32_t t0 = 32 * (warp - kPlaceWarps); t0 < n; t0 += kBring) {
+      const uint64_t* block = rows + (b * batch + t0) * (2 * W);
+      const uint32_t m = min(32u, n - t0);
+      uint64_t t[2 * W], r[2 * W];
+      load_term<W>(block + min(static_cast<uint32_t>(lane), m - 1) * (2 * W), t);
+      uint32_t mine = 0;
+#pragma unroll 4
+      for (uint32_t j = 0; j < m; ++j) {
+        load_term<W>(block + j * (2 * W), r);
+        const uint32_t c = __ballot_sync(0xffffffffu, !row_accepts<W>(t, r));
+        if (lane == static_cast<int>(j)) mine = c & ((1u << j) - 1u);
+      }
+      if (lane < static_cast<int>(m)) conflicts[b * batch + t0 + lane] = mine;
     }
-    uint32_t found = G0;
-    if (FULL) {
-      // found by group_search_full_kernel (UINT_MAX: no group accepts)
-      found = min(lb[i], G0);
+  };
+  uint64_t basis[2 * W];
+#pragma unroll
+  for (int e = 0; e < 2 * W; ++e) basis[e] = 0;
+  bool used = false;
+  if (warp >= kPlaceWarps) bring(0);
+  __syncthreads();
+  int cur = 0;
+  while (true) {
+    const uint32_t n = s_n[cur];
+    if (n == 0) break;
+    read += n;
+    if (warp >= kPlaceWarps) {
+      bring(cur ^ 1);
     } else {
-      for (uint32_t g0 = 0; g0 < G0; g0 += 32) {
-        const uint32_t g = g0 + lane;
-        bool ok = false;
-        if (g < G0) {
-          uint64_t r[2 * W];
-          load_row<W>(rows + static_cast<size_t>(g) * (2 * W), r);
-          ok = row_accepts<W>(t, r);
+      constexpr int kShare = 32 / kPlaceWarps;
+      for (uint32_t t0 = 0; t0 < n; t0 += 32) {
+        const uint64_t* block = rows + (cur * batch + t0) * (2 * W);
+        const uint32_t m = min(32u, n - t0);
+        bool ok[kShare];
+#pragma unroll
+        for (int i = 0; i < kShare; ++i) {
+          const uint32_t j = warp * kShare + i;
+          uint64_t t[2 * W];
+          load_term<W>(block + min(j, m - 1) * (2 * W), t);
+          ok[i] = row_accepts<W>(t, basis) && j < m;
         }
-        const unsigned b = __ballot_sync(0xffffffffu, ok);
-        if (b) {
-          found = g0 + __ffs(b) - 1;
-          break;
+        uint32_t mask = 0;
+#pragma unroll
+        for (int i = 0; i < kShare; ++i) {
+          const uint32_t a = __ballot_sync(0xffffffffu, ok[i]);
+          if (lane == i) mask = a;
         }
+        uint32_t* all = s_accepts[(t0 >> 5) & 1];
+        if (lane < kShare) all[warp * kShare + lane] = mask;
+        asm volatile("bar.sync 2, %0;" ::"n"(32 * kPlaceWarps) : "memory");
+        uint32_t joined;
+        const uint32_t mine = place_terms(all[lane], lane < static_cast<int>(m) ? conflicts[cur * batch + t0 + lane] : 0,
+                                          s_in[warp], &joined);
+        if (warp == 0 && lane < static_cast<int>(m)) got[t0 + lane] = mine;
+        used |= joined != 0;
+        for (; joined; joined &= joined - 1) {
+          uint64_t t[2 * W];
+          load_term<W>(block + (__ffs(joined) - 1) * (2 * W), t);
+#pragma unroll
+          for (int e = 0; e < 2 * W; ++e) basis[e] |= t[e];
+        }
+        __syncwarp();
       }
     }
-    __syncwarp();
-    if (lane == 0) lb[i] = found;
-    if (FULL) {
-      // which of the 32 groups from the bound accept the term now
-      const uint32_t g = found + lane;
-      const bool ok = g < G0 && members_commute<W>(t, ox, oz, next, first[g]);
-      const unsigned m = __ballot_sync(0xffffffffu, ok);
-      if (lane == 0) lbm[i] = m;
+    __syncthreads();
+    // the placed terms' groups, and the others to the next stage, in order
+    for (uint32_t k0 = 0; k0 < n; k0 += kQwcThreads) {
+      const uint32_t k = k0 + tid;
+      const uint32_t id = k < n ? ids[cur * batch + k] : 0, g = k < n ? got[k] : 0;
+      const bool left = k < n && g == UINT_MAX;
+      if (k < n && !left) pipe.group_of[id] = pipe.base + stage * kStageGroups + g;
+      const uint32_t b = __ballot_sync(0xffffffffu, left);
+      if (lane == 0) s_left[warp] = __popc(b);
+      __syncthreads();
+      uint32_t at = written + __popc(b & ((1u << lane) - 1u));
+      uint32_t sum = 0;
+      for (int w = 0; w < kQwcThreads / 32; ++w) {
+        if (w < warp) at += s_left[w];
+        sum += s_left[w];
+      }
+      if (left) __stcg(pipe.list + at, id);
+      written += sum;
+      __syncthreads();
     }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
+    cur ^= 1;
+  }
+  if (tid == 0) {
+    __threadfence();
+    *const_cast<volatile unsigned long long*>(pipe.status + stage) = kDone | written;
+  }
+  if (warp == 0) {
+    const uint32_t u = __ballot_sync(0xffffffffu, used);
+    if (lane == 0 && u) atomicMax(&ctl->groups, pipe.base + stage * kStageGroups + __popc(u));
   }
 }
 
-// qwc placement of a chunk's staged term rows by one warp.  Lane j owns the
-// groups g with g % 32 == j: any 32 consecutive groups hold one group of each
-// lane, so a round over [g0, g0 + 32) has lane j check g0 + ((j - g0) & 31),
-// and a basis row is only ever read and written by its owner (no cross-lane
-// ordering is needed).  One warp reduction per round gives the smallest
-// accepting group; its owner ORs the term into the row.  The fast loop runs
-// the first round of each term (most terms end there) and leaves at the first
-// term it cannot place; that term's later rounds (or its new group) are
-// handled outside it, and the fast loop resumes.  Keeping the rare path out of
-// the per-term loop keeps the loop free of nested warp-synchronous control
-// flow.  B holds the basis rows: shared memory (SMEM) or global memory.
-template <int W, bool SMEM>
-__device__ __forceinline__ uint32_t place_qwc(const uint64_t* st, const uint32_t* slb, uint32_t* sgid, uint32_t n,
-                                              uint32_t G, uint64_t* B) {
-  const uint32_t lane = threadIdx.x & 31;
-  auto row_at = [&](uint32_t g) { return SMEM ? B + g * (2 * W) : B + static_cast<size_t>(g) * (2 * W); };
-  uint32_t k = 0;
-  while (k < n) {
+constexpr int kFullMost = 31;   // most terms of a batch: a warp each, and one that brings the next batch
+constexpr uint32_t kScan = 8;   // members checked with a group per lane
+
+// members of each group that a full-mode stage keeps in shared memory
+template <int W>
+constexpr int kKept = 320 / W;
+// words of the m-th members of the 32 groups, and one against bank conflicts
+template <int W>
+constexpr int kMemberRow = 2 * W * 32 + 1;
+
+// Full mode: a batch of up to 31 terms, a warp each.  A warp checks its term
+// against the first 8 members of all groups, a group per lane: of most groups
+// one of them anticommutes.  The groups that are left are checked one after
+// another, a member per lane.  Warp 0 then places the batch in order
+// (place_terms), while one more warp brings the next batch and the table of
+// which of its terms anticommute.  32,768 terms on 128 qubits in 708 groups: 5.0
+// ms (before: 60 ms; with a group per lane for all members, which 32 warps load
+// again and again: 7.8 ms).
+template <int W>
+__global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl* ctl) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  uint64_t* members = reinterpret_cast<uint64_t*>(raw);  // [kKept][kMemberRow]
+  __shared__ __align__(16) uint64_t term[2][kFullMost + 1][2 * W];
+  __shared__ uint32_t ids[2][kFullMost + 1], against[2][kFullMost + 1];
+  __shared__ uint32_t accepts[32], place[32], slot[32], s_in[32];
+  __shared__ uint32_t count[kStageGroups], first[kStageGroups], last[kStageGroups];
+  __shared__ uint32_t s_stage, s_n[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bringer = static_cast<int>(pipe.batch);
+  constexpr uint32_t kIn = kKept<W>;
+  if (tid == 0) s_stage = atomicAdd(&ctl->ticket, 1u);
+  if (tid < kStageGroups) count[tid] = 0;
+  __syncthreads();
+  const uint32_t stage = s_stage;
+  uint32_t read = 0, written = 0;
+  auto bring = [&](int b) {
+    uint32_t n = 0;
+    if (lane == 0) n = wait_terms(pipe, stage, read, pipe.batch, ctl);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    __threadfence();  // lane 0 saw the count: the others read what lies below it
     uint64_t t[2 * W], r[2 * W];
-    uint32_t l = 0;
-    for (; k < n; ++k) {
-      load_row<W>(st + k * (2 * W), t);
-      l = slb[k];
-      const uint32_t g = l + ((lane - l) & 31u);
-      bool ok = false;
-      if (g < G) {
-        load_row<W>(row_at(g), r);
-        ok = row_accepts<W>(t, r);
-      }
-      const uint32_t best = __reduce_min_sync(0xffffffffu, ok ? g : UINT_MAX);
-      if (best == UINT_MAX) break;
-      if (best % 32 == lane) {
+    const bool has = lane < static_cast<int>(n);
+    const uint32_t id = has ? stream_term(pipe, stage, read + lane) : 0;
 #pragma unroll
-        for (int e = 0; e < 2 * W; ++e) r[e] |= t[e];
-        store_row<W>(row_at(best), r);
-      }
-      if (lane == 0) sgid[k] = best;
+    for (int w = 0; w < W; ++w) {
+      t[w] = has ? __ldg(pipe.ox + static_cast<size_t>(id) * W + w) : 0;
+      t[W + w] = has ? __ldg(pipe.oz + static_cast<size_t>(id) * W + w) : 0;
     }
-    if (k >= n) break;
-    // term k: the rounds after the first, then a new group if none accepts
-    uint32_t best = UINT_MAX;
-    for (uint32_t g0 = l + 32; best == UINT_MAX && g0 < G; g0 += 32) {
-      const uint32_t g = g0 + ((lane - g0) & 31u);
-      bool ok = false;
-      if (g < G) {
-        load_row<W>(row_at(g), r);
-        ok = row_accepts<W>(t, r);
-      }
-      best = __reduce_min_sync(0xffffffffu, ok ? g : UINT_MAX);
-    }
-    const bool fresh = best == UINT_MAX;
-    if (fresh) best = G;
-    if (best % 32 == lane) {
+    if (has) {
+      ids[b][lane] = id;
 #pragma unroll
-      for (int e = 0; e < 2 * W; ++e) r[e] = fresh ? t[e] : (r[e] | t[e]);
-      store_row<W>(row_at(best), r);
+      for (int e = 0; e < 2 * W; ++e) term[b][lane][e] = t[e];
     }
-    if (fresh) ++G;
-    if (lane == 0) sgid[k] = best;
-    ++k;
-  }
-  return G;
-}
-
-// Full-mode placement of a chunk's staged term rows by one warp.  A term's
-// bound group l accepted it at the chunk's start, so the fast loop checks it
-// only against the chunk's members placed in l so far (lane-parallel over the
-// chunk's earlier terms, one vote).  A term that fails, or had no bound, goes
-// through the groups in first-fit order outside the fast loop: the window
-// groups that accepted it at the chunk's start (lbm), again against the
-// chunk's members only; the older groups beyond the window, by a walk of their
-// whole member list; the groups opened during the chunk, whose members are all
-// chunk members.  sgid[k] is written by lane k % 32, the lane that reads it in
-// the fast loop; the slow path starts with a warp barrier so that every lane
-// sees all group ids and list links written so far.
-template <int W>
-__device__ __forceinline__ uint32_t place_full(const uint64_t* __restrict__ ox, const uint64_t* __restrict__ oz,
-                                               const uint64_t* st, const uint32_t* slb, const uint32_t* smask,
-                                               uint32_t* sgid, uint32_t n, uint32_t c0, uint32_t G0, uint32_t* first,
-                                               uint32_t* last, uint32_t* next) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t G = G0;
-  // no member placed in group g among the chunk's first k terms anticommutes with t
-  auto chunk_members_commute = [&](const uint64_t (&t)[2 * W], uint32_t g, uint32_t k) {
-    for (uint32_t q = 0; q < k; ++q)
-      if (sgid[q] == g && anticommutes<W>(t, st + q * (2 * W))) return false;
-    return true;
+    __syncwarp();
+    uint32_t mine = 0;
+    for (uint32_t j = 0; j < n; ++j) {
+      load_term<W>(term[b][j], r);
+      const uint32_t c = __ballot_sync(0xffffffffu, anticommutes<W>(t, r));
+      if (lane == static_cast<int>(j)) mine = c & ((1u << j) - 1u);
+    }
+    if (has) against[b][lane] = mine;
+    if (lane == 0) s_n[b] = n;
   };
-  auto place = [&](uint32_t k, uint32_t best, bool fresh) {
-    if ((k & 31u) == lane) sgid[k] = best;
+  if (warp == bringer) bring(0);
+  __syncthreads();
+  int cur = 0;
+  while (true) {
+    const uint32_t n = s_n[cur];
+    if (n == 0) break;
+    read += n;
+    if (warp == bringer) {
+      bring(cur ^ 1);
+    } else if (warp < static_cast<int>(n)) {
+      uint64_t t[2 * W], r[2 * W];
+      load_term<W>(term[cur][warp], t);
+      const uint32_t c = count[lane], in = min(c, kIn);
+      bool ok = true;
+      const uint32_t scan = min(in, kScan);
+#pragma unroll 4
+      for (uint32_t k = 0; k < kScan; ++k) {
+        if (k < scan) {
+          const uint64_t* row = members + k * kMemberRow<W> + lane;
+#pragma unroll
+          for (int e = 0; e < 2 * W; ++e) r[e] = row[32 * e];
+          ok = ok && !anticommutes<W>(t, r);
+        }
+      }
+      uint32_t a = __ballot_sync(0xffffffffu, ok);
+      for (uint32_t rest = a & __ballot_sync(0xffffffffu, in > kScan); rest; rest &= rest - 1) {
+        const int g = __ffs(rest) - 1;
+        const uint32_t all = __shfl_sync(0xffffffffu, in, g);
+        bool bad = false;
+        for (uint32_t k0 = kScan; k0 < all; k0 += 32) {
+          const uint32_t k = k0 + lane;
+          if (k < all) {
+            const uint64_t* row = members + k * kMemberRow<W> + g;
+#pragma unroll
+            for (int e = 0; e < 2 * W; ++e) r[e] = row[32 * e];
+            bad = anticommutes<W>(t, r);
+          }
+          if (__any_sync(0xffffffffu, bad)) {
+            a &= ~(1u << g);
+            break;
+          }
+        }
+      }
+      bool still = (a >> lane) & 1u;
+      if (still && c > kIn) {
+        const volatile uint32_t* next = pipe.next;
+        for (uint32_t m = first[lane]; still && m != UINT_MAX; m = next[m]) {
+#pragma unroll
+          for (int w = 0; w < W; ++w) {
+            r[w] = __ldg(pipe.ox + static_cast<size_t>(m) * W + w);
+            r[W + w] = __ldg(pipe.oz + static_cast<size_t>(m) * W + w);
+          }
+          still = !anticommutes<W>(t, r);
+        }
+      }
+      a = __ballot_sync(0xffffffffu, still);
+      if (lane == 0) accepts[warp] = a;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const bool has = lane < static_cast<int>(n);
+      uint32_t joined;
+      const uint32_t mine = place_terms(has ? accepts[lane] : 0, has ? against[cur][lane] : 0, s_in, &joined);
+      uint32_t c = count[lane];
+      s_in[lane] = joined;
+      place[lane] = mine;
+      __syncwarp();
+      // a term's place in its group: behind the members and the batch's earlier terms
+      const uint32_t before = mine == UINT_MAX ? 0 : count[mine] + __popc(s_in[mine] & ((1u << lane) - 1u));
+      slot[lane] = before;
+      __syncwarp();
+      for (uint32_t rest = joined; rest; rest &= rest - 1, ++c) {
+        if (c < kIn) continue;
+        const uint32_t id = ids[cur][__ffs(rest) - 1];
+        pipe.next[id] = UINT_MAX;
+        if (c == kIn) first[lane] = id;
+        else pipe.next[last[lane]] = id;
+        last[lane] = id;
+      }
+      count[lane] = c;
+      const bool left = has && mine == UINT_MAX;
+      const uint32_t b = __ballot_sync(0xffffffffu, left);
+      if (left) __stcg(pipe.list + written + __popc(b & ((1u << lane) - 1u)), ids[cur][lane]);
+      else if (has) pipe.group_of[ids[cur][lane]] = pipe.base + stage * kStageGroups + mine;
+      written += __popc(b);
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
+    }
+    __syncthreads();
+    if (warp < static_cast<int>(n) && place[warp] != UINT_MAX && slot[warp] < kIn && lane < 2 * W)
+      members[slot[warp] * kMemberRow<W> + 32 * lane + place[warp]] = term[cur][warp][lane];
+    cur ^= 1;
+    __syncthreads();
+  }
+  if (warp == 0) {
     if (lane == 0) {
-      const uint32_t i = c0 + k;
-      next[i] = UINT_MAX;
-      if (fresh) first[best] = i;
-      else next[last[best]] = i;
-      last[best] = i;
+      __threadfence();
+      *const_cast<volatile unsigned long long*>(pipe.status + stage) = kDone | written;
     }
-  };
-  uint32_t k = 0;
-  while (k < n) {
-    uint64_t t[2 * W];
-    uint32_t l = 0;
-    for (; k < n; ++k) {
-      load_row<W>(st + k * (2 * W), t);
-      l = slb[k];
-      if (l >= G0) break;
-      bool bad = false;
-      for (uint32_t q = lane; q < k; q += 32)
-        if (sgid[q] == l && anticommutes<W>(t, st + q * (2 * W))) bad = true;
-      if (__any_sync(0xffffffffu, bad)) break;
-      place(k, l, false);
-    }
-    if (k >= n) break;
-    __syncwarp();
-    const uint32_t m = smask[k];
-    uint32_t best = UINT_MAX;
-    {
-      const uint32_t g = l + lane;
-      const bool ok = l < G0 && lane > 0 && g < G0 && ((m >> lane) & 1u) && chunk_members_commute(t, g, k);
-      best = __reduce_min_sync(0xffffffffu, ok ? g : UINT_MAX);
-    }
-    for (uint32_t g0 = l + 32; best == UINT_MAX && g0 < G0; g0 += 32) {
-      const uint32_t g = g0 + lane;
-      const bool ok = g < G0 && members_commute<W>(t, ox, oz, next, first[g]);
-      best = __reduce_min_sync(0xffffffffu, ok ? g : UINT_MAX);
-    }
-    for (uint32_t g0 = G0; best == UINT_MAX && g0 < G; g0 += 32) {
-      const uint32_t g = g0 + lane;
-      const bool ok = g < G && chunk_members_commute(t, g, k);
-      best = __reduce_min_sync(0xffffffffu, ok ? g : UINT_MAX);
-    }
-    const bool fresh = best == UINT_MAX;
-    if (fresh) best = G;
-    place(k, best, fresh);
-    if (fresh) ++G;
-    __syncwarp();
-    ++k;
+    const uint32_t u = __ballot_sync(0xffffffffu, count[lane] > 0);
+    if (lane == 0 && u) atomicMax(&ctl->groups, pipe.base + stage * kStageGroups + __popc(u));
   }
-  return G;
-}
-
-// One CTA: its threads stage the chunk's term rows and bounds (and, in qwc
-// mode, the basis rows when every group of the chunk fits) in shared memory;
-// warp 0 places the terms in order; the threads then write the basis rows
-// back and the chunk's group ids out.
-template <int W, bool FULL>
-__global__ void __launch_bounds__(kResolveThreads) group_resolve_kernel(
-    const uint64_t* __restrict__ ox, const uint64_t* __restrict__ oz, uint32_t c0, uint32_t c1, uint32_t cap, uint64_t* __restrict__ rows, uint32_t* __restrict__ first, uint32_t* __restrict__ last,
-    uint32_t* __restrict__ next, const uint32_t* __restrict__ lb, const uint32_t* __restrict__ lbm,
-    uint32_t* __restrict__ group_of, uint32_t* __restrict__ n_groups) {
-  extern __shared__ __align__(16) unsigned char rraw[];
-  __shared__ uint32_t s_G;
-  const uint32_t n = c1 - c0;
-  uint64_t* st = reinterpret_cast<uint64_t*>(rraw);         // [kChunk][2W] term rows
-  uint64_t* sb = st + kChunk * (2 * W);                       // [cap][2W] basis rows
-  uint32_t* slb = reinterpret_cast<uint32_t*>(sb + static_cast<size_t>(cap) * (2 * W));
-  uint32_t* sgid = slb + kChunk;
-  uint32_t* smask = sgid + kChunk;
-  const uint32_t G0 = *n_groups;
-  const bool in_smem = !FULL && static_cast<uint64_t>(G0) + n <= cap;
-  for (uint32_t k = threadIdx.x; k < n * W; k += blockDim.x) {
-    const uint32_t kk = k / W, w = k - kk * W;
-    st[kk * (2 * W) + w] = ox[static_cast<size_t>(c0) * W + k];
-    st[kk * (2 * W) + W + w] = oz[static_cast<size_t>(c0) * W + k];
-  }
-  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
-    slb[k] = lb[c0 + k];
-    if (FULL) smask[k] = lbm[c0 + k];
-  }
-  if (in_smem) {
-    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(rows);
-    ulonglong2* dst = reinterpret_cast<ulonglong2*>(sb);
-    for (uint32_t k = threadIdx.x; k < G0 * W; k += blockDim.x) dst[k] = src[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t G = G0;
-    if (!FULL) {
-      G = in_smem ? place_qwc<W, true>(st, slb, sgid, n, G0, sb) : place_qwc<W, false>(st, slb, sgid, n, G0, rows);
-    } else {
-      G = place_full<W>(ox, oz, st, slb, smask, sgid, n, c0, G0, first, last, next);
-    }
-    if (threadIdx.x == 0) {
-      *n_groups = G;
-      s_G = G;
-    }
-  }
-  __syncthreads();
-  if (in_smem) {
-    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(sb);
-    ulonglong2* dst = reinterpret_cast<ulonglong2*>(rows);
-    for (uint32_t k = threadIdx.x; k < s_G * W; k += blockDim.x) dst[k] = src[k];
-  }
-  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) group_of[c0 + k] = sgid[k];
 }
 
 // 64-bit sort keys from group ids; carried index = processing position.
@@ -452,49 +535,56 @@ __global__ void group_out_kernel(const uint32_t* __restrict__ order, const uint3
   }
 }
 
-// Chunk lengths the autotuner chooses among (the measured defaults above are
-// candidates 2 and 1); every chunk length gives the same groups.
-constexpr uint32_t kQwcChunks[] = {256, 512, 1024};
-constexpr uint32_t kFullChunks[] = {64, 96, 128, 192};
-static_assert(kQwcChunks[2] == kChunk && kFullChunks[1] == kChunkFull, "defaults are candidates");
+// Terms per batch that the autotuner chooses among (candidates 1 and 3 are the
+// defaults); every batch gives the same groups.
+constexpr uint32_t kQwcBatches[] = {128, 256, 512};
+constexpr uint32_t kFullBatches[] = {8, 16, 24, 31};
+static_assert(kQwcBatches[2] <= kQwcMost && kFullBatches[3] <= kFullMost, "staging holds a batch");
 
+// Runs the stages, as many as the device holds at once; where terms are left
+// behind the last of them, those through as many again.
 template <int W>
-void run_greedy(int device, bool full, const uint64_t* ox, const uint64_t* oz, uint32_t T, uint64_t* rows,
-                uint32_t* first, uint32_t* last, uint32_t* next, uint32_t* lb, uint32_t* lbm, uint32_t* gid,
-                uint32_t* ng, cudaStream_t s, uint32_t chunk) {
-  const auto& props = wg::device_props(device);
-  auto* kb = full ? group_bound_kernel<W, true> : group_bound_kernel<W, false>;
-  auto* kr = full ? group_resolve_kernel<W, true> : group_resolve_kernel<W, false>;
-  // term rows, bounds, bound masks and group ids of a chunk, then as many basis rows as fit
-  // beside the kernel's static shared memory
-  cudaFuncAttributes fa{};
-  wg::check_cuda(cudaFuncGetAttributes(&fa, kr), "query group resolve attributes");
-  const size_t stage = static_cast<size_t>(kChunk) * (16 * W + 12);
-  const size_t smem_max = static_cast<size_t>(props.max_smem_optin) - fa.sharedSizeBytes;
-  const uint32_t cap = full || smem_max <= stage ? 0u : static_cast<uint32_t>((smem_max - stage) / (16 * W));
-  const size_t smem = stage + static_cast<size_t>(cap) * 16 * W;
-  wg::check_cuda(cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                 "set group resolve shared memory");
-  wg::check_cuda(cudaMemsetAsync(ng, 0, 4, s), "clear group count");
-  const unsigned max_blocks = static_cast<unsigned>(props.sm_count) * 8;
-  if (chunk == 0 || chunk > static_cast<uint32_t>(kChunk)) chunk = full ? kChunkFull : kChunk;  // staging holds kChunk
-  for (uint32_t c0 = 0; c0 < T; c0 += chunk) {
-    const uint32_t c1 = T - c0 > chunk ? c0 + chunk : T;
-    const unsigned blocks = std::min<unsigned>(max_blocks, (c1 - c0 + kBoundThreads / 32 - 1) / (kBoundThreads / 32));
+uint32_t run_pipeline(int device, bool full, Pipe pipe, uint32_t T, cudaStream_t s) {
+  const uint32_t stages = static_cast<uint32_t>(wg::device_props(device).sm_count);
+  const size_t zero_bytes = sizeof(unsigned long long) * stages + sizeof(PipeControl);
+  wg::Scratch zero(zero_bytes, s);
+  pipe.status = zero.as<unsigned long long>();
+  auto* ctl = reinterpret_cast<PipeControl*>(pipe.status + stages);
+  const size_t smem = full ? sizeof(uint64_t) * kKept<W> * kMemberRow<W>
+                           : 2 * static_cast<size_t>(pipe.batch) * (16 * W + 8) + 4 * static_cast<size_t>(pipe.batch);
+  if (full) {
+    wg::check_cuda(cudaFuncSetAttribute(group_full_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(smem)),
+                   "set grouping shared memory");
+  } else {
+    wg::check_cuda(cudaFuncSetAttribute(group_qwc_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(smem)),
+                   "set grouping shared memory");
+  }
+  pipe.n = T;
+  pipe.fresh = 1;
+  pipe.base = 0;
+  std::vector<unsigned char> host(zero_bytes);
+  while (true) {
+    wg::check_cuda(cudaMemsetAsync(zero.get(), 0, zero_bytes, s), "clear grouping state");
+    const uint32_t need = std::min<uint32_t>(stages, (pipe.n + kStageGroups - 1) / kStageGroups);
     if (full) {
-      wg::check_cuda(cudaMemsetAsync(lb + c0, 0xff, 4 * static_cast<size_t>(c1 - c0), s), "clear bounds");
-      const unsigned sblocks = std::min<unsigned>(
-          max_blocks, ((c1 - c0) * kBoundSplit + kBoundThreads / 32 - 1) / (kBoundThreads / 32));
-      WG_TIMED("group_search_full_kernel", s,
-        group_search_full_kernel<W><<<sblocks, kBoundThreads, 0, s>>>(ox, oz, c0, c1, first, next, ng, lb));
-      wg::check_launch("launch group bound search");
+      WG_TIMED("group_full_kernel", s,
+        group_full_kernel<W><<<need, 32 * (pipe.batch + 1), smem, s>>>(pipe, ctl));
+    } else {
+      WG_TIMED("group_qwc_kernel", s, group_qwc_kernel<W><<<need, kQwcThreads, smem, s>>>(pipe, ctl));
     }
-    WG_TIMED("group_bound_kernel", s,
-      kb<<<blocks, kBoundThreads, 0, s>>>(ox, oz, c0, c1, rows, first, next, ng, lb, lbm));
-    wg::check_launch("launch group bounds");
-    WG_TIMED("group_resolve_kernel", s,
-      kr<<<1, kResolveThreads, smem, s>>>(ox, oz, c0, c1, cap, rows, first, last, next, lb, lbm, gid, ng));
-    wg::check_launch("launch group resolve");
+    wg::check_launch("launch grouping");
+    wg::check_cuda(cudaMemcpyAsync(host.data(), zero.get(), zero_bytes, cudaMemcpyDeviceToHost, s), "read grouping state");
+    wg::check_cuda(cudaStreamSynchronize(s), "grouping");
+    const auto* st = reinterpret_cast<const unsigned long long*>(host.data());
+    const auto* c = reinterpret_cast<const PipeControl*>(st + stages);
+    if (c->timeout) throw wg::Error(WG_ERR_TIMEOUT, "grouping: a stage waited too long for its predecessor");
+    const uint32_t left = static_cast<uint32_t>(st[need - 1] & ~kDone);
+    if (left == 0) return c->groups;
+    pipe.n = left;
+    pipe.fresh = 0;
+    pipe.base += need * kStageGroups;
   }
 }
 
@@ -853,55 +943,52 @@ int wg_group_commuting(int device, size_t words, size_t n_terms, const uint64_t*
       wg::check_cuda(cudaMemsetAsync(ox.get(), 0, 8 * T, s), "clear masks");
       wg::check_cuda(cudaMemsetAsync(oz.get(), 0, 8 * T, s), "clear masks");
     }
-    wg::Scratch rows(16 * Wa * T, s), first(4 * T, s), last(4 * T, s), next(4 * T, s), lb(4 * T, s), lbm(4 * T, s),
-        gid(4 * T, s), ng(4, s);
     const bool full = mode_full != 0;
     const uint32_t T32 = static_cast<uint32_t>(T);
-    wg::Scratch trows(W > 4 ? 16 * Wa * T : 0, s);
-    if (W > 4) {
+    wg::Scratch gid(4 * T, s), next(4 * T, s);
+    uint32_t G = 0;
+    if (W <= 4) {
+      wg::Scratch list(4 * T, s);
+      auto place = [&](uint32_t batch) {
+        Pipe pipe{};
+        pipe.ox = ox.as<uint64_t>();
+        pipe.oz = oz.as<uint64_t>();
+        pipe.list = list.as<uint32_t>();
+        pipe.group_of = gid.as<uint32_t>();
+        pipe.next = next.as<uint32_t>();
+        pipe.batch = batch;
+        switch (W) {
+          case 0:
+          case 1: G = run_pipeline<1>(device, full, pipe, T32, s); break;
+          case 2: G = run_pipeline<2>(device, full, pipe, T32, s); break;
+          case 3: G = run_pipeline<3>(device, full, pipe, T32, s); break;
+          default: G = run_pipeline<4>(device, full, pipe, T32, s); break;
+        }
+      };
+      // terms per batch: the autotuner's choice for (mode, words, log2 terms)
+      const uint32_t* cands = full ? kFullBatches : kQwcBatches;
+      bool done = false;
+      const int choice = wg::tune_choose(
+          full ? wg::kTuneGroupFull : wg::kTuneGroupQwc, W, wg::ceil_log2(T), 0, full ? 3 : 1, true, s,
+          [&](int c) {
+            place(cands[c]);
+            return true;
+          },
+          &done);
+      if (!done) place(cands[choice]);
+    } else {
+      wg::Scratch rows(16 * Wa * T, s), first(4 * T, s), last(4 * T, s), lb(4 * T, s), lbm(4 * T, s), ng(4, s),
+          trows(16 * Wa * T, s);
       WG_TIMED("interleave_rows_kernel", s,
         interleave_rows_kernel<<<wg::grid_for(T * W, kThreads, device, 4), kThreads, 0, s>>>(
             ox.as<uint64_t>(), oz.as<uint64_t>(), T, W, trows.as<uint64_t>()));
       wg::check_launch("launch interleave rows");
+      run_greedy_n(device, full, W, trows.as<uint64_t>(), T32, rows.as<uint64_t>(), first.as<uint32_t>(),
+                   last.as<uint32_t>(), next.as<uint32_t>(), lb.as<uint32_t>(), lbm.as<uint32_t>(),
+                   gid.as<uint32_t>(), ng.as<uint32_t>(), s);
+      wg::check_cuda(cudaMemcpyAsync(&G, ng.get(), 4, cudaMemcpyDeviceToHost, s), "read group count");
+      wg::check_cuda(cudaStreamSynchronize(s), "group greedy");
     }
-    auto greedy = [&](uint32_t chunk) {
-      auto* r = rows.as<uint64_t>();
-      auto* f = first.as<uint32_t>();
-      auto* l = last.as<uint32_t>();
-      auto* nx = next.as<uint32_t>();
-      auto* b = lb.as<uint32_t>();
-      auto* bm = lbm.as<uint32_t>();
-      auto* gi = gid.as<uint32_t>();
-      auto* n = ng.as<uint32_t>();
-      const uint64_t* px = ox.as<uint64_t>();
-      const uint64_t* pz = oz.as<uint64_t>();
-      switch (W) {
-        case 0:
-        case 1: run_greedy<1>(device, full, px, pz, T32, r, f, l, nx, b, bm, gi, n, s, chunk); break;
-        case 2: run_greedy<2>(device, full, px, pz, T32, r, f, l, nx, b, bm, gi, n, s, chunk); break;
-        case 3: run_greedy<3>(device, full, px, pz, T32, r, f, l, nx, b, bm, gi, n, s, chunk); break;
-        case 4: run_greedy<4>(device, full, px, pz, T32, r, f, l, nx, b, bm, gi, n, s, chunk); break;
-        default: run_greedy_n(device, full, W, trows.as<uint64_t>(), T32, r, f, l, nx, b, bm, gi, n, s); break;
-      }
-    };
-    if (W <= 4) {
-      // chunk length: the autotuner's choice for (mode, words, log2 terms)
-      const uint32_t* cands = full ? kFullChunks : kQwcChunks;
-      bool done = false;
-      const int choice = wg::tune_choose(
-          full ? wg::kTuneGroupFull : wg::kTuneGroupQwc, W, wg::ceil_log2(T), 0, full ? 1 : 2, true, s,
-          [&](int c) {
-            greedy(cands[c]);
-            return true;
-          },
-          &done);
-      if (!done) greedy(cands[choice]);
-    } else {
-      greedy(0);
-    }
-    uint32_t G = 0;
-    wg::check_cuda(cudaMemcpyAsync(&G, ng.get(), 4, cudaMemcpyDeviceToHost, s), "read group count");
-    wg::check_cuda(cudaStreamSynchronize(s), "group greedy");
     // Stable partition of processing positions by group id.
     wg::Scratch gkeys(8 * T, s), pos(4 * T, s);
     widen_ids_kernel<<<wg::grid_for(T, kThreads, device, 4), kThreads, 0, s>>>(gid.as<uint32_t>(), T,

@@ -332,6 +332,41 @@ __global__ void __launch_bounds__(256) soa_check_kernel(const uint64_t* __restri
   if (mixed) ctl->mixed = 1;
 }
 
+// The runs of equal codes in stable key order, a thread per run; ctl->mixed
+// where a run of more than kTieRun items holds several keys.
+constexpr uint32_t kTieRun = 64;
+
+__global__ void __launch_bounds__(256) soa_ties_kernel(const uint64_t* __restrict__ code, uint32_t* order,
+                                                       const uint64_t* __restrict__ packed, size_t n, int words,
+                                                       SortControl* ctl) {
+  auto compare = [&](uint32_t a, uint32_t b) {
+    for (int w = 0; w < words; ++w) {
+      const uint64_t u = packed[static_cast<size_t>(w) * n + a], v = packed[static_cast<size_t>(w) * n + b];
+      if (u != v) return u < v ? -1 : 1;
+    }
+    return 0;
+  };
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i + 1 < n;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    if (code[i + 1] != code[i] || (i > 0 && code[i - 1] == code[i])) continue;
+    size_t e = i + 2;
+    while (e < n && e - i <= kTieRun && code[e] == code[i]) ++e;
+    if (e - i > kTieRun) {
+      // a long run of one key is in order as it is; of several, or too long to see: the words
+      bool same = true;
+      for (e = i + 1; e < n && code[e] == code[i] && same; ++e) same = e - i < 4096 && compare(order[i], order[e]) == 0;
+      if (!same) ctl->mixed = 1;
+      continue;
+    }
+    for (size_t q = i + 1; q < e; ++q) {
+      const uint32_t o = order[q];
+      size_t r = q;
+      for (; r > i && compare(order[r - 1], o) > 0; --r) order[r] = order[r - 1];
+      order[r] = o;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) soa_gather_kernel(SoaWords src, int K, const uint32_t* __restrict__ order,
                                                          const uint32_t* __restrict__ idx, uint64_t* __restrict__ keys,
                                                          uint32_t* __restrict__ out) {
@@ -382,7 +417,8 @@ void radix_sort_keys(int device, size_t n, int K, Scratch& keys, Scratch& idx, c
   }
   if (n > 0xffffffffull) throw_invalid("sort item count exceeds the index range");
   KeyBits kb = key_bits(device, K, n, src, size_t{0}, src, s);
-  const CodeSpec spec = choose_code(kb, n);
+  CodeSpec spec = choose_code(kb, n);
+  if (!spec.exact) spec.nb = 64;  // ties cost more here than in a reduction
   const int passes = kb.B == 0 ? 0 : (spec.nb + 7) / 8;
   if (passes == 0) return;  // every key is the same
   const size_t tiles = pair_tiles(n);
@@ -419,6 +455,14 @@ void radix_sort_keys(int device, size_t n, int K, Scratch& keys, Scratch& idx, c
     // the look-backs' outcome is known only here
     check_cuda(cudaMemcpyAsync(&h, b.control, sizeof(h), cudaMemcpyDeviceToHost, s), "read sort state");
     check_cuda(cudaStreamSynchronize(s), "read sort state");
+    if (h.mixed && !h.timeout) {
+      check_cuda(cudaMemsetAsync(b.control, 0, sizeof(SortControl), s), "clear sort state");
+      WG_TIMED("soa_ties_kernel", s,
+        soa_ties_kernel<<<g, 256, 0, s>>>(b.k0, b.i0, packed.as<uint64_t>(), n, spec.words, b.control));
+      check_launch("launch sort ties");
+      check_cuda(cudaMemcpyAsync(&h, b.control, sizeof(h), cudaMemcpyDeviceToHost, s), "read sort state");
+      check_cuda(cudaStreamSynchronize(s), "read sort state");
+    }
   }
   if (h.mixed && !h.timeout) {
     allow_smem(soa_word_kernel, digit_smem(kMaxPasses));

@@ -115,9 +115,11 @@ KeyBits key_bits(int device, int K, size_t na, const A& a, size_t nc, const C& c
   std::vector<unsigned long long> h(words);
   wg::check_cuda(cudaMemcpyAsync(h.data(), f, sizeof(uint64_t) * words, cudaMemcpyDeviceToHost, s), "read key bits");
   wg::check_cuda(cudaStreamSynchronize(s), "read key bits");
+  unsigned long long constant[2] = {0, 0};  // set bits that every key of a list has
   for (int k = 0; k < K; ++k) {
     unsigned long long vary = 0, ored = 0;
     for (int y = 0; y < lists; ++y) {
+      constant[y] += __builtin_popcountll(~h[(2 * y + 1) * K + k]);
       vary |= h[2 * y * K + k] & h[(2 * y + 1) * K + k];
       ored |= h[2 * y * K + k];
     }
@@ -126,8 +128,8 @@ KeyBits key_bits(int device, int K, size_t na, const A& a, size_t nc, const C& c
     for (int b = 0; b < 64; b += 8) kb.ored_digits += ((ored >> b) & 0xffu) != 0;
   }
   const double B = std::max(1, kb.B);
-  const double p = std::min(1.0, static_cast<double>(h[4 * K]) / (B * static_cast<double>(na)));
-  const double q = nc > 0 ? std::min(1.0, static_cast<double>(h[4 * K + 1]) / (B * static_cast<double>(nc))) : 0.0;
+  const double p = std::min(1.0, static_cast<double>(h[4 * K] - constant[0] * na) / (B * static_cast<double>(na)));
+  const double q = nc > 0 ? std::min(1.0, static_cast<double>(h[4 * K + 1] - constant[1] * nc) / (B * static_cast<double>(nc))) : 0.0;
   kb.density = p * (1.0 - q) + q * (1.0 - p);
   return kb;
 }
