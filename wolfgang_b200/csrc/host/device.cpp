@@ -347,6 +347,11 @@ DeviceBuffer commutation_bits(const DevicePauliSum::Impl& l, const DevicePauliSu
   return bits;
 }
 
+void commutation_flags(const DevicePauliSum::Impl& l, const DevicePauliSum::Impl& r, std::uint8_t* out) {
+  abi::check(wg_commutation_flags(l.device, l.words, l.x.as<std::uint64_t>(), l.z.as<std::uint64_t>(), l.num_terms,
+                                  r.x.as<std::uint64_t>(), r.z.as<std::uint64_t>(), r.num_terms, out, nullptr));
+}
+
 }  // namespace
 
 void DevicePauliSum::commutes_with_into(const DevicePauliSum& rhs, std::span<std::uint8_t> output,
@@ -361,25 +366,9 @@ void DevicePauliSum::commutes_with_into(const DevicePauliSum& rhs, std::span<std
   if (output.size() != entries)
     throw std::invalid_argument("CUDA commutes_with output buffer size does not match entry count");
   if (entries == 0) return;
-  const std::size_t pitch = (rhs.impl_->num_terms + 31) / 32;
-  DeviceBuffer bits = commutation_bits(*impl_, *rhs.impl_, pitch, 0);
   DeviceBuffer flags(impl_->device, entries);
-  abi::check(wg_bits_to_u8(impl_->device, bits.as<std::uint32_t>(), impl_->num_terms, rhs.impl_->num_terms, pitch,
-                           flags.as<std::uint8_t>(), nullptr));
+  commutation_flags(*impl_, *rhs.impl_, flags.as<std::uint8_t>());
   flags.download(output.data(), entries);
-}
-
-DeviceCommutationMatrix DevicePauliSum::commutes_with_device(const DevicePauliSum& rhs,
-                                                             std::size_t max_commutation_matrix_entries) const {
-  if (!impl_ || !rhs.impl_) moved_from();
-  validate_same_accelerator_context("CUDA commutes_with_device", {AcceleratorBackend::Cuda, impl_->device},
-                                    {AcceleratorBackend::Cuda, rhs.impl_->device});
-  if (impl_->num_qubits != rhs.impl_->num_qubits)
-    throw std::invalid_argument("PauliSum commutes_with requires the same num_qubits");
-  (void)guards::commutation_entries(impl_->num_terms, rhs.impl_->num_terms, max_commutation_matrix_entries);
-  DeviceCommutationMatrix out = DeviceCommutationMatrix::empty(impl_->num_terms, rhs.impl_->num_terms, impl_->device);
-  commutes_with_device_into(rhs, out, max_commutation_matrix_entries);
-  return out;
 }
 
 DeviceCommutationBits DevicePauliSum::commutes_with_bits(const DevicePauliSum& rhs, std::size_t max_entries,
@@ -460,6 +449,26 @@ DeviceCommutationMatrix DeviceCommutationMatrix::empty(std::size_t rows, std::si
   return DeviceCommutationMatrix(std::move(impl));
 }
 
+DeviceCommutationMatrix DevicePauliSum::commutes_with_device(const DevicePauliSum& rhs,
+                                                             std::size_t max_commutation_matrix_entries) const {
+  if (!impl_ || !rhs.impl_) moved_from();
+  validate_same_accelerator_context("CUDA commutes_with_device", {AcceleratorBackend::Cuda, impl_->device},
+                                    {AcceleratorBackend::Cuda, rhs.impl_->device});
+  if (impl_->num_qubits != rhs.impl_->num_qubits)
+    throw std::invalid_argument("PauliSum commutes_with requires the same num_qubits");
+  (void)guards::commutation_entries(impl_->num_terms, rhs.impl_->num_terms, max_commutation_matrix_entries);
+  // every entry is written: no need of empty()'s zeros
+  auto mi = std::make_unique<DeviceCommutationMatrix::Impl>();
+  mi->rows = impl_->num_terms;
+  mi->cols = rhs.impl_->num_terms;
+  mi->entries = guards::product(mi->rows, mi->cols, "device commutation matrix");
+  mi->device = impl_->device;
+  if (mi->entries) mi->data = DeviceBuffer(mi->device, mi->entries);
+  DeviceCommutationMatrix out(std::move(mi));
+  commutes_with_device_into(rhs, out, max_commutation_matrix_entries);
+  return out;
+}
+
 void DevicePauliSum::commutes_with_device_into(const DevicePauliSum& rhs, DeviceCommutationMatrix& output,
                                                std::size_t max_commutation_matrix_entries) const {
   if (!impl_ || !rhs.impl_) moved_from();
@@ -476,10 +485,7 @@ void DevicePauliSum::commutes_with_device_into(const DevicePauliSum& rhs, Device
       output.impl_->entries != entries)
     throw std::invalid_argument("CUDA commutes_with_device output shape does not match operand term counts");
   if (entries == 0) return;
-  const std::size_t pitch = (rhs.impl_->num_terms + 31) / 32;
-  DeviceBuffer bits = commutation_bits(*impl_, *rhs.impl_, pitch, 0);
-  abi::check(wg_bits_to_u8(impl_->device, bits.as<std::uint32_t>(), impl_->num_terms, rhs.impl_->num_terms, pitch,
-                           output.impl_->data.as<std::uint8_t>(), nullptr));
+  commutation_flags(*impl_, *rhs.impl_, output.impl_->data.as<std::uint8_t>());
   abi::check(wg_stream_synchronize(impl_->device, nullptr));
 }
 

