@@ -172,162 +172,250 @@ __global__ void fill_ones_kernel(uint32_t* bits, size_t rows, size_t cols, size_
 }
 
 // ---------------------------------------------------------------------------
-// algo 2: bit-plane XOR.  For a block of 32*LW*32 rhs columns, plane (q,
-// X|Z) is the bit-vector over the block of the rhs x/z bits on qubit q.  Row
-// l's output word j is the complement of XOR over q in supp(l) of
-// (lx_q ? Zplane_q[j] : 0) ^ (lz_q ? Xplane_q[j] : 0).  Per output word that
-// is ~weight(l) shared-memory reads instead of 32 * (4W LOP3 + POPC), so for
-// sparse terms the kernel is bound by issue, not by POPC.  Each lane owns LW
-// consecutive output words of a row (read as one LW-word vector per plane):
-// LW = 4 with 1,024 threads for large products of 1-2 mask words (planes take
-// up to 128 KB of shared memory), LW = 2 with 256 threads otherwise.
+// algo 2: bit-plane XOR.  For a block of 1024 LW rhs columns, the planes of qubit
+// q are the bit-vectors over the block of the columns that anticommute there with
+// an X (their z bits), a Z (their x bits) and a Y (x ^ z).  Row l's output word j
+// is the complement of the XOR, over l's support, of word j of the plane of l's
+// letter: weight(l) shared-memory reads of LW words per lane instead of 32
+// (4 W LOP3 + POPC) per word.
+//
+// Bound by the shared-memory data path (88 % of its wavefronts used): LW wavefronts
+// per set qubit, row and 32 LW words, beside LW for the output and about 3 for the
+// row's list.  131,072^2 terms of 128 qubits, weight 6.4, 2.15 GB of output: 0.64 ms
+// (with X and Z planes, 256 equal CTAs and planes built by ballots 1.07 ms).
+//   - Three planes per qubit, not two with a Y reading both.
+//   - A warp takes up to 32 rows; lane r lists row r's planes (16-bit vector
+//     indexes, kRowList of them, 24-byte rows: 2-way bank conflicts), which the
+//     warp then reads four at a time as a broadcast.  A longer row is listed mask
+//     word by mask word by the whole warp when its turn comes.
+//   - The launch holds as many CTAs as the device runs at once, and each takes an
+//     equal run of (column block, row) pairs: a block's planes are built once or
+//     twice per CTA, and no last wave runs part empty.
+//   - The planes are built by 32x32 bit transposes; plane vector v of qubit q lies
+//     at v ^ (q & 31), so that the 32 qubits that a warp writes at a time fall
+//     into different banks.
+//   - A lane's LW words are consecutive where the output can be written as
+//     vectors, else 32 apart, so that each store is 32 consecutive words.
 constexpr int kMaxConfiguredDevices = 64;
-constexpr int kRowList = 16;  // plane offsets listed per row; rows with more set bits loop over their masks
+constexpr int kRowList = 12;   // planes listed per row beforehand
+constexpr int kListBytes = 32 * kRowList * 2 + 64 * 2 + 32;  // per warp: lists, one long row's word, counts
+
+constexpr size_t plane_smem(int W, int LW, int threads) {
+  return static_cast<size_t>(64 * W) * 3 * 32 * LW * 4 + static_cast<size_t>(threads / 32) * kListBytes;
+}
+
+// Bit i of lane t's result: bit t of lane i's v.
+__device__ __forceinline__ uint32_t transpose32(uint32_t v, int lane) {
+#pragma unroll
+  for (int s = 16, k = 0; s >= 1; s >>= 1, ++k) {
+    constexpr uint32_t kLow[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+    const uint32_t m = kLow[k];  // columns with bit s clear
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, v, s);
+    v = (lane & s) ? ((v & ~m) | ((y & ~m) >> s)) : ((v & m) | ((y & m) << s));
+  }
+  return v;
+}
 
 template <int LW>
-__device__ __forceinline__ void xor_plane(uint32_t (&acc)[LW], const uint32_t* planes, int vec) {
+struct WordVec;
+template <>
+struct WordVec<2> {
+  using type = uint2;
+};
+template <>
+struct WordVec<4> {
+  using type = uint4;
+};
+
+template <int LW>
+__device__ __forceinline__ void load_words(uint32_t (&w)[LW], const typename WordVec<LW>::type& v) {
+  w[0] = v.x;
+  w[1] = v.y;
   if constexpr (LW == 4) {
-    const uint4 v = reinterpret_cast<const uint4*>(planes)[vec];
-    acc[0] ^= v.x;
-    acc[1] ^= v.y;
-    acc[2] ^= v.z;
-    acc[3] ^= v.w;
-  } else {
-    static_assert(LW == 2, "two or four output words per lane");
-    const uint2 v = reinterpret_cast<const uint2*>(planes)[vec];
-    acc[0] ^= v.x;
-    acc[1] ^= v.y;
+    w[2] = v.z;
+    w[3] = v.w;
   }
+}
+
+template <int LW>
+__device__ __forceinline__ typename WordVec<LW>::type make_words(const uint32_t (&w)[LW]) {
+  if constexpr (LW == 4)
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  else
+    return make_uint2(w[0], w[1]);
+}
+
+// acc ^= the cnt planes of a list (8-byte aligned).
+template <int LW>
+__device__ __forceinline__ void xor_list(uint32_t (&acc)[LW], const typename WordVec<LW>::type* planes,
+                                         const uint16_t* list, int cnt, int lane) {
+  const uint2* l4 = reinterpret_cast<const uint2*>(list);
+  auto plane = [&](uint32_t (&w)[LW], uint32_t entry) { load_words<LW>(w, planes[entry ^ static_cast<uint32_t>(lane)]); };
+  int k = 0;
+  for (; k + 4 <= cnt; k += 4) {
+    const uint2 e = l4[k >> 2];
+    uint32_t a[LW], b[LW], c[LW], d[LW];
+    plane(a, e.x & 0xffffu);
+    plane(b, e.x >> 16);
+    plane(c, e.y & 0xffffu);
+    plane(d, e.y >> 16);
+#pragma unroll
+    for (int h = 0; h < LW; ++h) acc[h] ^= a[h] ^ b[h] ^ c[h] ^ d[h];
+  }
+  if (k < cnt) {
+    const uint2 e = l4[k >> 2];
+    uint32_t a[LW];
+    plane(a, e.x & 0xffffu);
+    if (k + 1 < cnt) {
+      uint32_t b[LW];
+      plane(b, e.x >> 16);
+#pragma unroll
+      for (int h = 0; h < LW; ++h) a[h] ^= b[h];
+    }
+    if (k + 2 < cnt) {
+      uint32_t c[LW];
+      plane(c, e.y & 0xffffu);
+#pragma unroll
+      for (int h = 0; h < LW; ++h) a[h] ^= c[h];
+    }
+#pragma unroll
+    for (int h = 0; h < LW; ++h) acc[h] ^= a[h];
+  }
+}
+
+// List entry of qubit q for a letter with bits (x, z): the plane's vector 0 is at
+// its index 32 (3 q + letter) + (q & 31).
+__device__ __forceinline__ uint16_t plane_entry(int q, uint32_t x, uint32_t z) {
+  return static_cast<uint16_t>(((q * 3 + static_cast<int>(x + 2 * z) - 1) << 5) | (q & 31));
 }
 
 template <int W, int LW, int THREADS>
 __global__ void __launch_bounds__(THREADS) commute_plane_kernel(
     const uint64_t* __restrict__ lx, const uint64_t* __restrict__ lz, size_t n_l,
     const uint64_t* __restrict__ rx, const uint64_t* __restrict__ rz, size_t n_r,
-    uint32_t* __restrict__ bits, size_t pitch, size_t rows_per_cta) {
-  constexpr int kWordsCta = 32 * LW;  // output words per row per CTA
+    uint32_t* __restrict__ bits, size_t pitch, size_t total, size_t per_cta) {
+  using Vec = typename WordVec<LW>::type;
+  constexpr int kWordsCta = 32 * LW;  // output words per row and column block
   constexpr int kWarpsCta = THREADS / 32;
-  // planes[(q*2 + 0)*kWordsCta + j] = X bits of rhs block word j on qubit q; +1 = Z bits.
-  // In LW-word vectors a plane is 32 vectors long, so plane p starts at vector 32p.
-  extern __shared__ __align__(16) uint32_t planes[];
+  extern __shared__ __align__(16) unsigned char smem[];
+  Vec* planes = reinterpret_cast<Vec*>(smem);
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const size_t col0 = static_cast<size_t>(blockIdx.x) * (32 * kWordsCta);
+  unsigned char* mine = smem + static_cast<size_t>(64 * W) * 3 * kWordsCta * 4 + warp * kListBytes;
+  uint16_t* lists = reinterpret_cast<uint16_t*>(mine);                  // [32][kRowList]
+  uint16_t* longs = reinterpret_cast<uint16_t*>(mine + 32 * kRowList * 2);  // [64]
+  uint8_t* counts = mine + 32 * kRowList * 2 + 128;                     // [32]
   const size_t words_needed = (n_r + 31) / 32;
-  // Build: warp handles block words j = warp, warp + kWarpsCta, ...; lane t
-  // loads column col0 + 32j + t once, then one ballot per (qubit, x|z) gives a
-  // plane word.
-  for (int j = warp; j < kWordsCta; j += kWarpsCta) {
-    const size_t c = col0 + 32 * static_cast<size_t>(j) + lane;
-    const bool ok = c < n_r;
+  const bool vectors = pitch % LW == 0 && (reinterpret_cast<uintptr_t>(bits) & (4 * LW - 1)) == 0;
+  const int jstep = vectors ? 1 : 32, jmul = vectors ? LW : 1;  // lane's word h of a block: jmul lane + jstep h
+
+  // per_cta <= total, and the pairs run block by block
+  size_t at = min(total, static_cast<size_t>(blockIdx.x) * per_cta);
+  const size_t end = min(total, at + per_cta);
+  while (at < end) {
+    const size_t block = at / n_l, row0 = at - block * n_l;
+    const size_t row1 = min(n_l, row0 + (end - at));
+    at += row1 - row0;
+    const size_t col0 = block * (32 * kWordsCta);
+    __syncthreads();  // the planes of the block before are read
+    for (int v = warp; v < 32; v += kWarpsCta) {
 #pragma unroll
-    for (int w = 0; w < W; ++w) {
-      const uint64_t vx = ok ? __ldg(rx + c * W + w) : 0;
-      const uint64_t vz = ok ? __ldg(rz + c * W + w) : 0;
-#pragma unroll 8
-      for (int b = 0; b < 64; ++b) {
-        const uint32_t px = __ballot_sync(0xffffffffu, (vx >> b) & 1u);
-        const uint32_t pz = __ballot_sync(0xffffffffu, (vz >> b) & 1u);
-        if (lane == (b & 31)) {
-          const int q = w * 64 + b;
-          planes[(q * 2 + 0) * kWordsCta + j] = px;
-          planes[(q * 2 + 1) * kWordsCta + j] = pz;
+      for (int w = 0; w < W; ++w) {
+        uint64_t vx[LW], vz[LW];
+#pragma unroll
+        for (int h = 0; h < LW; ++h) {
+          const size_t c = col0 + 32 * static_cast<size_t>(jmul * v + jstep * h) + lane;
+          vx[h] = c < n_r ? __ldg(rx + c * W + w) : 0;
+          vz[h] = c < n_r ? __ldg(rz + c * W + w) : 0;
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t x[LW], z[LW], y[LW];
+#pragma unroll
+          for (int h = 0; h < LW; ++h) {
+            x[h] = transpose32(static_cast<uint32_t>(vx[h] >> (32 * half)), lane);
+            z[h] = transpose32(static_cast<uint32_t>(vz[h] >> (32 * half)), lane);
+            y[h] = x[h] ^ z[h];
+          }
+          const int q = w * 64 + half * 32 + lane;
+          Vec* p = planes + static_cast<size_t>(q) * 96 + (v ^ lane);  // q & 31 == lane
+          p[0] = make_words<LW>(z);   // X on the left
+          p[32] = make_words<LW>(x);  // Z
+          p[64] = make_words<LW>(y);  // Y
         }
       }
     }
-  }
-  __syncthreads();
-  // lane covers output words LW*lane .. LW*lane + LW - 1 of the block
-  uint32_t valid[LW];
-  bool write_ok[LW];
-  size_t wi[LW];
+    __syncthreads();
+    uint32_t valid[LW];
+    bool write_ok[LW];
+    const size_t wi0 = block * kWordsCta + static_cast<size_t>(jmul * lane);
 #pragma unroll
-  for (int h = 0; h < LW; ++h) {
-    const int j = LW * lane + h;
-    const size_t c_first = col0 + 32 * static_cast<size_t>(j);
-    valid[h] = c_first >= n_r ? 0u : (n_r - c_first < 32 ? (1u << (n_r - c_first)) - 1u : 0xffffffffu);
-    wi[h] = static_cast<size_t>(blockIdx.x) * kWordsCta + j;
-    write_ok[h] = wi[h] < words_needed;
-  }
-  const size_t row0 = static_cast<size_t>(blockIdx.y) * rows_per_cta;
-  const size_t row1 = min(n_l, row0 + rows_per_cta);
-  // A warp takes 32 rows at a time: lane r loads row rbase + r (coalesced)
-  // and lists the plane offsets its row selects (set X bits select rhs Z
-  // planes, set Z bits rhs X planes); each row's list is then read by the
-  // whole warp (a broadcast, two offsets per 32-bit read), so a lane's work
-  // per set bit is one LW-word shared-memory load and LW XORs.  A row with
-  // more than kRowList set bits has its masks broadcast by shuffles and walked
-  // bit by bit instead.
-  __shared__ uint16_t lists[kWarpsCta][32][kRowList];
-  __shared__ uint8_t counts[kWarpsCta][32];
-  for (size_t rbase = row0 + 32 * static_cast<size_t>(warp); rbase < row1; rbase += 32 * kWarpsCta) {
-    const size_t my = rbase + lane;
-    uint64_t mx[W], mz[W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-      mx[w] = my < row1 ? __ldg(lx + my * W + w) : 0;
-      mz[w] = my < row1 ? __ldg(lz + my * W + w) : 0;
+    for (int h = 0; h < LW; ++h) {
+      const size_t wi = wi0 + static_cast<size_t>(jstep * h);
+      write_ok[h] = wi < words_needed;
+      valid[h] = !write_ok[h] ? 0u : (n_r - 32 * wi < 32 ? (1u << (n_r - 32 * wi)) - 1u : 0xffffffffu);
     }
-    {
+    // up to 32 rows to a warp at a time, fewer where the CTA's run is short
+    const size_t batch = min(static_cast<size_t>(32), (row1 - row0 + kWarpsCta - 1) / kWarpsCta);
+    for (size_t rbase = row0 + batch * warp; rbase < row1; rbase += batch * kWarpsCta) {
+      const int nrows = static_cast<int>(min(batch, row1 - rbase));
+      const size_t my = rbase + lane;
+      uint64_t mx[W], mz[W];
       int cnt = 0;
 #pragma unroll
       for (int w = 0; w < W; ++w) {
-        for (uint64_t m = mx[w]; m; m &= m - 1) {
-          if (cnt < kRowList) lists[warp][lane][cnt] = static_cast<uint16_t>(((w * 64 + __ffsll(m) - 1) * 2 + 1) * 32);
-          ++cnt;
-        }
-        for (uint64_t m = mz[w]; m; m &= m - 1) {
-          if (cnt < kRowList) lists[warp][lane][cnt] = static_cast<uint16_t>(((w * 64 + __ffsll(m) - 1) * 2) * 32);
-          ++cnt;
-        }
+        mx[w] = lane < nrows ? __ldg(lx + my * W + w) : 0;
+        mz[w] = lane < nrows ? __ldg(lz + my * W + w) : 0;
+        cnt += __popcll(mx[w] | mz[w]);
       }
-      counts[warp][lane] = static_cast<uint8_t>(cnt <= kRowList ? cnt : 255);
-    }
-    __syncwarp();
-    const int nrows = row1 - rbase < 32 ? static_cast<int>(row1 - rbase) : 32;
-    for (int rr = 0; rr < nrows; ++rr) {
-      uint32_t acc[LW];
+      counts[lane] = static_cast<uint8_t>(cnt <= kRowList ? cnt : 255);
+      if (cnt <= kRowList) {
+        uint16_t* l = lists + lane * kRowList;
 #pragma unroll
-      for (int h = 0; h < LW; ++h) acc[h] = 0u;
-      const int cnt = counts[warp][rr];
-      if (cnt != 255) {
-        const uint32_t* l2 = reinterpret_cast<const uint32_t*>(lists[warp][rr]);
-        int k = 0;
-        for (; k + 1 < cnt; k += 2) {
-          const uint32_t pr = l2[k >> 1];
-          xor_plane<LW>(acc, planes, static_cast<int>(pr & 0xffffu) + lane);
-          xor_plane<LW>(acc, planes, static_cast<int>(pr >> 16) + lane);
-        }
-        if (k < cnt) xor_plane<LW>(acc, planes, lists[warp][rr][k] + lane);
-      } else {
+        for (int w = 0; w < W; ++w)
+          for (uint64_t m = mx[w] | mz[w]; m; m &= m - 1) {
+            const int b = __ffsll(static_cast<long long>(m)) - 1;
+            *l++ = plane_entry(w * 64 + b, static_cast<uint32_t>(mx[w] >> b) & 1u, static_cast<uint32_t>(mz[w] >> b) & 1u);
+          }
+      }
+      __syncwarp();
+      uint32_t* out = bits + rbase * pitch + wi0;
+      for (int rr = 0; rr < nrows; ++rr, out += pitch) {
+        uint32_t acc[LW];
 #pragma unroll
-        for (int w = 0; w < W; ++w) {
-          const uint64_t ax = __shfl_sync(0xffffffffu, mx[w], rr);
-          const uint64_t az = __shfl_sync(0xffffffffu, mz[w], rr);
+        for (int h = 0; h < LW; ++h) acc[h] = 0xffffffffu;
+        const int n = counts[rr];
+        if (n != 255) {
+          xor_list<LW>(acc, planes, lists + rr * kRowList, n, lane);
+        } else {
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int qb = w * 64 + half * 32;
-            for (uint32_t m = static_cast<uint32_t>(ax >> (32 * half)); m; m &= m - 1)
-              xor_plane<LW>(acc, planes, ((qb + __ffs(m) - 1) * 2 + 1) * 32 + lane);
-            for (uint32_t m = static_cast<uint32_t>(az >> (32 * half)); m; m &= m - 1)
-              xor_plane<LW>(acc, planes, ((qb + __ffs(m) - 1) * 2 + 0) * 32 + lane);
+          for (int w = 0; w < W; ++w) {
+            const uint64_t ax = __shfl_sync(0xffffffffu, mx[w], rr), az = __shfl_sync(0xffffffffu, mz[w], rr);
+            const uint64_t m = ax | az;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              const int b = 32 * half + lane;
+              if ((m >> b) & 1u)
+                longs[__popcll(m & ((1ull << b) - 1))] =
+                    plane_entry(w * 64 + b, static_cast<uint32_t>(ax >> b) & 1u, static_cast<uint32_t>(az >> b) & 1u);
+            }
+            __syncwarp();
+            xor_list<LW>(acc, planes, longs, __popcll(m), lane);
+            __syncwarp();  // before the next word's list
           }
         }
-      }
-      uint32_t* out = bits + (rbase + rr) * pitch + wi[0];
-      if (write_ok[LW - 1] && (reinterpret_cast<uintptr_t>(out) & (4 * LW - 1)) == 0) {
-        if constexpr (LW == 4)
-          *reinterpret_cast<uint4*>(out) =
-              make_uint4(~acc[0] & valid[0], ~acc[1] & valid[1], ~acc[2] & valid[2], ~acc[3] & valid[3]);
-        else
-          *reinterpret_cast<uint2*>(out) = make_uint2(~acc[0] & valid[0], ~acc[1] & valid[1]);
-      } else {
 #pragma unroll
-        for (int h = 0; h < LW; ++h)
-          if (write_ok[h]) out[h] = ~acc[h] & valid[h];
+        for (int h = 0; h < LW; ++h) acc[h] &= valid[h];
+        if (vectors && write_ok[LW - 1]) {
+          *reinterpret_cast<Vec*>(out) = make_words<LW>(acc);
+        } else {
+#pragma unroll
+          for (int h = 0; h < LW; ++h)
+            if (write_ok[h]) out[jstep * h] = acc[h];
+        }
       }
+      __syncwarp();  // every lane is done with this batch's lists
     }
-    __syncwarp();  // every lane is done with this batch's lists
   }
 }
 
@@ -353,58 +441,61 @@ void launch_ballot(const uint64_t* lx, const uint64_t* lz, size_t n_l, const uin
 
 template <int W, int LW, int THREADS>
 void launch_plane_as(const uint64_t* lx, const uint64_t* lz, size_t n_l, const uint64_t* rx, const uint64_t* rz,
-                     size_t n_r, uint32_t* bits, size_t pitch, int device, cudaStream_t s, size_t max_rows = 16384) {
-  constexpr int kWordsCta = 32 * LW;
+                     size_t n_r, uint32_t* bits, size_t pitch, int device, cudaStream_t s, size_t max_rows) {
+  constexpr size_t kColsCta = 1024 * LW;
+  constexpr size_t smem = plane_smem(W, LW, THREADS);
+  static_assert(smem <= 227 * 1024, "planes and lists of one CTA");
   auto* kernel = commute_plane_kernel<W, LW, THREADS>;
-  const size_t smem = static_cast<size_t>(64 * W) * 2 * kWordsCta * sizeof(uint32_t);
   // The shared-memory opt-in is per device and per kernel; set once per device
   // (std::call_once also orders host threads that launch concurrently).
   static std::once_flag configured[kMaxConfiguredDevices];
+  static int resident[kMaxConfiguredDevices];  // CTAs that an SM runs at once
   if (device < 0 || device >= kMaxConfiguredDevices) wg::throw_invalid("CUDA device ordinal is out of range");
   std::call_once(configured[device], [&] {  // a throw leaves the flag unset: the next call retries
     wg::check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                    "configure bit-plane commutation");
+    int ctas = 0;
+    wg::check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, kernel, THREADS, smem),
+                   "configure bit-plane commutation");
+    resident[device] = std::max(1, ctas);
   });
-  const size_t col_blocks = (n_r + 32 * kWordsCta - 1) / (32 * kWordsCta);
-  // Enough row chunks to fill the machine (at least four CTAs per SM); as many
-  // rows per CTA as that allows, to amortise the plane building: on 262,144^2
-  // terms 2,048 rows per CTA took 5.93 ms, 4,096 4.57, 8,192 3.88, 16,384 3.52
-  // (32,768 rows at two CTAs per SM 3.80: the last wave runs part empty).
-  const size_t sms = wg::device_props(device).sm_count;
-  size_t rows_per_cta = max_rows;
-  while (rows_per_cta > 256 && col_blocks * ((n_l + rows_per_cta - 1) / rows_per_cta) < 4 * sms)
-    rows_per_cta /= 2;
-  size_t row_chunks = (n_l + rows_per_cta - 1) / rows_per_cta;
-  while (row_chunks > 65535) {
-    rows_per_cta *= 2;
-    row_chunks = (n_l + rows_per_cta - 1) / rows_per_cta;
-  }
-  dim3 grid(static_cast<unsigned>(col_blocks), static_cast<unsigned>(row_chunks));
+  const size_t blocks = (n_r + kColsCta - 1) / kColsCta;
+  const size_t total = wg::checked_mul(blocks, n_l, "commutation bit matrix");
+  // A CTA for each one that the device runs at once, while it has kMinRows rows to
+  // build a block's planes for; more of them with max_rows.
+  constexpr size_t kMinRows = 64;
+  const size_t most = static_cast<size_t>(wg::device_props(device).sm_count) * static_cast<size_t>(resident[device]);
+  size_t ctas = std::min(most, (total + kMinRows - 1) / kMinRows);
+  if (max_rows) ctas = std::max(ctas, std::min<size_t>(1u << 20, (total + max_rows - 1) / max_rows));
+  const size_t per_cta = (total + ctas - 1) / ctas;
   WG_TIMED("commute_plane_kernel", s,
-    kernel<<<grid, THREADS, smem, s>>>(lx, lz, n_l, rx, rz, n_r, bits, pitch, rows_per_cta));
+    (kernel<<<static_cast<unsigned>(ctas), THREADS, smem, s>>>(lx, lz, n_l, rx, rz, n_r, bits, pitch, total,
+                                                               per_cta)));
   wg::check_launch("launch commutation (bit-plane)");
 }
 
 // Candidates of the commutation autotuner (wg_tune.cu) on 1-4 mask words:
 //   0 ballot kernel;
-//   1 bit-plane, two output words per lane, 256 threads (2,048-column tiles);
-//   2 bit-plane, four output words per lane, 1,024 threads (4,096-column
-//     tiles; 1-2 mask words only: the planes of 4,096 columns take 64 KB of
-//     shared memory per mask word and side);
-//   3, 4 as 1, 2 with at most 2,048 lhs rows per CTA (more CTAs, each
-//     building its plane tile for fewer rows).
+//   1 bit-plane, two output words per lane (2,048-column blocks);
+//   2 bit-plane, four output words per lane (4,096-column blocks; 1-2 mask words
+//     only: the planes of 4,096 columns take 96 KB of shared memory per word);
+//   3, 4 as 1, 2 with at most 2,048 rows per CTA (more CTAs than run at once).
 // Returns false when the candidate does not serve this width.
+// Two words per lane: as many threads as let an SM hold 32 warps beside the planes.
 template <int W>
 bool launch_candidate_w(int c, const uint64_t* lx, const uint64_t* lz, size_t n_l, const uint64_t* rx,
                         const uint64_t* rz, size_t n_r, uint32_t* bits, size_t pitch, int device, cudaStream_t s) {
   switch (c) {
     case 0: launch_ballot<W>(lx, lz, n_l, rx, rz, n_r, bits, pitch, s); return true;
-    case 1: launch_plane_as<W, 2, 256>(lx, lz, n_l, rx, rz, n_r, bits, pitch, device, s); return true;
-    case 3: launch_plane_as<W, 2, 256>(lx, lz, n_l, rx, rz, n_r, bits, pitch, device, s, 2048); return true;
+    case 1:
+    case 3:
+      launch_plane_as<W, 2, W == 1 ? 256 : W == 2 ? 512 : 1024>(lx, lz, n_l, rx, rz, n_r, bits, pitch, device, s,
+                                                                c == 1 ? 0 : 2048);
+      return true;
     case 2:
     case 4:
       if constexpr (W <= 2) {
-        launch_plane_as<W, 4, 1024>(lx, lz, n_l, rx, rz, n_r, bits, pitch, device, s, c == 2 ? 16384 : 2048);
+        launch_plane_as<W, 4, 1024>(lx, lz, n_l, rx, rz, n_r, bits, pitch, device, s, c == 2 ? 0 : 2048);
         return true;
       }
       return false;
@@ -423,14 +514,13 @@ bool launch_candidate(int c, size_t words, const uint64_t* lx, const uint64_t* l
   }
 }
 
-// The measured default tile for the bit-plane kernel: four output words per
-// lane and 1,024 threads (4,096-column tiles) for one or two mask words when
-// both sides are large: 5.9 against 7.2 ms on 262,144^2 terms.  Smaller
-// products keep two words per lane and 256 threads, where the wider tile's
-// plane building would not be amortised over enough rows (32,768^2 terms: 433
-// against 253 us).
+// The measured default block of the bit-plane kernel.  With 4,096 columns (1-2 mask
+// words) a row's list and loop are paid half as often as with 2,048: 131,072^2 terms
+// of 128 qubits, weight 12.5, 1.24 against 2.24 ms; 16,384^2 46 against 64 us;
+// 4,099^2 27.5 both, and smaller products 10-20 % behind.  Up to 2,048 columns the
+// wider block would be half empty.
 int default_plane_candidate(size_t W, size_t n_l, size_t n_r) {
-  return (W <= 2 && n_l >= 65536 && n_r >= 65536) ? 2 : 1;
+  return (W <= 2 && n_r > 2048 && n_l >= (size_t{1} << 26) / n_r) ? 2 : 1;
 }
 
 // Default choice between the two algorithms, from the sizes and the word
@@ -438,12 +528,12 @@ int default_plane_candidate(size_t W, size_t n_l, size_t n_r) {
 // no synchronisation, and a call that uses it can be captured in a CUDA graph.
 // Cost model per output word:
 //   ballot: 32 pairs * (4W LOP3 + 1 POPC + pack)  ~ 32 * (4W + 2) instructions
-//   plane : about 8 per set bit of the lhs row (find bit, offsets, 16-byte
-//           shared load, XORs) + 16, plus the plane tile built once per CTA.
-// The plane kernel wins up to a mean lhs weight of (32(4W+2) - 16) / 8, i.e.
-// 22 set qubits at one word and 38 at two: every workload of this path's
-// benchmark set is far below that (k-local and sparse operators of weight
-// 2-8).  Small products keep the ballot kernel (no tile to amortise).  Callers
+//   plane : one 16-byte shared load (4 wavefronts a warp) per set qubit of the
+//           lhs row and four words, plus the planes built once per CTA.
+// Measured on 131,072^2 terms with a quarter of the bits set (weight 9 of 20, 56
+// of 128, 109 of 250): 0.72, 3.9 and 9.9 ms against the ballot kernel's 12.9, 16.7
+// and 35.9.  Small products keep the ballot kernel (no planes to build): 256^2 and
+// 20 qubits 14 us by ballots, 10 by planes, 64^2 8 and 10.  Callers
 // that know the weight pass algo 1 or 2 themselves, and the autotuner's cached
 // measurement replaces this rule for shape classes it has searched.
 int default_algo(size_t W, size_t n_l, size_t n_r) {

@@ -3,14 +3,15 @@
 // Tuned operations and their candidates (every candidate gives identical
 // results; only the time differs):
 //   commute     wg_commutation_bits with algo 0, 1-4 mask words:
-//               0 ballot kernel; 1 bit-plane, 2,048-column tiles (256
-//               threads); 2 bit-plane, 4,096-column tiles (1,024 threads, 1-2
-//               words); 3 and 4 the same two tiles with at most 2,048 lhs rows
-//               per CTA instead of up to 16,384;
+//               0 ballot kernel; 1 bit-plane, 2,048-column blocks; 2 bit-plane,
+//               4,096-column blocks (1-2 words); 3 and 4 the same two with at
+//               most 2,048 rows per CTA instead of one run for each CTA that
+//               the device holds;
 //   bucket      the bucketed sort's target items per fine bucket:
 //               640, 768, 896, 1,024, 1,280;
-//   group_qwc   group_commuting chunk length, qwc mode: 256, 512, 1,024;
-//   group_full  group_commuting chunk length, full mode: 64, 96, 128, 192.
+//   group_qwc   group_commuting, terms per batch of a stage, qwc mode: 128, 256,
+//               512 (above 4 mask words the chunk length);
+//   group_full  the same in full mode: 8, 16, 24, 31.
 // Classes: commute (words, log2 n_lhs, log2 n_rhs); bucket (words, log2
 // products or terms, 0); group_* (words, log2 terms, 0), logs rounded up.
 
