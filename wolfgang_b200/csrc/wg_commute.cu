@@ -116,15 +116,22 @@ __global__ void __launch_bounds__(kThreads) commute_generic_kernel(
 // Dense uint8 flags straight from the masks, without the bit matrix.  A warp
 // holds the masks of 32 COLS columns (a lane's columns are 32 apart, so that each
 // of its stores is 32 consecutive bytes of the warp) and sweeps rows.  Per pair: 4
-// LOP3 per mask word, a population count, a byte store.  4,099^2 flags of 20 qubits:
-// 23 us of kernel, 36 us a call, against 36 + 27 us of the bit matrix and its
-// expansion, 88 us a call.
-template <int W, int COLS>
-__global__ void __launch_bounds__(kThreads) commute_flags_kernel(
+// LOP3 per mask word, a population count (a quarter of the issue rate of a LOP3), a
+// byte store.  One wave of CTAs, each warp with as many rows as that leaves it, and
+// the next row's masks loaded ahead: 4,099^2 flags of 20 qubits 28 us a call (36 with
+// 1.4 waves and no loads ahead; 88 through the bit matrix, 36 + 27 us of kernels).
+template <int W>
+constexpr int kFlagCols = W <= 2 ? 8 : 4;  // columns of a lane
+template <int W>
+constexpr int kFlagCtas = W == 1 ? 4 : 2;  // CTAs per SM that the registers are held down to
+
+template <int W>
+__global__ void __launch_bounds__(kThreads, kFlagCtas<W>) commute_flags_kernel(
     const uint64_t* __restrict__ lx, const uint64_t* __restrict__ lz, size_t n_l, const uint64_t* __restrict__ rx,
     const uint64_t* __restrict__ rz, size_t n_r, uint8_t* __restrict__ out, uint32_t rows_per_warp) {
+  constexpr int COLS = kFlagCols<W>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t col0 = static_cast<size_t>(blockIdx.x) * (32 * COLS) + lane;
+  const size_t tile = static_cast<size_t>(blockIdx.x) * (32 * COLS), col0 = tile + lane;
   uint64_t cx[COLS][W], cz[COLS][W];
 #pragma unroll
   for (int k = 0; k < COLS; ++k) {
@@ -136,24 +143,45 @@ __global__ void __launch_bounds__(kThreads) commute_flags_kernel(
     }
   }
   const size_t row0 = (static_cast<size_t>(blockIdx.y) * kWarps + warp) * rows_per_warp;
-  const size_t row1 = min(n_l, row0 + rows_per_warp);
-  const bool whole = static_cast<size_t>(blockIdx.x + 1) * (32 * COLS) <= n_r;
-#pragma unroll 2
-  for (size_t row = row0; row < row1; ++row) {
-    uint64_t ax[W], az[W];
+  if (row0 >= n_l) return;
+  const int rows = static_cast<int>(min(n_l - row0, static_cast<size_t>(rows_per_warp)));
+  uint8_t* o = out + row0 * n_r + col0;
+  lx += row0 * W;
+  lz += row0 * W;
+  auto flag = [&](const uint64_t(&ax)[W], const uint64_t(&az)[W], int k) {
+    uint32_t acc = 0;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      ax[w] = __ldg(lx + row * W + w);
-      az[w] = __ldg(lz + row * W + w);
+      acc ^= static_cast<uint32_t>(ax[w]) & static_cast<uint32_t>(cz[k][w]);
+      acc ^= static_cast<uint32_t>(az[w]) & static_cast<uint32_t>(cx[k][w]);
+      acc ^= static_cast<uint32_t>(ax[w] >> 32) & static_cast<uint32_t>(cz[k][w] >> 32);
+      acc ^= static_cast<uint32_t>(az[w] >> 32) & static_cast<uint32_t>(cx[k][w] >> 32);
     }
-    uint8_t* o = out + row * n_r + col0;
+    return static_cast<uint8_t>(~__popc(acc) & 1);
+  };
+  // the next row's masks are in flight while a row is worked on
+  uint64_t nx[W], nz[W];
 #pragma unroll
-    for (int k = 0; k < COLS; ++k) {
-      uint64_t acc = 0;
+  for (int w = 0; w < W; ++w) nx[w] = __ldg(lx + w), nz[w] = __ldg(lz + w);
+  const int mine = static_cast<int>(min(static_cast<size_t>(COLS), (max(n_r, col0) - col0 + 31) / 32));
+  const bool whole = tile + 32 * COLS <= n_r;
+  for (int r = 0; r < rows; ++r, o += n_r) {
+    uint64_t ax[W], az[W];
+    const size_t next = static_cast<size_t>(min(r + 1, rows - 1)) * W;
 #pragma unroll
-      for (int w = 0; w < W; ++w) acc ^= (ax[w] & cz[k][w]) ^ (az[w] & cx[k][w]);
-      const uint32_t folded = static_cast<uint32_t>(acc) ^ static_cast<uint32_t>(acc >> 32);
-      if (whole || col0 + 32 * k < n_r) o[32 * k] = static_cast<uint8_t>(~__popc(folded) & 1);
+    for (int w = 0; w < W; ++w) {
+      ax[w] = nx[w];
+      az[w] = nz[w];
+      nx[w] = __ldg(lx + next + w);
+      nz[w] = __ldg(lz + next + w);
+    }
+    if (whole) {
+#pragma unroll
+      for (int k = 0; k < COLS; ++k) o[32 * k] = flag(ax, az, k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < COLS; ++k)
+        if (k < mine) o[32 * k] = flag(ax, az, k);
     }
   }
 }
@@ -541,20 +569,21 @@ int default_algo(size_t W, size_t n_l, size_t n_r) {
   return 2;
 }
 
-template <int W, int COLS>
+template <int W>
 void launch_flags(const uint64_t* lx, const uint64_t* lz, size_t n_l, const uint64_t* rx, const uint64_t* rz,
                   size_t n_r, uint8_t* out, int device, cudaStream_t s) {
-  const size_t tiles = (n_r + 32 * COLS - 1) / (32 * COLS);
-  // One wave of 32 warps an SM while a warp has no more than 64 rows: it reads
-  // its columns once for them all.
-  const size_t warps = static_cast<size_t>(wg::device_props(device).sm_count) * 32;
-  size_t rows = std::min<size_t>(64, std::max<size_t>(1, n_l * tiles / warps));
+  constexpr int kCols = 32 * kFlagCols<W>;
+  const size_t tiles = (n_r + kCols - 1) / kCols;
+  // One wave of CTAs while a warp has no more than 64 rows: it reads its columns
+  // once for them all.
+  const size_t ctas = static_cast<size_t>(wg::device_props(device).sm_count) * kFlagCtas<W>;
+  const size_t chunks = std::max<size_t>(1, ctas / tiles);  // along the rows
+  size_t rows = std::min<size_t>(64, (n_l + chunks * kWarps - 1) / (chunks * kWarps));
   while ((n_l + rows * kWarps - 1) / (rows * kWarps) > 65535) rows *= 2;
-  if (rows > 0xffffffffu || tiles > 0x7fffffffu) wg::throw_invalid("commutation matrix exceeds the launch grid");
+  if (rows > 0x7fffffffu || tiles > 0x7fffffffu) wg::throw_invalid("commutation matrix exceeds the launch grid");
   const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>((n_l + rows * kWarps - 1) / (rows * kWarps)));
   WG_TIMED("commute_flags_kernel", s,
-    (commute_flags_kernel<W, COLS><<<grid, kThreads, 0, s>>>(lx, lz, n_l, rx, rz, n_r, out,
-                                                             static_cast<uint32_t>(rows))));
+    commute_flags_kernel<W><<<grid, kThreads, 0, s>>>(lx, lz, n_l, rx, rz, n_r, out, static_cast<uint32_t>(rows)));
   wg::check_launch("launch commutation flags");
 }
 
@@ -562,10 +591,10 @@ void launch_flags(const uint64_t* lx, const uint64_t* lz, size_t n_l, const uint
 bool commutation_flags(int device, size_t words, const uint64_t* lx, const uint64_t* lz, size_t n_l,
                        const uint64_t* rx, const uint64_t* rz, size_t n_r, uint8_t* out, cudaStream_t s) {
   switch (words) {
-    case 1: launch_flags<1, 8>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
-    case 2: launch_flags<2, 8>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
-    case 3: launch_flags<3, 4>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
-    case 4: launch_flags<4, 4>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 1: launch_flags<1>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 2: launch_flags<2>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 3: launch_flags<3>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
+    case 4: launch_flags<4>(lx, lz, n_l, rx, rz, n_r, out, device, s); return true;
     default: return false;
   }
 }
