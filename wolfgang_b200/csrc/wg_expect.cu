@@ -22,7 +22,8 @@
 // Forward.  A warp holds 32 x 16 amplitudes of the tile.  The sums of 8 terms
 // over them are matrix products: signs (8 terms x 4 amplitudes) times t (4
 // amplitudes x 8), FP64 m8n8k4, 16 of them a component whatever the number of
-// terms; what is left of the columns is added up with the terms' signs.
+// terms; what is left of the columns is added up with the terms' signs.  A
+// sub-group's even and odd terms are taken together, from the same loads.
 //
 // Adjoint.  (H psi)[j] = sum_g F_g(j^x) psi[j^x].  F's real part at j is an entry
 // of a table of the 2^8 sign patterns of the sub-group's even terms, its
@@ -54,7 +55,7 @@ constexpr int kTileMax = 1 << kTileBits;
 constexpr int kPiece = 8;                // terms per sub-group of either parity of y
 constexpr int kSegSubs = 16;             // sub-groups of one class staged at a time (adjoint)
 constexpr int kSegEntries = 2048;        // and their table entries
-constexpr int kChunkPieces = 32;         // pieces of one forward item
+constexpr int kChunkPieces = 128;        // pieces of one forward item
 constexpr int kFwdThreads = 512;         // two sets of 256 x 16 amplitudes = a tile
 constexpr int kFwdInner = 8;             // warps of a set
 constexpr int kAdjThreads = 512;         // x 8 amplitudes = a tile
@@ -66,11 +67,14 @@ struct __align__(16) FwdPiece {
   uint32_t xlo;              // x within the tile
   uint32_t xhi;              // and above it
   uint32_t t0;
-  uint16_t nk, odd;
+  uint8_t nk, odd;
+  uint8_t pair;              // even terms, and the next piece has the sub-group's odd ones: taken together
+  uint8_t turn;              // the set of threads that takes it (kDirect: of a chunk that reads psi itself)
   uint32_t zlo[kPiece];      // z within the tile
   uint32_t zhi[kPiece];      // and above it
 };
 static_assert(sizeof(FwdPiece) == 80, "copied in 16-byte pieces");
+constexpr uint8_t kDirect = 0x80;
 
 // A sub-group: terms [t0, t0 + nre) of even y, then nim of odd y.  A sign word has the even terms' signs in bits
 // 3-10, the odd ones' in bits 19-26: byte offsets into the tables.
@@ -199,9 +203,9 @@ __device__ __forceinline__ void copy_wait() {
 }
 
 // Two tile buffers.  complex128 amplitudes are copied as they are, the next
-// tile into the other buffer; complex64 ones are copied into the second
-// buffer and widened from there into the first (once for all groups of a
-// class: the conversions would cost as much as the products).
+// tile into the other buffer; complex64 ones are copied into the halves of the
+// second buffer by turns and widened from there into the first (once for all
+// groups of a class: the conversions would cost as much as the products).
 template <typename Amp>
 struct TileBuffers {
   static constexpr bool kWide = sizeof(Amp) == 16;
@@ -222,7 +226,7 @@ struct TileBuffers {
         else to[i] = make_double2(0.0, 0.0);
       }
     } else {
-      float2* to = reinterpret_cast<float2*>(b1);
+      float2* to = reinterpret_cast<float2*>(b1) + slot * kTileMax;
       for (int i = threadIdx.x; i < size; i += blockDim.x) {
         if (i < have) copy_async<8>(to + i, from + i);
         else to[i] = make_float2(0.0f, 0.0f);
@@ -231,8 +235,8 @@ struct TileBuffers {
   }
   // complex64: the fetched tile, widened (all copies of this thread are done;
   // each thread widens what it fetched)
-  __device__ __forceinline__ void widen(int m) {
-    const float2* from = reinterpret_cast<const float2*>(b1);
+  __device__ __forceinline__ void widen(int m, int slot) {
+    const float2* from = reinterpret_cast<const float2*>(b1) + slot * kTileMax;
     for (int i = threadIdx.x; i < (1 << m); i += blockDim.x) {
       const float2 v = from[i];
       b0[i] = make_double2(static_cast<double>(v.x), static_cast<double>(v.y));
@@ -248,7 +252,7 @@ __device__ __forceinline__ double flip(double v, uint32_t sign) {
 
 struct FwdShared {
   double2 tile[2][kTileMax];
-  double acc[kFwdInner][kChunkPieces * 32];  // by warp, piece, term and column quarter
+  double acc[kFwdInner][kChunkPieces * kPiece];  // by warp, piece and term
   FwdPiece piece[kChunkPieces];
   uint32_t seg_xhi[kChunkPieces];
   uint32_t seg_at[kChunkPieces + 1];
@@ -275,55 +279,77 @@ struct Layout {
   __device__ __forceinline__ uint32_t off8(int r) const { return static_cast<uint32_t>(r) << (m() - 3); }
 };
 
-// Adds a piece's sums over tile J to acc (the lane's place): a is the thread's
-// part of tile J, src the tile that x pairs it with.  Amplitude bits of the
-// tile: 0-1 lane % 4 (the products' inner index, with t's bits m-4 to m-2), 2-4
-// lane / 4 (the columns, with t's bit m-1), 5 to m-5 the warp.
-template <int M>
-__device__ __forceinline__ void forward_piece(const Layout<M>& lay, const FwdPiece& pd, const double2* src,
-                                              const c128 (&a)[16], uint32_t J, int tt, int lane, double* acc) {
-  constexpr uint32_t kSign = 0x80000000u;
-  const int m = lay.m();
-  const uint32_t at = static_cast<uint32_t>(tt) ^ pd.xlo;
-  double t[16];
-  if (pd.odd) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const double2 v = src[at ^ lay.off16(q)];
-      t[q] = fma(v.x, a[q].im, -(v.y * a[q].re));
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const double2 v = src[at ^ lay.off16(q)];
-      t[q] = fma(v.x, a[q].re, v.y * a[q].im);
-    }
+// Signs of a piece's terms for the products: the lane's term is lane / 4.
+struct TermSigns {
+  uint32_t zlo, one, e0, e1, e2;
+  __device__ __forceinline__ TermSigns(const FwdPiece& pd, uint32_t J, uint32_t where, int m, int lane) {
+    constexpr uint32_t kSign = 0x80000000u;
+    zlo = pd.zlo[lane >> 2];
+    one = 0x3ff00000u ^ (static_cast<uint32_t>(__popc((zlo & where) ^ (pd.zhi[lane >> 2] & J))) << 31);
+    e0 = (zlo << (35 - m)) & kSign;
+    e1 = (zlo << (34 - m)) & kSign;
+    e2 = (zlo << (33 - m)) & kSign;
   }
-  // the lane's term is lane / 4; its sign at the lane's and warp's share of the inner bits
-  const uint32_t zlo = pd.zlo[lane >> 2], zhi = pd.zhi[lane >> 2];
-  const uint32_t where = static_cast<uint32_t>(tt) & ~28u;
-  const uint32_t one = 0x3ff00000u ^ (static_cast<uint32_t>(__popc((zlo & where) ^ (zhi & J))) << 31);
-  const uint32_t e0 = (zlo << (35 - m)) & kSign, e1 = (zlo << (34 - m)) & kSign, e2 = (zlo << (33 - m)) & kSign;
-  double c00 = 0.0, c01 = 0.0, c10 = 0.0, c11 = 0.0;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
+  // +-1 for step k of the inner bits
+  __device__ __forceinline__ double at(int k) const {
     uint32_t hi = one;
     if (k & 1) hi ^= e0;
     if (k & 2) hi ^= e1;
     if (k & 4) hi ^= e2;
-    const double s = __hiloint2double(static_cast<int>(hi), 0);
-    mma_f64(c00, c01, s, t[k]);
-    mma_f64(c10, c11, s, t[8 + k]);
+    return __hiloint2double(static_cast<int>(hi), 0);
   }
-  const uint32_t bit2 = zlo << 29;
-  const double v = (c00 + flip(c01, bit2)) + flip(c10 + flip(c11, bit2), zlo << (32 - m));
-  *acc += flip(v, static_cast<uint32_t>(__popc((zlo >> 3) & (lane & 3))) << 31);
+};
+
+// Adds a piece's sums over tile J to acc[0..7] (kParts 1: even terms, 2: odd ones), or a pair's to those and the
+// next eight (3): a is the thread's part of tile J, load the tile that x pairs it with.  Amplitude bits of the
+// tile: 0-1 lane % 4 (the products' inner index, with t's bits m-4 to m-2), 2-4 lane / 4 (the columns, with t's
+// bit m-1), 5 to m-5 the warp.  An amplitude's products follow its load at once: four independent chains of a
+// pair keep the pipe busy while the next loads are under way.
+template <int M, int kParts, class Load>
+__device__ __forceinline__ void forward_unit(const Layout<M>& lay, const FwdPiece* pd, const Load& load,
+                                             const c128 (&a)[16], uint32_t J, int tt, int lane, double* acc) {
+  const int m = lay.m();
+  const uint32_t at = static_cast<uint32_t>(tt) ^ pd->xlo, where = static_cast<uint32_t>(tt) & ~28u;
+  constexpr int kCount = kParts == 3 ? 2 : 1;
+  const TermSigns first(pd[0], J, where, m, lane), second(pd[kCount - 1], J, where, m, lane);
+  double c[kCount][4] = {};
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const double s0 = first.at(k), s1 = kCount == 2 ? second.at(k) : 0.0;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int q = k + 8 * half;
+      const double2 v = load(at ^ lay.off16(q));
+      const double re = fma(v.x, a[q].re, v.y * a[q].im), im = fma(v.x, a[q].im, -(v.y * a[q].re));
+      mma_f64(c[0][2 * half], c[0][2 * half + 1], s0, kParts == 2 ? im : re);
+      if constexpr (kCount == 2) mma_f64(c[1][2 * half], c[1][2 * half + 1], s1, im);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kCount; ++i) {
+    const uint32_t zlo = i ? second.zlo : first.zlo, bit2 = zlo << 29;
+    double v = (c[i][0] + flip(c[i][1], bit2)) + flip(c[i][2] + flip(c[i][3], bit2), zlo << (32 - m));
+    v = flip(v, static_cast<uint32_t>(__popc((zlo >> 3) & (lane & 3))) << 31);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    if ((lane & 3) == 0) acc[kPiece * i + (lane >> 2)] += v;
+  }
+}
+
+template <int M, class Load>
+__device__ __forceinline__ void forward_any(const Layout<M>& lay, const FwdPiece* pd, const Load& load,
+                                            const c128 (&a)[16], uint32_t J, int tt, int lane, double* acc) {
+  if (pd->pair) forward_unit<M, 3>(lay, pd, load, a, J, tt, lane, acc);
+  else if (pd->odd) forward_unit<M, 2>(lay, pd, load, a, J, tt, lane, acc);
+  else forward_unit<M, 1>(lay, pd, load, a, J, tt, lane, acc);
 }
 
 // A CTA takes (chunk of pieces, range of tiles) items.  24 qubits, 20,000 terms
-// in 1,699 groups: 50 ms (before, with 16 masked sums a pair: 87 ms); 20 qubits,
-// 4,096 terms in 2,526 groups: 2.2 ms (4.5).  Bound by instruction issue: the
-// matrix products are 15 of the 50 ms, a tile's fetch hides behind them.
+// in 1,699 groups: 40 ms (87 ms with 16 masked sums a pair; 50 ms with a piece's
+// loads before its products, the parities apart and 32 pieces a chunk); 20
+// qubits, 4,096 terms in 2,526 groups: 2.0 ms (4.5).  Bound by the FP64 pipe, 61 %
+// busy (47 % products, 14 % the t's): four warps a scheduler (tile J takes half of
+// the registers) do not cover all of the chains' latency.
 template <typename Amp>
 __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(BatchDev B) {
   extern __shared__ __align__(16) unsigned char raw[];
@@ -350,94 +376,108 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(BatchDev
       const uint4* from = reinterpret_cast<const uint4*>(P.piece + piece0);
       uint4* to = reinterpret_cast<uint4*>(sh.piece);
       for (uint32_t i = tid; i < pieces * (sizeof(FwdPiece) / 16); i += kFwdThreads) to[i] = from[i];
-      for (int i = tid; i < kFwdInner * kChunkPieces * 32; i += kFwdThreads) (&sh.acc[0][0])[i] = 0.0;
-      if (warp == 0) {
-        const uint32_t xhi = lane < static_cast<int>(pieces) ? P.piece[piece0 + lane].xhi : 0;
-        const uint32_t before = __shfl_up_sync(0xffffffffu, xhi, 1);
-        const bool head = lane < static_cast<int>(pieces) && (lane == 0 || xhi != before);
-        const uint32_t heads = __ballot_sync(0xffffffffu, head);
-        if (head) {
-          const int at = __popc(heads & ((1u << lane) - 1u));
-          sh.seg_xhi[at] = xhi;
-          sh.seg_at[at] = lane;
+      for (uint32_t i = lane; i < pieces * kPiece; i += 32)
+        if (warp < kFwdInner) sh.acc[warp][i] = 0.0;
+      if (warp == kFwdInner) {
+        uint32_t segs = 0;
+        for (uint32_t at = 0; at < pieces; at += 32) {
+          const uint32_t i = at + lane;
+          const bool in = i < pieces;
+          const uint32_t xhi = in ? P.piece[piece0 + i].xhi : 0;
+          const bool head = in && (i == 0 || xhi != P.piece[piece0 + i - 1].xhi);
+          const uint32_t heads = __ballot_sync(0xffffffffu, head);
+          if (head) {
+            const uint32_t to = segs + __popc(heads & ((1u << lane) - 1u));
+            sh.seg_xhi[to] = xhi;
+            sh.seg_at[to] = i;
+          }
+          segs += __popc(heads);
         }
         if (lane == 0) {
-          sh.segs = __popc(heads);
-          sh.seg_at[__popc(heads)] = pieces;
+          sh.segs = segs;
+          sh.seg_at[segs] = pieces;
         }
       }
     }
     __syncthreads();
     const uint32_t segs = sh.segs;
     // thread tt of the tile holds amplitudes tt + (q << m-4); the sets of
-    // threads (two for tiles of 2^12, more for smaller ones) take the pieces in
-    // turn: while one brings its operands in, the other's products run
+    // threads (two for tiles of 2^12, more for smaller ones) take a piece each
     const int tt = tid & ((1 << (m - 4)) - 1);
-    const uint32_t slice = tid >> (m - 4), slices = kFwdThreads >> (m - 4);
-    // (tile, segment) steps: a segment with x above the tile pairs J with
-    // J ^ xhi once, from the side whose lowest bit of xhi is clear
-    auto next_step = [&](uint32_t& J, uint32_t& g) {
-      while (J < J1) {
-        for (; g < segs; ++g) {
-          const uint32_t xhi = sh.seg_xhi[g];
-          if (xhi == 0 || !((J >> (__ffs(static_cast<int>(xhi)) - 1)) & 1u)) return true;
-        }
-        g = 0;
-        ++J;
-      }
-      return false;
-    };
-    TileBuffers<Amp> buf{sh.tile[0], sh.tile[1]};
-    constexpr bool kWide = TileBuffers<Amp>::kWide;
-    uint32_t J = J0, g = 0, have = 0xffffffffu;
-    bool more = next_step(J, g);
-    int slot = 0;
-    if (more) buf.fetch(psi, J ^ sh.seg_xhi[g], m, n, 0);
-    copy_commit();
+    const uint32_t slice = tid >> (m - 4);
     c128 a[16];
-    while (more) {
-      uint32_t Jn = J, gn = g + 1;
-      const bool more_n = next_step(Jn, gn);
-      if (kWide) {
+    auto load_own = [&](uint32_t J) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const uint64_t b = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(q) << (m - 4));
+        a[q] = (b >> n) == 0 ? load_amp<Amp>(psi, b) : c128{0.0, 0.0};
+      }
+    };
+    double* const acc = sh.acc[tt >> 5];
+    // a segment with x above the tile pairs J with J ^ xhi once, from the side
+    // whose lowest bit of xhi is clear
+    auto this_side = [](uint32_t J, uint32_t xhi) { return xhi == 0 || !((J >> (__ffs(static_cast<int>(xhi)) - 1)) & 1u); };
+    if (sh.piece[0].turn & kDirect) {
+      // hardly two pieces of a class: each reads the paired tile itself, and
+      // nothing waits for the others
+      for (uint32_t J = J0; J < J1; ++J) {
+        load_own(J);
+        for (uint32_t i = 0; i < pieces; i += sh.piece[i].pair ? 2 : 1) {
+          const FwdPiece* pd = sh.piece + i;
+          if ((pd->turn & ~kDirect) != slice || !this_side(J, pd->xhi)) continue;
+          const Amp* from = static_cast<const Amp*>(psi) + (static_cast<uint64_t>(J ^ pd->xhi) << kTileBits);
+          auto load = [&](uint32_t i) {
+            const c128 v = load_amp<Amp>(from, i);
+            return make_double2(v.re, v.im);
+          };
+          forward_any(Layout<kTileBits>{kTileBits}, pd, load, a, J, tt, lane, acc + kPiece * i);
+        }
+      }
+    } else {
+      // (tile, segment) steps
+      auto next_step = [&](uint32_t& J, uint32_t& g) {
+        while (J < J1) {
+          for (; g < segs; ++g)
+            if (this_side(J, sh.seg_xhi[g])) return true;
+          g = 0;
+          ++J;
+        }
+        return false;
+      };
+      TileBuffers<Amp> buf{sh.tile[0], sh.tile[1]};
+      constexpr bool kWide = TileBuffers<Amp>::kWide;
+      uint32_t J = J0, g = 0, have = 0xffffffffu;
+      bool more = next_step(J, g);
+      int slot = 0;
+      if (more) buf.fetch(psi, J ^ sh.seg_xhi[g], m, n, 0);
+      copy_commit();
+      while (more) {
+        uint32_t Jn = J, gn = g + 1;
+        const bool more_n = next_step(Jn, gn);
         if (more_n) buf.fetch(psi, Jn ^ sh.seg_xhi[gn], m, n, slot ^ 1);
         copy_commit();
-      }
-      if (have != J) {
-        have = J;
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const uint64_t b = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(q) << (m - 4));
-          a[q] = (b >> n) == 0 ? load_amp<Amp>(psi, b) : c128{0.0, 0.0};
+        if (have != J) {
+          have = J;
+          load_own(J);
         }
-      }
-      if (kWide) {
         copy_wait<1>();
-      } else {
-        copy_wait<0>();
-        buf.widen(m);
+        if (!kWide) buf.widen(m, slot);
+        __syncthreads();
+        const double2* src = kWide && slot ? buf.b1 : buf.b0;
+        auto load = [&](uint32_t i) { return src[i]; };
+        const uint32_t i1 = sh.seg_at[g + 1];
+        for (uint32_t i = sh.seg_at[g]; i < i1; i += sh.piece[i].pair ? 2 : 1) {
+          const FwdPiece* pd = sh.piece + i;
+          if (pd->turn != slice) continue;
+          if (m == kTileBits) forward_any(Layout<kTileBits>{m}, pd, load, a, J, tt, lane, acc + kPiece * i);
+          else forward_any(Layout<0>{m}, pd, load, a, J, tt, lane, acc + kPiece * i);
+        }
+        __syncthreads();
+        J = Jn;
+        g = gn;
+        more = more_n;
+        slot ^= 1;
       }
-      __syncthreads();
-      if (!kWide) {
-        if (more_n) buf.fetch(psi, Jn ^ sh.seg_xhi[gn], m, n, 0);
-        copy_commit();
-      }
-      const double2* src = kWide && slot ? buf.b1 : buf.b0;
-      const uint32_t i1 = sh.seg_at[g + 1];
-      double* acc = sh.acc[tt >> 5] + lane;
-      if (m == kTileBits) {
-        const Layout<kTileBits> lay{m};
-        for (uint32_t i = sh.seg_at[g]; i < i1; ++i)
-          if ((i & 1u) == slice) forward_piece(lay, sh.piece[i], src, a, J, tt, lane, acc + 32 * i);
-      } else {
-        const Layout<0> lay{m};
-        for (uint32_t i = sh.seg_at[g]; i < i1; ++i)
-          if ((i & (slices - 1)) == slice) forward_piece(lay, sh.piece[i], src, a, J, tt, lane, acc + 32 * i);
-      }
-      __syncthreads();
-      J = Jn;
-      g = gn;
-      more = more_n;
-      slot ^= 1;
     }
     copy_wait<0>();
     __syncthreads();
@@ -446,26 +486,30 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(BatchDev
       if (k % kPiece >= pd.nk) continue;
       double s = 0.0;
 #pragma unroll
-      for (int v = 0; v < kFwdInner; ++v) {
-        const double* row = sh.acc[v] + 4 * k;
-        s += (row[0] + row[1]) + (row[2] + row[3]);
-      }
+      for (int v = 0; v < kFwdInner; ++v) s += sh.acc[v][k];
       P.partial[static_cast<uint64_t>(pd.t0 + k % kPiece) * P.ranges + range] = s;
     }
   }
 }
 
-// e_k from the ranges' partial sums (in order), scaled by the pairing factor
-// and scattered to original term order; flat over every pair's terms.
+// e_k from the ranges' partial sums (eight lanes a term, in a fixed order:
+// one thread took 17 us for 256 ranges), scaled by the pairing factor and
+// scattered to original term order; flat over every pair's terms.
 __global__ void __launch_bounds__(kThreads) expect_finish_terms_kernel(BatchDev B) {
-  for (uint64_t f = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; f < B.n_terms;
-       f += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+  const uint32_t lane = threadIdx.x & 7;
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x / 8;
+  const uint64_t first = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) / 8;
+  for (uint64_t f0 = first; f0 - (threadIdx.x & 31) / 8 < B.n_terms; f0 += stride) {  // a warp leaves together
+    const uint64_t f = min(f0, B.n_terms - 1);
     const uint32_t p = upper_index<uint64_t>(B.term_base, B.np + 1, f);
     const PlanDev& P = B.plans[p];
     const uint32_t k = static_cast<uint32_t>(f - B.term_base[p]);
     const double* part = P.partial + static_cast<uint64_t>(k) * P.ranges;
     double s = 0.0;
-    for (uint32_t c = 0; c < P.ranges; ++c) s += part[c];
+    for (uint32_t c = lane; c < P.ranges; c += 8) s += part[c];
+#pragma unroll
+    for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane != 0 || f0 >= B.n_terms) continue;
     const uint32_t ty = P.ty[k];
     const double e = ((ty & 3u) == 1 || (ty & 3u) == 2) ? -s : s;
     B.evals[p][P.torig[k]] = ty & (kDiagFlag | kTwiceFlag) ? e : 2.0 * e;
@@ -630,21 +674,12 @@ __global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(BatchDev
       const bool last = g + 1 == g1;
       const SegDev after = P.seg[min(g + 2, g1 - 1)];  // a step ahead of its use
       const bool fresh_n = !last && nx.xhi != sg.xhi;
-      if (kWide) {
-        if (fresh_n) buf.fetch(psi, J ^ nx.xhi, m, n, slot ^ 1);
-        if (!last) fetch_stage(nx, stage ^ 1);
-        copy_commit();
-        copy_wait<1>();
-      } else {
-        copy_wait<0>();
-        if (fresh) buf.widen(m);
-      }
+      if (fresh_n) buf.fetch(psi, J ^ nx.xhi, m, n, slot ^ 1);
+      if (!last) fetch_stage(nx, stage ^ 1);
+      copy_commit();
+      copy_wait<1>();
+      if (!kWide && fresh) buf.widen(m, slot);
       __syncthreads();
-      if (!kWide) {
-        if (fresh_n) buf.fetch(psi, J ^ nx.xhi, m, n, 0);
-        if (!last) fetch_stage(nx, stage ^ 1);
-        copy_commit();
-      }
       const double2* src = kWide && slot ? buf.b1 : buf.b0;
       const AdjStage& st = sh.stage[stage];
       if (m == kTileBits) {
@@ -874,8 +909,9 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
         pd.xlo = ad.xlo;
         pd.xhi = static_cast<uint32_t>(gx >> m);
         pd.t0 = static_cast<uint32_t>(t0);
-        pd.nk = static_cast<uint16_t>(nk);
-        pd.odd = static_cast<uint16_t>(half);
+        pd.nk = static_cast<uint8_t>(nk);
+        pd.odd = static_cast<uint8_t>(half);
+        if (half && nk && ad.nre) piece.back().pair = 1;
         for (uint32_t kk = 0; kk < nk; ++kk, ++t0) {
           const uint32_t o = all[from + kk];
           torig[t0] = o;
@@ -943,7 +979,33 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   const size_t sets = (static_cast<size_t>(kFwdThreads) * 16) >> m;
   const size_t chunk_pieces = std::min<size_t>(
       kChunkPieces, std::max<size_t>(sets, (NP * d.tiles + 4 * sms - 1) / (4 * sms)));
-  for (size_t i = 0; i < NP; i += chunk_pieces) chunk.push_back(static_cast<uint32_t>(std::min(NP, i + chunk_pieces)));
+  std::vector<uint32_t> load(sets);
+  for (size_t i = 0; i < NP;) {
+    size_t e = i, units = 0, segs = 0;
+    while (e < NP && e - i + 1 + piece[e].pair <= chunk_pieces) {
+      segs += e == i || piece[e].xhi != piece[e - 1].xhi;
+      ++units;
+      e += 1 + piece[e].pair;
+    }
+    // Staging a class's tile pays where more than a piece or two of it follow: 21
+    // qubits, 16 terms of as many classes, complex64, 105 us staged and 60 direct.
+    const bool direct = m == kTileBits && static_cast<int>(n) > m && 4 * units <= 5 * segs;
+    // the sets' turns: the least loaded one of the segment's (of the chunk's
+    // where nothing is staged); a last pair is shared by two equally loaded ones
+    std::fill(load.begin(), load.end(), 0u);
+    for (size_t k = i; k < e;) {
+      if (!direct && k > i && piece[k].xhi != piece[k - 1].xhi) std::fill(load.begin(), load.end(), 0u);
+      const size_t next = k + 1 + piece[k].pair;
+      const size_t to = static_cast<size_t>(std::min_element(load.begin(), load.end()) - load.begin());
+      const bool last = !direct && (next >= e || piece[next].xhi != piece[k].xhi);
+      if (piece[k].pair && last && std::count(load.begin(), load.end(), load[to]) > 1) piece[k].pair = 0;
+      load[to] += 1u + piece[k].pair;
+      piece[k].turn = static_cast<uint8_t>(to | (direct ? kDirect : 0));
+      k += 1 + piece[k].pair;
+    }
+    chunk.push_back(static_cast<uint32_t>(e));
+    i = e;
+  }
   d.chunks = static_cast<uint32_t>(chunk.size() - 1);
   d.ranges = static_cast<uint32_t>(
       std::max<size_t>(1, std::min<size_t>({d.tiles, 256, (8 * sms + d.chunks - 1) / d.chunks})));
@@ -1140,7 +1202,8 @@ void run_batch(const wg_expect_batch_s& b, cudaStream_t s) {
   }
   const unsigned wave = static_cast<unsigned>(b.sms) * 8;
   if (d.n_terms) {
-    const unsigned grid = static_cast<unsigned>(std::min<uint64_t>((d.n_terms + kThreads - 1) / kThreads, wave));
+    const unsigned grid =
+        static_cast<unsigned>(std::min<uint64_t>((8 * d.n_terms + kThreads - 1) / kThreads, wave));
     WG_TIMED("expect_finish_terms_kernel", s, expect_finish_terms_kernel<<<grid, kThreads, 0, s>>>(d));
     wg::check_launch("launch expectation finish");
   }
