@@ -309,6 +309,9 @@ int wg_expect_plan_destroy(wg_expect_plan_t plan);
 /* Replaces the coefficients of a plan (same terms, new values; device buffer
  * of 2*n_terms doubles in the plan's original term order). */
 int wg_expect_plan_set_coeffs(wg_expect_plan_t plan, const double* coeffs, wg_stream_t stream);
+/* The same with real coefficients (device buffer of n_terms doubles): a
+ * Hermitian operator's, as an optimiser holds them. */
+int wg_expect_plan_set_real_coeffs(wg_expect_plan_t plan, const double* coeffs, wg_stream_t stream);
 int wg_expect_plan_info(wg_expect_plan_t plan, size_t* n_groups, size_t* n_terms);
 /* Forward and adjoint in one x-grouped pass.  Any output may be NULL:
  *   result[2]        E = sum_k c_k <psi|P_k|psi> (device, complex128);

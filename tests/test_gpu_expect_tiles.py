@@ -61,3 +61,44 @@ def test_tiles(cuda, oracle, n, T, patterns, real):
     assert abs(complex(*res.tolist()) - oracle.expectation(n, x, z, c2, psi)) <= BOUND
     assert np.max(np.abs(hp.cpu().numpy() - oracle.hpsi(n, x, z, c2, psi))) <= BOUND
     plan.close()
+
+
+@pytest.mark.parametrize("n,T,patterns", [(3, 1, 1), (12, 512, 60), (12, 513, 60), (13, 1, 1), (13, 3, 3), (14, 40, 40),
+                                          (15, 16, 16), (16, 12, 6), (16, 700, 300)])
+def test_few_terms_a_class_and_single_calls(cuda, oracle, n, T, patterns):
+    """Chunks whose pieces read the paired tile themselves; sums joined in one block up to
+    512 terms; one pair in the kernel's parameter or several in a table, with and without
+    outputs: the same bits."""
+    torch = cuda
+    from wolfgang_b200.expectation import ExpectationBatch, ExpectationPlan
+
+    rng = np.random.default_rng(zlib.crc32(repr(("calls", n, T, patterns)).encode()))
+    x, z = operator(rng, n, T, patterns)
+    c = rng.normal(size=T) / np.sqrt(T)
+    host = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+    host /= np.linalg.norm(host)
+    other = ExpectationPlan((4, x[:3] & np.uint64(15), z[:3] & np.uint64(15), c[:3].astype(np.complex128)))
+    for dtype in (np.complex128, np.complex64):
+        stored = host.astype(dtype)
+        psi, wide = torch.from_numpy(stored).cuda(), stored.astype(np.complex128)
+        plan = ExpectationPlan((n, x, z, np.zeros(T, np.complex128)))
+        plan.set_coefficients(torch.from_numpy(c).cuda())  # real ones as they are
+        res, ev, hp = plan.run(psi, terms=True, hpsi=True)
+        assert abs(complex(*res.tolist()) - oracle.expectation(n, x, z, c.astype(np.complex128), wide)) <= BOUND
+        assert np.max(np.abs(ev.cpu().numpy() - oracle.term_expectations(n, x, z, wide))) <= BOUND
+        assert np.max(np.abs(hp.cpu().numpy() - oracle.hpsi(n, x, z, c.astype(np.complex128), wide))) <= BOUND
+        assert plan.run(psi)[0].tolist() == res.tolist()
+        small = torch.from_numpy(stored[:16].copy()).cuda()
+        batch = ExpectationBatch([other, plan], [small, psi])
+        batch.run()
+        assert batch.values[1].tolist() == res.tolist()
+        assert torch.equal(batch.term_values[1][:T], ev) and torch.equal(batch.hpsi[1], hp)
+        one = ExpectationBatch([plan], [psi])
+        one.run()
+        assert one.values[0].tolist() == res.tolist() and torch.equal(one.hpsi[0], hp)
+        plan.set_coefficients(torch.from_numpy(c.astype(np.complex128)).cuda())
+        again = plan.run(psi, terms=True, hpsi=True)
+        assert again[0].tolist() == res.tolist() and torch.equal(again[2], hp)
+        for o in (batch, one, plan):
+            o.close()
+    other.close()

@@ -90,6 +90,7 @@ _SIGNATURES: dict[str, list] = {
     "wg_expect_plan_create": [_i, _sz, _sz, _vp, _vp, _vp, _pvp, _vp],
     "wg_expect_plan_destroy": [_vp],
     "wg_expect_plan_set_coeffs": [_vp, _vp, _vp],
+    "wg_expect_plan_set_real_coeffs": [_vp, _vp, _vp],
     "wg_expect_plan_info": [_vp, _psz, _psz],
     "wg_expect_plan_run": [_vp, _vp, _i, _vp, _vp, _vp, _vp],
     "wg_expectation": [_i, _sz, _sz, _vp, _vp, _vp, _vp, _i, ctypes.POINTER(_d), _vp],

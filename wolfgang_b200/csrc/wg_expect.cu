@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -49,6 +50,9 @@ namespace {
 using wgd::c128;
 
 constexpr int kThreads = 256;
+constexpr int kTotalThreads = 1024;      // of the block that sums up a pair
+constexpr uint64_t kJoinSums = 8192;     // partial sums
+constexpr size_t kJoinTerms = 512;       // and terms of a pair up to which that block also sums its terms
 constexpr int kTileBits = 12;            // amplitudes per tile: 2^12 at most
 constexpr int kTileMin = 9;              // and 2^9 at least (zeros above 2^n)
 constexpr int kTileMax = 1 << kTileBits;
@@ -106,13 +110,16 @@ struct PlanDev {
   uint32_t T, G, S, NP, NS;  // terms, groups, sub-groups, pieces, segments
   uint32_t tiles;            // 2^(n - m)
   uint32_t chunks, ranges;   // forward items: chunks of pieces x ranges of tiles
+  uint32_t splits;           // parts of the segments that an adjoint tile is split into
+  uint32_t joined;           // one block sums the partial sums of all terms and E
   const FwdPiece* piece;     // [NP]
   AdjSub* asub;              // [S]
   const SegDev* seg;         // [NS]
   const uint32_t* chunk;     // [chunks + 1] first piece of a chunk
+  const uint32_t* bounds;    // [splits + 1] segments of the splits
   const uint32_t* ty;        // [T] y mod 4 | flags
   const uint32_t* torig;     // [T] original index of sorted term
-  const double* coeffs;      // [2T] original-order coefficients
+  double* coeffs;            // [2T] original-order coefficients
   double* table;             // adjoint tables of the part of c_k (-i)^y that its y makes it
                              // (real where y is even)
   double* other;             // and of the other part (read where AdjSub::mixed)
@@ -123,8 +130,7 @@ struct wg_plan_host {
   int device;
   PlanDev dev;
   size_t n_groups = 0;
-  std::vector<uint32_t> bounds;  // segments of the adjoint's splits: splits + 1 bounds
-  wg::Scratch blob, coeffs, table, partial;
+  wg::Scratch mem;  // all of the above
 };
 
 }  // namespace
@@ -156,24 +162,29 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Device work tables of one batched launch (kernel parameter, by value).
+// One (operator, statevector) pair of a launch.
+struct PairDev {
+  PlanDev plan;
+  const void* psi;
+  double* evals;    // e_k outputs (original order); null where the plan joins its sums and nobody asked
+  double* result;   // E output or null
+  double* hpsi;     // H psi output or null
+  double2* part;    // splits x 2^n partial H psi, or null
+};
+
+// A launch over one or several pairs (kernel parameter).  A single pair travels in
+// the parameter itself: nothing to allocate, copy or free for a call.
 struct BatchDev {
-  const PlanDev* plans;       // [np]
+  const PairDev* pairs;       // [np], null for a single one
   const uint64_t* item_base;  // [np+1] forward items per pair
-  const uint64_t* term_base;  // [np+1] flat term offsets
+  const uint64_t* term_base;  // [np+1] flat term offsets (0 for pairs whose sums are joined)
   const uint64_t* tile_base;  // [np+1] adjoint items (0 for pairs without H psi): tiles x splits
   const uint64_t* amp_base;   // [np+1] amplitudes of the pairs whose adjoint is split
-  const uint32_t* splits;     // [np] parts of the segments an adjoint tile is split into
-  const uint32_t* split_at;   // [np] first entry of the pair's splits + 1 segment bounds
-  const uint32_t* bounds;
-  const void* const* psis;    // [np]
-  double* const* evals;       // [np] e_k outputs (original order)
-  double* const* results;     // [np] E outputs or null
-  double* const* hpsis;       // [np] H psi outputs or null
-  double2* const* parts;      // [np] splits x 2^n partial H psi, or null
-  unsigned long long* counters;  // [2] forward / adjoint work queues
+  unsigned long long* counters;  // [2] forward / adjoint work queues; null: an item for every CTA
   uint32_t np;
   uint64_t n_items, n_terms, n_tiles, n_amps;
+  PairDev one;
+  __device__ __forceinline__ const PairDev& pair(uint32_t p) const { return pairs ? pairs[p] : one; }
 };
 
 template <typename T>
@@ -186,6 +197,20 @@ __device__ __forceinline__ uint32_t upper_index(const T* base, uint32_t n, T v) 
     else hi = mid;
   }
   return lo;
+}
+
+// The pair that flat index v belongs to; v becomes the index within the pair.
+__device__ __forceinline__ uint32_t find_pair(const BatchDev& B, const uint64_t* base, uint64_t& v) {
+  if (!B.pairs) return 0;
+  const uint32_t p = upper_index<uint64_t>(base, B.np + 1, v);
+  v -= base[p];
+  return p;
+}
+
+__device__ __forceinline__ void copy_pair(PairDev& to, const PairDev& from) {
+  static_assert(sizeof(PairDev) % 8 == 0, "copied in 8-byte pieces");
+  if (threadIdx.x < sizeof(PairDev) / 8)
+    reinterpret_cast<uint64_t*>(&to)[threadIdx.x] = reinterpret_cast<const uint64_t*>(&from)[threadIdx.x];
 }
 
 // ------------------------------------------------------------- tiles
@@ -258,6 +283,7 @@ struct FwdShared {
   uint32_t seg_at[kChunkPieces + 1];
   uint32_t segs;
   unsigned long long item;
+  PairDev pair;
 };
 static_assert(sizeof(FwdShared) <= 227 * 1024, "shared memory of an SM");
 
@@ -351,20 +377,25 @@ __device__ __forceinline__ void forward_any(const Layout<M>& lay, const FwdPiece
 // busy (47 % products, 14 % the t's): four warps a scheduler (tile J takes half of
 // the registers) do not cover all of the chains' latency.
 template <typename Amp>
-__global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(BatchDev B) {
+__global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(const __grid_constant__ BatchDev B) {
   extern __shared__ __align__(16) unsigned char raw[];
   FwdShared& sh = *reinterpret_cast<FwdShared*>(raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  while (true) {
+  for (uint64_t turn = blockIdx.x;; turn += gridDim.x) {
     __syncthreads();
-    if (tid == 0) sh.item = atomicAdd(B.counters, 1ull);
-    __syncthreads();
-    const uint64_t item = sh.item;
+    uint64_t item = turn;
+    if (B.counters) {
+      if (tid == 0) sh.item = atomicAdd(B.counters, 1ull);
+      __syncthreads();
+      item = sh.item;
+    }
     if (item >= B.n_items) break;
-    const uint32_t p = upper_index<uint64_t>(B.item_base, B.np + 1, item);
-    const PlanDev& P = B.plans[p];
-    const void* psi = B.psis[p];
-    const uint32_t r = static_cast<uint32_t>(item - B.item_base[p]);
+    copy_pair(sh.pair, B.pair(find_pair(B, B.item_base, item)));
+    __syncthreads();
+    const PairDev& Q = sh.pair;
+    const PlanDev& P = Q.plan;
+    const void* psi = Q.psi;
+    const uint32_t r = static_cast<uint32_t>(item);
     // ranges outermost: the CTAs that run together meet the same tiles in L2
     const uint32_t range = r / P.chunks, chunk = r - range * P.chunks;
     const uint32_t piece0 = P.chunk[chunk], pieces = P.chunk[chunk + 1] - piece0;
@@ -492,43 +523,75 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(BatchDev
   }
 }
 
-// e_k from the ranges' partial sums (eight lanes a term, in a fixed order:
-// one thread took 17 us for 256 ranges), scaled by the pairing factor and
-// scattered to original term order; flat over every pair's terms.
-__global__ void __launch_bounds__(kThreads) expect_finish_terms_kernel(BatchDev B) {
-  const uint32_t lane = threadIdx.x & 7;
+// e_k from the sum over all pairs
+__device__ __forceinline__ double scaled(double s, uint32_t ty) {
+  const double e = ((ty & 3u) == 1 || (ty & 3u) == 2) ? -s : s;
+  return ty & (kDiagFlag | kTwiceFlag) ? e : 2.0 * e;
+}
+
+// e_k from the ranges' partial sums, scaled by the pairing factor, by eight lanes
+// in a fixed order (one thread took 17 us for 256 ranges); every lane gets it.
+__device__ __forceinline__ double term_value(const PlanDev& P, uint32_t k, uint32_t lane8) {
+  const double* part = P.partial + static_cast<uint64_t>(k) * P.ranges;
+  double s = 0.0;
+#pragma unroll 8
+  for (uint32_t c = lane8; c < P.ranges; c += 8) s += part[c];
+#pragma unroll
+  for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return scaled(s, P.ty[k]);
+}
+
+// The term values in original order; flat over the terms of the pairs whose sums
+// are not joined.
+__global__ void __launch_bounds__(kThreads) expect_finish_terms_kernel(const __grid_constant__ BatchDev B) {
+  const uint32_t lane8 = threadIdx.x & 7;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x / 8;
   const uint64_t first = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) / 8;
   for (uint64_t f0 = first; f0 - (threadIdx.x & 31) / 8 < B.n_terms; f0 += stride) {  // a warp leaves together
-    const uint64_t f = min(f0, B.n_terms - 1);
-    const uint32_t p = upper_index<uint64_t>(B.term_base, B.np + 1, f);
-    const PlanDev& P = B.plans[p];
-    const uint32_t k = static_cast<uint32_t>(f - B.term_base[p]);
-    const double* part = P.partial + static_cast<uint64_t>(k) * P.ranges;
-    double s = 0.0;
-    for (uint32_t c = lane; c < P.ranges; c += 8) s += part[c];
-#pragma unroll
-    for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane != 0 || f0 >= B.n_terms) continue;
-    const uint32_t ty = P.ty[k];
-    const double e = ((ty & 3u) == 1 || (ty & 3u) == 2) ? -s : s;
-    B.evals[p][P.torig[k]] = ty & (kDiagFlag | kTwiceFlag) ? e : 2.0 * e;
+    uint64_t k = min(f0, B.n_terms - 1);
+    const PairDev& Q = B.pair(find_pair(B, B.term_base, k));
+    const double e = term_value(Q.plan, static_cast<uint32_t>(k), lane8);
+    if (lane8 == 0 && f0 < B.n_terms) Q.evals[Q.plan.torig[k]] = e;
   }
 }
 
-// E_p = sum_k c_k e_k, one block per pair, tree reduction in a fixed order.
-__global__ void __launch_bounds__(kThreads) expect_total_kernel(BatchDev B) {
-  __shared__ double sre[kThreads / 32], sim[kThreads / 32];
+// E_p = sum_k c_k e_k, one block per pair, tree reduction in a fixed order; where
+// the plan says so, the term values too.
+__global__ void __launch_bounds__(kTotalThreads) expect_total_kernel(const __grid_constant__ BatchDev B) {
+  __shared__ double sre[kTotalThreads / 32], sim[kTotalThreads / 32];
   for (uint32_t p = blockIdx.x; p < B.np; p += gridDim.x) {
-    double* out = B.results[p];
-    if (!out) continue;
-    const PlanDev& P = B.plans[p];
-    const double* ev = B.evals[p];
+    const PairDev& Q = B.pair(p);
+    const PlanDev& P = Q.plan;
+    if (!Q.result && !P.joined) continue;
     double re = 0.0, im = 0.0;
-    for (uint32_t k = threadIdx.x; k < P.T; k += blockDim.x) {
-      re += P.coeffs[2 * k] * ev[k];
-      im += P.coeffs[2 * k + 1] * ev[k];
+    if (P.joined && P.ranges < 8) {
+      for (uint32_t k = threadIdx.x; k < P.T; k += kTotalThreads) {
+        double s = 0.0;
+        for (uint32_t c = 0; c < P.ranges; ++c) s += P.partial[static_cast<uint64_t>(k) * P.ranges + c];
+        const double e = scaled(s, P.ty[k]);
+        const uint32_t o = P.torig[k];
+        if (Q.evals) Q.evals[o] = e;
+        re += P.coeffs[2 * o] * e;
+        im += P.coeffs[2 * o + 1] * e;
+      }
+    } else if (P.joined) {
+      const uint32_t lane8 = threadIdx.x & 7;
+      for (uint32_t k0 = threadIdx.x / 8; k0 - (threadIdx.x & 31) / 8 < P.T; k0 += kTotalThreads / 8) {
+        const uint32_t k = min(k0, P.T - 1);
+        const double e = term_value(P, k, lane8);
+        if (lane8 != 0 || k0 >= P.T) continue;
+        const uint32_t o = P.torig[k];
+        if (Q.evals) Q.evals[o] = e;
+        re += P.coeffs[2 * o] * e;
+        im += P.coeffs[2 * o + 1] * e;
+      }
+    } else {
+      for (uint32_t k = threadIdx.x; k < P.T; k += kTotalThreads) {
+        re += P.coeffs[2 * k] * Q.evals[k];
+        im += P.coeffs[2 * k + 1] * Q.evals[k];
+      }
     }
+    __syncwarp();
     re = warp_sum(re);
     im = warp_sum(im);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -538,13 +601,13 @@ __global__ void __launch_bounds__(kThreads) expect_total_kernel(BatchDev B) {
     }
     __syncthreads();
     if (warp == 0) {
-      re = lane < kThreads / 32 ? sre[lane] : 0.0;
-      im = lane < kThreads / 32 ? sim[lane] : 0.0;
+      re = lane < kTotalThreads / 32 ? sre[lane] : 0.0;
+      im = lane < kTotalThreads / 32 ? sim[lane] : 0.0;
       re = warp_sum(re);
       im = warp_sum(im);
-      if (lane == 0) {
-        out[0] = re;
-        out[1] = im;
+      if (lane == 0 && Q.result) {
+        Q.result[0] = re;
+        Q.result[1] = im;
       }
     }
     __syncthreads();
@@ -562,6 +625,7 @@ struct AdjShared {
   double2 tile[2][kTileMax];
   AdjStage stage[2];
   unsigned long long item;
+  PairDev pair;
 };
 static_assert(sizeof(AdjShared) <= 227 * 1024, "shared memory of an SM");
 
@@ -629,25 +693,29 @@ __device__ __forceinline__ void adjoint_sub(const Layout<M>& lay, const AdjSub& 
 // table): 44 ms on 24 qubits with 20,000 terms (80 ms with tables of complex
 // entries and psi read through L1).
 template <typename Amp>
-__global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(BatchDev B) {
+__global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(const __grid_constant__ BatchDev B) {
   extern __shared__ __align__(16) unsigned char raw[];
   AdjShared& sh = *reinterpret_cast<AdjShared*>(raw);
   const int tid = threadIdx.x, lane = tid & 31;
   constexpr bool kWide = TileBuffers<Amp>::kWide;
-  while (true) {
+  for (uint64_t turn = blockIdx.x;; turn += gridDim.x) {
     __syncthreads();
-    if (tid == 0) sh.item = atomicAdd(B.counters + 1, 1ull);
-    __syncthreads();
-    const uint64_t item = sh.item;
+    uint64_t item = turn;
+    if (B.counters) {
+      if (tid == 0) sh.item = atomicAdd(B.counters + 1, 1ull);
+      __syncthreads();
+      item = sh.item;
+    }
     if (item >= B.n_tiles) break;
-    const uint32_t p = upper_index<uint64_t>(B.tile_base, B.np + 1, item);
-    const PlanDev& P = B.plans[p];
-    const void* psi = B.psis[p];
-    const uint32_t splits = B.splits[p];
-    const uint64_t rest = item - B.tile_base[p];
+    copy_pair(sh.pair, B.pair(find_pair(B, B.tile_base, item)));
+    __syncthreads();
+    const PairDev& Q = sh.pair;
+    const PlanDev& P = Q.plan;
+    const void* psi = Q.psi;
+    const uint32_t splits = P.splits;
     // tiles outermost: the CTAs that run together share tiles and segments
-    const uint32_t J = static_cast<uint32_t>(rest / splits), split = static_cast<uint32_t>(rest - static_cast<uint64_t>(J) * splits);
-    const uint32_t g0 = B.bounds[B.split_at[p] + split], g1 = B.bounds[B.split_at[p] + split + 1];
+    const uint32_t J = static_cast<uint32_t>(item / splits), split = static_cast<uint32_t>(item - static_cast<uint64_t>(J) * splits);
+    const uint32_t g0 = P.bounds[split], g1 = P.bounds[split + 1];
     const int m = P.m, n = P.n;
     const int tt = tid & ((1 << (m - 3)) - 1);
     const uint32_t slice = tid >> (m - 3), slices = kAdjThreads >> (m - 3);
@@ -726,7 +794,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(BatchDev
       }
     }
     if (slice == 0) {
-      double2* out = splits > 1 ? B.parts[p] + (static_cast<uint64_t>(split) << n) : reinterpret_cast<double2*>(B.hpsis[p]);
+      double2* out = splits > 1 ? Q.part + (static_cast<uint64_t>(split) << n) : reinterpret_cast<double2*>(Q.hpsi);
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const uint64_t j = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(r) << (m - 3));
@@ -737,21 +805,22 @@ __global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(BatchDev
 }
 
 // H psi of the pairs whose segments were split, summed over the splits in order.
-__global__ void __launch_bounds__(kThreads) expect_join_kernel(BatchDev B) {
+__global__ void __launch_bounds__(kThreads) expect_join_kernel(const __grid_constant__ BatchDev B) {
   for (uint64_t f = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; f < B.n_amps;
        f += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-    const uint32_t p = upper_index<uint64_t>(B.amp_base, B.np + 1, f);
-    const uint64_t j = f - B.amp_base[p];
-    const double2* part = B.parts[p] + j;
-    const uint32_t splits = B.splits[p];
-    const int n = B.plans[p].n;
+    uint64_t j = f;
+    const PairDev& Q = B.pair(find_pair(B, B.amp_base, j));
+    const double2* part = Q.part + j;
+    const uint32_t splits = Q.plan.splits;
+    const int n = Q.plan.n;
     double2 s = part[0];
+#pragma unroll 8
     for (uint32_t k = 1; k < splits; ++k) {
       const double2 v = part[static_cast<uint64_t>(k) << n];
       s.x += v.x;
       s.y += v.y;
     }
-    reinterpret_cast<double2*>(B.hpsis[p])[j] = s;
+    reinterpret_cast<double2*>(Q.hpsi)[j] = s;
   }
 }
 
@@ -760,8 +829,9 @@ __global__ void __launch_bounds__(kThreads) expect_join_kernel(BatchDev B) {
 // The adjoint's tables from the coefficients, a warp per sub-group: entry q of
 // a piece is the sum of its terms' c_k (-i)^y_k (i^y, and (-1)^y for the signs,
 // which are those at j where the adjoint needs them at j ^ x), with the sign of
-// bit kk of q, in order.
-__global__ void plan_tables_kernel(PlanDev P) {
+// bit kk of q, in order.  The coefficients come from `from` (original order,
+// `reals` doubles each) and go to the plan too: every term lies in one sub-group.
+__global__ void plan_tables_kernel(PlanDev P, const double* __restrict__ from, int reals) {
   const uint32_t lane = threadIdx.x & 31;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < P.S; i += (gridDim.x * blockDim.x) >> 5) {
     AdjSub& sd = P.asub[i];
@@ -769,7 +839,11 @@ __global__ void plan_tables_kernel(PlanDev P) {
     double own = 0.0, other = 0.0;
     if (lane < static_cast<uint32_t>(sd.nre) + sd.nim) {
       const uint32_t k = sd.t0 + lane, o = P.torig[k];
-      const c128 d = wgd::rotate(c128{P.coeffs[2 * o], P.coeffs[2 * o + 1]}, (4u - (P.ty[k] & 3u)) & 3u);
+      const c128 c = reals == 2 ? c128{from[2 * static_cast<size_t>(o)], from[2 * static_cast<size_t>(o) + 1]}
+                                : c128{from[o], 0.0};
+      P.coeffs[2 * static_cast<size_t>(o)] = c.re;
+      P.coeffs[2 * static_cast<size_t>(o) + 1] = c.im;
+      const c128 d = wgd::rotate(c, (4u - (P.ty[k] & 3u)) & 3u);
       const bool odd = P.ty[k] & 1u;
       own = odd ? d.im : d.re;
       other = odd ? d.re : d.im;
@@ -798,10 +872,11 @@ __global__ void plan_tables_kernel(PlanDev P) {
   }
 }
 
-void refresh_coeffs(const wg_plan_host& h, cudaStream_t s) {
+void refresh_coeffs(const wg_plan_host& h, const double* from, int reals, cudaStream_t s) {
   const PlanDev& P = h.dev;
   if (P.T == 0) return;
-  plan_tables_kernel<<<wg::grid_for(32 * static_cast<size_t>(P.S), kThreads, h.device, 8), kThreads, 0, s>>>(P);
+  plan_tables_kernel<<<wg::grid_for(32 * static_cast<size_t>(P.S), kThreads, h.device, 8), kThreads, 0, s>>>(P, from,
+                                                                                                             reals);
   wg::check_launch("launch adjoint tables");
 }
 
@@ -817,8 +892,10 @@ struct Blob {
   }
 };
 
+// adjoint = false: for E alone, on this stream only (no sub-groups, segments or
+// tables, no wait).
 wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const uint64_t* z, const double* c,
-                        cudaStream_t s) {
+                        bool adjoint, cudaStream_t s) {
   if (n > 63) wg::throw_invalid("expectation_statevector requires num_qubits <= 63");
   if (T > 0xffffffffull) wg::throw_invalid("expectation supports at most 2^32-1 terms");
   std::unique_ptr<wg_plan_host> p(new wg_plan_host());
@@ -829,14 +906,7 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   d.T = static_cast<uint32_t>(T);
   d.m = std::max(kTileMin, std::min(static_cast<int>(n), kTileBits));
   d.tiles = static_cast<int>(n) > d.m ? 1u << std::min<int>(31, static_cast<int>(n) - d.m) : 1u;
-  p->coeffs.reset(std::max<size_t>(16, 16 * T), s);
-  if (T) wg::check_cuda(cudaMemcpyAsync(p->coeffs.get(), c, 16 * T, cudaMemcpyDeviceToDevice, s), "copy coefficients");
-  d.coeffs = p->coeffs.as<double>();
-  if (T == 0) {
-    wg::check_cuda(cudaStreamSynchronize(s), "build plan");
-    p->coeffs.rebind(nullptr);
-    return p.release();
-  }
+  if (T == 0) return p.release();
   // masks to the host; the plan's tables are built there
   const int words = n == 0 ? 0 : 1;
   std::vector<uint64_t> hx(T, 0), hz(T, 0);
@@ -856,7 +926,7 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   std::iota(order.begin(), order.end(), 0u);
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return hx[a] < hx[b]; });
   const int m = d.m;
-  std::vector<uint32_t> ty(T), torig(T), seg_cost, chunk{0};
+  std::vector<uint32_t> ty(T), torig(T), seg_cost, chunk{0}, bounds;
   std::vector<FwdPiece> piece;
   std::vector<AdjSub> asub;
   std::vector<SegDev> seg;
@@ -919,12 +989,13 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
                    (gx == 0 ? kDiagFlag : (gx >> m) == 0 ? kTwiceFlag : 0u);
           pd.zlo[kk] = static_cast<uint32_t>(hz[o] & ((uint64_t{1} << m) - 1));
           pd.zhi[kk] = ad.zhi[half * kPiece + kk] = static_cast<uint32_t>(hz[o] >> m);
-          for (int q = 0; q < m; ++q) plane[q] |= static_cast<uint32_t>((hz[o] >> q) & 1u) << (3 + 16 * half + kk);
+          for (int q = 0; adjoint && q < m; ++q) plane[q] |= static_cast<uint32_t>((hz[o] >> q) & 1u) << (3 + 16 * half + kk);
         }
         if (nk) piece.push_back(pd);
         entries += uint64_t{1} << nk;
       }
       entries += entries & 1u;  // staged in 16-byte pieces
+      if (!adjoint) continue;
       for (int q = 0; q < 5; ++q)
         for (int l = 0; l < (1 << q); ++l) ad.lane[l | 1 << q] = ad.lane[l] ^ plane[q];
       for (int q = 5; q < m - 3; ++q)
@@ -946,7 +1017,7 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   const size_t slices = static_cast<size_t>(kTileMax) >> m;
   const size_t seg_subs = std::min<size_t>(
       kSegSubs, std::max<size_t>(slices, (S * d.tiles + 2 * sms - 1) / (2 * sms)));
-  for (size_t i = 0; i < S;) {
+  for (size_t i = 0; i < S;) {  // none without the adjoint
     size_t e = i + 1;
     while (e < S && e - i < seg_subs && xhi_of(e) == xhi_of(i) && tab_end(e) - asub[i].tab <= kSegEntries) ++e;
     // work of a segment, in hundredths of a tile's fetch: the tile, and its
@@ -961,18 +1032,19 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   // The adjoint's tiles are split by segments until there are about four items
   // an SM.  The plan alone sets the splits, so that a pair's H psi has the same
   // bits in every batch.
-  {
+  if (adjoint) {
     const size_t NS = seg.size();
     const size_t splits = std::max<size_t>(1, std::min<size_t>({(4 * sms + d.tiles / 2) / d.tiles, NS, 64}));
-    p->bounds.push_back(0);
+    bounds.push_back(0);
     for (size_t k = 1; k < splits; ++k) {
       // the segment at which k / splits of the work is done; each split takes one at least
       const uint32_t to = static_cast<uint32_t>(static_cast<uint64_t>(seg_cost.back()) * k / splits);
       size_t at = static_cast<size_t>(std::lower_bound(seg_cost.begin(), seg_cost.end(), to) - seg_cost.begin()) + 1;
-      at = std::min(std::max<size_t>(at, p->bounds.back() + 1), NS - (splits - k));
-      p->bounds.push_back(static_cast<uint32_t>(at));
+      at = std::min(std::max<size_t>(at, bounds.back() + 1), NS - (splits - k));
+      bounds.push_back(static_cast<uint32_t>(at));
     }
-    p->bounds.push_back(static_cast<uint32_t>(NS));
+    bounds.push_back(static_cast<uint32_t>(NS));
+    d.splits = static_cast<uint32_t>(splits);
   }
   // Forward items: chunks of pieces (their sums stay in shared memory) times
   // ranges of tiles; about eight items an SM where there is the work.
@@ -1014,30 +1086,38 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   d.NS = static_cast<uint32_t>(seg.size());
   d.G = static_cast<uint32_t>(groups);
   p->n_groups = groups;
+  d.joined = T <= kJoinTerms && static_cast<uint64_t>(T) * d.ranges <= kJoinSums;
   Blob blob;
   const size_t o_piece = blob.put(piece), o_asub = blob.put(asub), o_seg = blob.put(seg), o_chunk = blob.put(chunk),
-               o_ty = blob.put(ty), o_torig = blob.put(torig);
-  p->blob.reset(blob.bytes.size(), s);
-  wg::check_cuda(cudaMemcpyAsync(p->blob.get(), blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice, s),
+               o_bounds = blob.put(bounds), o_ty = blob.put(ty), o_torig = blob.put(torig);
+  const size_t o_coeffs = (blob.bytes.size() + 15) & ~size_t{15}, o_partial = o_coeffs + 16 * T;
+  const size_t o_table = (o_partial + 8 * static_cast<uint64_t>(T) * d.ranges + 15) & ~size_t{15};
+  p->mem.reset(o_table + (adjoint ? 16 * entries : 0), s);
+  wg::check_cuda(cudaMemcpyAsync(p->mem.get(), blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice, s),
                  "upload plan");
-  auto* base = static_cast<unsigned char*>(p->blob.get());
+  auto* base = static_cast<unsigned char*>(p->mem.get());
   d.piece = reinterpret_cast<const FwdPiece*>(base + o_piece);
   d.asub = reinterpret_cast<AdjSub*>(base + o_asub);
   d.seg = reinterpret_cast<const SegDev*>(base + o_seg);
   d.chunk = reinterpret_cast<const uint32_t*>(base + o_chunk);
+  d.bounds = reinterpret_cast<const uint32_t*>(base + o_bounds);
   d.ty = reinterpret_cast<const uint32_t*>(base + o_ty);
   d.torig = reinterpret_cast<const uint32_t*>(base + o_torig);
-  p->table.reset(16 * entries, s);
-  p->partial.reset(8 * static_cast<uint64_t>(T) * d.ranges, s);
-  d.table = p->table.as<double>();
+  d.coeffs = reinterpret_cast<double*>(base + o_coeffs);
+  d.partial = reinterpret_cast<double*>(base + o_partial);
+  d.table = reinterpret_cast<double*>(base + o_table);
   d.other = d.table + entries;
-  d.partial = p->partial.as<double>();
-  refresh_coeffs(*p, s);
+  if (!adjoint) {
+    // the caller's coefficients outlive the call; the upload's source is staged
+    d.coeffs = const_cast<double*>(c);
+    return p.release();
+  }
+  refresh_coeffs(*p, c, 2, s);
   // pageable source above: wait until the plan image is on the device
   wg::check_cuda(cudaStreamSynchronize(s), "build plan");
-  // The plan outlives the caller's stream: release its buffers on the legacy
+  // The plan outlives the caller's stream: release its memory on the legacy
   // default stream.
-  for (wg::Scratch* b : {&p->blob, &p->coeffs, &p->table, &p->partial}) b->rebind(nullptr);
+  p->mem.rebind(nullptr);
   return p.release();
 }
 
@@ -1059,17 +1139,28 @@ struct wg_expect_batch_s {
   int dtype = WG_DTYPE_C128;
   int sms = 0;
   BatchDev dev{};
-  wg::Scratch table;
-  wg::Scratch parts;  // partial H psi of the pairs whose adjoint is split
-  std::vector<wg::Scratch> evtmp;
+  wg::Scratch table;  // the pairs and the work queues
+  wg::Scratch parts;  // partial H psi of the pairs whose adjoint is split, term values that nobody asked for
 };
 
 namespace {
 
-template <class K>
-void allow_smem(K kernel, size_t bytes) {
-  wg::check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
-                 "set expectation shared memory");
+constexpr int kMaxDevices = 64;
+
+// The kernels' shared memory, set once per device.
+void allow_smem(int device) {
+  static std::once_flag done[kMaxDevices];
+  if (device < 0 || device >= kMaxDevices) wg::throw_invalid("CUDA device ordinal is out of range");
+  std::call_once(done[device], [] {  // a throw leaves the flag unset: the next call retries
+    auto allow = [](auto* kernel, size_t bytes) {
+      wg::check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+                     "set expectation shared memory");
+    };
+    allow(expect_forward_kernel<double2>, sizeof(FwdShared));
+    allow(expect_forward_kernel<float2>, sizeof(FwdShared));
+    allow(expect_adjoint_kernel<double2>, sizeof(AdjShared));
+    allow(expect_adjoint_kernel<float2>, sizeof(AdjShared));
+  });
 }
 
 wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int dtype, cudaStream_t s) {
@@ -1078,65 +1169,56 @@ wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int
   b->device = device;
   b->dtype = dtype;
   b->sms = wg::device_props(device).sm_count;
-  if (dtype == WG_DTYPE_C128) {
-    allow_smem(expect_forward_kernel<double2>, sizeof(FwdShared));
-    allow_smem(expect_adjoint_kernel<double2>, sizeof(AdjShared));
-  } else {
-    allow_smem(expect_forward_kernel<float2>, sizeof(FwdShared));
-    allow_smem(expect_adjoint_kernel<float2>, sizeof(AdjShared));
-  }
+  allow_smem(device);
   const size_t np = specs.size();
   if (np > 0xffffffffull) wg::throw_invalid("too many pairs in one batch");
-  std::vector<PlanDev> plans(np);
+  std::vector<PairDev> pairs(np);
   std::vector<uint64_t> item_base(np + 1, 0), term_base(np + 1, 0), tile_base(np + 1, 0), amp_base(np + 1, 0);
-  std::vector<uint32_t> splits(np, 1), split_at(np, 0), bounds;
-  std::vector<uint64_t> part_at(np, 0);
-  std::vector<const void*> psis(np);
-  std::vector<double*> evals(np), results(np), hpsis(np);
-  std::vector<double2*> parts(np, nullptr);
-  b->evtmp.resize(np);
-  uint64_t part_amps = 0;
+  uint64_t bytes = 0;  // of the partial H psi and the term values, then where they lie
+  std::vector<uint64_t> part_at(np, 0), ev_at(np, 0);
   for (size_t i = 0; i < np; ++i) {
     const PlanDev& P = specs[i].plan->dev;
     // tile numbers are 32 bits; no device holds a larger state
     if (P.n > kTileBits + 31) wg::throw_invalid("expectation_statevector: the statevector exceeds device memory");
-    plans[i] = P;
-    psis[i] = specs[i].psi;
+    pairs[i] = PairDev{P, specs[i].psi, specs[i].term_values, specs[i].result, specs[i].hpsi, nullptr};
     item_base[i + 1] = item_base[i] + (P.T ? static_cast<uint64_t>(P.chunks) * P.ranges : 0);
-    term_base[i + 1] = term_base[i] + P.T;
-    const bool adj = specs[i].hpsi != nullptr && P.T != 0;
+    term_base[i + 1] = term_base[i] + (P.joined ? 0 : P.T);
     tile_base[i + 1] = tile_base[i];
     amp_base[i + 1] = amp_base[i];
-    if (adj) {
-      const auto& own = specs[i].plan->bounds;
-      splits[i] = static_cast<uint32_t>(own.size() - 1);
-      split_at[i] = static_cast<uint32_t>(bounds.size());
-      bounds.insert(bounds.end(), own.begin(), own.end());
-      tile_base[i + 1] += static_cast<uint64_t>(P.tiles) * splits[i];
-      if (splits[i] > 1) {
+    if (specs[i].hpsi && P.T) {
+      tile_base[i + 1] += static_cast<uint64_t>(P.tiles) * P.splits;
+      if (P.splits > 1) {
         amp_base[i + 1] += uint64_t{1} << P.n;
-        part_at[i] = part_amps;
-        part_amps += static_cast<uint64_t>(splits[i]) << P.n;
+        part_at[i] = bytes;
+        bytes += static_cast<uint64_t>(P.splits) << (P.n + 4);
       }
     }
-    if (specs[i].term_values) {
-      evals[i] = specs[i].term_values;
-    } else {
-      b->evtmp[i].reset(8 * std::max<uint32_t>(1, P.T), s);
-      b->evtmp[i].rebind(nullptr);
-      evals[i] = b->evtmp[i].as<double>();
+    if (!specs[i].term_values && !P.joined && P.T) {
+      ev_at[i] = bytes;
+      bytes += (8 * static_cast<uint64_t>(P.T) + 15) & ~uint64_t{15};
     }
-    results[i] = specs[i].result;
-    hpsis[i] = specs[i].hpsi;
   }
-  if (part_amps) {
-    b->parts.reset(16 * part_amps, s);
+  if (bytes) {
+    b->parts.reset(bytes, s);
     b->parts.rebind(nullptr);
-    for (size_t i = 0; i < np; ++i)
-      if (splits[i] > 1) parts[i] = b->parts.as<double2>() + part_at[i];
+    auto* base = b->parts.as<unsigned char>();
+    for (size_t i = 0; i < np; ++i) {
+      const PlanDev& P = pairs[i].plan;
+      if (pairs[i].hpsi && P.T && P.splits > 1) pairs[i].part = reinterpret_cast<double2*>(base + part_at[i]);
+      if (!pairs[i].evals && !P.joined && P.T) pairs[i].evals = reinterpret_cast<double*>(base + ev_at[i]);
+    }
   }
-  if (bounds.empty()) bounds.push_back(0);
-  // one device block, 8-byte pieces first
+  BatchDev& d = b->dev;
+  d.np = static_cast<uint32_t>(np);
+  d.n_items = item_base[np];
+  d.n_terms = term_base[np];
+  d.n_tiles = tile_base[np];
+  d.n_amps = amp_base[np];
+  // A queue where some CTA takes several items: which side of a pairing a tile is
+  // on makes them uneven (21 qubits, 16 terms: 112 us taking turns, 60 queued).
+  const bool queue = np > 1 || std::max(d.n_items, d.n_tiles) > static_cast<uint64_t>(b->sms);
+  if (np == 1) d.one = pairs[0];
+  if (!queue) return b.release();
   std::vector<unsigned char> host;
   auto put = [&](const void* src, size_t n) {
     const size_t at = (host.size() + 15) & ~size_t{15};
@@ -1145,46 +1227,28 @@ wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int
     return at;
   };
   const unsigned long long zero[2] = {0, 0};
-  const size_t o_plans = put(plans.data(), sizeof(PlanDev) * np);
-  const size_t o_item = put(item_base.data(), 8 * (np + 1));
-  const size_t o_term = put(term_base.data(), 8 * (np + 1));
-  const size_t o_tile = put(tile_base.data(), 8 * (np + 1));
-  const size_t o_amp = put(amp_base.data(), 8 * (np + 1));
-  const size_t o_splits = put(splits.data(), 4 * np);
-  const size_t o_at = put(split_at.data(), 4 * np);
-  const size_t o_bounds = put(bounds.data(), 4 * bounds.size());
-  const size_t o_psis = put(psis.data(), 8 * np);
-  const size_t o_evals = put(evals.data(), 8 * np);
-  const size_t o_res = put(results.data(), 8 * np);
-  const size_t o_hpsi = put(hpsis.data(), 8 * np);
-  const size_t o_parts = put(parts.data(), 8 * np);
   const size_t o_cnt = put(zero, sizeof(zero));
+  size_t o_pairs = 0, o_item = 0, o_term = 0, o_tile = 0, o_amp = 0;
+  if (np > 1) {
+    o_pairs = put(pairs.data(), sizeof(PairDev) * np);
+    o_item = put(item_base.data(), 8 * (np + 1));
+    o_term = put(term_base.data(), 8 * (np + 1));
+    o_tile = put(tile_base.data(), 8 * (np + 1));
+    o_amp = put(amp_base.data(), 8 * (np + 1));
+  }
   b->table.reset(host.size(), s);
   b->table.rebind(nullptr);
+  auto* base = static_cast<unsigned char*>(b->table.get());
+  d.counters = reinterpret_cast<unsigned long long*>(base + o_cnt);
+  if (np == 1) return b.release();
   // pageable source: the call returns once the bytes are staged
   wg::check_cuda(cudaMemcpyAsync(b->table.get(), host.data(), host.size(), cudaMemcpyHostToDevice, s),
                  "upload work table");
-  auto* base = static_cast<unsigned char*>(b->table.get());
-  BatchDev& d = b->dev;
-  d.plans = reinterpret_cast<const PlanDev*>(base + o_plans);
+  d.pairs = reinterpret_cast<const PairDev*>(base + o_pairs);
   d.item_base = reinterpret_cast<const uint64_t*>(base + o_item);
   d.term_base = reinterpret_cast<const uint64_t*>(base + o_term);
   d.tile_base = reinterpret_cast<const uint64_t*>(base + o_tile);
   d.amp_base = reinterpret_cast<const uint64_t*>(base + o_amp);
-  d.splits = reinterpret_cast<const uint32_t*>(base + o_splits);
-  d.split_at = reinterpret_cast<const uint32_t*>(base + o_at);
-  d.bounds = reinterpret_cast<const uint32_t*>(base + o_bounds);
-  d.psis = reinterpret_cast<const void* const*>(base + o_psis);
-  d.evals = reinterpret_cast<double* const*>(base + o_evals);
-  d.results = reinterpret_cast<double* const*>(base + o_res);
-  d.hpsis = reinterpret_cast<double* const*>(base + o_hpsi);
-  d.parts = reinterpret_cast<double2* const*>(base + o_parts);
-  d.counters = reinterpret_cast<unsigned long long*>(base + o_cnt);
-  d.np = static_cast<uint32_t>(np);
-  d.n_items = item_base[np];
-  d.n_terms = term_base[np];
-  d.n_tiles = tile_base[np];
-  d.n_amps = amp_base[np];
   return b.release();
 }
 
@@ -1192,7 +1256,7 @@ wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int
 void run_batch(const wg_expect_batch_s& b, cudaStream_t s) {
   const BatchDev& d = b.dev;
   if (d.np == 0) return;
-  wg::check_cuda(cudaMemsetAsync(d.counters, 0, 16, s), "reset work queues");
+  if (d.counters) wg::check_cuda(cudaMemsetAsync(d.counters, 0, 16, s), "reset work queues");
   const unsigned persistent = static_cast<unsigned>(b.sms);  // one CTA an SM: its tiles fill the shared memory
   if (d.n_items) {
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(d.n_items, persistent));
@@ -1208,7 +1272,7 @@ void run_batch(const wg_expect_batch_s& b, cudaStream_t s) {
     wg::check_launch("launch expectation finish");
   }
   WG_TIMED("expect_total_kernel", s,
-           expect_total_kernel<<<std::min<uint32_t>(d.np, 65535u), kThreads, 0, s>>>(d));
+           expect_total_kernel<<<std::min<uint32_t>(d.np, 65535u), kTotalThreads, 0, s>>>(d));
   wg::check_launch("launch expectation total");
   if (d.n_tiles) {
     const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(d.n_tiles, persistent));
@@ -1239,7 +1303,6 @@ void run_specs(int device, const std::vector<RunSpec>& specs, int dtype, cudaStr
   // stream-ordered release after the kernels that read the tables
   b->table.rebind(s);
   b->parts.rebind(s);
-  for (auto& e : b->evtmp) e.rebind(s);
 }
 
 std::vector<RunSpec> batch_specs(int device, size_t n_pairs, const wg_expect_plan_t* plans, const void* const* psis,
@@ -1267,7 +1330,7 @@ int wg_expect_plan_create(int device, size_t n_qubits, size_t n_terms, const uin
     *plan = nullptr;
     if (n_qubits > 63) wg::throw_invalid("expectation_statevector requires num_qubits <= 63");
     wg::DeviceGuard g(device);
-    std::unique_ptr<wg_plan_host> p(make_plan(device, n_qubits, n_terms, x, z, coeffs, stream));
+    std::unique_ptr<wg_plan_host> p(make_plan(device, n_qubits, n_terms, x, z, coeffs, true, stream));
     *plan = reinterpret_cast<wg_expect_plan_t>(new wg_expect_plan_s{std::move(*p)});
   });
 }
@@ -1284,11 +1347,15 @@ int wg_expect_plan_set_coeffs(wg_expect_plan_t plan, const double* coeffs, wg_st
   return wg::guarded([&] {
     if (!plan) wg::throw_invalid("expectation plan is null");
     wg::DeviceGuard g(plan->h.device);
-    const PlanDev& P = plan->h.dev;
-    if (P.T == 0) return;
-    wg::check_cuda(cudaMemcpyAsync(plan->h.coeffs.get(), coeffs, 16ull * P.T, cudaMemcpyDeviceToDevice, stream),
-                   "copy coefficients");
-    refresh_coeffs(plan->h, stream);
+    refresh_coeffs(plan->h, coeffs, 2, stream);
+  });
+}
+
+int wg_expect_plan_set_real_coeffs(wg_expect_plan_t plan, const double* coeffs, wg_stream_t stream) {
+  return wg::guarded([&] {
+    if (!plan) wg::throw_invalid("expectation plan is null");
+    wg::DeviceGuard g(plan->h.device);
+    refresh_coeffs(plan->h, coeffs, 1, stream);
   });
 }
 
@@ -1321,7 +1388,7 @@ int wg_expectation(int device, size_t n_qubits, size_t n_terms, const uint64_t* 
     if (!psi) wg::throw_invalid("CUDA statevector data pointer must be non-null");
     wg::DeviceGuard g(device);
     cudaStream_t s = stream;
-    std::unique_ptr<wg_plan_host> p(make_plan(device, n_qubits, n_terms, x, z, coeffs, s));
+    std::unique_ptr<wg_plan_host> p(make_plan(device, n_qubits, n_terms, x, z, coeffs, false, s));
     wg::Scratch res(16, s);
     run_specs(device, {RunSpec{p.get(), psi, res.as<double>(), nullptr, nullptr}}, psi_dtype, s);
     wg::check_cuda(cudaMemcpyAsync(result_host, res.get(), 16, cudaMemcpyDeviceToHost, s), "read expectation");

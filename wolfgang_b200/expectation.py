@@ -100,10 +100,14 @@ class ExpectationPlan:
 
     def set_coefficients(self, coeffs: torch.Tensor) -> None:
         """Replace the coefficients (same terms, original order) in place."""
-        c = coeffs.to(device=f"cuda:{self.device}", dtype=torch.complex128).contiguous()
+        # float64 coefficients go in as they are
+        real = coeffs.dtype == torch.float64
+        c = coeffs.to(device=f"cuda:{self.device}", dtype=torch.float64 if real else torch.complex128)
+        c = c.resolve_neg().resolve_conj().contiguous()
         if c.numel() != self.T:
             raise ValueError("coefficient count must match the plan's term count")
-        capi.call("wg_expect_plan_set_coeffs", self.handle, c.data_ptr(), _stream())
+        capi.call("wg_expect_plan_set_real_coeffs" if real else "wg_expect_plan_set_coeffs", self.handle, c.data_ptr(),
+                  _stream())
         self._coeff_tensor = c  # keep alive until the copy has run
 
     def run(self, psi: torch.Tensor, terms: bool = False, hpsi: bool = False):
