@@ -384,17 +384,14 @@ def bench_products(args, world, rank, torch) -> dict:
     U = U_last[0]
 
     # roofline: algorithmic bytes per launch of each kernel (the bytes a launch
-    # must move at minimum): keys are 2W words + a 4-byte index per item.
-    rec = 8 * 2 * W + 4
+    # must move at minimum): an item is an 8-byte key code and a 4-byte product
+    # index; operand gathers hit L2 and are not counted.
     per_launch = {
-        "products_kernel": P * (rec + 16),                    # write keys+index+coefficient
-        "radix_scatter_kernel": P * 2 * rec,                  # read + write keys and index
-        "radix_hist_kernel": P * 8,                           # read one key word
-        "seg_head_kernel": P * (8 * 2 * W + 4),               # read keys, write flag
-        "seg_reduce_kernel": P * (4 + 16) + U * 20,           # idx + gathered coefficient, sums
-        "write_out_kernel": U * (8 * 2 * W + 16),
-        # bucketed path: an item is a 4-byte product index; codes are 8 bytes;
-        # operand gathers hit L2 and are not counted
+        "code_kernel": P * 8,                                  # write the codes
+        "radix_pass_kernel": P * 2 * 12,                       # codes and indices in and out
+        "reduce_kernel": P * 12 + U * (4 + 16),                # codes and indices in; survivors' index and sum out
+        "write_kernel": U * (4 + 16) + U * (8 * 2 * W + 16),   # survivors in, the U terms out
+        # --sort bucket
         "bucket_coarse_kernel": P * 4,                         # write the item index
         "bucket_fine_kernel": P * (4 + 8 + 4),                 # idx in, code + idx out (one pass)
         "bucket_final_kernel": P * (8 + 4) + U * (4 + 16),     # code + idx in; survivors' idx + sum out
@@ -877,8 +874,8 @@ def bench_products_batch(args, world, rank, torch) -> dict:
     # launched directly with the profiler on (outside the timed region)
     _, prof, _, _ = timed_steps(torch, max(1, args.steps // 2), 1, batch.run)
     peak, kind = peaks()
-    rl = roofline(prof, {"pbatch_sums_kernel": 4 * batch.n_products + 24 * batch.n_keys,
-                         "pbatch_write_kernel": batch.n_keys * 12 + batch.n_keys * (16 * w + 16)}, peak, kind)
+    # codes in; every key's term out
+    rl = roofline(prof, {"pbatch_pass_kernel": 4 * batch.n_products + batch.n_keys * (16 * w + 16)}, peak, kind)
     out = {"metric": "batched products terms/s", "value": world * P / (t * 1e-3), "unit": "terms/s",
            "ms_per_step": t,
            "config": {"workload": f"{len(pairs) * world} uneven products A_p*B_p, 64 qubits, 16-4096 terms a side, "

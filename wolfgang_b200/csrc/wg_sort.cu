@@ -247,8 +247,9 @@ CodeSpec choose_code(const KeyBits& kb, size_t n) {
   // A pass costs more than the ties that its bits would tell apart as long as
   // some 28 bits more than log2 n are there: on 67,108,864 products of
   // 100-qubit local terms passes and reduction take 6.17 ms with 64 bits, 5.75
-  // with 56 and 6.50 with 48.
-  c.nb = c.exact ? std::max(1, kb.B) : n <= (size_t{1} << 20) ? 48 : n <= (size_t{1} << 28) ? 56 : 64;
+  // with 56 and 6.50 with 48; on 536,870,912 the whole call 70.6 with 64, 67.6
+  // with 56.
+  c.nb = c.exact ? std::max(1, kb.B) : n <= (size_t{1} << 20) ? 48 : n <= (size_t{1} << 30) ? 56 : 64;
   c.k = 0;
   if (!c.exact && kb.density > 0.0 && kb.density < 0.45) {
     // the remainder's width that suits a mean gap of 1 / density
