@@ -57,7 +57,7 @@ int wg_device_info(int ordinal, char* name, size_t name_cap, int* cc_major,
  * Tuned: the commutation kernel and its tile and rows per CTA (algo 0 of
  * wg_commutation_bits, 1-4 mask words), the bucketed sort's fine-bucket
  * target (wg_pauli_products / wg_simplify when wg_set_bucket_fine_target is
- * 0), and the group_commuting chunk length.  A class is (operation, mask
+ * 0), and the terms that a group_commuting stage takes at a time.  A class is (operation, mask
  * words, ceil log2 of the sizes).  Every candidate gives identical results.
  *   WG_TUNE_OFF     the measured defaults always;
  *   WG_TUNE_CACHED  (default) cached choices, the defaults elsewhere: no call
