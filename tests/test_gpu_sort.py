@@ -97,3 +97,28 @@ def test_not_finite(cuda, oracle, T, bad):
     c[T // 3] = bad
     for rtol in (0.0, 0.5):
         assert same(G.simplify(n, x, z, c, 1e-12, rtol), oracle.simplify(n, x, z, c, 1e-12, rtol))
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 63, 64, 65, 127, 129, 1024, 1900, 2047, 2048, 2049])
+@pytest.mark.parametrize("windows", [(0, 0, 0, 0), (1, 0, 0, 0), (5, 6, 0, 0), (26, 27, 0, 0), (27, 27, 0, 0),
+                                     (53, 0, 0, 0), (54, 0, 0, 0), (13, 13, 13, 14), (2, 0, 0, 52)])
+def test_windows_of_small_calls(cuda, oracle, T, windows):
+    """Up to 2,048 items whose varying bits lie in windows of 53 bits together are sorted as
+    one value with their number; constant bits within and beside the windows; duplicates."""
+    rng = seeded("windows", T, windows)
+    base = rng.integers(0, 1 << 62, size=4, dtype=np.uint64)
+    words = np.repeat(base[None, :], T, axis=0)
+    for k, width in enumerate(windows):
+        if width:
+            low = int(rng.integers(0, 63 - width)) if width < 63 else 0
+            pool = rng.integers(0, 1 << width, size=max(1, T // 3), dtype=np.uint64)
+            pool[0], pool[-1] = 0, (1 << width) - 1
+            mask = np.uint64(((1 << width) - 1) << low)
+            words[:, k] = (words[:, k] & ~mask) | (rng.choice(pool, size=T) << np.uint64(low))
+    order = (0, 2), (1, 3)  # key order x0, z0, x1, z1
+    x, z = (np.ascontiguousarray(words[:, list(o)]) for o in order)
+    c = coefficients(rng, T)
+    n = 126
+    assert same(G.simplify(n, x, z, c), oracle.simplify(n, x, z, c))
+    if windows[2] == windows[3] == 0:
+        assert same(G.simplify(62, x[:, :1], z[:, :1], c), oracle.simplify(62, x[:, :1].copy(), z[:, :1].copy(), c))
