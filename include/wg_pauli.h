@@ -45,6 +45,11 @@ typedef struct CUstream_st* wg_stream_t;
 /* ------------------------------------------------------------ runtime ---- */
 const char* wg_last_error(void);
 int wg_abi_version(void);
+/* Polls after which a kernel of this thread's calls stops waiting for an
+ * earlier block of its own launch (radix passes, grouping stages) and the call
+ * fails with WG_ERR_TIMEOUT; the context stays usable.  0 (the default)
+ * restores the library's limits, some seconds.  No reference counterpart. */
+int wg_set_wait_limit(unsigned polls);
 /* Device discovery; replaces DevicePauliSum::cuda_status()
  * (include/wolfgang/device_pauli_sum.hpp:111, src/cuda/device_pauli_sum.cu:286-335). */
 int wg_device_count(int* count);

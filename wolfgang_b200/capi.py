@@ -63,6 +63,7 @@ _SIGNATURES: dict[str, list] = {
     "wg_kernel_launches": [ctypes.POINTER(ctypes.c_ulonglong)],
     "wg_profile_enable": [_i],
     "wg_profile_report": [ctypes.c_char_p, _sz],
+    "wg_set_wait_limit": [ctypes.c_uint],
     "wg_commutation_bits": [_i, _sz, _vp, _vp, _sz, _vp, _vp, _sz, _vp, _sz, _i, _vp],
     "wg_bits_to_u8": [_i, _vp, _sz, _sz, _sz, _vp, _vp],
     "wg_commutation_flags": [_i, _sz, _vp, _vp, _sz, _vp, _vp, _sz, _vp, _vp],

@@ -95,6 +95,9 @@ struct DeviceProps {
   size_t total_mem = 0;
 };
 const DeviceProps& device_props(int device);
+// Polls after which a kernel's wait for an earlier CTA of its launch gives up:
+// the calling thread's setting (wg_set_wait_limit), else `fallback`.
+uint32_t wait_limit(uint32_t fallback);
 int current_device();
 
 // Grid size for a grid-stride kernel: a whole number of waves of `per_sm`

@@ -79,6 +79,12 @@ void prof_record(const char* name, cudaStream_t s, bool begin) {
   g_prof_free.push_back(e);
 }
 
+namespace {
+thread_local unsigned t_wait_limit = 0;
+}  // namespace
+
+uint32_t wait_limit(uint32_t fallback) { return t_wait_limit ? t_wait_limit : fallback; }
+
 int current_device() {
   int d = 0;
   check_cuda(cudaGetDevice(&d), "get current device");
@@ -371,6 +377,13 @@ extern "C" {
 const char* wg_last_error(void) { return g_last_error.c_str(); }
 
 int wg_abi_version(void) { return 1; }
+
+int wg_set_wait_limit(unsigned polls) {
+  return guarded([&] {
+    if (polls > (1u << 30)) throw_invalid("wait limit must be at most 2^30 polls (0: the default)");
+    t_wait_limit = polls;
+  });
+}
 
 int wg_device_count(int* count) {
   return guarded([&] {

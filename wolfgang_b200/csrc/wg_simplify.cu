@@ -432,6 +432,10 @@ __global__ void __launch_bounds__(kThreads, 4) reduce_kernel(Items items, const 
   extern __shared__ __align__(16) unsigned char raw[];
   ReduceSmem& sm = *reinterpret_cast<ReduceSmem*>(raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (ctl->timeout) {  // item numbers are not all in place
+    if (tid == 0) counts[blockIdx.x] = 0;
+    return;
+  }
   const size_t t0 = static_cast<size_t>(blockIdx.x) * kTile;
   const int own = static_cast<int>(min(static_cast<size_t>(kTile), n - t0));
   const double thr = threshold.value();

@@ -29,7 +29,7 @@ constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kItems = 8;
 constexpr int kTile = kThreads * kItems;
-constexpr int kSpinLimit = 1 << 24;
+constexpr uint32_t kSpinLimit = 1u << 24;  // unless wg_set_wait_limit says otherwise
 constexpr int kLook = 8;
 
 // A status word: value (56 bits) | pass + 1 (6 bits) | state (2 bits).  The
@@ -59,7 +59,7 @@ template <bool kHigh>  // the digit lies in the code's upper half
 static __global__ void __launch_bounds__(kThreads, 3) radix_pass_kernel(
     const uint64_t* __restrict__ kin, uint64_t* __restrict__ kout, const uint32_t* __restrict__ iin,
     uint32_t* __restrict__ iout, uint32_t n, int pass, const uint32_t* __restrict__ base,
-    unsigned long long* status, SortControl* ctl) {
+    unsigned long long* status, SortControl* ctl, uint32_t limit) {
   extern __shared__ __align__(16) unsigned char raw[];
   PassSmem& sm = *reinterpret_cast<PassSmem*>(raw);
   uint32_t* warp_count = reinterpret_cast<uint32_t*>(sm.keys);  // [kWarps][kDigits]
@@ -150,7 +150,7 @@ static __global__ void __launch_bounds__(kThreads, 3) radix_pass_kernel(
     // kLook predecessors are read at a time: one after another their latency
     // is what a pass spends (5,000,000 pairs: 70 us a pass one by one)
     const volatile unsigned long long* look = st;
-    int spins = 0;
+    uint32_t spins = 0;
     for (uint32_t t = tile; t > 0;) {
       unsigned long long v[kLook];
 #pragma unroll
@@ -167,7 +167,7 @@ static __global__ void __launch_bounds__(kThreads, 3) radix_pass_kernel(
         used = e + 1;
       }
       if (total) break;
-      if (used == 0 && ++spins > kSpinLimit) {
+      if (used == 0 && ++spins >= limit) {
         ctl->timeout = 1;
         break;
       }
@@ -234,7 +234,8 @@ void sort_pairs(size_t n, PairBuffers& b, int count, bool implied, cudaStream_t 
     auto* kernel = p < 4 ? radix_pass_kernel<false> : radix_pass_kernel<true>;
     WG_TIMED("radix_pass_kernel", s,
       kernel<<<tiles, kThreads, sizeof(PassSmem), s>>>(b.k0, b.k1, implied && p == 0 ? nullptr : b.i0, b.i1,
-                                                       static_cast<uint32_t>(n), p, b.hist, b.status, b.control));
+                                                       static_cast<uint32_t>(n), p, b.hist, b.status, b.control,
+                                                       wg::wait_limit(kSpinLimit)));
     wg::check_launch("launch radix pass");
     std::swap(b.k0, b.k1);
     std::swap(b.i0, b.i1);
@@ -325,6 +326,7 @@ __global__ void __launch_bounds__(256) soa_check_kernel(const uint64_t* __restri
                                                         const uint32_t* __restrict__ order,
                                                         const uint64_t* __restrict__ packed, size_t n, int words,
                                                         SortControl* ctl) {
+  if (ctl->timeout) return;  // the order is not whole
   bool mixed = false;
   for (size_t i = 1 + blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {

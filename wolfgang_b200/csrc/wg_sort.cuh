@@ -107,7 +107,7 @@ constexpr size_t digit_smem(int passes) { return sizeof(uint32_t) * kDigits * kH
 // Device words that a sort writes for the host.
 struct SortControl {
   uint32_t ticket[kMaxPasses];  // next tile of each pass
-  uint32_t timeout;             // a look-back gave up
+  uint32_t timeout;             // a look-back gave up: codes and item numbers are not all in place, nothing may follow them
   uint32_t mixed;               // a run of equal codes needs the full keys
   uint32_t infinite;            // some |c| is infinite
   uint32_t survivors;
