@@ -91,13 +91,16 @@ struct Pipe {
   uint32_t base;                 // first group of the first stage
   uint32_t batch;                // terms taken at a time
   uint32_t* group_of;
-  uint32_t* next;                // full mode: members that do not fit in shared memory, linked
+  // full mode: members that do not fit in shared memory, in blocks of kBlock<W>
+  uint64_t* more;                // [blocks][2 W][kBlock<W>] their words
+  uint32_t* next;                // [blocks] a group's next block
 };
 
 struct PipeControl {
   uint32_t ticket;
   uint32_t timeout;
   uint32_t groups;  // groups opened so far
+  uint32_t blocks;  // blocks of members taken so far (full mode)
 };
 
 // Terms that stage s can read, and whether more may come; waits until `want`
@@ -350,11 +353,25 @@ constexpr int kKept = 320 / W;
 // words of the m-th members of the 32 groups, and one against bank conflicts
 template <int W>
 constexpr int kMemberRow = 2 * W * 32 + 1;
+// members of a block beyond those: 2 KB of words
+template <int W>
+constexpr uint32_t kBlock = W == 1 ? 128 : W == 2 ? 64 : 32;
+
+// Blocks that T terms can need: full ones, and a last one for each group with
+// more than kKept members.
+template <int W>
+constexpr size_t member_blocks(size_t T) {
+  return T / kBlock<W> + T / (kKept<W> + 1) + 1;
+}
 
 // Full mode: a batch of up to 31 terms, a warp each.  A warp checks its term
 // against the first 8 members of all groups, a group per lane: of most groups
 // one of them anticommutes.  The groups that are left are checked one after
-// another, a member per lane.  Warp 0 then places the batch in order
+// another, a member per lane, also behind those in shared memory: the words of
+// the members beyond lie in blocks of 2 KB, word by word, that all the batch's
+// warps read at about the same time (through L1; one lane that followed a linked
+// list of members took 811 ms for 16,384 Z strings on 40 qubits, 1,207 ms on
+// 128: this takes 25.5 and 37 ms).  Warp 0 then places the batch in order
 // (place_terms), while one more warp brings the next batch and the table of
 // which of its terms anticommute.  32,768 terms on 128 qubits in 708 groups: 5.0
 // ms (before: 60 ms; with a group per lane for all members, which 32 warps load
@@ -365,12 +382,12 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
   uint64_t* members = reinterpret_cast<uint64_t*>(raw);  // [kKept][kMemberRow]
   __shared__ __align__(16) uint64_t term[2][kFullMost + 1][2 * W];
   __shared__ uint32_t ids[2][kFullMost + 1], against[2][kFullMost + 1];
-  __shared__ uint32_t accepts[32], place[32], slot[32], s_in[32];
-  __shared__ uint32_t count[kStageGroups], first[kStageGroups], last[kStageGroups];
+  __shared__ uint32_t accepts[32], place[32], slot[32], block[32], s_in[32];
+  __shared__ uint32_t count[kStageGroups], first[kStageGroups], last[kStageGroups];  // members, first and last block
   __shared__ uint32_t s_stage, s_n[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bringer = static_cast<int>(pipe.batch);
-  constexpr uint32_t kIn = kKept<W>;
+  constexpr uint32_t kIn = kKept<W>, kMore = kBlock<W>;
   if (tid == 0) s_stage = atomicAdd(&ctl->ticket, 1u);
   if (tid < kStageGroups) count[tid] = 0;
   __syncthreads();
@@ -447,19 +464,30 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
           }
         }
       }
-      bool still = (a >> lane) & 1u;
-      if (still && c > kIn) {
-        const volatile uint32_t* next = pipe.next;
-        for (uint32_t m = first[lane]; still && m != UINT_MAX; m = next[m]) {
+      // this CTA wrote the blocks before its last barrier: plain loads see them
+      for (uint32_t rest = a & __ballot_sync(0xffffffffu, c > kIn); rest; rest &= rest - 1) {
+        const int g = __ffs(rest) - 1;
+        uint32_t left = __shfl_sync(0xffffffffu, c, g) - kIn;
+        for (uint32_t blk = first[g], after;; blk = after) {
+          after = pipe.next[blk];  // on its way meanwhile; not set for a last block, nor used
+          const uint64_t* words = pipe.more + static_cast<size_t>(blk) * (2 * W * kMore);
+          bool bad = false;
 #pragma unroll
-          for (int w = 0; w < W; ++w) {
-            r[w] = __ldg(pipe.ox + static_cast<size_t>(m) * W + w);
-            r[W + w] = __ldg(pipe.oz + static_cast<size_t>(m) * W + w);
+          for (uint32_t k0 = 0; k0 < kMore; k0 += 32) {
+            if (k0 + lane < left) {
+#pragma unroll
+              for (int e = 0; e < 2 * W; ++e) r[e] = words[e * kMore + k0 + lane];
+              bad |= anticommutes<W>(t, r);
+            }
           }
-          still = !anticommutes<W>(t, r);
+          if (__any_sync(0xffffffffu, bad)) {
+            a &= ~(1u << g);
+            break;
+          }
+          if (left <= kMore) break;
+          left -= kMore;
         }
       }
-      a = __ballot_sync(0xffffffffu, still);
       if (lane == 0) accepts[warp] = a;
     }
     __syncthreads();
@@ -477,11 +505,13 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
       __syncwarp();
       for (uint32_t rest = joined; rest; rest &= rest - 1, ++c) {
         if (c < kIn) continue;
-        const uint32_t id = ids[cur][__ffs(rest) - 1];
-        pipe.next[id] = UINT_MAX;
-        if (c == kIn) first[lane] = id;
-        else pipe.next[last[lane]] = id;
-        last[lane] = id;
+        if ((c - kIn) % kMore == 0) {
+          const uint32_t fresh = atomicAdd(&ctl->blocks, 1u);  // below member_blocks(terms)
+          if (c == kIn) first[lane] = fresh;
+          else pipe.next[last[lane]] = fresh;
+          last[lane] = fresh;
+        }
+        block[__ffs(rest) - 1] = last[lane];
       }
       count[lane] = c;
       const bool left = has && mine == UINT_MAX;
@@ -494,8 +524,11 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
       if (lane == 0) *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
     }
     __syncthreads();
-    if (warp < static_cast<int>(n) && place[warp] != UINT_MAX && slot[warp] < kIn && lane < 2 * W)
-      members[slot[warp] * kMemberRow<W> + 32 * lane + place[warp]] = term[cur][warp][lane];
+    if (warp < static_cast<int>(n) && place[warp] != UINT_MAX && lane < 2 * W) {
+      const uint32_t k = slot[warp];
+      if (k < kIn) members[k * kMemberRow<W> + 32 * lane + place[warp]] = term[cur][warp][lane];
+      else pipe.more[(static_cast<size_t>(block[warp]) * (2 * W) + lane) * kMore + (k - kIn) % kMore] = term[cur][warp][lane];
+    }
     cur ^= 1;
     __syncthreads();
   }
@@ -560,6 +593,14 @@ uint32_t run_pipeline(int device, bool full, Pipe pipe, uint32_t T, cudaStream_t
     wg::check_cuda(cudaFuncSetAttribute(group_qwc_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         static_cast<int>(smem)),
                    "set grouping shared memory");
+  }
+  wg::Scratch more, next;
+  if (full) {
+    const size_t blocks = member_blocks<W>(T);
+    more.reset(sizeof(uint64_t) * 2 * W * kBlock<W> * blocks, s);
+    next.reset(sizeof(uint32_t) * blocks, s);
+    pipe.more = more.as<uint64_t>();
+    pipe.next = next.as<uint32_t>();
   }
   pipe.n = T;
   pipe.fresh = 1;
@@ -945,7 +986,7 @@ int wg_group_commuting(int device, size_t words, size_t n_terms, const uint64_t*
     }
     const bool full = mode_full != 0;
     const uint32_t T32 = static_cast<uint32_t>(T);
-    wg::Scratch gid(4 * T, s), next(4 * T, s);
+    wg::Scratch gid(4 * T, s);
     uint32_t G = 0;
     if (W <= 4) {
       wg::Scratch list(4 * T, s);
@@ -955,7 +996,6 @@ int wg_group_commuting(int device, size_t words, size_t n_terms, const uint64_t*
         pipe.oz = oz.as<uint64_t>();
         pipe.list = list.as<uint32_t>();
         pipe.group_of = gid.as<uint32_t>();
-        pipe.next = next.as<uint32_t>();
         pipe.batch = batch;
         switch (W) {
           case 0:
@@ -977,7 +1017,7 @@ int wg_group_commuting(int device, size_t words, size_t n_terms, const uint64_t*
           &done);
       if (!done) place(cands[choice]);
     } else {
-      wg::Scratch rows(16 * Wa * T, s), first(4 * T, s), last(4 * T, s), lb(4 * T, s), lbm(4 * T, s), ng(4, s),
+      wg::Scratch rows(16 * Wa * T, s), first(4 * T, s), last(4 * T, s), next(4 * T, s), lb(4 * T, s), lbm(4 * T, s), ng(4, s),
           trows(16 * Wa * T, s);
       WG_TIMED("interleave_rows_kernel", s,
         interleave_rows_kernel<<<wg::grid_for(T * W, kThreads, device, 4), kThreads, 0, s>>>(
