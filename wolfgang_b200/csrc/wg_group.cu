@@ -76,10 +76,12 @@ constexpr int kBoundSplit = 8;
 // it has read k or more of its predecessor's, so the predecessor's unread ones
 // are further on.  status[s] tells how many there are (and kDone when there will
 // be no more).  Stages take their number by a ticket, so that whoever a stage
-// waits for is already running; the waits are bounded all the same.
+// waits for is already running.  A stage may see no term for as long as an earlier
+// one takes them all, so a wait gives up only when no stage has taken a batch for
+// kPollLimit polls.
 constexpr int kStageGroups = 32;
 constexpr unsigned long long kDone = 1ull << 63;
-constexpr int kPollLimit = 1 << 26;
+constexpr uint32_t kPollLimit = 1u << 26;  // unless wg_set_wait_limit says otherwise
 
 struct Pipe {
   const uint64_t* ox;            // terms in processing order
@@ -90,6 +92,7 @@ struct Pipe {
   unsigned long long* status;    // [stages], zeroed
   uint32_t base;                 // first group of the first stage
   uint32_t batch;                // terms taken at a time
+  uint32_t limit;                // polls without progress before a wait gives up
   uint32_t* group_of;
   // full mode: members that do not fit in shared memory, in blocks of kBlock<W>
   uint64_t* more;                // [blocks][2 W][kBlock<W>] their words
@@ -101,6 +104,7 @@ struct PipeControl {
   uint32_t timeout;
   uint32_t groups;  // groups opened so far
   uint32_t blocks;  // blocks of members taken so far (full mode)
+  uint32_t beat;    // batches that all stages have taken
 };
 
 // Terms that stage s can read, and whether more may come; waits until `want`
@@ -109,16 +113,25 @@ __device__ __forceinline__ uint32_t wait_terms(const Pipe& p, uint32_t s, uint32
                                                PipeControl* ctl) {
   if (s == 0) return min(want, p.n - have);
   const volatile unsigned long long* st = p.status + s - 1;
-  for (int spins = 0;; ++spins) {
+  const volatile uint32_t* beat = &ctl->beat;
+  uint32_t seen = 0;
+  bool watched = false;
+  for (uint32_t spins = 1;; ++spins) {
     const unsigned long long v = *st;
     const uint32_t there = static_cast<uint32_t>(v & ~kDone) - have;
     if (there >= want || (v & kDone)) {
       __threadfence();
       return min(there, want);
     }
-    if (spins > kPollLimit) {
-      ctl->timeout = 1;
-      return 0;
+    if (spins >= p.limit) {
+      const uint32_t now = *beat;
+      if (watched && now == seen) {
+        ctl->timeout = 1;
+        return 0;
+      }
+      watched = true;
+      seen = now;
+      spins = 0;
     }
     __nanosleep(64);
   }
@@ -331,7 +344,10 @@ __global__ void __launch_bounds__(kQwcThreads) group_qwc_kernel(Pipe pipe, PipeC
     }
     __threadfence();
     __syncthreads();
-    if (tid == 0) *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
+    if (tid == 0) {
+      *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
+      atomicAdd(&ctl->beat, 1u);
+    }
     cur ^= 1;
   }
   if (tid == 0) {
@@ -521,7 +537,10 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
       written += __popc(b);
       __threadfence();
       __syncwarp();
-      if (lane == 0) *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
+      if (lane == 0) {
+        *const_cast<volatile unsigned long long*>(pipe.status + stage) = written;
+        atomicAdd(&ctl->beat, 1u);
+      }
     }
     __syncthreads();
     if (warp < static_cast<int>(n) && place[warp] != UINT_MAX && lane < 2 * W) {
@@ -997,6 +1016,7 @@ int wg_group_commuting(int device, size_t words, size_t n_terms, const uint64_t*
         pipe.list = list.as<uint32_t>();
         pipe.group_of = gid.as<uint32_t>();
         pipe.batch = batch;
+        pipe.limit = wg::wait_limit(kPollLimit);
         switch (W) {
           case 0:
           case 1: G = run_pipeline<1>(device, full, pipe, T32, s); break;
