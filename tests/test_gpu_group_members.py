@@ -1,5 +1,5 @@
 """Full-mode groups with more members than a stage keeps in shared memory (320 / words):
-the others lie in blocks of 32 to 128 in device memory."""
+the others lie in blocks of 128 in device memory."""
 
 from __future__ import annotations
 

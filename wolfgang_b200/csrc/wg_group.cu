@@ -94,8 +94,8 @@ struct Pipe {
   uint32_t batch;                // terms taken at a time
   uint32_t limit;                // polls without progress before a wait gives up
   uint32_t* group_of;
-  // full mode: members that do not fit in shared memory, in blocks of kBlock<W>
-  uint64_t* more;                // [blocks][2 W][kBlock<W>] their words
+  // full mode: members that do not fit in shared memory, in blocks of kBlock
+  uint64_t* more;                // [blocks][2 W][kBlock] their words
   uint32_t* next;                // [blocks] a group's next block
 };
 
@@ -369,25 +369,25 @@ constexpr int kKept = 320 / W;
 // words of the m-th members of the 32 groups, and one against bank conflicts
 template <int W>
 constexpr int kMemberRow = 2 * W * 32 + 1;
-// members of a block beyond those: 2 KB of words
-template <int W>
-constexpr uint32_t kBlock = W == 1 ? 128 : W == 2 ? 64 : 32;
+// members of a block beyond those (of 32 at 4 words, 2 KB: 8,192 Z strings on 250
+// qubits 36 against 13 ms, 16,384 random terms on 200 3.65 against 3.3 ms)
+constexpr uint32_t kBlock = 128;
 
 // Blocks that T terms can need: full ones, and a last one for each group with
 // more than kKept members.
 template <int W>
 constexpr size_t member_blocks(size_t T) {
-  return T / kBlock<W> + T / (kKept<W> + 1) + 1;
+  return T / kBlock + T / (kKept<W> + 1) + 1;
 }
 
 // Full mode: a batch of up to 31 terms, a warp each.  A warp checks its term
 // against the first 8 members of all groups, a group per lane: of most groups
 // one of them anticommutes.  The groups that are left are checked one after
 // another, a member per lane, also behind those in shared memory: the words of
-// the members beyond lie in blocks of 2 KB, word by word, that all the batch's
+// the members beyond lie in blocks of 128, word by word, that all the batch's
 // warps read at about the same time (through L1; one lane that followed a linked
 // list of members took 811 ms for 16,384 Z strings on 40 qubits, 1,207 ms on
-// 128: this takes 25.5 and 37 ms).  Warp 0 then places the batch in order
+// 128: this takes 25.5 and 35 ms).  Warp 0 then places the batch in order
 // (place_terms), while one more warp brings the next batch and the table of
 // which of its terms anticommute.  32,768 terms on 128 qubits in 708 groups: 5.0
 // ms (before: 60 ms; with a group per lane for all members, which 32 warps load
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
   __shared__ uint32_t s_stage, s_n[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bringer = static_cast<int>(pipe.batch);
-  constexpr uint32_t kIn = kKept<W>, kMore = kBlock<W>;
+  constexpr uint32_t kIn = kKept<W>;
   if (tid == 0) s_stage = atomicAdd(&ctl->ticket, 1u);
   if (tid < kStageGroups) count[tid] = 0;
   __syncthreads();
@@ -486,13 +486,13 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
         uint32_t left = __shfl_sync(0xffffffffu, c, g) - kIn;
         for (uint32_t blk = first[g], after;; blk = after) {
           after = pipe.next[blk];  // on its way meanwhile; not set for a last block, nor used
-          const uint64_t* words = pipe.more + static_cast<size_t>(blk) * (2 * W * kMore);
+          const uint64_t* words = pipe.more + static_cast<size_t>(blk) * (2 * W * kBlock);
           bool bad = false;
 #pragma unroll
-          for (uint32_t k0 = 0; k0 < kMore; k0 += 32) {
+          for (uint32_t k0 = 0; k0 < kBlock; k0 += 32) {
             if (k0 + lane < left) {
 #pragma unroll
-              for (int e = 0; e < 2 * W; ++e) r[e] = words[e * kMore + k0 + lane];
+              for (int e = 0; e < 2 * W; ++e) r[e] = words[e * kBlock + k0 + lane];
               bad |= anticommutes<W>(t, r);
             }
           }
@@ -500,8 +500,8 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
             a &= ~(1u << g);
             break;
           }
-          if (left <= kMore) break;
-          left -= kMore;
+          if (left <= kBlock) break;
+          left -= kBlock;
         }
       }
       if (lane == 0) accepts[warp] = a;
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
       __syncwarp();
       for (uint32_t rest = joined; rest; rest &= rest - 1, ++c) {
         if (c < kIn) continue;
-        if ((c - kIn) % kMore == 0) {
+        if ((c - kIn) % kBlock == 0) {
           const uint32_t fresh = atomicAdd(&ctl->blocks, 1u);  // below member_blocks(terms)
           if (c == kIn) first[lane] = fresh;
           else pipe.next[last[lane]] = fresh;
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(1024) group_full_kernel(Pipe pipe, PipeControl
     if (warp < static_cast<int>(n) && place[warp] != UINT_MAX && lane < 2 * W) {
       const uint32_t k = slot[warp];
       if (k < kIn) members[k * kMemberRow<W> + 32 * lane + place[warp]] = term[cur][warp][lane];
-      else pipe.more[(static_cast<size_t>(block[warp]) * (2 * W) + lane) * kMore + (k - kIn) % kMore] = term[cur][warp][lane];
+      else pipe.more[(static_cast<size_t>(block[warp]) * (2 * W) + lane) * kBlock + (k - kIn) % kBlock] = term[cur][warp][lane];
     }
     cur ^= 1;
     __syncthreads();
@@ -616,7 +616,7 @@ uint32_t run_pipeline(int device, bool full, Pipe pipe, uint32_t T, cudaStream_t
   wg::Scratch more, next;
   if (full) {
     const size_t blocks = member_blocks<W>(T);
-    more.reset(sizeof(uint64_t) * 2 * W * kBlock<W> * blocks, s);
+    more.reset(sizeof(uint64_t) * 2 * W * kBlock * blocks, s);
     next.reset(sizeof(uint32_t) * blocks, s);
     pipe.more = more.as<uint64_t>();
     pipe.next = next.as<uint32_t>();
