@@ -178,26 +178,51 @@ struct PairRun {
   uint32_t below;          // survivors in its first segment's tile below that segment
 };
 
-// The pair of sorted position j, not before pair p.
-__device__ __forceinline__ uint32_t pair_from(const PairNum* __restrict__ pairs, uint32_t p, uint64_t j) {
-  while (j >= pairs[p].item_end) ++p;
-  return p;
+// The pair of sorted position j, one of lo to hi.
+__device__ __forceinline__ uint32_t pair_within(const PairNum* __restrict__ pairs, uint32_t lo, uint32_t hi, uint64_t j) {
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (j < pairs[mid].item_end) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
 }
 
 // rtol > 0: each pair's largest |product|, ahead of the pass that needs it
 // (non-negative doubles order like their bits; a NaN never replaces the running
 // maximum, std::max's rule).
-__global__ void __launch_bounds__(kThreads) pbatch_max_kernel(const PairNum* __restrict__ pairs,
+__global__ void __launch_bounds__(kThreads) pbatch_max_kernel(const PairNum* __restrict__ pairs, uint32_t n_pairs,
                                                               const uint32_t* __restrict__ code, size_t N,
                                                               PairRun* __restrict__ run) {
   uint32_t p = 0;
   for (size_t j = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; j < N;
        j += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    p = pair_from(pairs, p, j);
+    if (j >= pairs[p].item_end) p = pair_within(pairs, p + 1, n_pairs - 1, j);
     const c128 c = coded_product(pairs[p], code[j]);
     const double m = wgd::hypot_ref(c.re, c.im);
     if (m > __longlong_as_double(static_cast<long long>(run[p].max)))
       atomicMax(&run[p].max, static_cast<unsigned long long>(__double_as_longlong(m)));
+  }
+}
+
+// The pairs' counts, spread over the launch (kept holds the survivors before each
+// tile where something was culled).  rtol = 0 (`infinite`): a pair with an infinite
+// |product| has the threshold atol + 0 * inf, a NaN, and keeps nothing.
+__device__ __forceinline__ void write_counts(const PairNum* __restrict__ pairs, uint32_t n_pairs,
+                                             const uint32_t* __restrict__ tile_of, bool infinite, const PairRun* run,
+                                             const uint32_t* kept, uint32_t tiles, uint64_t* __restrict__ counts) {
+  for (uint64_t p = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; p < n_pairs;
+       p += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    uint64_t c = pairs[p].n_seg;
+    if (c && run[p].culled) {
+      // up to where the next pair with segments begins
+      uint64_t q = p + 1;
+      while (q < n_pairs && pairs[q].n_seg == 0) ++q;
+      const uint32_t end = q < n_pairs ? kept[tile_of[q]] + run[q].below : kept[tiles];
+      c = end - (kept[tile_of[p]] + run[p].below);
+    }
+    if (infinite && isinf(__longlong_as_double(static_cast<long long>(run[p].max)))) c = 0;
+    counts[p] = c;
   }
 }
 
@@ -218,12 +243,15 @@ constexpr int kStage = kTile + kThreads;  // products staged at a time
 // another in a chain.
 template <int WT, int MAX, bool REDO>
 __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
-    const PairNum* __restrict__ pairs, const uint32_t* __restrict__ tile_seg, const uint32_t* __restrict__ seg_start,
+    const PairNum* __restrict__ pairs, uint32_t n_pairs, const uint32_t* __restrict__ tile_seg, const uint32_t* __restrict__ seg_start,
     const uint32_t* __restrict__ seg_pair, const uint64_t* __restrict__ seg_keys, const uint32_t* __restrict__ code,
     int Wrt, double atol, double rtol, PairRun* run, uint32_t* __restrict__ any, uint32_t* __restrict__ kept,
     const uint32_t* __restrict__ tile_of, uint64_t* __restrict__ ox, uint64_t* __restrict__ oz,
-    double2* __restrict__ oc) {
-  if (REDO && *any == 0) return;
+    double2* __restrict__ oc, uint64_t* __restrict__ counts) {
+  if (REDO) {
+    write_counts(pairs, n_pairs, tile_of, MAX == kMaxInf, run, kept, gridDim.x, counts);
+    if (*any == 0) return;
+  }
   __shared__ double2 prod[kStage];
   __shared__ uint32_t bits[kTile / 32];
   __shared__ uint32_t rank[kTile / 32 + 1];
@@ -237,13 +265,14 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
   if (REDO) {
     // nothing to do unless a pair of the tile has culled segments
     bool redo = false;
-    for (uint32_t p = seg_pair[s0]; p <= seg_pair[s1 - 1]; ++p) redo |= run[p].culled != 0;
-    if (!redo) return;
+    for (uint32_t p = seg_pair[s0] + tid; p <= seg_pair[s1 - 1]; p += kThreads) redo |= run[p].culled != 0;
+    if (!__syncthreads_or(redo)) return;
   }
   const uint32_t j0 = seg_start[s0], j1 = seg_start[s1];
   const uint32_t staged = min(j1 - j0, static_cast<uint32_t>(kStage));
-  // products [from, from + count) into prod[0..]; the loads of a thread's
-  // products are in flight together
+  const uint32_t p0 = seg_pair[s0], p1 = seg_pair[s1 - 1];  // the tile's pairs: all others are searched among these
+  // products [from, from + count) of pairs p to p1 into prod[0..]; the loads of
+  // a thread's products are in flight together
   auto stage = [&](uint32_t p, uint32_t from, uint32_t count) {
     constexpr int kPer = kStage / kThreads;
     uint32_t c[kPer], own[kPer];
@@ -256,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
       const uint32_t i = k * kThreads + tid;
-      if (i < count) p = pair_from(pairs, p, from + i);
+      if (i < count) p = pair_within(pairs, p, p1, from + i);
       own[k] = p;
       const PairNum& P = pairs[p];
       const uint32_t nr = static_cast<uint32_t>(P.n_r), q = c[k] >> 2;  // below 2^30
@@ -289,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
     begin[k] = __ldg(seg_start + s) - j0;
     end[k] = __ldg(seg_start + s + 1) - j0;
   }
-  stage(seg_pair[s0], j0, staged);
+  stage(p0, j0, staged);
   __syncthreads();
   ulonglong2 key[WT == 1 ? kRounds : 1];  // on their way while the sums are formed
   if constexpr (WT == 1) {
@@ -309,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
   for (uint32_t from = j0 + staged; from < j1; from += kStage) {
     const uint32_t count = min(j1 - from, static_cast<uint32_t>(kStage));
     __syncthreads();
-    stage(seg_pair[s1 - 1], from, count);
+    stage(p1, from, count);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kRounds; ++k)
@@ -388,54 +417,46 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
   }
 }
 
-// One CTA, between the pass and its repetition: where something was culled,
-// the tiles' survivor counts become the survivors before each tile; the pairs'
-// counts.  rtol = 0: a pair with an infinite |product| has the threshold
-// atol + 0 * inf, a NaN, and keeps nothing.
-__global__ void __launch_bounds__(1024) pbatch_counts_kernel(const PairNum* __restrict__ pairs, size_t n_pairs,
-                                                             const uint32_t* __restrict__ tile_of, int infinite,
-                                                             const PairRun* __restrict__ run,
-                                                             const uint32_t* __restrict__ any, uint32_t* kept,
-                                                             size_t tiles, uint64_t* __restrict__ counts) {
+// One CTA, between the pass and its repetition: where something was culled, the
+// tiles' survivor counts become the survivors before each tile.
+__global__ void __launch_bounds__(1024) pbatch_scan_kernel(const uint32_t* __restrict__ any, uint32_t* kept,
+                                                           size_t tiles) {
+  constexpr int kPer = 8;  // consecutive tiles of a thread
   __shared__ uint32_t sums[32];
-  __shared__ uint32_t carry;
+  if (!*any) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (*any) {
-    if (tid == 0) carry = 0;
-    __syncthreads();
-    for (size_t t0 = 0; t0 < tiles; t0 += 1024) {
-      const size_t t = t0 + tid;
-      const uint32_t c = t < tiles ? kept[t] : 0;
-      uint32_t incl = c;
+  uint32_t carry = 0;
+  for (size_t t0 = 0; t0 < tiles; t0 += 1024 * kPer) {
+    uint32_t c[kPer], sum = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (lane == 31) sums[warp] = incl;
-      __syncthreads();
-      uint32_t before = carry;
-      for (int w = 0; w < warp; ++w) before += sums[w];
-      if (t < tiles) kept[t] = before + incl - c;
-      __syncthreads();
-      if (tid == 1023) carry = before + incl;
-      __syncthreads();
+    for (int e = 0; e < kPer; ++e) {
+      const size_t t = t0 + static_cast<size_t>(tid) * kPer + e;
+      c[e] = t < tiles ? kept[t] : 0;
     }
-    if (tid == 0) kept[tiles] = carry;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) sum += c[e];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) sums[warp] = incl;
+    __syncthreads();
+    uint32_t at = carry + incl - sum;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) at += sums[w];
+      carry += sums[w];
+    }
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const size_t t = t0 + static_cast<size_t>(tid) * kPer + e;
+      if (t < tiles) kept[t] = at;
+      at += c[e];
+    }
     __syncthreads();
   }
-  for (size_t p = tid; p < n_pairs; p += 1024) {
-    uint64_t c = pairs[p].n_seg;
-    if (c && run[p].culled) {
-      // up to where the next pair with segments begins
-      size_t q = p + 1;
-      while (q < n_pairs && pairs[q].n_seg == 0) ++q;
-      const uint32_t end = q < n_pairs ? kept[tile_of[q]] + run[q].below : kept[tiles];
-      c = end - (kept[tile_of[p]] + run[p].below);
-    }
-    if (infinite && isinf(__longlong_as_double(static_cast<long long>(run[p].max)))) c = 0;
-    counts[p] = c;
-  }
+  if (tid == 0) kept[tiles] = carry;
 }
 
 }  // namespace
@@ -604,23 +625,23 @@ void run_batch(wg_products_batch_s& b, cudaStream_t s) {
   auto* code = b.code.as<uint32_t>();
   if (max_mode == kMaxFull) {
     WG_TIMED("pbatch_max_kernel", s,
-      pbatch_max_kernel<<<wg::grid_for(b.N, kThreads, device, 8), kThreads, 0, s>>>(pairs, code, b.N, run));
+      pbatch_max_kernel<<<wg::grid_for(b.N, kThreads, device, 8), kThreads, 0, s>>>(pairs, static_cast<uint32_t>(b.n_pairs),
+                                                                                       code, b.N, run));
     wg::check_launch("launch batch maxima");
   }
   auto pass = [&](auto* kernel, const char* name) {
     WG_TIMED(name, s,
       kernel<<<static_cast<unsigned>(b.tiles), kThreads, 0, s>>>(
-          pairs, b.tile_seg.as<uint32_t>(), b.seg_start.as<uint32_t>(), b.seg_pair.as<uint32_t>(),
+          pairs, static_cast<uint32_t>(b.n_pairs), b.tile_seg.as<uint32_t>(), b.seg_start.as<uint32_t>(), b.seg_pair.as<uint32_t>(),
           b.seg_keys.as<uint64_t>(), code, b.W, b.atol, b.rtol, run, any, b.kept.as<uint32_t>(),
-          b.tile_of.as<uint32_t>(), b.out_x.as<uint64_t>(), b.out_z.as<uint64_t>(), b.out_c.as<double2>()));
+          b.tile_of.as<uint32_t>(), b.out_x.as<uint64_t>(), b.out_z.as<uint64_t>(), b.out_c.as<double2>(),
+          b.counts.as<uint64_t>()));
     wg::check_launch("launch batch pass");
   };
   auto both = [&](auto* first, auto* again) {
     pass(first, "pbatch_pass_kernel");
-    WG_TIMED("pbatch_counts_kernel", s,
-      pbatch_counts_kernel<<<1, 1024, 0, s>>>(pairs, b.n_pairs, b.tile_of.as<uint32_t>(), max_mode == kMaxInf ? 1 : 0,
-                                              run, any, b.kept.as<uint32_t>(), b.tiles, b.counts.as<uint64_t>()));
-    wg::check_launch("launch batch counts");
+    WG_TIMED("pbatch_scan_kernel", s, pbatch_scan_kernel<<<1, 1024, 0, s>>>(any, b.kept.as<uint32_t>(), b.tiles));
+    wg::check_launch("launch batch scan");
     pass(again, "pbatch_redo_kernel");
   };
   auto width = [&](auto w) {
