@@ -178,6 +178,13 @@ struct PairRun {
   uint32_t below;          // survivors in its first segment's tile below that segment
 };
 
+// Sums that the pass leaves for its repetition: those of the tiles in which it
+// found a pair with culled sums.
+struct SavedSums {
+  double2* sum;     // [segments]
+  uint32_t* saved;  // [tiles]
+};
+
 // The pair of sorted position j, one of lo to hi.
 __device__ __forceinline__ uint32_t pair_within(const PairNum* __restrict__ pairs, uint32_t lo, uint32_t hi, uint64_t j) {
   while (lo < hi) {
@@ -238,16 +245,21 @@ constexpr int kStage = kTile + kThreads;  // products staged at a time
 // coefficients come from L2).  47,800,000 products of 64 pairs on 64 qubits:
 // 0.91 ms and 0.03 ms for the repetition's early exits.  Before, a thread per
 // segment chased start, code and coefficients one after another (0.99 ms), and
-// cull, scan and write-out re-read every sum (0.65 ms).  Ranks from a look-back
+// cull, scan and write-out re-read every sum (0.65 ms).  Where a tile's pairs are
+// known to have culled sums by the time it is done, it keeps its sums for the
+// repetition, and leaves out the writing if the tile has one pair only: 98,600,000
+// products of 64 squares on 64 qubits, 5,200,000 of 39,750,000 sums culled, 2.8 ms
+// (4.7 ms with all products formed twice and a mark by every culled sum; 2.9 ms in
+// four passes).  Ranks from a look-back
 // over the tiles measured 2.7 ms: the tiles of one large pair wait for one
 // another in a chain.
 template <int WT, int MAX, bool REDO>
 __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
     const PairNum* __restrict__ pairs, uint32_t n_pairs, const uint32_t* __restrict__ tile_seg, const uint32_t* __restrict__ seg_start,
     const uint32_t* __restrict__ seg_pair, const uint64_t* __restrict__ seg_keys, const uint32_t* __restrict__ code,
-    int Wrt, double atol, double rtol, PairRun* run, uint32_t* __restrict__ any, uint32_t* __restrict__ kept,
+    int Wrt, double atol, double rtol, PairRun* run, uint32_t* any, uint32_t* __restrict__ kept,
     const uint32_t* __restrict__ tile_of, uint64_t* __restrict__ ox, uint64_t* __restrict__ oz,
-    double2* __restrict__ oc, uint64_t* __restrict__ counts) {
+    double2* __restrict__ oc, uint64_t* __restrict__ counts, SavedSums keeper) {
   if (REDO) {
     write_counts(pairs, n_pairs, tile_of, MAX == kMaxInf, run, kept, gridDim.x, counts);
     if (*any == 0) return;
@@ -259,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
   const int W = WT > 0 ? WT : Wrt;
   const uint32_t s0 = tile_seg[blockIdx.x], s1 = tile_seg[blockIdx.x + 1];
   if (s0 == s1) {
-    if (!REDO && tid == 0) kept[blockIdx.x] = 0;
+    if (!REDO && tid == 0) kept[blockIdx.x] = keeper.saved[blockIdx.x] = 0;
     return;
   }
   if (REDO) {
@@ -270,7 +282,10 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
   }
   const uint32_t j0 = seg_start[s0], j1 = seg_start[s1];
   const uint32_t staged = min(j1 - j0, static_cast<uint32_t>(kStage));
-  const uint32_t p0 = seg_pair[s0], p1 = seg_pair[s1 - 1];  // the tile's pairs: all others are searched among these
+  const uint32_t p0 = seg_pair[s0], p1 = seg_pair[s1 - 1];  // the tile's first and last pair
+  // pairs that other tiles have found culled sums of (a hint: of the first 256)
+  const bool known = !REDO && static_cast<uint32_t>(tid) <= p1 - p0 && __ldcg(&run[p0 + tid].culled) != 0;
+  const bool again = REDO && keeper.saved[blockIdx.x] != 0;
   // products [from, from + count) of pairs p to p1 into prod[0..]; the loads of
   // a thread's products are in flight together
   auto stage = [&](uint32_t p, uint32_t from, uint32_t count) {
@@ -318,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
     begin[k] = __ldg(seg_start + s) - j0;
     end[k] = __ldg(seg_start + s + 1) - j0;
   }
-  stage(p0, j0, staged);
+  if (!again) stage(p0, j0, staged);
   __syncthreads();
   ulonglong2 key[WT == 1 ? kRounds : 1];  // on their way while the sums are formed
   if constexpr (WT == 1) {
@@ -330,12 +345,17 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
   for (int k = 0; k < kRounds; ++k) {
     sum[k] = {0.0, 0.0};
     if (s0 + k * kThreads + tid >= s1) continue;
+    if (again) {
+      const double2 v = __ldcs(keeper.sum + s0 + k * kThreads + tid);
+      sum[k] = {v.x, v.y};
+      continue;
+    }
     const uint32_t e = min(end[k], staged);
     for (uint32_t q = begin[k]; q < e; ++q) sum[k] = wgd::cadd(sum[k], c128{prod[q].x, prod[q].y});
   }
   // the last segment may go on behind the staged products: all threads form
   // them, its thread goes on adding
-  for (uint32_t from = j0 + staged; from < j1; from += kStage) {
+  for (uint32_t from = j0 + staged; !again && from < j1; from += kStage) {
     const uint32_t count = min(j1 - from, static_cast<uint32_t>(kStage));
     __syncthreads();
     stage(p1, from, count);
@@ -345,6 +365,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
       if (s0 + k * kThreads + tid == s1 - 1)
         for (uint32_t q = 0; q < count; ++q) sum[k] = wgd::cadd(sum[k], c128{prod[q].x, prod[q].y});
   }
+  bool culls = known;
 #pragma unroll
   for (int k = 0; k < kRounds; ++k) {
     keep[k] = false;
@@ -361,14 +382,27 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
       const bool plain = !isnan(acc.re) && !isnan(acc.im);
       keep[k] = (plain && (fabs(acc.re) > thr || fabs(acc.im) > thr)) || wgd::hypot_ref(acc.re, acc.im) > thr;
       if (!REDO && !keep[k]) {
-        run[p].culled = 1;
-        *any = 1;
+        if (p0 != p1 && __ldcg(&run[p].culled) == 0) run[p].culled = 1;
+        culls = true;
       }
     }
     const uint32_t v = __ballot_sync(0xffffffffu, keep[k]);
     if (lane == 0) bits[k * (kThreads / 32) + warp] = v;
   }
-  __syncthreads();
+  const bool save = __syncthreads_or(culls) && !REDO;
+  if (save) {
+    // a store by every thread with a culled sum would take its turn in L2: 2 ms for 5,000,000
+    if (tid == 0) {
+      if (p0 == p1 && !known) run[p0].culled = 1;
+      if (__ldcg(any) == 0) *any = 1;
+    }
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k) {
+      const uint32_t s = s0 + k * kThreads + tid;
+      if (s < s1) __stcs(keeper.sum + s, make_double2(sum[k].re, sum[k].im));
+    }
+  }
+  if (!REDO && tid == 0) keeper.saved[blockIdx.x] = save;
   if (warp == 0) {
     static_assert(kTile / 32 == 32, "one warp scans the tile");
     const uint32_t c = __popc(bits[lane]);
@@ -400,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, 4) pbatch_pass_kernel(
       // kept holds the survivors of all tiles before
       o = base + (kept[blockIdx.x] + below) - (kept[tile_of[p]] + run[p].below);
     }
-    if (!keep[k]) continue;
+    if (!keep[k] || (save && p0 == p1)) continue;  // one pair: the repetition writes all of it
     if constexpr (WT == 1) {
       ox[o] = key[k].x;
       oz[o] = key[k].y;
@@ -479,6 +513,7 @@ struct wg_products_batch_s {
   wg::Scratch tile_seg;         // uint32[tiles + 1]: first segment that starts in a tile
   wg::Scratch tile_of;          // uint32[n_pairs]: tile of a pair's first segment
   wg::Scratch run, kept;        // PairRun[n_pairs] and `any`, cleared by every run; uint32[tiles + 1]
+  wg::Scratch sums, saved;      // double2[S], uint32[tiles]: SavedSums
   size_t tiles = 0;
   wg::Scratch out_x, out_z, out_c, counts;
 };
@@ -600,6 +635,8 @@ void build_batch(wg_products_batch_s& b, const uint64_t* const* lhs_x, const uin
   }
   b.run.reset(sizeof(PairRun) * np + 16, s);
   b.kept.reset(sizeof(uint32_t) * (b.tiles + 1), s);
+  b.sums.reset(sizeof(double2) * S, s);
+  b.saved.reset(sizeof(uint32_t) * b.tiles, s);
   b.out_x.reset(sizeof(uint64_t) * S * W, s);
   b.out_z.reset(sizeof(uint64_t) * S * W, s);
   b.out_c.reset(sizeof(double) * 2 * S, s);
@@ -635,7 +672,7 @@ void run_batch(wg_products_batch_s& b, cudaStream_t s) {
           pairs, static_cast<uint32_t>(b.n_pairs), b.tile_seg.as<uint32_t>(), b.seg_start.as<uint32_t>(), b.seg_pair.as<uint32_t>(),
           b.seg_keys.as<uint64_t>(), code, b.W, b.atol, b.rtol, run, any, b.kept.as<uint32_t>(),
           b.tile_of.as<uint32_t>(), b.out_x.as<uint64_t>(), b.out_z.as<uint64_t>(), b.out_c.as<double2>(),
-          b.counts.as<uint64_t>()));
+          b.counts.as<uint64_t>(), SavedSums{b.sums.as<double2>(), b.saved.as<uint32_t>()}));
     wg::check_launch("launch batch pass");
   };
   auto both = [&](auto* first, auto* again) {
