@@ -161,16 +161,6 @@ __global__ void pbatch_count_kernel(const uint32_t* __restrict__ seg_pair, size_
 // product with a part beyond 2^1022 or not finite.
 __device__ __noinline__ double product_magnitude(double re, double im) { return wgd::hypot_ref(re, im); }
 
-// The product of a sorted position's code (FP64, no FMA: the reference's rounding).
-__device__ __forceinline__ c128 coded_product(const PairNum& P, uint32_t code) {
-  const uint32_t nr = static_cast<uint32_t>(P.n_r);  // below 2^30
-  const uint32_t q = code >> 2;
-  const uint32_t l = nr == 1 ? q : static_cast<uint32_t>(__umul64hi(static_cast<uint64_t>(q), P.div_m));
-  const double2 av = __ldg(reinterpret_cast<const double2*>(P.lc) + l);
-  const double2 bv = __ldg(reinterpret_cast<const double2*>(P.rc) + (q - l * nr));
-  return wgd::rotate(wgd::cmul(c128{av.x, av.y}, c128{bv.x, bv.y}), code & 3u);
-}
-
 // What a run learns of its pairs (cleared by every run).
 struct PairRun {
   unsigned long long max;  // bits of the largest |product|, as far as the mode needs it
@@ -195,20 +185,73 @@ __device__ __forceinline__ uint32_t pair_within(const PairNum* __restrict__ pair
   return lo;
 }
 
+constexpr int kTile = 1024;      // products whose segments a CTA owns: those that start there
+
+// Products of a warp of pbatch_max_kernel, ROUND of a lane in flight together.
+template <int ROUND>
+constexpr int kMaxItems = ROUND == 1 ? 32 : 64 * ROUND;
+
 // rtol > 0: each pair's largest |product|, ahead of the pass that needs it
 // (non-negative doubles order like their bits; a NaN never replaces the running
-// maximum, std::max's rule).
-__global__ void __launch_bounds__(kThreads) pbatch_max_kernel(const PairNum* __restrict__ pairs, uint32_t n_pairs,
+// maximum, std::max's rule).  A warp takes consecutive products.  The hypot is
+// formed only of products that may exceed what is known: |c| <= sqrt(2) max(|re|,
+// |im|), and a NaN fails the comparison.  18,000,000 products of 20,000 pairs
+// 0.16 ms (0.46 with a look and an atomic by every product).  ROUND = 1 where there
+// are few products: what counts then is the chain of one warp's loads.
+template <int ROUND>
+__global__ void __launch_bounds__(kThreads) pbatch_max_kernel(const PairNum* __restrict__ pairs,
+                                                              const uint32_t* __restrict__ tile_seg,
+                                                              const uint32_t* __restrict__ seg_pair,
                                                               const uint32_t* __restrict__ code, size_t N,
-                                                              PairRun* __restrict__ run) {
-  uint32_t p = 0;
-  for (size_t j = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; j < N;
-       j += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    if (j >= pairs[p].item_end) p = pair_within(pairs, p + 1, n_pairs - 1, j);
-    const c128 c = coded_product(pairs[p], code[j]);
-    const double m = wgd::hypot_ref(c.re, c.im);
-    if (m > __longlong_as_double(static_cast<long long>(run[p].max)))
+                                                              PairRun* run) {
+  const int lane = threadIdx.x & 31;
+  const size_t warps = static_cast<size_t>(gridDim.x) * (kThreads / 32);
+  auto known = [&](uint32_t p) { return __longlong_as_double(static_cast<long long>(__ldcg(&run[p].max))); };
+  // of the lanes that come here together for one pair, those with the largest upper half
+  auto put = [&](uint32_t p, double m) {
+    const uint32_t peers = __match_any_sync(__activemask(), p), high = static_cast<uint32_t>(__double2hiint(m));
+    if (__reduce_max_sync(peers, high) == high && m > 0.0)
       atomicMax(&run[p].max, static_cast<unsigned long long>(__double_as_longlong(m)));
+  };
+  for (size_t w = (blockIdx.x * static_cast<size_t>(kThreads) + threadIdx.x) >> 5; w * kMaxItems<ROUND> < N; w += warps) {
+    const size_t j0 = w * kMaxItems<ROUND>, end = min(N, j0 + kMaxItems<ROUND>);
+    // the pairs of the segments that start in the tile, and of the one that reaches into it
+    const size_t tile = j0 / kTile;
+    const uint32_t first = tile_seg[tile], past = tile_seg[tile + 1];
+    const uint32_t lo = seg_pair[first ? first - 1 : 0], hi = seg_pair[past - 1];
+    uint32_t p = pair_within(pairs, lo, hi, min(j0 + lane, end - 1));
+    double most = known(p), best = 0.0;  // best: what this lane found above what was known
+    for (size_t j = j0 + lane; j - lane < end; j += 32 * ROUND) {
+      uint32_t own[ROUND], c[ROUND];
+      double2 u[ROUND], v[ROUND];
+#pragma unroll
+      for (int k = 0; k < ROUND; ++k) c[k] = __ldg(code + min(j + 32 * k, end - 1));
+#pragma unroll
+      for (int k = 0; k < ROUND; ++k) {
+        own[k] = pair_within(pairs, k ? own[k - 1] : p, hi, min(j + 32 * k, end - 1));
+        const PairNum& P = pairs[own[k]];
+        const uint32_t nr = static_cast<uint32_t>(P.n_r), q = c[k] >> 2;  // below 2^30
+        const uint32_t l = nr == 1 ? q : static_cast<uint32_t>(__umul64hi(static_cast<uint64_t>(q), P.div_m));
+        u[k] = __ldg(reinterpret_cast<const double2*>(P.lc) + l);
+        v[k] = __ldg(reinterpret_cast<const double2*>(P.rc) + (q - l * nr));
+      }
+#pragma unroll
+      for (int k = 0; k < ROUND; ++k) {
+        // behind the end: the last product once more
+        if (own[k] != p) {
+          put(p, best);
+          p = own[k];
+          most = known(p);
+          best = 0.0;
+        }
+        const c128 t = wgd::cmul(c128{u[k].x, u[k].y}, c128{v[k].x, v[k].y});  // the phase leaves |c| as it is
+        if (1.5 * fabs(t.re) <= most && 1.5 * fabs(t.im) <= most) continue;
+        const double m = product_magnitude(t.re, t.im);
+        if (m > most) most = best = m;
+      }
+    }
+    __syncwarp();
+    put(p, best);
   }
 }
 
@@ -233,7 +276,6 @@ __device__ __forceinline__ void write_counts(const PairNum* __restrict__ pairs, 
   }
 }
 
-constexpr int kTile = 1024;             // products whose segments a CTA owns: those that start there
 constexpr int kStage = kTile + kThreads;  // products staged at a time
 
 // The numeric pass.  All threads form products (coalesced codes, gathers of
@@ -673,9 +715,13 @@ void run_batch(wg_products_batch_s& b, cudaStream_t s) {
   auto* pairs = b.pairs.as<PairNum>();
   auto* code = b.code.as<uint32_t>();
   if (max_mode == kMaxFull) {
-    WG_TIMED("pbatch_max_kernel", s,
-      pbatch_max_kernel<<<wg::grid_for(b.N, kThreads, device, 8), kThreads, 0, s>>>(pairs, static_cast<uint32_t>(b.n_pairs),
-                                                                                       code, b.N, run));
+    auto maxima = [&](auto* kernel, int items) {
+      const unsigned g = wg::grid_for(b.N, kThreads / 32 * items, device, 4);
+      WG_TIMED("pbatch_max_kernel", s,
+        kernel<<<g, kThreads, 0, s>>>(pairs, b.tile_seg.as<uint32_t>(), b.seg_pair.as<uint32_t>(), code, b.N, run));
+    };
+    if (b.N < (size_t{1} << 20)) maxima(pbatch_max_kernel<1>, kMaxItems<1>);
+    else maxima(pbatch_max_kernel<4>, kMaxItems<4>);
     wg::check_launch("launch batch maxima");
   }
   auto pass = [&](auto* kernel, const char* name) {
