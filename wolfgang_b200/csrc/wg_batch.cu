@@ -199,7 +199,7 @@ constexpr int kMaxItems = ROUND == 1 ? 32 : 64 * ROUND;
 // 0.16 ms (0.46 with a look and an atomic by every product).  ROUND = 1 where there
 // are few products: what counts then is the chain of one warp's loads.
 template <int ROUND>
-__global__ void __launch_bounds__(kThreads) pbatch_max_kernel(const PairNum* __restrict__ pairs,
+__global__ void __launch_bounds__(kThreads, ROUND == 1 ? 8 : 4) pbatch_max_kernel(const PairNum* __restrict__ pairs,
                                                               const uint32_t* __restrict__ tile_seg,
                                                               const uint32_t* __restrict__ seg_pair,
                                                               const uint32_t* __restrict__ code, size_t N,
@@ -715,13 +715,13 @@ void run_batch(wg_products_batch_s& b, cudaStream_t s) {
   auto* pairs = b.pairs.as<PairNum>();
   auto* code = b.code.as<uint32_t>();
   if (max_mode == kMaxFull) {
-    auto maxima = [&](auto* kernel, int items) {
-      const unsigned g = wg::grid_for(b.N, kThreads / 32 * items, device, 4);
+    auto maxima = [&](auto* kernel, int items, int ctas) {  // resident CTAs an SM
+      const unsigned g = wg::grid_for(b.N, kThreads / 32 * items, device, ctas);
       WG_TIMED("pbatch_max_kernel", s,
         kernel<<<g, kThreads, 0, s>>>(pairs, b.tile_seg.as<uint32_t>(), b.seg_pair.as<uint32_t>(), code, b.N, run));
     };
-    if (b.N < (size_t{1} << 20)) maxima(pbatch_max_kernel<1>, kMaxItems<1>);
-    else maxima(pbatch_max_kernel<4>, kMaxItems<4>);
+    if (b.N < (size_t{1} << 20)) maxima(pbatch_max_kernel<1>, kMaxItems<1>, 8);
+    else maxima(pbatch_max_kernel<4>, kMaxItems<4>, 4);
     wg::check_launch("launch batch maxima");
   }
   auto pass = [&](auto* kernel, const char* name) {
