@@ -63,6 +63,9 @@ constexpr int kChunkPieces = 128;        // pieces of one forward item
 constexpr int kFwdThreads = 512;         // two sets of 256 x 16 amplitudes = a tile
 constexpr int kFwdInner = 8;             // warps of a set
 constexpr int kAdjThreads = 512;         // x 8 amplitudes = a tile
+// Least work of a split, in the costs of make_plan (a sub-group 90): its sums are written
+// and read again.  Half of it where these are less than a whole tile's.
+constexpr uint32_t kSplitCost = 400;
 constexpr uint32_t kDiagFlag = 4;        // ty bit: the term's group has x == 0
 constexpr uint32_t kTwiceFlag = 8;       // ty bit: the forward pass meets every pair of the group twice
 
@@ -73,12 +76,12 @@ struct __align__(16) FwdPiece {
   uint32_t t0;
   uint8_t nk, odd;
   uint8_t pair;              // even terms, and the next piece has the sub-group's odd ones: taken together
-  uint8_t turn;              // the set of threads that takes it (kDirect: of a chunk that reads psi itself)
+  uint8_t turn;              // the set of threads that takes it
   uint32_t zlo[kPiece];      // z within the tile
   uint32_t zhi[kPiece];      // and above it
 };
 static_assert(sizeof(FwdPiece) == 80, "copied in 16-byte pieces");
-constexpr uint8_t kDirect = 0x80;
+constexpr uint32_t kReads = 0x80000000u;  // chunk bit: its pieces read psi themselves
 
 // A sub-group: terms [t0, t0 + nre) of even y, then nim of odd y.  A sign word has the even terms' signs in bits
 // 3-10, the odd ones' in bits 19-26: byte offsets into the tables.
@@ -115,7 +118,7 @@ struct PlanDev {
   const FwdPiece* piece;     // [NP]
   AdjSub* asub;              // [S]
   const SegDev* seg;         // [NS]
-  const uint32_t* chunk;     // [chunks + 1] first piece of a chunk
+  const uint32_t* chunk;     // [chunks + 1] first piece of a chunk | kReads
   const uint32_t* bounds;    // [splits + 1] segments of the splits
   const uint32_t* ty;        // [T] y mod 4 | flags
   const uint32_t* torig;     // [T] original index of sorted term
@@ -130,6 +133,8 @@ struct wg_plan_host {
   int device;
   PlanDev dev;
   size_t n_groups = 0;
+  uint32_t chunk_most = 0;   // pieces of the largest chunk
+  uint64_t tile_cost = 0;    // the adjoint's work on a tile, in SegDev's costs
   wg::Scratch mem;  // all of the above
 };
 
@@ -170,6 +175,9 @@ struct PairDev {
   double* result;   // E output or null
   double* hpsi;     // H psi output or null
   double2* part;    // splits x 2^n partial H psi, or null
+  uint32_t group;   // chunks of a forward item
+  uint32_t per_range;  // forward items of a range of tiles
+  uint64_t fold;    // an adjoint item takes all splits of its tile, one after another
 };
 
 // A launch over one or several pairs (kernel parameter).  A single pair travels in
@@ -281,7 +289,7 @@ struct FwdShared {
   FwdPiece piece[kChunkPieces];
   uint32_t seg_xhi[kChunkPieces];
   uint32_t seg_at[kChunkPieces + 1];
-  uint32_t segs;
+  uint32_t segs, reads;
   unsigned long long item;
   PairDev pair;
 };
@@ -397,8 +405,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(const __
     const void* psi = Q.psi;
     const uint32_t r = static_cast<uint32_t>(item);
     // ranges outermost: the CTAs that run together meet the same tiles in L2
-    const uint32_t range = r / P.chunks, chunk = r - range * P.chunks;
-    const uint32_t piece0 = P.chunk[chunk], pieces = P.chunk[chunk + 1] - piece0;
+    const uint32_t range = r / Q.per_range, chunk = (r - range * Q.per_range) * Q.group;
+    const uint32_t taken = min(Q.group, P.chunks - chunk);
+    const uint32_t piece0 = P.chunk[chunk] & ~kReads, pieces = (P.chunk[chunk + taken] & ~kReads) - piece0;
     const int m = P.m, n = P.n;
     const uint32_t J0 = static_cast<uint32_t>(static_cast<uint64_t>(P.tiles) * range / P.ranges);
     const uint32_t J1 = static_cast<uint32_t>(static_cast<uint64_t>(P.tiles) * (range + 1) / P.ranges);
@@ -410,7 +419,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(const __
       for (uint32_t i = lane; i < pieces * kPiece; i += 32)
         if (warp < kFwdInner) sh.acc[warp][i] = 0.0;
       if (warp == kFwdInner) {
-        uint32_t segs = 0;
+        uint32_t segs = 0, reads = kReads;  // of all of the item's chunks
+        for (uint32_t c = lane; c < taken; c += 32) reads &= P.chunk[chunk + c];
         for (uint32_t at = 0; at < pieces; at += 32) {
           const uint32_t i = at + lane;
           const bool in = i < pieces;
@@ -424,7 +434,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(const __
           }
           segs += __popc(heads);
         }
+        const bool all = __all_sync(0xffffffffu, (reads & kReads) != 0);
         if (lane == 0) {
+          sh.reads = all;
           sh.segs = segs;
           sh.seg_at[segs] = pieces;
         }
@@ -448,14 +460,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) expect_forward_kernel(const __
     // a segment with x above the tile pairs J with J ^ xhi once, from the side
     // whose lowest bit of xhi is clear
     auto this_side = [](uint32_t J, uint32_t xhi) { return xhi == 0 || !((J >> (__ffs(static_cast<int>(xhi)) - 1)) & 1u); };
-    if (sh.piece[0].turn & kDirect) {
+    if (sh.reads) {
       // hardly two pieces of a class: each reads the paired tile itself, and
       // nothing waits for the others
       for (uint32_t J = J0; J < J1; ++J) {
         load_own(J);
         for (uint32_t i = 0; i < pieces; i += sh.piece[i].pair ? 2 : 1) {
           const FwdPiece* pd = sh.piece + i;
-          if ((pd->turn & ~kDirect) != slice || !this_side(J, pd->xhi)) continue;
+          if (pd->turn != slice || !this_side(J, pd->xhi)) continue;
           const Amp* from = static_cast<const Amp*>(psi) + (static_cast<uint64_t>(J ^ pd->xhi) << kTileBits);
           auto load = [&](uint32_t i) {
             const c128 v = load_amp<Amp>(from, i);
@@ -712,10 +724,12 @@ __global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(const __
     const PairDev& Q = sh.pair;
     const PlanDev& P = Q.plan;
     const void* psi = Q.psi;
-    const uint32_t splits = P.splits;
+    const uint32_t splits = P.splits, parts = Q.fold ? 1 : splits;  // items of a tile
     // tiles outermost: the CTAs that run together share tiles and segments
-    const uint32_t J = static_cast<uint32_t>(item / splits), split = static_cast<uint32_t>(item - static_cast<uint64_t>(J) * splits);
-    const uint32_t g0 = P.bounds[split], g1 = P.bounds[split + 1];
+    const uint32_t J = static_cast<uint32_t>(item / parts);
+    uint32_t split = static_cast<uint32_t>(item - static_cast<uint64_t>(J) * parts);
+    const uint32_t g0 = P.bounds[split], g1 = P.bounds[Q.fold ? splits : split + 1];
+    uint32_t split_end = P.bounds[split + 1];
     const int m = P.m, n = P.n;
     const int tt = tid & ((1 << (m - 3)) - 1);
     const uint32_t slice = tid >> (m - 3), slices = kAdjThreads >> (m - 3);
@@ -765,6 +779,51 @@ __global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(const __
         }
       }
       __syncthreads();
+      if (g + 1 == split_end) {
+        // the split's sums: stored, or added to those of the splits before (the order of expect_join_kernel)
+        if (slices > 1) {
+          // the slices' sums, slice by slice, behind the tile (what is fetched meanwhile lies in front)
+          if (slice > 0) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+              const uint32_t j = tt + (static_cast<uint32_t>(r) << (m - 3));
+              sh.tile[0][(slice << m) + j] = make_double2(acc[r].re, acc[r].im);
+            }
+          }
+          __syncthreads();
+          if (slice == 0) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+              const uint32_t j = tt + (static_cast<uint32_t>(r) << (m - 3));
+              for (uint32_t v = 1; v < slices; ++v) {
+                const double2 o = sh.tile[0][(v << m) + j];
+                acc[r].re += o.x;
+                acc[r].im += o.y;
+              }
+            }
+          }
+        }
+        if (slice == 0) {
+          double2* out = parts > 1 ? Q.part + (static_cast<uint64_t>(split) << n) : reinterpret_cast<double2*>(Q.hpsi);
+          const bool add = parts == 1 && split > 0;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const uint64_t j = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(r) << (m - 3));
+            if ((j >> n) != 0) continue;
+            double2 v = make_double2(acc[r].re, acc[r].im);
+            if (add) {
+              const double2 before = out[j];
+              v.x += before.x;
+              v.y += before.y;
+            }
+            out[j] = v;
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) acc[r] = {0.0, 0.0};
+        ++split;
+        if (!last) split_end = P.bounds[split + 1];
+      }
       if (fresh_n) slot ^= 1;
       fresh = fresh_n;
       stage ^= 1;
@@ -772,35 +831,6 @@ __global__ void __launch_bounds__(kAdjThreads, 1) expect_adjoint_kernel(const __
       nx = after;
     }
     copy_wait<0>();
-    if (slices > 1) {
-      // the slices' sums, slice by slice (the tile buffers are free)
-      __syncthreads();
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const uint32_t j = tt + (static_cast<uint32_t>(r) << (m - 3));
-        sh.tile[0][(slice << m) + j] = make_double2(acc[r].re, acc[r].im);
-      }
-      __syncthreads();
-      if (slice == 0) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const uint32_t j = tt + (static_cast<uint32_t>(r) << (m - 3));
-          for (uint32_t v = 1; v < slices; ++v) {
-            const double2 o = sh.tile[0][(v << m) + j];
-            acc[r].re += o.x;
-            acc[r].im += o.y;
-          }
-        }
-      }
-    }
-    if (slice == 0) {
-      double2* out = splits > 1 ? Q.part + (static_cast<uint64_t>(split) << n) : reinterpret_cast<double2*>(Q.hpsi);
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const uint64_t j = (static_cast<uint64_t>(J) << m) + tt + (static_cast<uint32_t>(r) << (m - 3));
-        if ((j >> n) == 0) out[j] = make_double2(acc[r].re, acc[r].im);
-      }
-    }
   }
 }
 
@@ -1030,11 +1060,12 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
     i = e;
   }
   // The adjoint's tiles are split by segments until there are about four items
-  // an SM.  The plan alone sets the splits, so that a pair's H psi has the same
-  // bits in every batch.
+  // an SM.  The plan alone sets the splits and with them the order of the sums, so
+  // that a pair's H psi has the same bits in every batch, however that runs them.
   if (adjoint) {
     const size_t NS = seg.size();
-    const size_t splits = std::max<size_t>(1, std::min<size_t>({(4 * sms + d.tiles / 2) / d.tiles, NS, 64}));
+    const size_t splits = std::max<size_t>(
+        1, std::min<size_t>({(4 * sms + d.tiles / 2) / d.tiles, NS, 64, seg_cost.back() / (m < kTileBits ? kSplitCost / 2 : kSplitCost)}));
     bounds.push_back(0);
     for (size_t k = 1; k < splits; ++k) {
       // the segment at which k / splits of the work is done; each split takes one at least
@@ -1044,6 +1075,7 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
       bounds.push_back(static_cast<uint32_t>(at));
     }
     bounds.push_back(static_cast<uint32_t>(NS));
+    p->tile_cost = seg_cost.back();
     d.splits = static_cast<uint32_t>(splits);
   }
   // Forward items: chunks of pieces (their sums stay in shared memory) times
@@ -1052,6 +1084,7 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
   const size_t chunk_pieces = std::min<size_t>(
       kChunkPieces, std::max<size_t>(sets, (NP * d.tiles + 4 * sms - 1) / (4 * sms)));
   std::vector<uint32_t> load(sets);
+  bool was_direct = false;
   for (size_t i = 0; i < NP;) {
     size_t e = i, units = 0, segs = 0;
     while (e < NP && e - i + 1 + piece[e].pair <= chunk_pieces) {
@@ -1064,7 +1097,11 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
     const bool direct = m == kTileBits && static_cast<int>(n) > m && 4 * units <= 5 * segs;
     // the sets' turns: the least loaded one of the segment's (of the chunk's
     // where nothing is staged); a last pair is shared by two equally loaded ones
-    std::fill(load.begin(), load.end(), 0u);
+    // A class that goes on from the chunk before goes on with its loads: an item may
+    // take several chunks together.
+    const bool goes_on = !direct && i > 0 && !was_direct && piece[i].xhi == piece[i - 1].xhi;
+    if (!goes_on) std::fill(load.begin(), load.end(), 0u);
+    was_direct = direct;
     for (size_t k = i; k < e;) {
       if (!direct && k > i && piece[k].xhi != piece[k - 1].xhi) std::fill(load.begin(), load.end(), 0u);
       const size_t next = k + 1 + piece[k].pair;
@@ -1072,9 +1109,11 @@ wg_plan_host* make_plan(int device, size_t n, size_t T, const uint64_t* x, const
       const bool last = !direct && (next >= e || piece[next].xhi != piece[k].xhi);
       if (piece[k].pair && last && std::count(load.begin(), load.end(), load[to]) > 1) piece[k].pair = 0;
       load[to] += 1u + piece[k].pair;
-      piece[k].turn = static_cast<uint8_t>(to | (direct ? kDirect : 0));
+      piece[k].turn = static_cast<uint8_t>(to);
       k += 1 + piece[k].pair;
     }
+    if (direct) chunk.back() |= kReads;
+    p->chunk_most = std::max(p->chunk_most, static_cast<uint32_t>(e - i));
     chunk.push_back(static_cast<uint32_t>(e));
     i = e;
   }
@@ -1163,34 +1202,93 @@ void allow_smem(int device) {
   });
 }
 
-wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int dtype, cudaStream_t s) {
+// How a batch divides its pairs.  A plan is divided as if it had the device for itself;
+// among others a pair takes several of its chunks in one forward item, and the splits
+// of a tile one after another in one adjoint item: what an item fetches, and the sums
+// that a split writes and reads, then serve more terms.  Neither changes a bit.  64
+// pairs of 14 qubits and 1,000 terms with H psi 2.47 -> 1.05 ms, 400 of 100 terms 6.5
+// -> 1.63; 30 pairs of 8 to 18 qubits 2.02 -> 1.77; and no partial H psi for most pairs
+// (up to 37 MB each, now 1 GB at most in all: the tiles that are still split are fewer
+// than three an SM, of 64 splits at most).
+struct Division {
+  double forward = 0.0;  // pieces x tiles of a forward item, at most
+  double adjoint = 0.0;  // tiles of at most this cost are one adjoint item
+};
+
+// Forward items: four for every SM, and at least eight pieces x tiles.  Adjoint items:
+// a tile that is no more than 1.35 of an SM's share of the batch, as long as the SMs'
+// last turn at such tiles is not mostly empty, else of a third.
+Division divide_batch(const std::vector<RunSpec>& specs, int sms) {
+  Division d;
+  if (specs.size() <= 1) return d;
+  double fwd = 0.0, adj = 0.0;
+  for (const RunSpec& r : specs) {
+    fwd += static_cast<double>(r.plan->dev.NP) * r.plan->dev.tiles;
+    if (r.hpsi) adj += static_cast<double>(r.plan->tile_cost) * r.plan->dev.tiles;
+  }
+  d.forward = std::max(8.0, fwd / (4.0 * sms));
+  const double share = adj / sms;
+  d.adjoint = 1.35 * share;
+  uint64_t large = 0;  // items above a third of the share
+  for (const RunSpec& r : specs) {
+    const double cost = static_cast<double>(r.plan->tile_cost);
+    if (r.hpsi && cost > share / 3.0 && cost <= d.adjoint) large += r.plan->dev.tiles;
+  }
+  const uint64_t turns = (large + sms - 1) / sms;
+  if (3 * large < 2 * turns * sms) d.adjoint = share / 3.0;
+  return d;
+}
+
+// The pairs in order of their adjoint items' work, largest first: the queue ends with
+// the small ones.
+std::vector<RunSpec> by_work(const std::vector<RunSpec>& specs) {
+  std::vector<RunSpec> out(specs);
+  std::stable_sort(out.begin(), out.end(), [](const RunSpec& a, const RunSpec& b) {
+    return a.plan->tile_cost * (a.hpsi ? 1 : 0) > b.plan->tile_cost * (b.hpsi ? 1 : 0);
+  });
+  return out;
+}
+
+wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& given, int dtype, cudaStream_t s) {
   if (dtype != WG_DTYPE_C128 && dtype != WG_DTYPE_C64) wg::throw_invalid("psi dtype must be complex64 or complex128");
   std::unique_ptr<wg_expect_batch_s> b(new wg_expect_batch_s());
   b->device = device;
   b->dtype = dtype;
   b->sms = wg::device_props(device).sm_count;
   allow_smem(device);
+  const std::vector<RunSpec> specs = by_work(given);
   const size_t np = specs.size();
   if (np > 0xffffffffull) wg::throw_invalid("too many pairs in one batch");
   std::vector<PairDev> pairs(np);
   std::vector<uint64_t> item_base(np + 1, 0), term_base(np + 1, 0), tile_base(np + 1, 0), amp_base(np + 1, 0);
+  const Division division = divide_batch(specs, b->sms);
   uint64_t bytes = 0;  // of the partial H psi and the term values, then where they lie
   std::vector<uint64_t> part_at(np, 0), ev_at(np, 0);
   for (size_t i = 0; i < np; ++i) {
     const PlanDev& P = specs[i].plan->dev;
     // tile numbers are 32 bits; no device holds a larger state
     if (P.n > kTileBits + 31) wg::throw_invalid("expectation_statevector: the statevector exceeds device memory");
-    pairs[i] = PairDev{P, specs[i].psi, specs[i].term_values, specs[i].result, specs[i].hpsi, nullptr};
-    item_base[i + 1] = item_base[i] + (P.T ? static_cast<uint64_t>(P.chunks) * P.ranges : 0);
+    const wg_plan_host& h = *specs[i].plan;
+    uint32_t group = 1;
+    if (np > 1 && P.T) {
+      const double chunk_work = static_cast<double>(P.NP) / P.chunks * P.tiles / P.ranges;  // of an item of one chunk
+      group = static_cast<uint32_t>(
+          std::max(1.0, std::min<double>(division.forward / chunk_work, kChunkPieces / h.chunk_most)));
+    }
+    const bool fold = P.splits > 1 && static_cast<double>(h.tile_cost) <= division.adjoint;
+    const uint32_t parts = fold ? 1 : P.splits;
+    pairs[i] = PairDev{P, specs[i].psi, specs[i].term_values, specs[i].result, specs[i].hpsi, nullptr, group,
+                       (P.chunks + group - 1) / group, fold};
+    item_base[i + 1] = item_base[i] + (P.T ? static_cast<uint64_t>(pairs[i].per_range) * P.ranges : 0);
     term_base[i + 1] = term_base[i] + (P.joined ? 0 : P.T);
     tile_base[i + 1] = tile_base[i];
     amp_base[i + 1] = amp_base[i];
     if (specs[i].hpsi && P.T) {
-      tile_base[i + 1] += static_cast<uint64_t>(P.tiles) * P.splits;
-      if (P.splits > 1) {
+      tile_base[i + 1] += static_cast<uint64_t>(P.tiles) * parts;
+      if (parts > 1) {
         amp_base[i + 1] += uint64_t{1} << P.n;
         part_at[i] = bytes;
-        bytes += static_cast<uint64_t>(P.splits) << (P.n + 4);
+        bytes += static_cast<uint64_t>(parts) << (P.n + 4);
       }
     }
     if (!specs[i].term_values && !P.joined && P.T) {
@@ -1204,7 +1302,7 @@ wg_expect_batch_s* make_batch(int device, const std::vector<RunSpec>& specs, int
     auto* base = b->parts.as<unsigned char>();
     for (size_t i = 0; i < np; ++i) {
       const PlanDev& P = pairs[i].plan;
-      if (pairs[i].hpsi && P.T && P.splits > 1) pairs[i].part = reinterpret_cast<double2*>(base + part_at[i]);
+      if (pairs[i].hpsi && P.T && P.splits > 1 && !pairs[i].fold) pairs[i].part = reinterpret_cast<double2*>(base + part_at[i]);
       if (!pairs[i].evals && !P.joined && P.T) pairs[i].evals = reinterpret_cast<double*>(base + ev_at[i]);
     }
   }
