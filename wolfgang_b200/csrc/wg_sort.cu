@@ -277,17 +277,34 @@ struct SoaWords {
 };
 
 __global__ void __launch_bounds__(256) soa_code_kernel(SoaWords src, int K, const unsigned long long* __restrict__ bits,
-                                                       CodeSpec spec, int passes, uint64_t* __restrict__ packed,
-                                                       uint64_t* __restrict__ code, uint32_t* hist) {
+                                                       CodeSpec spec, int passes, uint64_t* __restrict__ code,
+                                                       uint32_t* hist) {
   extern __shared__ uint32_t sh[];
   clear_digits(sh, passes);
   __syncthreads();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < src.n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    pack_key(bits, K, [&](int k) { return src(i, k); },
-             [&](int w, uint64_t v) { packed[static_cast<size_t>(w) * src.n + i] = v; }, spec.words);
+    // the packed key's words as the code asks for them, one after another
+    int k = 0, base = 0;  // next key word, varying bits before it
+    uint64_t rest = 0;    // of that word, what belongs to the next packed one
     bool whole;
-    const uint64_t c = key_code(spec, [&](int w) { return packed[static_cast<size_t>(w) * src.n + i]; }, &whole);
+    const uint64_t c = key_code(spec, [&](int w) {
+      uint64_t cur = rest;
+      rest = 0;
+      while (k < K && base < 64 * (w + 1)) {
+        const uint64_t m = bits[k];
+        uint64_t v = src(i, k) & m;
+        while (v) {
+          const int b = 63 - __clzll(static_cast<long long>(v));
+          v ^= uint64_t{1} << b;
+          const int r = base + __popcll(m & ~((uint64_t{2} << b) - 1));
+          (r < 64 * (w + 1) ? cur : rest) |= 0x8000000000000000ull >> (r & 63);
+        }
+        base += __popcll(m);
+        ++k;
+      }
+      return cur;
+    }, &whole);
     code[i] = c;
     count_digits(sh, c, passes);
   }
@@ -295,25 +312,19 @@ __global__ void __launch_bounds__(256) soa_code_kernel(SoaWords src, int K, cons
   store_digits(sh, passes, hist);
 }
 
-// The packed words alone.
-__global__ void __launch_bounds__(256) soa_pack_kernel(SoaWords src, int K, const unsigned long long* __restrict__ bits,
-                                                       int words, uint64_t* __restrict__ packed) {
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < src.n;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x)
-    pack_key(bits, K, [&](int k) { return src(i, k); },
-             [&](int w, uint64_t v) { packed[static_cast<size_t>(w) * src.n + i] = v; }, words);
-}
-
-// The top 8 * passes bits of one packed word as code, read through the order so far.
-__global__ void __launch_bounds__(256) soa_word_kernel(const uint64_t* __restrict__ packed, size_t n, int w, int passes,
-                                                       const uint32_t* __restrict__ order, uint64_t* __restrict__ code,
-                                                       uint32_t* hist) {
+// The varying bits of key word k as code, read through the order so far.
+__global__ void __launch_bounds__(256) soa_word_kernel(SoaWords src, int k, const unsigned long long* __restrict__ bits,
+                                                       int passes, const uint32_t* __restrict__ order,
+                                                       uint64_t* __restrict__ code, uint32_t* hist) {
   extern __shared__ uint32_t sh[];
   clear_digits(sh, passes);
   __syncthreads();
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
+  const uint64_t m = bits[k];
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < src.n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const uint64_t c = packed[static_cast<size_t>(w) * n + (order ? order[i] : i)] >> (64 - 8 * passes);
+    uint64_t c = 0;
+    for (uint64_t v = src(order ? order[i] : i, k) & m; v; v &= v - 1)
+      c |= uint64_t{1} << __popcll(m & ((v & (0 - v)) - 1));
     code[i] = c;
     count_digits(sh, c, passes);
   }
@@ -323,16 +334,16 @@ __global__ void __launch_bounds__(256) soa_word_kernel(const uint64_t* __restric
 
 // Equal neighbouring codes of unequal keys: the codes did not sort the keys.
 __global__ void __launch_bounds__(256) soa_check_kernel(const uint64_t* __restrict__ code,
-                                                        const uint32_t* __restrict__ order,
-                                                        const uint64_t* __restrict__ packed, size_t n, int words,
+                                                        const uint32_t* __restrict__ order, SoaWords src, int K,
                                                         SortControl* ctl) {
+  const size_t n = src.n;
   if (ctl->timeout) return;  // the order is not whole
   bool mixed = false;
   for (size_t i = 1 + blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     if (code[i] != code[i - 1]) continue;
     const size_t a = order[i], b = order[i - 1];
-    for (int w = 0; w < words; ++w) mixed |= packed[static_cast<size_t>(w) * n + a] != packed[static_cast<size_t>(w) * n + b];
+    for (int k = 0; k < K; ++k) mixed |= src(a, k) != src(b, k);
   }
   if (mixed) ctl->mixed = 1;
 }
@@ -342,11 +353,11 @@ __global__ void __launch_bounds__(256) soa_check_kernel(const uint64_t* __restri
 constexpr uint32_t kTieRun = 64;
 
 __global__ void __launch_bounds__(256) soa_ties_kernel(const uint64_t* __restrict__ code, uint32_t* order,
-                                                       const uint64_t* __restrict__ packed, size_t n, int words,
-                                                       SortControl* ctl) {
+                                                       SoaWords src, int K, SortControl* ctl) {
+  const size_t n = src.n;
   auto compare = [&](uint32_t a, uint32_t b) {
-    for (int w = 0; w < words; ++w) {
-      const uint64_t u = packed[static_cast<size_t>(w) * n + a], v = packed[static_cast<size_t>(w) * n + b];
+    for (int k = 0; k < K; ++k) {
+      const uint64_t u = src(a, k), v = src(b, k);
       if (u != v) return u < v ? -1 : 1;
     }
     return 0;
@@ -373,14 +384,19 @@ __global__ void __launch_bounds__(256) soa_ties_kernel(const uint64_t* __restric
 }
 
 __global__ void __launch_bounds__(256) soa_gather_kernel(SoaWords src, int K, const uint32_t* __restrict__ order,
-                                                         const uint32_t* __restrict__ idx, uint64_t* __restrict__ keys,
-                                                         uint32_t* __restrict__ out) {
+                                                         uint64_t* __restrict__ keys) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < src.n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const uint32_t o = order[i];
     for (int k = 0; k < K; ++k) keys[static_cast<size_t>(k) * src.n + i] = src(o, k);
-    out[i] = idx[o];
   }
+}
+
+__global__ void __launch_bounds__(256) soa_index_kernel(size_t n, const uint32_t* __restrict__ order,
+                                                        const uint32_t* __restrict__ idx, uint32_t* __restrict__ out) {
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x)
+    out[i] = idx[order[i]];
 }
 
 __global__ void __launch_bounds__(kBlockSortThreads) soa_block_kernel(SoaWords src, int K,
@@ -404,13 +420,16 @@ namespace wg {
 
 // Keys varying in at most 64 bits are sorted by those bits; wider ones by
 // their codes, and only if some equal codes turn out to stand for different
-// keys by all their packed words.  `alike`: the keys are known to agree in long
+// keys by all their words.  `alike`: the keys are known to agree in long
 // stretches, so that codes would tie: the words at once.
+// Device memory beside the keys and indices: 24 bytes an item while the pairs are
+// sorted, then 4 and a second copy of the indices, then of the keys.
 void radix_sort_keys(int device, size_t n, int K, Scratch& keys, Scratch& idx, cudaStream_t s, bool alike) {
   if (n <= 1 || K == 0) return;
+  if (n > 0xffffffffull) throw_invalid("sort item count exceeds the index range");
   const SoaWords src{keys.as<uint64_t>(), n};
-  Scratch keys2(sizeof(uint64_t) * K * n, s), idx2(sizeof(uint32_t) * n, s);
   if (n <= static_cast<size_t>(kBlockSortItems)) {
+    Scratch keys2(sizeof(uint64_t) * K * n, s), idx2(sizeof(uint32_t) * n, s);
     allow_smem(soa_block_kernel, sizeof(BlockSort));
     WG_TIMED("soa_block_kernel", s,
       soa_block_kernel<<<1, kBlockSortThreads, sizeof(BlockSort), s>>>(src, K, idx.as<uint32_t>(),
@@ -420,75 +439,84 @@ void radix_sort_keys(int device, size_t n, int K, Scratch& keys, Scratch& idx, c
     std::swap(idx, idx2);
     return;
   }
-  if (n > 0xffffffffull) throw_invalid("sort item count exceeds the index range");
   KeyBits kb = key_bits(device, K, n, src, size_t{0}, src, s);
   CodeSpec spec = choose_code(kb, n);
   if (!spec.exact) spec.nb = 64;  // ties cost more here than in a reduction
   const int passes = kb.B == 0 ? 0 : (spec.nb + 7) / 8;
   if (passes == 0) return;  // every key is the same
+  const auto* bits = kb.masks.as<unsigned long long>();
   const size_t tiles = pair_tiles(n);
-  Scratch pairs(2 * (sizeof(uint64_t) + sizeof(uint32_t)) * n, s), packed(sizeof(uint64_t) * spec.words * n, s);
+  // the codes and one of the item arrays go when the order, in the other, is known
+  Scratch pairs((2 * sizeof(uint64_t) + sizeof(uint32_t)) * n, s), order(sizeof(uint32_t) * n, s);
   const size_t zero_bytes = sizeof(uint64_t) * kDigits * tiles + sizeof(uint32_t) * kDigits * kMaxPasses + sizeof(SortControl);
   Scratch zero(zero_bytes, s);
   check_cuda(cudaMemsetAsync(zero.get(), 0, zero_bytes, s), "clear sort state");
   PairBuffers b{};
   b.k0 = pairs.as<uint64_t>();
   b.k1 = b.k0 + n;
-  b.i0 = reinterpret_cast<uint32_t*>(b.k1 + n);
-  b.i1 = b.i0 + n;
+  b.i0 = order.as<uint32_t>();
+  b.i1 = reinterpret_cast<uint32_t*>(b.k1 + n);
+  if (passes % 2) std::swap(b.i0, b.i1);
   b.status = zero.as<unsigned long long>();
   b.hist = reinterpret_cast<uint32_t*>(b.status + kDigits * tiles);
   b.control = reinterpret_cast<SortControl*>(b.hist + kDigits * kMaxPasses);
   const unsigned g = grid_for(n, 256, device, 4);
   SortControl h{};
-  h.mixed = alike && !spec.exact;
-  if (h.mixed) {
-    WG_TIMED("soa_pack_kernel", s,
-      soa_pack_kernel<<<g, 256, 0, s>>>(src, K, kb.masks.as<unsigned long long>(), spec.words, packed.as<uint64_t>()));
-    check_launch("launch sort words");
-  } else {
+  auto outcome = [&] {  // of the look-backs too, which is known only now
+    check_cuda(cudaMemcpyAsync(&h, b.control, sizeof(h), cudaMemcpyDeviceToHost, s), "read sort state");
+    check_cuda(cudaStreamSynchronize(s), "read sort state");
+    if (h.timeout) throw Error(WG_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors");
+  };
+  bool by_words = alike && !spec.exact;
+  if (!by_words) {
     allow_smem(soa_code_kernel, digit_smem(kMaxPasses));
     WG_TIMED("soa_code_kernel", s,
-      soa_code_kernel<<<g, 256, digit_smem(passes), s>>>(src, K, kb.masks.as<unsigned long long>(), spec, passes,
-                                                         packed.as<uint64_t>(), b.k0, b.hist));
+      soa_code_kernel<<<g, 256, digit_smem(passes), s>>>(src, K, bits, spec, passes, b.k0, b.hist));
     check_launch("launch sort codes");
     sort_pairs(n, b, passes, true, s);
     if (!spec.exact) {
-      soa_check_kernel<<<g, 256, 0, s>>>(b.k0, b.i0, packed.as<uint64_t>(), n, spec.words, b.control);
+      soa_check_kernel<<<g, 256, 0, s>>>(b.k0, b.i0, src, K, b.control);
       check_launch("launch sort check");
     }
-    // the look-backs' outcome is known only here
-    check_cuda(cudaMemcpyAsync(&h, b.control, sizeof(h), cudaMemcpyDeviceToHost, s), "read sort state");
-    check_cuda(cudaStreamSynchronize(s), "read sort state");
-    if (h.mixed && !h.timeout) {
+    outcome();
+    if (h.mixed) {
       check_cuda(cudaMemsetAsync(b.control, 0, sizeof(SortControl), s), "clear sort state");
-      WG_TIMED("soa_ties_kernel", s,
-        soa_ties_kernel<<<g, 256, 0, s>>>(b.k0, b.i0, packed.as<uint64_t>(), n, spec.words, b.control));
+      WG_TIMED("soa_ties_kernel", s, soa_ties_kernel<<<g, 256, 0, s>>>(b.k0, b.i0, src, K, b.control));
       check_launch("launch sort ties");
-      check_cuda(cudaMemcpyAsync(&h, b.control, sizeof(h), cudaMemcpyDeviceToHost, s), "read sort state");
-      check_cuda(cudaStreamSynchronize(s), "read sort state");
+      outcome();
     }
+    by_words = h.mixed != 0;
   }
-  if (h.mixed && !h.timeout) {
+  if (by_words) {
     allow_smem(soa_word_kernel, digit_smem(kMaxPasses));
-    for (int w = spec.words - 1; w >= 0 && !h.timeout; --w) {
-      const int count = (std::min(64, kb.B - 64 * w) + 7) / 8;
+    bool first = true;
+    for (int k = K - 1; k >= 0; --k) {
+      const int count = (kb.vary[k] + 7) / 8;
+      if (count == 0) continue;
       check_cuda(cudaMemsetAsync(zero.get(), 0, zero_bytes, s), "clear sort state");
       WG_TIMED("soa_word_kernel", s,
-        soa_word_kernel<<<g, 256, digit_smem(count), s>>>(packed.as<uint64_t>(), n, w, count,
-                                                        w == spec.words - 1 ? nullptr : b.i0, b.k0, b.hist));
+        soa_word_kernel<<<g, 256, digit_smem(count), s>>>(src, k, bits, count, first ? nullptr : b.i0, b.k0, b.hist));
       check_launch("launch sort word");
-      sort_pairs(n, b, count, w == spec.words - 1, s);
-      check_cuda(cudaMemcpyAsync(&h, b.control, sizeof(h), cudaMemcpyDeviceToHost, s), "read sort state");
-      check_cuda(cudaStreamSynchronize(s), "read sort state");
+      sort_pairs(n, b, count, first, s);
+      first = false;
+      outcome();
     }
   }
-  if (h.timeout) throw Error(WG_ERR_TIMEOUT, "radix sort: a tile waited too long for its predecessors");
+  if (b.i0 != order.as<uint32_t>())
+    check_cuda(cudaMemcpyAsync(order.get(), b.i0, order.size(), cudaMemcpyDeviceToDevice, s), "copy sort order");
+  pairs.release();
+  zero.release();
+  {
+    Scratch idx2(sizeof(uint32_t) * n, s);
+    soa_index_kernel<<<g, 256, 0, s>>>(n, order.as<uint32_t>(), idx.as<uint32_t>(), idx2.as<uint32_t>());
+    check_launch("launch sort index");
+    std::swap(idx, idx2);
+  }
+  Scratch keys2(sizeof(uint64_t) * K * n, s);
   WG_TIMED("soa_gather_kernel", s,
-  soa_gather_kernel<<<g, 256, 0, s>>>(src, K, b.i0, idx.as<uint32_t>(), keys2.as<uint64_t>(), idx2.as<uint32_t>()));
+    soa_gather_kernel<<<g, 256, 0, s>>>(src, K, order.as<uint32_t>(), keys2.as<uint64_t>()));
   check_launch("launch sort gather");
   std::swap(keys, keys2);
-  std::swap(idx, idx2);
 }
 
 }  // namespace wg

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "wg_common.cuh"
 
 namespace wgo {
@@ -138,7 +140,8 @@ struct KeyBits {
   int ored;           // bits set in some key
   int ored_digits;    // 8-bit digits holding such a bit
   double density;     // mean share of set bits among the varying ones
-  wg::Scratch masks;  // device: varying bits per key word (K words)
+  std::vector<int> vary;  // varying bits per key word
+  wg::Scratch masks;      // device: the same as masks (K words)
 };
 CodeSpec choose_code(const KeyBits& kb, size_t n);
 

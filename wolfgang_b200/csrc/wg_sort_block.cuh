@@ -123,7 +123,8 @@ KeyBits key_bits(int device, int K, size_t na, const A& a, size_t nc, const C& c
       vary |= h[2 * y * K + k] & h[(2 * y + 1) * K + k];
       ored |= h[2 * y * K + k];
     }
-    kb.B += __builtin_popcountll(vary);
+    kb.vary.push_back(__builtin_popcountll(vary));
+    kb.B += kb.vary.back();
     kb.ored += __builtin_popcountll(ored);
     for (int b = 0; b < 64; b += 8) kb.ored_digits += ((ored >> b) & 0xffu) != 0;
   }
