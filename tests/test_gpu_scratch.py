@@ -68,3 +68,37 @@ def test_grouping_order(cuda, peak, n):
     used = peak(lambda: capi.call("wg_group_commuting", 0, w, T, G.ptr(dx), G.ptr(dz), 0, order.ctypes.data_as(to),
                                   sizes.ctypes.data_as(to), ctypes.byref(count), None))
     assert used < (16 * (1 + 2 * w) + 16) * T
+
+
+@pytest.mark.parametrize("n,T", [(20, 1_400_000), (100, 900_000)])
+def test_simplify(cuda, peak, n, T):
+    """A code, a sum and two item numbers a term, and the packed key (8 bytes for 64 of the 2 n
+    varying bits); the sizes keep the call below the 64 MiB from which the workspace, which
+    stays for later calls, takes its place."""
+    bytes_a_term = 32 + 8 * ((2 * n + 63) // 64)
+    rng = np.random.default_rng(n)
+    x, z = strings(rng, n, T)
+    dx, dz, dc = G.operator_on_device(x, z, rng.normal(size=T) + 0j)
+    out = [ctypes.c_void_p() for _ in range(3)]
+    terms = ctypes.c_size_t()
+    used = peak(lambda: capi.call("wg_simplify", 0, (n + 63) // 64, T, G.ptr(dx), G.ptr(dz), G.ptr(dc), 1e-12, 0.0,
+                                  *(ctypes.byref(p) for p in out), ctypes.byref(terms), None))
+    assert 0 < terms.value <= 1600 and used < (bytes_a_term + 3) * T
+    for p in out:
+        capi.call("wg_free", 0, p, None)
+
+
+@pytest.mark.parametrize("n", [20, 100])
+def test_products(cuda, peak, n):
+    rng = np.random.default_rng(n)
+    T = 1300
+    x, z = strings(rng, n, T)
+    dx, dz, dc = G.operator_on_device(x, z, rng.normal(size=T) + 0j)
+    side = G.ptr(dx), G.ptr(dz), G.ptr(dc), T
+    out = [ctypes.c_void_p() for _ in range(3)]
+    terms = ctypes.c_size_t()
+    used = peak(lambda: capi.call("wg_pauli_products", 0, (n + 63) // 64, *side, *side, capi.WG_PRODUCTS_SIMPLIFY,
+                                  1e-12, 0.0, *(ctypes.byref(p) for p in out), ctypes.byref(terms), None))
+    assert terms.value > 0 and used < (32 + 3) * T * T + 48 * terms.value
+    for p in out:
+        capi.call("wg_free", 0, p, None)

@@ -428,7 +428,8 @@ __global__ void __launch_bounds__(kThreads, 4) reduce_kernel(Items items, const 
                                                              CodeSpec spec, Threshold threshold,
                                                              uint32_t* __restrict__ out_idx,
                                                              double2* __restrict__ out_c,
-                                                             uint32_t* __restrict__ counts, SortControl* ctl) {
+                                                             uint32_t* __restrict__ counts,
+                                                             uint32_t* __restrict__ starts, SortControl* ctl) {
   extern __shared__ __align__(16) unsigned char raw[];
   ReduceSmem& sm = *reinterpret_cast<ReduceSmem*>(raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -536,7 +537,8 @@ __global__ void __launch_bounds__(kThreads, 4) reduce_kernel(Items items, const 
   __syncthreads();
   if (warp == 0) rank_bits(sm.keep, kSpanWords, sm.rank);
   __syncthreads();
-  const size_t o0 = static_cast<size_t>(blockIdx.x) * kSpan;
+  // survivors from the tile's first run on: no more than it has items, so the tiles' lie one behind another
+  const size_t o0 = t0 + first;
   for (int p = tid; p < kSpan; p += kThreads) {
     const uint32_t k = sm.keep[p >> 5];
     if (!((k >> (p & 31)) & 1u)) continue;
@@ -589,7 +591,10 @@ __global__ void __launch_bounds__(kThreads, 4) reduce_kernel(Items items, const 
     }
   }
   if (inf) ctl->infinite = 1;
-  if (tid == 0) counts[blockIdx.x] = kept;
+  if (tid == 0) {
+    counts[blockIdx.x] = kept;
+    starts[blockIdx.x] = static_cast<uint32_t>(o0);
+  }
 }
 
 // The survivors of each tile at their ranks: a CTA per tile.
@@ -597,11 +602,13 @@ template <class Items>
 __global__ void __launch_bounds__(kThreads) write_kernel(Items items, const uint32_t* __restrict__ sidx,
                                                          const double2* __restrict__ sc,
                                                          const uint32_t* __restrict__ counts,
+                                                         const uint32_t* __restrict__ starts,
                                                          const uint32_t* __restrict__ offsets,
                                                          uint64_t* __restrict__ ox, uint64_t* __restrict__ oz,
                                                          double2* __restrict__ oc) {
   const uint32_t m = counts[blockIdx.x];
-  const size_t o0 = offsets[blockIdx.x], i0 = static_cast<size_t>(blockIdx.x) * kSpan;
+  if (m == 0) return;
+  const size_t o0 = offsets[blockIdx.x], i0 = starts[blockIdx.x];
 #pragma unroll 4
   for (uint32_t r = threadIdx.x; r < m; r += kThreads) {
     items.store(sidx[i0 + r], o0 + r, ox, oz);
@@ -806,14 +813,18 @@ int sort_reduce(int device, int W, Items items, uint32_t n, const KeyBits& kb, c
                 Pieces& mem, int wide, const Outputs& out, cudaStream_t s) {
   const int passes = (spec.nb + 7) / 8;
   const size_t tiles = pair_tiles(n), parts = (static_cast<size_t>(n) + kTile - 1) / kTile;
+  // Sums take the place of one code array and sums' items that of one item array:
+  // the codes of the sorted order are to end in the other.
   PairBuffers b{};
-  b.k0 = mem.take<uint64_t>(n);
-  b.k1 = mem.take<uint64_t>(n);
+  auto* codes = mem.take<uint64_t>(n);
+  auto* sc = mem.take<double2>(n);
+  b.k0 = codes;
+  b.k1 = reinterpret_cast<uint64_t*>(sc);
+  if (passes % 2) std::swap(b.k0, b.k1);
   b.i0 = mem.take<uint32_t>(n);
   b.i1 = mem.take<uint32_t>(n);
-  auto* sc = mem.take<double2>(parts * kSpan);
-  auto* sidx = mem.take<uint32_t>(parts * kSpan);
   auto* counts = mem.take<uint32_t>(parts);
+  auto* starts = mem.take<uint32_t>(parts);
   auto* offsets = mem.take<uint32_t>(parts);
   auto* scan = mem.take<uint32_t>(wgs::scan_workspace(parts));
   auto* max_bits = mem.take<unsigned long long>(1);
@@ -833,8 +844,8 @@ int sort_reduce(int device, int W, Items items, uint32_t n, const KeyBits& kb, c
   auto reduce = [&](auto* kernel) {
     wg::allow_smem(kernel, sizeof(ReduceSmem));
     WG_TIMED("reduce_kernel", s,
-      kernel<<<static_cast<unsigned>(parts), kThreads, sizeof(ReduceSmem), s>>>(items, b.k0, b.i0, n, spec, thr, sidx,
-                                                                              sc, counts, b.control));
+      kernel<<<static_cast<unsigned>(parts), kThreads, sizeof(ReduceSmem), s>>>(items, b.k0, b.i0, n, spec, thr, b.i1,
+                                                                              sc, counts, starts, b.control));
     wg::check_launch("launch reduce");
     wgs::exclusive_scan_ws<uint32_t>(counts, offsets, parts, &b.control->survivors, scan, s);
     return read_control(b.control, s);
@@ -867,7 +878,8 @@ int sort_reduce(int device, int W, Items items, uint32_t n, const KeyBits& kb, c
   if (U == 0) return algo;
   wg::Scratch ox(sizeof(uint64_t) * W * U, s), oz(sizeof(uint64_t) * W * U, s), oc(sizeof(double) * 2 * U, s);
   WG_TIMED("write_kernel", s,
-    write_kernel<<<static_cast<unsigned>(parts), kThreads, 0, s>>>(items, sidx, sc, counts, offsets, ox.as<uint64_t>(),
+    write_kernel<<<static_cast<unsigned>(parts), kThreads, 0, s>>>(items, b.i1, sc, counts, starts, offsets,
+                                                                 ox.as<uint64_t>(),
                                                                  oz.as<uint64_t>(), oc.as<double2>()));
   wg::check_launch("launch simplify output");
   wg::check_cuda(cudaStreamSynchronize(s), "synchronize simplify");
@@ -881,8 +893,8 @@ int sort_reduce(int device, int W, Items items, uint32_t n, const KeyBits& kb, c
 size_t sort_reduce_bytes(size_t n) {
   using WS = wg::Workspace;
   const size_t tiles = pair_tiles(n), parts = (n + kTile - 1) / kTile;
-  return 2 * WS::rounded(8 * n) + 2 * WS::rounded(4 * n) + WS::rounded(16 * parts * kSpan) +
-         WS::rounded(4 * parts * kSpan) + 2 * WS::rounded(4 * parts) + WS::rounded(4 * wgs::scan_workspace(parts)) +
+  return WS::rounded(8 * n) + WS::rounded(16 * n) + 2 * WS::rounded(4 * n) + 3 * WS::rounded(4 * parts) +
+         WS::rounded(4 * wgs::scan_workspace(parts)) +
          WS::rounded(8) + WS::rounded(8 * kDigits * tiles + 4 * kDigits * kMaxPasses + sizeof(SortControl));
 }
 
