@@ -102,3 +102,43 @@ def test_products(cuda, peak, n):
     assert terms.value > 0 and used < (32 + 3) * T * T + 48 * terms.value
     for p in out:
         capi.call("wg_free", 0, p, None)
+
+
+_GIVE_BACK = """
+import ctypes, numpy as np, torch
+from wolfgang_b200 import capi
+n, T = 20, 20_000_000
+x = torch.randint(0, 1 << n, (T, 1), device="cuda") & 1023
+z = torch.zeros_like(x)
+c = torch.zeros(T, dtype=torch.complex128, device="cuda") + 1
+out, terms = [ctypes.c_void_p() for _ in range(3)], ctypes.c_size_t()
+def simplify():
+    torch.cuda.synchronize()
+    capi.call("wg_simplify", 0, 1, T, x.data_ptr(), z.data_ptr(), c.data_ptr(), 1e-12, 0.0,
+              *(ctypes.byref(p) for p in out), ctypes.byref(terms), None)
+    assert terms.value == 1024
+    for p in out:
+        capi.call("wg_free", 0, p, None)
+simplify()
+torch.cuda.empty_cache()
+filler = torch.empty(torch.cuda.mem_get_info()[0] - (2 << 30), dtype=torch.uint8, device="cuda")
+free = torch.cuda.mem_get_info()[0]
+held = 40 * T  # the workspace of the call above, at least
+p = ctypes.c_void_p()
+capi.call("wg_malloc", 0, free + held // 2, None, ctypes.byref(p))
+capi.call("wg_free", 0, p, None)
+simplify()
+print("given back")
+"""
+
+
+def test_workspace_is_given_back_when_room_is_short(cuda):
+    """With all but 2 GiB of the device taken, an allocation that fits only where the workspace
+    of an earlier call lay; the next large call takes a new one."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parents[1]
+    run = subprocess.run([sys.executable, "-c", _GIVE_BACK], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0 and "given back" in run.stdout, run.stderr[-2000:]

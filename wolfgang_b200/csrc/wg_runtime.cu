@@ -126,6 +126,32 @@ const DeviceProps& device_props(int device) {
   return p;
 }
 
+namespace {
+constexpr int kMaxDevices = 64;
+// The devices' workspaces.  A holder has mu; every one has synchronised its stream
+// by the time it lets go.
+struct WorkspaceSlot {
+  std::mutex mu;
+  void* base = nullptr;
+  size_t cap = 0;
+};
+WorkspaceSlot g_workspace[kMaxDevices];
+thread_local bool t_holds_workspace = false;
+
+// Gives the current device's workspace back to the pool if nobody holds it.
+bool give_back_workspace(cudaStream_t s) {
+  int device = -1;
+  if (t_holds_workspace || cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return false;
+  WorkspaceSlot& w = g_workspace[device];
+  std::unique_lock<std::mutex> lk(w.mu, std::try_to_lock);
+  if (!lk.owns_lock() || !w.base) return false;
+  pool_free(w.base, s);
+  w.base = nullptr;
+  w.cap = 0;
+  return true;
+}
+}  // namespace
+
 void* pool_alloc(size_t bytes, cudaStream_t s) {
   if (bytes == 0) return nullptr;
   long f = g_fail_after.load();
@@ -134,7 +160,13 @@ void* pool_alloc(size_t bytes, cudaStream_t s) {
     if (f == 1) throw Error(WG_ERR_OOM, "CUDA allocate device buffer failed: out of memory (injected)");
   }
   void* p = nullptr;
-  check_cuda(cudaMallocAsync(&p, bytes, s), "allocate device buffer");
+  cudaError_t e = cudaMallocAsync(&p, bytes, s);
+  // large calls share the workspace, which stays with the device: not while others need the room
+  if (e == cudaErrorMemoryAllocation && give_back_workspace(s)) {
+    (void)cudaGetLastError();
+    e = cudaMallocAsync(&p, bytes, s);
+  }
+  check_cuda(e, "allocate device buffer");
   return p;
 }
 
@@ -313,16 +345,6 @@ void staged_copy(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, 
   check_cuda(cudaStreamSynchronize(s), "synchronize staged copy");
 }
 
-namespace {
-constexpr int kMaxDevices = 64;
-struct WorkspaceSlot {
-  std::mutex mu;
-  void* base = nullptr;
-  size_t cap = 0;
-};
-WorkspaceSlot g_workspace[kMaxDevices];
-}  // namespace
-
 Workspace::Workspace(int device, size_t bytes, cudaStream_t s) : device_(device) {
   if (device < 0 || device >= kMaxDevices) throw_invalid("CUDA device ordinal is out of range");
   WorkspaceSlot& w = g_workspace[device];
@@ -332,20 +354,32 @@ Workspace::Workspace(int device, size_t bytes, cudaStream_t s) : device_(device)
       if (w.base) pool_free(w.base, s);
       w.base = nullptr;
       w.cap = 0;
-      // some headroom, so that slightly larger calls reuse the block
+      // some headroom, so that slightly larger calls reuse the block, where there is room for it
+      t_holds_workspace = true;
       const size_t want = bytes + bytes / 8;
-      w.base = pool_alloc(want, s);
-      w.cap = want;
+      try {
+        w.base = pool_alloc(want, s);
+        w.cap = want;
+      } catch (const Error& e) {
+        if (e.code != WG_ERR_OOM) throw;
+        w.base = pool_alloc(bytes, s);
+        w.cap = bytes;
+      }
     }
   } catch (...) {
+    t_holds_workspace = false;
     w.mu.unlock();
     throw;
   }
+  t_holds_workspace = true;
   p_ = static_cast<char*>(w.base);
   end_ = p_ + w.cap;
 }
 
-Workspace::~Workspace() { g_workspace[device_].mu.unlock(); }
+Workspace::~Workspace() {
+  t_holds_workspace = false;
+  g_workspace[device_].mu.unlock();
+}
 
 void* Workspace::take(size_t bytes) {
   const size_t r = rounded(bytes);
