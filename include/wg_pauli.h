@@ -258,22 +258,20 @@ int wg_products_batch_destroy(wg_products_batch_t batch);
  * wg_pauli_products.  No reference counterpart (the reference has one sort);
  * both algorithms give identical results, bit for bit.
  *   WG_SORT_AUTO    (default) up to 8,192 items one CTA sorts the full keys;
- *                   above, a radix sort of 64-bit codes that order like the
- *                   keys (the key's varying bits themselves where there are at
- *                   most 64), ties put in order by the keys.  Reported as
- *                   WG_SORT_BUCKET (sorted by key codes) for 1-2 mask words,
- *                   >= 2^20 items and keys that vary in more than 8 (one word)
- *                   or 5 (two words) of their 8-bit digits, as WG_SORT_LSD
- *                   otherwise and whenever codes tied so often that all words
- *                   of the keys were sorted;
- *   WG_SORT_LSD     the same sort, always reported as such;
+ *                   above, a radix sort of the keys' varying bits where there
+ *                   are at most 64, else of 64-bit codes that order like the
+ *                   keys, ties put in order by the keys, and of all words of
+ *                   the keys where codes tie too often;
+ *   WG_SORT_LSD     the radix sort of the varying bits of all words;
  *   WG_SORT_BUCKET  bucketed sort on 64-bit key codes (1-2 mask words, at most
  *                   255 significant key bits); falls back to WG_SORT_LSD when a
  *                   bucket of mixed keys stays over its capacity after being
  *                   split again, or one tie of key codes spans more than 16
  *                   distinct keys.
- * The setting is process-wide.  wg_last_sort_algorithm returns the algorithm
- * that produced the calling thread's last result (0 before any). */
+ * The setting is process-wide.  wg_last_sort_algorithm tells what put the
+ * calling thread's last result in order (0 before any): WG_SORT_LSD the keys'
+ * own bits; WG_SORT_BUCKET their 64-bit codes, in buckets where WG_SORT_BUCKET
+ * is set, by radix passes under WG_SORT_AUTO. */
 #define WG_SORT_AUTO 0
 #define WG_SORT_LSD 1
 #define WG_SORT_BUCKET 2

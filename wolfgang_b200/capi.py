@@ -177,7 +177,8 @@ def set_sort_algorithm(algo: int) -> int:
 
 
 def last_sort_algorithm() -> int:
-    """WG_SORT_LSD or WG_SORT_BUCKET: the algorithm of this thread's last simplify / products result."""
+    """WG_SORT_LSD (by the keys' own bits) or WG_SORT_BUCKET (by their 64-bit codes): what put
+    this thread's last simplify / products result in order."""
     return int(lib().wg_last_sort_algorithm())
 
 

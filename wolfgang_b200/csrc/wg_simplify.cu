@@ -807,10 +807,11 @@ class Pieces {
 };
 
 // Sorts and reduces n items; `where` points the items at their packed keys.
-// Returns the algorithm that gave the result.
+// Wide keys go by their codes under WG_SORT_AUTO only.  Returns what sorted them, for
+// wg_last_sort_algorithm: WG_SORT_LSD their own bits, WG_SORT_BUCKET their codes.
 template <class Items>
-int sort_reduce(int device, int W, Items items, uint32_t n, const KeyBits& kb, const CodeSpec& spec, Threshold thr,
-                Pieces& mem, int wide, const Outputs& out, cudaStream_t s) {
+int sort_reduce(int device, int W, Items items, uint32_t n, const CodeSpec& spec, Threshold thr,
+                Pieces& mem, const Outputs& out, cudaStream_t s) {
   const int passes = (spec.nb + 7) / 8;
   const size_t tiles = pair_tiles(n), parts = (static_cast<size_t>(n) + kTile - 1) / kTile;
   // Sums take the place of one code array and sums' items that of one item array:
@@ -850,16 +851,19 @@ int sort_reduce(int device, int W, Items items, uint32_t n, const KeyBits& kb, c
     wgs::exclusive_scan_ws<uint32_t>(counts, offsets, parts, &b.control->survivors, scan, s);
     return read_control(b.control, s);
   };
-  wg::check_cuda(cudaMemsetAsync(zero, 0, zero_bytes, s), "clear sort state");
-  wg::allow_smem(code_kernel<Items>, digit_smem(kMaxPasses));
-  WG_TIMED("code_kernel", s,
-    code_kernel<<<g, kThreads, digit_smem(passes), s>>>(items, n, spec, passes, b.k0, b.hist));
-  wg::check_launch("launch codes");
-  sort_pairs(n, b, passes, true, s);
-  SortControl h = spec.exact ? reduce(reduce_kernel<kByCode, Items>) : reduce(reduce_kernel<kChecked, Items>);
-  int algo = wide;
+  SortControl h{};
+  h.mixed = !spec.exact && wg::sort_algorithm() != WG_SORT_AUTO;
+  if (!h.mixed) {
+    wg::check_cuda(cudaMemsetAsync(zero, 0, zero_bytes, s), "clear sort state");
+    wg::allow_smem(code_kernel<Items>, digit_smem(kMaxPasses));
+    WG_TIMED("code_kernel", s,
+      code_kernel<<<g, kThreads, digit_smem(passes), s>>>(items, n, spec, passes, b.k0, b.hist));
+    wg::check_launch("launch codes");
+    sort_pairs(n, b, passes, true, s);
+    h = spec.exact ? reduce(reduce_kernel<kByCode, Items>) : reduce(reduce_kernel<kChecked, Items>);
+  }
+  const int algo = spec.exact || h.mixed ? WG_SORT_LSD : WG_SORT_BUCKET;
   if (h.mixed) {
-    algo = WG_SORT_LSD;
     wg::allow_smem(word_kernel<Items>, digit_smem(kMaxPasses));
     for (int w = spec.words - 1; w >= 0; --w) {
       const int count = (std::min(64, spec.B - 64 * w) + 7) / 8;
@@ -898,15 +902,6 @@ size_t sort_reduce_bytes(size_t n) {
          WS::rounded(8) + WS::rounded(8 * kDigits * tiles + 4 * kDigits * kMaxPasses + sizeof(SortControl));
 }
 
-// What wg_last_sort_algorithm reports for keys that are not narrow: under
-// WG_SORT_AUTO, 1-2 mask words, 2^20 items or more and keys with set bits in
-// more than 8 (one word) or 5 (two words) of their 8-bit digits are sorted by
-// key codes (WG_SORT_BUCKET), the rest by radix passes over whole keys.
-int reported(int W, size_t n, const KeyBits& kb) {
-  if (wg::sort_algorithm() != WG_SORT_AUTO || W < 1 || W > 2 || n < (size_t{1} << 20)) return WG_SORT_LSD;
-  return kb.ored <= 255 && kb.ored_digits > (W == 1 ? 8 : 5) ? WG_SORT_BUCKET : WG_SORT_LSD;
-}
-
 void simplify_terms(int device, int W, const uint64_t* x, const uint64_t* z, const double* c, size_t n,
                     const Threshold& thr, const Outputs& out, cudaStream_t s) {
   const OperandWords words{x, z, W};
@@ -926,8 +921,7 @@ void simplify_terms(int device, int W, const uint64_t* x, const uint64_t* z, con
                                                                         spec.words));
   wg::check_launch("launch pack");
   const uint32_t n32 = static_cast<uint32_t>(n);
-  const int wide = reported(W, n, kb);
-  auto go = [&](auto items) { wg::note_sort(sort_reduce(device, W, items, n32, kb, spec, thr, mem, wide, out, s)); };
+  auto go = [&](auto items) { wg::note_sort(sort_reduce(device, W, items, n32, spec, thr, mem, out, s)); };
   if (W == 1) go(TermItems<1>{x, z, c, 1, bits, spec.words});
   else if (W == 2) go(TermItems<2>{x, z, c, 2, bits, spec.words});
   else go(TermItems<0>{x, z, c, W, bits, spec.words});
@@ -956,8 +950,7 @@ void simplify_products(int device, int W, const uint64_t* lx, const uint64_t* lz
     pack_kernel<<<grid, kThreads, 0, s>>>(a, b, W, kb.masks.as<unsigned long long>(), spec.words));
   wg::check_launch("launch pack");
   const uint32_t n32 = static_cast<uint32_t>(P);
-  const int wide = reported(W, P, kb);
-  auto go = [&](auto items) { wg::note_sort(sort_reduce(device, W, items, n32, kb, spec, thr, mem, wide, out, s)); };
+  auto go = [&](auto items) { wg::note_sort(sort_reduce(device, W, items, n32, spec, thr, mem, out, s)); };
   const Divide by(n_r);
   if (W == 1) go(ProductItems<1>{a.rec, b.rec, 1, by, a.bits, b.bits, spec.words});
   else if (W == 2) go(ProductItems<2>{a.rec, b.rec, 2, by, a.bits, b.bits, spec.words});

@@ -137,8 +137,6 @@ struct KeyBits {
   bool side_by_side;  // two lists: the keys are XORs of one of each
   int K;              // key words (2 per mask word)
   int B;              // varying bits
-  int ored;           // bits set in some key
-  int ored_digits;    // 8-bit digits holding such a bit
   double density;     // mean share of set bits among the varying ones
   std::vector<int> vary;  // varying bits per key word
   wg::Scratch masks;      // device: the same as masks (K words)

@@ -117,16 +117,13 @@ KeyBits key_bits(int device, int K, size_t na, const A& a, size_t nc, const C& c
   wg::check_cuda(cudaStreamSynchronize(s), "read key bits");
   unsigned long long constant[2] = {0, 0};  // set bits that every key of a list has
   for (int k = 0; k < K; ++k) {
-    unsigned long long vary = 0, ored = 0;
+    unsigned long long vary = 0;
     for (int y = 0; y < lists; ++y) {
       constant[y] += __builtin_popcountll(~h[(2 * y + 1) * K + k]);
       vary |= h[2 * y * K + k] & h[(2 * y + 1) * K + k];
-      ored |= h[2 * y * K + k];
     }
     kb.vary.push_back(__builtin_popcountll(vary));
     kb.B += kb.vary.back();
-    kb.ored += __builtin_popcountll(ored);
-    for (int b = 0; b < 64; b += 8) kb.ored_digits += ((ored >> b) & 0xffu) != 0;
   }
   const double B = std::max(1, kb.B);
   const double p = std::min(1.0, static_cast<double>(h[4 * K] - constant[0] * na) / (B * static_cast<double>(na)));
