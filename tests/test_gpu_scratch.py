@@ -142,3 +142,32 @@ def test_workspace_is_given_back_when_room_is_short(cuda):
     root = Path(__file__).resolve().parents[1]
     run = subprocess.run([sys.executable, "-c", _GIVE_BACK], cwd=root, capture_output=True, text=True, timeout=300)
     assert run.returncode == 0 and "given back" in run.stdout, run.stderr[-2000:]
+
+
+@pytest.mark.parametrize("n", [20, 100])
+def test_small_results_keep_little(cuda, peak, n):
+    """100 sums of 8,000 terms that collect to 30 strings or fewer: 48 bytes a string, and at
+    most 64 KiB more for each (blocks for all terms would be 256 KB and more)."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    rng = np.random.default_rng(n)
+    T, w = 8000, (n + 63) // 64
+    x, z = strings(rng, n, T)
+    x[:], z[:] = x[rng.integers(0, 30, size=T)], z[0]
+    dx, dz, dc = G.operator_on_device(x, z, rng.normal(size=T) + 0j)
+    results = []
+
+    def used():
+        pool = runtime.cudaDeviceGetDefaultMemPool(0)[1]
+        return int(runtime.cudaMemPoolGetAttribute(pool, runtime.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)[1])
+
+    cuda.cuda.synchronize()
+    before = used()
+    for _ in range(100):
+        out, terms = [ctypes.c_void_p() for _ in range(3)], ctypes.c_size_t()
+        capi.call("wg_simplify", 0, w, T, G.ptr(dx), G.ptr(dz), G.ptr(dc), 1e-12, 0.0, *(ctypes.byref(p) for p in out),
+                  ctypes.byref(terms), None)
+        assert 0 < terms.value <= 30
+        results += out
+    assert used() - before < 100 * (65536 + 48 * 30)
+    for p in results:
+        capi.call("wg_free", 0, p, None)

@@ -767,7 +767,24 @@ void run_small(const SmallItems& in, size_t n, int W, const Threshold& thr, cons
   wg::check_launch("launch small simplify");
   const SortControl h = read_control(ctl, s);
   if (h.survivors == 0 || (thr.mode == 2 && h.infinite)) return;
-  *out.n = h.survivors;
+  // Blocks for all items are handed out unless more than kSpare bytes of them would
+  // never be used: exact ones take three allocations, copies and a wait (15 us).
+  const size_t U = h.survivors;
+  constexpr size_t kSpare = size_t{64} << 10;
+  if ((n - U) * (16 * static_cast<size_t>(W) + 16) > kSpare) {
+    auto exact = [&](wg::Scratch& all, size_t bytes) {
+      wg::Scratch own(bytes, s);
+      wg::check_cuda(cudaMemcpyAsync(own.get(), all.get(), bytes, cudaMemcpyDeviceToDevice, s), "copy small result");
+      std::swap(all, own);
+    };
+    if (W > 0) {
+      exact(ox, sizeof(uint64_t) * W * U);
+      exact(oz, sizeof(uint64_t) * W * U);
+    }
+    exact(oc, sizeof(double) * 2 * U);
+    wg::check_cuda(cudaStreamSynchronize(s), "copy small result");
+  }
+  *out.n = U;
   *out.x = static_cast<uint64_t*>(ox.detach());
   *out.z = static_cast<uint64_t*>(oz.detach());
   *out.c = static_cast<double*>(oc.detach());
