@@ -129,6 +129,7 @@ __device__ __forceinline__ uint32_t wait_terms(const Pipe& p, uint32_t s, uint32
     }
     if (spins >= p.limit) {
       unsigned long long now = 0;
+#pragma unroll 1
       for (uint32_t e = 1; e <= s; ++e) now += st[1 - static_cast<int>(e)];
       if (watched && now == seen) {
         ctl->timeout = 1;
