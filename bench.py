@@ -738,9 +738,8 @@ def bench_batched(args, world, rank, torch) -> dict:
     pc_total, _, _, _ = timed_steps(torch, max(1, args.steps // 2), 1, per_call)
     pc = pc_total / max(1, args.steps // 2)
 
-    # the plain per-call drop-in: wg_expectation (the path behind
-    # DevicePauliSum.expectation_statevector) builds its plan on every call and
-    # returns E only -- no gradient, so it does less than a batched evaluation
+    # one wg_expectation per pair: it builds the forward half of a plan on every
+    # call and returns E only -- no gradient, so it does less than a batched evaluation
     import ctypes as ct
 
     from wolfgang_b200.workloads import uneven_pair_operator as _upo
@@ -820,8 +819,8 @@ def bench_batched(args, world, rank, torch) -> dict:
                        "per_call_path": "one ExpectationPlan.run(terms, H psi) per pair, plans built once",
                        "one_shot_ms": os_ms, "batched_forward_ms": fwd_ms,
                        "batched_forward_over_one_shot": os_ms / fwd_ms,
-                       "one_shot_path": "wg_expectation per pair (DevicePauliSum.expectation_statevector's path: "
-                                        "plan built per call, E only), against the batch without gradients",
+                       "one_shot_path": "wg_expectation per pair (a forward-only plan built per call, E only), "
+                                        "against the batch without gradients",
                        "qubits": f"{args.min_qubits}..{args.max_qubits}"},
             "roofline": roofline(prof, {"expect_forward_kernel": fwd_bytes, "expect_adjoint_kernel": adj_bytes},
                                  *peaks()),

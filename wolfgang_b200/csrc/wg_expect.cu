@@ -701,7 +701,7 @@ __device__ __forceinline__ void adjoint_sub(const Layout<M>& lay, const AdjSub& 
 }
 
 // Output-stationary: a CTA owns tile J of H psi, 8 amplitudes a thread, and
-// walks the segments of its split.  Bound by shared-memory wavefronts (71 % of
+// walks the segments of its split.  Bound by shared-memory wavefronts (78 % of
 // the cycles; 8 an amplitude and sub-group at least: 4 for psi, 2 for either
 // table): 44 ms on 24 qubits with 20,000 terms (80 ms with tables of complex
 // entries and psi read through L1).
@@ -1214,8 +1214,8 @@ void allow_smem(int device) {
 // that a split writes and reads, then serve more terms.  Neither changes a bit.  64
 // pairs of 14 qubits and 1,000 terms with H psi 2.47 -> 1.05 ms, 400 of 100 terms 6.5
 // -> 1.63; 30 pairs of 8 to 18 qubits 2.02 -> 1.77; and no partial H psi for most pairs
-// (up to 37 MB each, now 1 GB at most in all: the tiles that are still split are fewer
-// than three an SM, of 64 splits at most).
+// (up to 37 MB each, now 2 GB at most in all: the tiles that are still split are at most
+// three an SM, of 64 splits and 64 KB each).
 struct Division {
   double forward = 0.0;  // pieces x tiles of a forward item, at most
   double adjoint = 0.0;  // tiles of at most this cost are one adjoint item

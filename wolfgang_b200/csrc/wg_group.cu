@@ -649,11 +649,13 @@ uint32_t run_pipeline(int device, bool full, Pipe pipe, uint32_t T, cudaStream_t
 }
 
 // ------------------------------------------------ any number of mask words
-// More than 4 mask words (over 256 qubits): the same chunked first-fit as
-// above, with each row read word by word from memory instead of held in
-// registers.  Term rows are interleaved once as trows[i] = [x words | z words]
-// (processing order); a chunk's term rows are staged in shared memory, the
-// qwc basis rows and the full-mode member lists stay in global memory.  The
+// More than 4 mask words (over 256 qubits): the first-fit by chunks of terms.  The
+// whole GPU finds for every term of a chunk the first group that accepts it among
+// those that the earlier chunks left (a lower bound: a group only ever accepts
+// less), then one warp places the chunk's terms in order from their bounds on.
+// Term rows are interleaved once as trows[i] = [x words | z words] (processing
+// order) and read word by word; a chunk's are staged in shared memory, the qwc
+// basis rows and the full-mode member lists (linked) stay in global memory.  The
 // chunk is shortened when its staged rows would not fit in shared memory.
 
 __device__ __forceinline__ bool row_accepts_n(const uint64_t* t, const uint64_t* b, int W) {
@@ -687,7 +689,8 @@ __global__ void interleave_rows_kernel(const uint64_t* __restrict__ ox, const ui
   }
 }
 
-// group_search_full_kernel for any width
+// Full mode: lb[i] = the first group of whose members none anticommutes with term i,
+// by kBoundSplit warps a term.
 __global__ void __launch_bounds__(kBoundThreads) group_search_full_n_kernel(
     const uint64_t* __restrict__ trows, int W, uint32_t c0, uint32_t c1, const uint32_t* __restrict__ first,
     const uint32_t* __restrict__ next, const uint32_t* __restrict__ n_groups, uint32_t* lb) {
@@ -714,7 +717,8 @@ __global__ void __launch_bounds__(kBoundThreads) group_search_full_n_kernel(
   }
 }
 
-// group_bound_kernel for any width
+// lb[i] = the first group that accepts term i (full mode: as found by the search);
+// full mode: lbm[i] = which of the 32 groups from there on do.
 __global__ void __launch_bounds__(kBoundThreads) group_bound_n_kernel(
     const uint64_t* __restrict__ trows, int W, uint32_t c0, uint32_t c1, const uint64_t* __restrict__ rows,
     const uint32_t* __restrict__ first, const uint32_t* __restrict__ next, const uint32_t* __restrict__ n_groups,
@@ -749,7 +753,8 @@ __global__ void __launch_bounds__(kBoundThreads) group_bound_n_kernel(
   }
 }
 
-// place_qwc for any width, basis rows in global memory (lane g % 32 owns row g)
+// Places a chunk's n terms in order, qwc, by one warp: lane g % 32 owns basis row g in
+// global memory.  Returns the number of groups.
 __device__ uint32_t place_qwc_n(const uint64_t* st, const uint32_t* slb, uint32_t* sgid, uint32_t n, uint32_t G,
                                 uint64_t* B, int W) {
   const uint32_t lane = threadIdx.x & 31;
@@ -787,7 +792,8 @@ __device__ uint32_t place_qwc_n(const uint64_t* st, const uint32_t* slb, uint32_
   return G;
 }
 
-// place_full for any width
+// The same in full mode: members that joined in this chunk are checked from its staged
+// rows, the others were by the bound.
 __device__ uint32_t place_full_n(const uint64_t* __restrict__ trows, const uint64_t* st, const uint32_t* slb,
                                  const uint32_t* smask, uint32_t* sgid, uint32_t n, uint32_t c0, uint32_t G0,
                                  uint32_t* first, uint32_t* last, uint32_t* next, int W) {
@@ -852,7 +858,7 @@ __device__ uint32_t place_full_n(const uint64_t* __restrict__ trows, const uint6
   return G;
 }
 
-// group_resolve_kernel for any width: stages up to `cap_terms` term rows
+// One CTA: stages the chunk's rows, up to cap_terms, and its first warp places them.
 __global__ void __launch_bounds__(kResolveThreads) group_resolve_n_kernel(
     const uint64_t* __restrict__ trows, int W, uint32_t c0, uint32_t c1, uint32_t cap_terms, uint64_t* rows,
     uint32_t* first, uint32_t* last, uint32_t* next, const uint32_t* __restrict__ lb,

@@ -9,8 +9,8 @@
 //               the device holds;
 //   bucket      the bucketed sort's target items per fine bucket:
 //               640, 768, 896, 1,024, 1,280;
-//   group_qwc   group_commuting, terms per batch of a stage, qwc mode: 128, 256,
-//               512 (above 4 mask words the chunk length);
+//   group_qwc   group_commuting up to 4 mask words, terms per batch of a stage, qwc
+//               mode: 128, 256, 512;
 //   group_full  the same in full mode: 8, 16, 24, 31.
 // Classes: commute (words, log2 n_lhs, log2 n_rhs); bucket (words, log2
 // products or terms, 0); group_* (words, log2 terms, 0), logs rounded up.
